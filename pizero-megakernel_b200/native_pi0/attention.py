@@ -113,9 +113,7 @@ class ResidentAttention:
     def forward(self):
         if not self.handle.value:
             raise RuntimeError("Attention instance is closed")
-        with torch.cuda.device(self.device):
-            _native.check(self.library.launch_attention(self.handle, torch.cuda.current_stream(self.device).cuda_stream),
-                          "Native attention launch")
+        _native.check(_native.launch(self.library.launch_attention, self.handle, self.device), "Native attention launch")
         return self.output
 
     def status(self):

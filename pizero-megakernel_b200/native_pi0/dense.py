@@ -164,8 +164,7 @@ class ResidentDense:
     def forward(self):
         if not self.handle.value:
             raise RuntimeError("Dense instance is closed")
-        with torch.cuda.device(self.device):
-            _native.check(self.library.launch_dense(self.handle, torch.cuda.current_stream(self.device).cuda_stream), "Native dense launch")
+        _native.check(_native.launch(self.library.launch_dense, self.handle, self.device), "Native dense launch")
         return self.logical_output
 
     def status(self):

@@ -60,9 +60,7 @@ class NativeLinearProgram:
     def forward(self):
         if not self.handle.value or any(not s.handle.value for s in self.stages):
             raise RuntimeError("Native program or child is closed")
-        with torch.cuda.device(self.device):
-            _native.check(self.library.launch_native_linear(self.handle, torch.cuda.current_stream(self.device).cuda_stream),
-                          "Native linear launch")
+        _native.check(_native.launch(self.library.launch_native_linear, self.handle, self.device), "Native linear launch")
         self.epoch += 1
         return self.output
 
@@ -141,9 +139,8 @@ class NativeStageProgram:
     def forward(self):
         if not self.handle.value:
             raise RuntimeError("Native stage program is closed")
-        with torch.cuda.device(self.device):
-            _native.check(self.library.launch_native_model(self.handle, torch.cuda.current_stream(self.device).cuda_stream,
-                                                           None, None, None, None), "Native stage program launch")
+        _native.check(_native.launch(self.library.launch_native_model, self.handle, self.device, None, None, None, None),
+                      "Native stage program launch")
         return self.operators[-1].output
 
     def status(self):

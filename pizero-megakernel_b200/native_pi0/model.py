@@ -902,10 +902,8 @@ class NativePi0:
         self.launch_range(begin, end, images, state, noise, tokens, new_epoch)
 
     def launch_range(self, begin, end, images, state, noise, tokens, new_epoch):
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream(self.device).cuda_stream
-            code = self.lib.launch_native_model_range(self.handle, stream, images.data_ptr(), state.data_ptr(), noise.data_ptr(),
-                                                      tokens.data_ptr(), begin, end, int(new_epoch))
+        code = _native.launch(self.lib.launch_native_model_range, self.handle, self.device, images.data_ptr(), state.data_ptr(),
+                              noise.data_ptr(), tokens.data_ptr(), begin, end, int(new_epoch))
         if code:
             raise RuntimeError(f"Native pi0 launch error {code}")
 

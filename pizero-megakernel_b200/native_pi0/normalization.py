@@ -93,9 +93,7 @@ class ResidentNorm:
     def forward(self):
         if not self.handle.value:
             raise RuntimeError("Normalization instance is closed")
-        with torch.cuda.device(self.device):
-            _native.check(self.library.launch_norm(self.handle, torch.cuda.current_stream(self.device).cuda_stream),
-                          "Native norm launch")
+        _native.check(_native.launch(self.library.launch_norm, self.handle, self.device), "Native norm launch")
         return self.output
 
     def status(self):

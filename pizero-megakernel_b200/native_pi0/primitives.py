@@ -164,9 +164,7 @@ class ResidentNVFP4:
     def forward(self):
         if not self._handle.value:
             raise RuntimeError("Native FP4 instance is closed")
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream(self.device)
-            _native.check(self._library.launch_resident_fp4(self._handle, stream.cuda_stream), "Native FP4 launch")
+        _native.check(_native.launch(self._library.launch_resident_fp4, self._handle, self.device), "Native FP4 launch")
         return self.output
 
     def status(self):
