@@ -337,10 +337,22 @@ int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begi
     p.wait_budget_ns = prog->budget_ns;
     p.in = in;
     p.debug = prog->h_debug;
-    if (prog->lean && !prog->h_debug && !p.timings) pi0_vm_kernel<true, false><<<prog->workers, kThreads, kSmemBytes, stream>>>(p);
-    else if (prog->lean && !prog->h_debug) pi0_vm_kernel<true><<<prog->workers, kThreads, kSmemBytes, stream>>>(p);
-    else pi0_vm_kernel<false><<<prog->workers, kThreads, kSmemBytes, stream>>>(p);
-    return cudaGetLastError();
+    // Programmatic stream serialisation: the CTAs are placed as soon as those of the kernel in front have exited and wait
+    // in the kernel for its completion (grid_dependency_wait).  Ordinary serialisation of back-to-back launches costs
+    // 2 - 4 us on B200, rounded up to multiples of 2.048 us: RMSNorm 51 x 1024 takes 8.2 us per call with it, 5.9 with this.
+    cudaLaunchAttribute serial{};
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(prog->workers);
+    config.blockDim = dim3(kThreads);
+    config.dynamicSmemBytes = kSmemBytes;
+    config.stream = stream;
+    config.attrs = &serial;
+    config.numAttrs = 1;
+    if (prog->lean && !prog->h_debug && !p.timings) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false>, p);
+    if (prog->lean && !prog->h_debug) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true>, p);
+    return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true>, p);
 }
 
 Op* as_op(void* h) {

@@ -31,6 +31,10 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 
+// Programmatic dependent launch: returns when every grid in front of this one in the stream has completed and its writes
+// are visible.  (Without the launch attribute it returns at once.)
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -87,6 +87,9 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
+    // Up to here nothing that other work on the stream writes was touched: launched with programmatic stream serialisation
+    // (launch_program), this CTA may be set up while the previous kernel's completion is still being processed.
+    grid_dependency_wait();
 
     const int4* stream = prog.code + static_cast<size_t>(blockIdx.x) * prog.length;
     // first instruction of the requested stage range (streams are sorted by stage)
