@@ -37,7 +37,7 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
         // been read by its MMAs before the first new copy lands (waits for the last release of each slot).
         int alive0 = 1;
         if (lane == 0)
-            for (int s = 0; s < kMaxStages && alive0; ++s)
+            for (int s = 0; s < kMaxStagesDense && alive0; ++s)
                 alive0 = mbar_wait(prog, ctl, &ctl->empty[s], ((p_bits >> s) & 1u) ^ 1u, stage_index) ? 1 : 0;
         alive0 = __shfl_sync(0xffffffffu, alive0, 0);
         if (!alive0) return;

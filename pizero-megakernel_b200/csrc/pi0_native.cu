@@ -400,7 +400,7 @@ int gemm_refresh(Op* op) {
     CUtensorMap host[2];
     const size_t row_bytes = operand_row_bytes(op->operands, op->k);
     int e = encode_operand(&host[0], op->a, op->m, row_bytes, g.a_box_rows);
-    if (!e) e = g.b_tiled ? encode_tiled(&host[1], op->b, op->n * (op->k / 256), kChunks * g.block_n)
+    if (!e) e = g.b_tiled ? encode_tiled(&host[1], op->b, op->n * static_cast<int>(row_bytes / 128), kChunks * g.block_n)
                           : encode_operand(&host[1], op->b, op->n, row_bytes, g.block_n);
     if (e) return e;
     if (!op->maps) {
@@ -425,7 +425,7 @@ int gemm_refresh(Op* op) {
     g.off_sfa = g.off_b + kChunks * 128 * g.block_n;
     g.off_sfb = g.off_sfa + sf_bytes;
     g.slot_stride = g.off_sfb + sf_bytes;
-    g.ring_stages = std::max(kStages, std::min(kMaxStages, kDataBytes / g.slot_stride));
+    g.ring_stages = std::max(kStages, std::min(op->operands == GEMM_NVFP4 ? kMaxStages : kMaxStagesDense, kDataBytes / g.slot_stride));
     if (g.slot_stride % 1024 || g.ring_stages * g.slot_stride > kDataBytes ||
         (kChunks - 1) * 128 * g.a_box_rows + kTileABytes > g.slot_stride)
         return cudaErrorInvalidValue;
@@ -668,16 +668,14 @@ extern "C" int configure_resident_fp4_rows(void* handle, int rows) {
 }
 extern "C" int configure_resident_fp4_weight_layout(void* handle, int tiled) {
     Op* op = as_op(handle);
-    if (!op || op->desc.kind != OP_GEMM || (tiled != 0 && tiled != 1) || (tiled && (op->k % 256 || op->operands != GEMM_NVFP4)))
+    if (!op || op->desc.kind != OP_GEMM || (tiled != 0 && tiled != 1) || (tiled && operand_row_bytes(op->operands, op->k) % 128))
         return cudaErrorInvalidValue;
     op->desc.p.gemm.b_tiled = tiled;
     return gemm_refresh(op);
 }
 extern "C" int configure_resident_fp4_tile(void* handle, int block_n) {
     Op* op = as_op(handle);
-    if (!op || op->desc.kind != OP_GEMM || (block_n != 128 && block_n != 64 && block_n != 32) ||
-        (block_n == 32 && op->operands != GEMM_NVFP4))
-        return cudaErrorInvalidValue;
+    if (!op || op->desc.kind != OP_GEMM || (block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
     op->desc.p.gemm.block_n = block_n;
     return gemm_refresh(op);
 }
@@ -842,7 +840,7 @@ extern "C" int configure_dense_rows(void* handle, int rows) {
 }
 extern "C" int configure_dense_tile(void* handle, int block_n) {
     Op* op = as_op(handle);
-    if (!op || op->desc.kind != OP_GEMM || op->operands == GEMM_NVFP4 || (block_n != 128 && block_n != 64)) return cudaErrorInvalidValue;
+    if (!op || op->desc.kind != OP_GEMM || op->operands == GEMM_NVFP4 || (block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
     op->desc.p.gemm.block_n = block_n;
     return gemm_refresh(op);
 }

@@ -10,7 +10,8 @@ namespace pi0 {
 // the rows that are really copied, as many slots as fit): kStages slots of kStageBytes for full tiles, up to
 // kMaxStages for the narrowest ones.
 constexpr int kStages = 3;                                   // slots in flight with full-size tiles (128 rows of A and of B)
-constexpr int kMaxStages = 5;                                // slots in flight with the narrowest tiles (64 rows of each)
+constexpr int kMaxStages = 5;                                // slots in flight with the narrowest NVFP4 tiles (64 rows of each) ...
+constexpr int kMaxStagesDense = 8;                           // ... and BF16 / FP8 tiles, whose slots cover less of K and carry no scales
 constexpr int kChunks = 2;                                   // 256-wide K chunks per slot
 constexpr int kTileABytes = 128 * 128;                       // one chunk of one operand: 128 rows x 128 bytes
 constexpr int kSfBytes = kChunks * 4 * 512;                  // scale atoms of one operand: four 64-wide K groups per chunk
@@ -33,8 +34,8 @@ struct alignas(16) Slot {
 };
 
 struct Ctl {
-    uint64_t full[kMaxStages];
-    uint64_t empty[kMaxStages];
+    uint64_t full[kMaxStagesDense];
+    uint64_t empty[kMaxStagesDense];
     uint64_t acc_full[2];
     uint64_t acc_empty[2];
     uint64_t ready[kRing];       // slot filled (32 asynchronous-copy arrivals of the prefetch warp)

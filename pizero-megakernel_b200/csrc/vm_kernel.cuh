@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
     const int warp = threadIdx.x >> 5;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kMaxStages; s++) {
+        for (int s = 0; s < kMaxStagesDense; s++) {
             mbar_init(&ctl->full[s], 1);
             mbar_init(&ctl->empty[s], 1);
         }
