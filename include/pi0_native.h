@@ -71,16 +71,17 @@ int configure_resident_fp4_stream_sums(void* handle, float* sums, int ld);
 int configure_resident_fp4_row_layernorm(void* handle, const float* sumsq, const float* sums, int parts, int width, float eps,
                                          const float* center);
 /* extension: logical row count (rows >= this are never stored; with at most 64 rows only 64 rows of A are
- * copied per tile) and output tile width: 128, 64, or 32 (NVFP4 operands only).  With 32-wide tiles the weight scales
+ * copied per tile) and output tile width: 128, 64, or 32.  With 32-wide NVFP4 tiles the weight scales
  * given at creation are read in a layout of their own: one 512-byte atom per (32-row tile, group of four 16-element
  * blocks) - [N / 32][K / 64][512] - holding the tile's 32 rows in the first 32-row sub-column of the atom (bytes
  * 16 r + b for row r, block b) and zeros elsewhere, i.e. four times the bytes of the standard layout.  Narrow tiles are
  * for projections of a few rows, whose time is the bytes one SM takes in and the serial epilogue of one tile. */
 int configure_resident_fp4_rows(void* handle, int rows);
 int configure_resident_fp4_tile(void* handle, int block_n);
-/* extension: tiled = 1 declares that B is stored tile-major (K a multiple of 256): for every output tile n and every
- * 256-wide K stage s the block_n x 128 bytes of that block are contiguous, at byte offset
- * ((n * K/256 + s) * block_n) * 128; one TMA box is then one contiguous read.  Set the tile width first. */
+/* extension: tiled = 1 declares that B is stored tile-major (rows of whole 128-byte pieces: K a multiple of 256 in NVFP4,
+ * 64 in BF16, 128 in FP8): for every output tile n and every 128-byte piece s of K the block_n x 128 bytes of that block are
+ * contiguous, at byte offset ((n * pieces + s) * block_n) * 128; one TMA box is then one contiguous read.  Set the tile
+ * width first. */
 int configure_resident_fp4_weight_layout(void* handle, int tiled);
 
 /* ------------------------------------------------------------------------------------------------------
@@ -122,9 +123,9 @@ int configure_dense_qkv_rope(void* handle, const void* cos, const void* sin, voi
  * buffer once and they stay zero.  Gives 72-wide SigLIP heads the 128-element pitch the tcgen05 attention tiles read
  * (configure_attention_head_pad).  No residual. */
 int configure_dense_head_pad(void* handle, int from, int to, int ld);
-/* extension: logical row count and output tile width (128 or 64) of a dense projection.  The NVFP4 GEMM's
- * configure_resident_fp4_{bf16, quantized, qkv_rope, rows, tile} calls accept dense handles too (a dense projection
- * may emit NVFP4 for an NVFP4 consumer); configure_resident_fp4_weight_layout does not. */
+/* extension: logical row count and output tile width (128, 64 or 32) of a dense projection.  The NVFP4 GEMM's
+ * configure_resident_fp4_{bf16, quantized, qkv_rope, rows, tile, weight_layout} calls accept dense handles too (a dense
+ * projection may emit NVFP4 for an NVFP4 consumer). */
 int configure_dense_rows(void* handle, int rows);
 int configure_dense_tile(void* handle, int block_n);
 

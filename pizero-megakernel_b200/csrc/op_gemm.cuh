@@ -3,10 +3,10 @@
 // FP8 E4M3 (kind::f8f6f4).  In every format a row of K is cut into 128-byte chunks and one MMA consumes 32 bytes of
 // each operand row (64 FP4, 16 BF16 or 32 FP8 elements), so the copy ring and the issue loop are the same code.
 //
-//   warp 0 / lane 0 : TMA producer  - operand tiles (128 B swizzled rows) and scale atoms into a ring of slots; the ring
-//                                     is laid out per GEMM: 3 slots of 72 KiB for full NVFP4 tiles, up to 5 for narrow ones
-//   warp 1          : MMA issuer    - warp-uniform loop, one elected lane issues tcgen05.cp (scales smem->TMEM, NVFP4
-//                                     only) and tcgen05.mma, 32 operand bytes of K each
+//   warps 0 and 3   : TMA producers - A and B tiles (128 B swizzled rows) and their scale atoms into a ring of slots; the
+//                                     ring is laid out per GEMM: 3 slots of 72 KiB for full NVFP4 tiles, more for narrow ones
+//   warp 1          : MMA issuer    - one elected thread issues tcgen05.cp (scales smem->TMEM, NVFP4 only) and
+//                                     tcgen05.mma, 32 operand bytes of K each
 //   warps 4..7      : epilogue      - tcgen05.ld of a 128xN FP32 accumulator (one row per thread), fused math, stores
 //
 // Two TMEM accumulators alternate, so the epilogue of tile t overlaps the MMAs of tile t+1. Pipeline positions live in
@@ -16,109 +16,93 @@
 
 namespace pi0 {
 
-// Whole warp 0: the dependency wait is lane-parallel, lane 0 issues the copies.
+// The copy warps: warp 0 (WEIGHTS = false) brings A and its scales, warp 3 (WEIGHTS = true) B and its scales; lane 0 of
+// each issues the copies and every slot's barrier expects one arrival from both.
 //
-// Weights never depend on another stage, so for the first tile of an instruction the B tiles and B scales of the
-// first slots are requested BEFORE the dependency wait (their bytes are announced with expect_tx without an
-// arrival); when the producers are done only the activation half (A, A scales) is still to be fetched.
+// Weights never depend on another stage, so warp 3 takes no part in the dependency wait: it fills whatever slots are free,
+// also those of the next GEMM instruction, and when the producers are done only the activation half is still to be
+// fetched.  One warp issuing all four copies of a slot (each costs the issuing thread about 65 cycles) was as slow as the
+// MMAs that read it.
+// The loop works on register copies of the descriptor: that lies in shared memory, and every asm statement with a memory
+// clobber would make the compiler read it again.
+template <bool WEIGHTS>
 __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, uint8_t* data, const StageDesc& st,
                                               int stage_index, int first, int count, PipeState& ps, long long* stamp) {
     const GemmParams& g = st.p.gemm;
     const int lane = lane_id();
-    uint32_t p_slot = ps.prod_slot, p_bits = ps.prod_bits;
-    const int chunks = (g.k_groups + 3) >> 2;                        // 256-wide K chunks
+    uint32_t slot = ps.prod_slot, bits = ps.prod_bits;
+    const int k_groups = g.k_groups, n_tiles = g.n_tiles, block_n = g.block_n, b_tiled = g.b_tiled;
+    const void* tmap = WEIGHTS ? g.tmap_b : g.tmap_a;
+    const uint8_t* scales = WEIGHTS ? g.sfb : g.sfa;
+    const int chunks = (k_groups + 3) >> 2;                          // 256-wide K chunks
     const int slots = (chunks + kChunks - 1) / kChunks;
-    const uint32_t a_bytes = static_cast<uint32_t>(kChunks) * 128u * static_cast<uint32_t>(g.a_box_rows);
-    const uint32_t b_bytes = static_cast<uint32_t>(kChunks) * 128u * static_cast<uint32_t>(g.block_n);
+    const uint32_t bytes = static_cast<uint32_t>(kChunks) * 128u * static_cast<uint32_t>(WEIGHTS ? block_n : g.a_box_rows);
     const uint32_t ring = static_cast<uint32_t>(g.ring_stages), stride = static_cast<uint32_t>(g.slot_stride);
-    const uint32_t sf_unit = g.operands == GEMM_NVFP4 ? 512u : 0u;      // scale-atom bytes per MMA group and operand
+    const uint32_t off = WEIGHTS ? static_cast<uint32_t>(g.off_b) : 0u, off_sf = static_cast<uint32_t>(WEIGHTS ? g.off_sfb : g.off_sfa);
+    const bool scaled = g.operands == GEMM_NVFP4;                    // scale atoms: 512 bytes per MMA group and operand
     if (ps.prod_geo != stride) {
         // Slots of the previous geometry overlap the new ones at other indices: every copy issued so far must have
         // been read by its MMAs before the first new copy lands (waits for the last release of each slot).
         int alive0 = 1;
         if (lane == 0)
             for (int s = 0; s < kMaxStagesDense && alive0; ++s)
-                alive0 = mbar_wait(prog, ctl, &ctl->empty[s], ((p_bits >> s) & 1u) ^ 1u, stage_index) ? 1 : 0;
+                alive0 = mbar_wait(prog, ctl, &ctl->empty[s], ((bits >> s) & 1u) ^ 1u, stage_index) ? 1 : 0;
         alive0 = __shfl_sync(0xffffffffu, alive0, 0);
         if (!alive0) return;
         ps.prod_geo = stride;
-        p_slot = 0;
+        slot = 0;
     }
     int current_band = -1;
     for (int t = first; t < first + count; ++t) {
-        const int m_tile = t / g.n_tiles, n_tile = t - m_tile * g.n_tiles;
-        const int band = tile_band(st, t);
-        // B scales: the 128-row atom that holds the tile's rows, or - 32-wide tiles - an atom of the tile's own
-        const int sfb_tile = g.block_n == 32 ? n_tile : (n_tile * g.block_n) >> 7;
-        int early = 0;                                               // slots whose weight half is already in flight
-        int alive = 1;
-        if (band != current_band) {
-            if (t == first) {
+        const int m_tile = t / n_tiles, n_tile = t - m_tile * n_tiles;
+        if (!WEIGHTS) {
+            const int band = tile_band(st, t);
+            if (band != current_band) {
+                if (!warp_wait_sources(prog, ctl, st, stage_index, band, band)) return;
                 if (lane == 0) {
-                    early = min(slots, g.ring_stages);
-                    for (int ks = 0; ks < early; ++ks) {
-                        const uint32_t s = (p_slot + ks) % ring;
-                        if (!mbar_wait(prog, ctl, &ctl->empty[s], ((p_bits >> s) & 1u) ^ 1u, stage_index)) { alive = 0; break; }
-                        const int groups = min(4 * kChunks, g.k_groups - ks * 4 * kChunks);
-                        uint8_t* slot = data + s * stride;
-                        mbar_expect_tx_only(&ctl->full[s], b_bytes + groups * sf_unit);
-                        if (g.b_tiled) tma_load_2d(slot + g.off_b, g.tmap_b, &ctl->full[s], 0, (n_tile * chunks + ks * kChunks) * g.block_n);
-                        else tma_load_3d(slot + g.off_b, g.tmap_b, &ctl->full[s], 0, n_tile * g.block_n, ks * kChunks);
-                        if (sf_unit)
-                            bulk_load(slot + g.off_sfb, g.sfb + (static_cast<size_t>(sfb_tile) * g.k_groups + ks * 4 * kChunks) * 512,
-                                      groups * 512u, &ctl->full[s]);
-                    }
+                    fence_proxy_async_global();
+                    if (current_band < 0)       // tell the epilogue warps: the sources of this instruction's first band are complete
+                        asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(&ctl->deps_seen))), "r"(ps.gemm_seq + 1u) : "memory");
+                    if (stamp && current_band < 0) stamp[1] = static_cast<long long>(global_ns());
                 }
-                early = __shfl_sync(0xffffffffu, early, 0);
-                alive = __shfl_sync(0xffffffffu, alive, 0);
-                if (!alive) return;
+                current_band = band;
             }
-            if (!warp_wait_sources(prog, ctl, st, stage_index, band, band)) return;
-            if (lane == 0) {
-                fence_proxy_async_global();
-                if (current_band < 0)       // tell the epilogue warps: the sources of this instruction's first band are complete
-                    asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(&ctl->deps_seen))), "r"(ps.gemm_seq + 1u) : "memory");
-                if (stamp && current_band < 0) stamp[1] = static_cast<long long>(global_ns());
-            }
-            current_band = band;
         }
+        int alive = 1;
         if (lane == 0) {
+            // B scales: the 128-row atom that holds the tile's rows, or - 32-wide tiles - an atom of the tile's own
+            const int sf_tile = !WEIGHTS ? m_tile : block_n == 32 ? n_tile : (n_tile * block_n) >> 7;
+            const uint8_t* sf = scales + static_cast<size_t>(sf_tile) * k_groups * 512;
             for (int ks = 0; ks < slots; ++ks) {
-                const uint32_t s = p_slot;
-                const int groups = min(4 * kChunks, g.k_groups - ks * 4 * kChunks);
-                uint8_t* slot = data + s * stride;
-                const bool weights_issued = ks < early;
-                if (!weights_issued && !mbar_wait(prog, ctl, &ctl->empty[s], ((p_bits >> s) & 1u) ^ 1u, stage_index)) { alive = 0; break; }
+                const uint32_t s = slot;
+                if (!mbar_wait(prog, ctl, &ctl->empty[s], ((bits >> s) & 1u) ^ 1u, stage_index)) { alive = 0; break; }
+                uint8_t* base = data + s * stride;
+                uint64_t* bar = &ctl->full[s];
+                const uint32_t sf_bytes = scaled ? static_cast<uint32_t>(min(4 * kChunks, k_groups - ks * 4 * kChunks)) * 512u : 0u;
                 // Boxes always deliver kChunks chunks (beyond K the copy engine fills zeros or, inside a padded
                 // allocation, bytes that no MMA reads).  a_box_rows < 128 (few logical rows): only the rows that
                 // exist are copied; the MMA still reads 128 rows, the rest lands in accumulator rows never stored.
-                mbar_expect_tx(&ctl->full[s], a_bytes + groups * sf_unit + (weights_issued ? 0u : b_bytes + groups * sf_unit));
-                tma_load_3d(slot, g.tmap_a, &ctl->full[s], 0, m_tile * 128, ks * kChunks);
-                if (sf_unit)
-                    bulk_load(slot + g.off_sfa, g.sfa + (static_cast<size_t>(m_tile) * g.k_groups + ks * 4 * kChunks) * 512, groups * 512u,
-                              &ctl->full[s]);
-                if (!weights_issued) {
-                    if (g.b_tiled) tma_load_2d(slot + g.off_b, g.tmap_b, &ctl->full[s], 0, (n_tile * chunks + ks * kChunks) * g.block_n);
-                    else tma_load_3d(slot + g.off_b, g.tmap_b, &ctl->full[s], 0, n_tile * g.block_n, ks * kChunks);
-                    if (sf_unit)
-                        bulk_load(slot + g.off_sfb, g.sfb + (static_cast<size_t>(sfb_tile) * g.k_groups + ks * 4 * kChunks) * 512,
-                                  groups * 512u, &ctl->full[s]);
-                }
-                p_bits ^= 1u << s;
-                p_slot = s + 1 == ring ? 0u : s + 1;
+                mbar_expect_tx(bar, bytes + sf_bytes);
+                if (WEIGHTS && b_tiled) tma_load_2d(base + off, tmap, bar, 0, (n_tile * chunks + ks * kChunks) * block_n);
+                else tma_load_3d(base + off, tmap, bar, 0, WEIGHTS ? n_tile * block_n : m_tile * 128, ks * kChunks);
+                if (scaled) bulk_load(base + off_sf, sf + static_cast<size_t>(ks) * (4 * kChunks * 512), sf_bytes, bar);
+                bits ^= 1u << s;
+                slot = s + 1 == ring ? 0u : s + 1;
             }
         }
         alive = __shfl_sync(0xffffffffu, alive, 0);
         if (!alive) return;
     }
-    ps.prod_slot = p_slot;
-    ps.prod_bits = p_bits;
+    ps.prod_slot = slot;
+    ps.prod_bits = bits;
 }
 
-// Whole warp 1, converged: the loop and all operand arithmetic are warp-uniform and only the tcgen05 instructions are
-// issued by one elected lane. (Run by a single lane inside a divergent branch, every descriptor and address has to be
-// moved from per-thread to uniform registers for each instruction, which measured about 250 cycles per 64-wide K
-// group and made this lane, not the copies or the tensor core, the pace of a narrow GEMM.)
+// Warp 1: one elected thread runs the whole loop - waits, scale copies, MMAs, commits - while the other lanes wait at the
+// end.  The queue in front of the tensor core holds only about two MMAs, so whatever the issuing thread does between two
+// slots is idle tensor time: with a warp-wide barrier vote and an election per slot a slot of eight MMAs cost 690 (BF16,
+// 32 columns) to 1050 cycles (NVFP4, 128 columns), alone it needs 325 and 740.  The barrier of the next slot is therefore
+// tested (without blocking) half-way through the current one, and a slot that has landed by then costs no wait at all.
+// The operand arithmetic starts from values broadcast over the warp, so that descriptors stay in uniform registers.
 // (One instantiation per operand format, so each issue loop carries only its own instructions.)
 template <int OPERANDS>
 __device__ __forceinline__ void gemm_mma(const VmProgram& prog, Ctl* ctl, uint8_t* data, uint32_t tmem_in, const StageDesc& st,
@@ -141,66 +125,75 @@ __device__ __forceinline__ void gemm_mma(const VmProgram& prog, Ctl* ctl, uint8_
     constexpr uint64_t kScaleHi = (1ull << 16) | (8ull << 32) | (1ull << 46);
     if (ps.mma_geo != stride) { ps.mma_geo = stride; ps.mma_slot = 0; }
     uint32_t slot = uniform_u32(ps.mma_slot), bits = uniform_u32(ps.mma_bits), it = uniform_u32(ps.mma_it), tile_no = uniform_u32(ps.mma_tile);
-    bool first_slot = true;
-    for (int t = first; t < first + count; ++t) {
-        const int n_tile = t % n_tiles;
-        const uint32_t buf = tile_no & 1u, acc_phase = (tile_no >> 1) & 1u;
-        if (!mbar_wait_warp(prog, ctl, &ctl->acc_empty[buf], acc_phase ^ 1u, stage_index)) return;
-        tc_fence_after();
-        const uint32_t d = tmem + buf * 128u;
-        // Scale rows of a 64-wide B tile sit in the 32-row sub-columns 0 or 2 of their 128-row atom (the scale operand of
-        // the MMA must start at an even sub-column); 32-wide tiles bring atoms of their own with the rows in sub-column 0.
-        const uint32_t sfb_sub = block_n == 32 ? 0u : static_cast<uint32_t>((n_tile * block_n) & 127) >> 5;
-        for (int ks = 0; ks < slots; ++ks) {
-            const uint32_t s = slot;
-            if (!mbar_wait_warp(prog, ctl, &ctl->full[s], (bits >> s) & 1u, stage_index)) return;
-            if (stamp && first_slot && lane_id() == 0) stamp[4] = static_cast<long long>(global_ns());
-            first_slot = false;
-            const int groups = min(4 * kChunks, k_groups - ks * 4 * kChunks);
-            const uint32_t a16 = data16 + s * stride16;
-            const uint32_t sf_cols = tmem + kSfCol0 + (it & 3u) * (4 * kChunks * 8);
-            if constexpr (OPERANDS != GEMM_NVFP4) {
-                // BF16 / FP8 rows: the same descriptors and the same 32-byte advance along K, no scale factors
-                if (elect_one()) {
+    const bool leader = elect_one();
+    if (leader) {
+        bool landed = false, alive = true;                   // landed: the current slot was seen full by the look-ahead
+        for (int t = first; alive && t < first + count; ++t) {
+            const int n_tile = t % n_tiles;
+            const uint32_t buf = tile_no & 1u, acc_phase = (tile_no >> 1) & 1u;
+            if (!mbar_wait(prog, ctl, &ctl->acc_empty[buf], acc_phase ^ 1u, stage_index)) break;
+            tc_fence_after();
+            const uint32_t d = tmem + buf * 128u;
+            // Scale rows of a 64-wide B tile sit in the 32-row sub-columns 0 or 2 of their 128-row atom (the scale operand of
+            // the MMA must start at an even sub-column); 32-wide tiles bring atoms of their own with the rows in sub-column 0.
+            const uint32_t sfb_sub = block_n == 32 ? 0u : static_cast<uint32_t>((n_tile * block_n) & 127) >> 5;
+            for (int ks = 0; ks < slots; ++ks) {
+                const uint32_t s = slot, next = s + 1 == ring ? 0u : s + 1;
+                if (!landed && !mbar_wait(prog, ctl, &ctl->full[s], (bits >> s) & 1u, stage_index)) { alive = false; break; }
+                if (stamp && t == first && ks == 0) stamp[4] = static_cast<long long>(global_ns());
+                const int groups = min(4 * kChunks, k_groups - ks * 4 * kChunks);
+                const uint32_t a16 = data16 + s * stride16;
+                const uint32_t sf_cols = tmem + kSfCol0 + (it & 3u) * (4 * kChunks * 8);
+                // Scales of group gi: smem -> tensor memory.  All copies of a slot are issued in front of its MMAs: alternating
+                // between the two kinds of instruction costs the tensor pipe about 20 cycles per group (slots of 8 groups,
+                // 128 x 32 / 64 / 128 tiles: 650 / 700 / 790 cycles alternating, 470 / 515 / 640 copies first).
+                auto copy_scales = [&](uint32_t gi) {
+                    tc_copy_sf(sf_cols + gi * 8, kScaleHi | static_cast<uint64_t>(a16 + off_sfa16 + gi * 32));
+                    tc_copy_sf(sf_cols + gi * 8 + 4, kScaleHi | static_cast<uint64_t>(a16 + off_sfb16 + gi * 32));
+                };
+                auto issue = [&](uint32_t gi, uint32_t acc) {
+                    const uint32_t chunk = gi >> 2, sub = gi & 3u;
+                    // 64 FP4, 16 BF16 or 32 FP8 elements = 32 bytes along K inside the 128-byte swizzled row: advance the start
+                    // address by 2 units
+                    const uint64_t da = kOperandHi | static_cast<uint64_t>(a16 + chunk * a_chunk16 + 2u * sub);
+                    const uint64_t db = kOperandHi | static_cast<uint64_t>(a16 + off_b16 + chunk * b_chunk16 + 2u * sub);
+                    if constexpr (OPERANDS == GEMM_NVFP4) tc_mma_nvfp4(d, da, db, idesc, sf_cols + gi * 8, sf_cols + gi * 8 + 4 + sfb_sub, acc);
+                    else if constexpr (OPERANDS == GEMM_BF16) tc_mma_f16(d, da, db, idesc, acc);
+                    else tc_mma_f8(d, da, db, idesc, acc);
+                };
+                if (groups == 4 * kChunks) {                 // a full slot: no branch between its MMAs
+                    if constexpr (OPERANDS == GEMM_NVFP4) {
 #pragma unroll
-                    for (int gi = 0; gi < 4 * kChunks; ++gi) {
-                        if (gi < groups) {
-                            const uint32_t chunk = static_cast<uint32_t>(gi) >> 2, sub = static_cast<uint32_t>(gi) & 3u;
-                            const uint64_t da = kOperandHi | static_cast<uint64_t>(a16 + chunk * a_chunk16 + 2u * sub);
-                            const uint64_t db = kOperandHi | static_cast<uint64_t>(a16 + off_b16 + chunk * b_chunk16 + 2u * sub);
-                            const uint32_t acc = gi != 0 ? 1u : static_cast<uint32_t>(ks != 0);
-                            if constexpr (OPERANDS == GEMM_BF16) tc_mma_f16(d, da, db, idesc, acc);
-                            else tc_mma_f8(d, da, db, idesc, acc);
-                        }
+                        for (uint32_t gi = 0; gi < 4 * kChunks; ++gi) copy_scales(gi);
                     }
-                    tc_commit(&ctl->empty[s]);
-                }
-            } else if (elect_one()) {
 #pragma unroll
-                for (int gi = 0; gi < 4 * kChunks; ++gi) {
-                    if (gi < groups) {
-                        const uint32_t chunk = static_cast<uint32_t>(gi) >> 2, sub = static_cast<uint32_t>(gi) & 3u;
-                        const uint32_t sfa_t = sf_cols + gi * 8, sfb_t = sfa_t + 4;
-                        tc_copy_sf(sfa_t, kScaleHi | static_cast<uint64_t>(a16 + off_sfa16 + gi * 32));
-                        tc_copy_sf(sfb_t, kScaleHi | static_cast<uint64_t>(a16 + off_sfb16 + gi * 32));
-                        // 64 FP4 = 32 bytes along K inside the 128-byte swizzled row: advance the start address by 2 units.
-                        tc_mma_nvfp4(d, kOperandHi | static_cast<uint64_t>(a16 + chunk * a_chunk16 + 2u * sub),
-                                     kOperandHi | static_cast<uint64_t>(a16 + off_b16 + chunk * b_chunk16 + 2u * sub), idesc, sfa_t,
-                                     sfb_t + sfb_sub, gi != 0 ? 1u : static_cast<uint32_t>(ks != 0));
+                    for (uint32_t gi = 0; gi < 4 * kChunks; ++gi) {
+                        if (gi == 2 * kChunks) landed = mbar_test_wait(&ctl->full[next], (bits >> next) & 1u);
+                        issue(gi, gi != 0 ? 1u : static_cast<uint32_t>(ks != 0));
+                    }
+                } else {
+                    landed = false;
+#pragma unroll 1
+                    for (uint32_t gi = 0; gi < static_cast<uint32_t>(groups); ++gi) {
+                        if constexpr (OPERANDS == GEMM_NVFP4) copy_scales(gi);
+                        issue(gi, static_cast<uint32_t>(ks != 0 || gi != 0));
                     }
                 }
                 tc_commit(&ctl->empty[s]);     // slot reusable once these MMAs have read it
+                bits ^= 1u << s;
+                slot = next;
+                it++;
             }
-            __syncwarp();
-            bits ^= 1u << s;
-            slot = s + 1 == ring ? 0u : s + 1;
-            it++;
+            if (alive) tc_commit(&ctl->acc_full[buf]);    // accumulator complete
+            tile_no++;
         }
-        if (elect_one()) tc_commit(&ctl->acc_full[buf]);    // accumulator complete
-        __syncwarp();
-        tile_no++;
     }
-    ps.mma_slot = slot; ps.mma_bits = bits; ps.mma_it = it; ps.mma_tile = tile_no;
+    __syncwarp();
+    const int from = __ffs(__ballot_sync(0xffffffffu, leader)) - 1;
+    ps.mma_slot = __shfl_sync(0xffffffffu, slot, from);
+    ps.mma_bits = __shfl_sync(0xffffffffu, bits, from);
+    ps.mma_it = __shfl_sync(0xffffffffu, it, from);
+    ps.mma_tile = __shfl_sync(0xffffffffu, tile_no, from);
     if (stamp && lane_id() == 0) stamp[5] = static_cast<long long>(global_ns());
 }
 
@@ -571,7 +564,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
     }
 }
 
-// Dispatch of one GEMM instruction onto the warp roles. Warps 2 and 3 have no role and fall through.
+// Dispatch of one GEMM instruction onto the warp roles. Warp 2 has no role and falls through.
 // LEAN: the kernel variant for programs made only of NVFP4 projections with the pi0 model's epilogues (the host checks
 // this when it builds a program); it carries neither the dense issue loops nor the other drain loops.
 template <bool LEAN>
@@ -580,8 +573,10 @@ __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl
                                                  PipeState& ps, long long* stamp) {
     const int warp = threadIdx.x >> 5;
     if (warp == 0) {
-        gemm_producer(prog, ctl, data, st, stage_index, first, count, ps, stamp);
+        gemm_producer<false>(prog, ctl, data, st, stage_index, first, count, ps, stamp);
         if (stamp && threadIdx.x == 0) stamp[3] = static_cast<long long>(global_ns());
+    } else if (warp == 3) {
+        gemm_producer<true>(prog, ctl, data, st, stage_index, first, count, ps, nullptr);
     } else if (warp == 1) {
         const int operands = st.p.gemm.operands;
         if (LEAN || operands == GEMM_NVFP4) gemm_mma<GEMM_NVFP4>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);

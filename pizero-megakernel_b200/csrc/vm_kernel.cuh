@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxStagesDense; s++) {
-            mbar_init(&ctl->full[s], 1);
+            mbar_init(&ctl->full[s], 2);            // one arrival per copy warp
             mbar_init(&ctl->empty[s], 1);
         }
         for (int b = 0; b < 2; b++) {

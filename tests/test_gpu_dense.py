@@ -52,6 +52,30 @@ def test_fp8_product_matches_fp32(m, n, k):
         assert torch.equal(op.forward(), got.bfloat16())
 
 
+@pytest.mark.parametrize("m,k,fp8", [(1, 64, False), (64, 192, False), (65, 1152, False), (128, 4096, False), (300, 640, False), (40, 384, True)])
+def test_narrow_and_tile_major_tiles_give_the_bits_of_the_default(m, k, fp8):
+    """32- and 64-wide tiles and tile-major weights sum over K in the same order as 128-wide row-major ones: equal bits.
+    K covers a single piece, odd piece counts (a half-filled last slot) and more slots than the ring holds."""
+    n = 384
+    a, b = operands(m, n, k, 7 + m + k)
+    if fp8:
+        a, b = a.float().to(torch.float8_e4m3fn), b.float().to(torch.float8_e4m3fn)
+    piece = 128 // a.element_size()
+    with ResidentDense(None, a, b, output_dtype=torch.float32) as op:
+        want = op.forward().clone()
+    assert relrms(want, a.float() @ b.float().T) <= 2e-5
+    for width in (128, 64, 32):
+        for tiled in (False, True):
+            with ResidentDense(None, a, b, output_dtype=torch.float32, workers=5) as op:
+                assert op.library.configure_dense_tile(op.handle, width) == 0
+                if tiled:
+                    rows, columns = op.b.shape
+                    op.b.copy_(op.b.view(rows // width, width, columns // piece, piece).permute(0, 2, 1, 3).reshape(rows, columns))
+                    assert op.library.configure_resident_fp4_weight_layout(op.handle, 1) == 0
+                assert torch.equal(op.forward(), want), (width, tiled)
+                assert op.status()["code"] == 0
+
+
 def test_bf16_epilogues_are_bit_exact_against_the_fp32_result():
     m, n, k = 200, 384, 512
     a, b = operands(m, n, k, 3)
