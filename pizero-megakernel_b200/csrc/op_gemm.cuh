@@ -61,8 +61,7 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
                 if (!warp_wait_sources(prog, ctl, st, stage_index, band, band)) return;
                 if (lane == 0) {
                     fence_proxy_async_global();
-                    if (current_band < 0)       // tell the epilogue warps: the sources of this instruction's first band are complete
-                        asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(&ctl->deps_seen))), "r"(ps.gemm_seq + 1u) : "memory");
+                    if (current_band < 0) word_set(&ctl->deps_seen, ps.gemm_seq + 1u);   // tell the draining warps: the sources of this instruction's first band are complete
                     if (stamp && current_band < 0) stamp[1] = static_cast<long long>(global_ns());
                 }
                 current_band = band;
@@ -212,27 +211,53 @@ __device__ __forceinline__ float gelu_sigmoid(float x) {
     return __fdividef(x, 1.f + __expf(-z));
 }
 
-// One 32-column chunk of one accumulator row (thread == row).
-// (Instantiated per epilogue kind: each accumulator drain carries only its own arithmetic and registers.)
+__device__ __forceinline__ void add_bf16x32(float2 (&v)[16], const uint4 (&u)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        v[4 * i + 0] = add2(v[4 * i + 0], unpack_bf16x2(u[i].x));
+        v[4 * i + 1] = add2(v[4 * i + 1], unpack_bf16x2(u[i].y));
+        v[4 * i + 2] = add2(v[4 * i + 2], unpack_bf16x2(u[i].z));
+        v[4 * i + 3] = add2(v[4 * i + 3], unpack_bf16x2(u[i].w));
+    }
+}
+// NVFP4 codes of 32 values times inv_gs (16 bytes) and the two block scales in one word.
+__device__ __forceinline__ uint4 quantize_32(const float2 (&v)[16], float inv_gs, uint32_t& codes) {
+    uint32_t words[4];
+    codes = 0;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        float2 h[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[i] = mul2(v[8 * half + i], make_float2(inv_gs, inv_gs));
+        uint32_t code;
+        const uint2 bytes = quantize_block16(h, 0, code);
+        words[2 * half] = bytes.x;
+        words[2 * half + 1] = bytes.y;
+        codes |= code << (8 * half);
+    }
+    return make_uint4(words[0], words[1], words[2], words[3]);
+}
+// One 32-column chunk of one accumulator row (thread == row); `res` holds the residual of the chunk (BF16) if there is one.
+// (Instantiated per epilogue kind: each accumulator drain carries only its own arithmetic and registers.  Values are kept as
+// pairs: the packed FP32 operations shorten the straight-line code that a drain executes once.)
 // LEAN: without the options only the BF16 model uses (rounding before the residual, GELU on BF16 output) and without ReLU^2.
 template <int EPI, bool LEAN = false>
-__device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const uint32_t (&raw)[32], int row, int col0,
-                                                    bool row_ok, float row_scale, float row_shift, float& sumsq, float& sum) {
-    float v[32];
+__device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const uint32_t (&raw)[32], const uint4 (&res)[4], int row, int col0,
+                                                    bool row_ok, float row_scale, float row_shift, float2& sumsq, float2& sum) {
+    float2 v[16];
     if (!row_ok) return;
 #pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(raw[i]) * row_scale;
+    for (int i = 0; i < 16; i++) v[i] = mul2(make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1])), make_float2(row_scale, row_scale));
     if constexpr (EPI == EPI_BF16_EXT || EPI == EPI_FP4) {
         if (g.col_center) {
             // folded LayerNorm: subtract the row mean's share, mean * rstd * (sum over K of weight row n)
             const float4* c4 = reinterpret_cast<const float4*>(g.col_center + col0);
+            const float2 shift = make_float2(row_shift, row_shift);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const float4 c = __ldg(c4 + i);
-                v[4 * i] = fmaf(row_shift, c.x, v[4 * i]);
-                v[4 * i + 1] = fmaf(row_shift, c.y, v[4 * i + 1]);
-                v[4 * i + 2] = fmaf(row_shift, c.z, v[4 * i + 2]);
-                v[4 * i + 3] = fmaf(row_shift, c.w, v[4 * i + 3]);
+                v[2 * i] = fma2(shift, make_float2(c.x, c.y), v[2 * i]);
+                v[2 * i + 1] = fma2(shift, make_float2(c.z, c.w), v[2 * i + 1]);
             }
         }
     }
@@ -240,7 +265,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         // interleaved (gate, up) column pairs -> 16 outputs = one scale block
         float h[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) h[i] = gelu_sigmoid(v[2 * i]) * v[2 * i + 1] * g.out_inv_gs;
+        for (int i = 0; i < 16; i++) h[i] = gelu_sigmoid(v[i].x) * v[i].y * g.out_inv_gs;
         uint32_t code;
         uint2 bytes = quantize_block16(h, 0, code);
         const int out_col = col0 >> 1;
@@ -253,8 +278,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         uint32_t w[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const float h0 = bf16_round(gelu_tanh(bf16_round(v[4 * i]))) * bf16_round(v[4 * i + 1]);
-            const float h1 = bf16_round(gelu_tanh(bf16_round(v[4 * i + 2]))) * bf16_round(v[4 * i + 3]);
+            const float h0 = bf16_round(gelu_tanh(bf16_round(v[2 * i].x))) * bf16_round(v[2 * i].y);
+            const float h1 = bf16_round(gelu_tanh(bf16_round(v[2 * i + 1].x))) * bf16_round(v[2 * i + 1].y);
             w[i] = pack_bf16x2(h0, h1);
         }
         uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo + (col0 >> 1));
@@ -262,136 +287,85 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
         return;
     }
-    const bool early_bias = !LEAN && EPI == EPI_BF16_EXT && g.bias && g.residual && g.round_before_residual;
-    if (early_bias) {
+    // (residual first, bias second: the order of the reference epilogue, whose BF16 result the tests reproduce bit for bit -
+    // but a projection that is rounded before the residual is added carries its bias by then)
+    auto add_bias = [&]() {
         const uint4* b = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(g.bias) + col0);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            uint4 u = __ldg(b + i);
-            float2 f;
-            f = unpack_bf16x2(u.x); v[8 * i + 0] += f.x; v[8 * i + 1] += f.y;
-            f = unpack_bf16x2(u.y); v[8 * i + 2] += f.x; v[8 * i + 3] += f.y;
-            f = unpack_bf16x2(u.z); v[8 * i + 4] += f.x; v[8 * i + 5] += f.y;
-            f = unpack_bf16x2(u.w); v[8 * i + 6] += f.x; v[8 * i + 7] += f.y;
-        }
-    }
+        const uint4 u[4] = {__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3)};
+        add_bf16x32(v, u);
+    };
+    const bool early_bias = !LEAN && EPI == EPI_BF16_EXT && g.bias && g.residual && g.round_before_residual;
+    if (early_bias) add_bias();
     if (g.residual) {
         if (!LEAN && EPI == EPI_BF16_EXT && g.round_before_residual) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = bf16_round(v[i]);
+            for (int i = 0; i < 16; i++) v[i] = make_float2(bf16_round(v[i].x), bf16_round(v[i].y));
         }
-        const uint4* r = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(g.residual) +
-                                                        static_cast<size_t>(row) * g.ldr + col0);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            uint4 u = __ldcg(r + i);
-            float2 f;
-            f = unpack_bf16x2(u.x); v[8 * i + 0] += f.x; v[8 * i + 1] += f.y;
-            f = unpack_bf16x2(u.y); v[8 * i + 2] += f.x; v[8 * i + 3] += f.y;
-            f = unpack_bf16x2(u.z); v[8 * i + 4] += f.x; v[8 * i + 5] += f.y;
-            f = unpack_bf16x2(u.w); v[8 * i + 6] += f.x; v[8 * i + 7] += f.y;
-        }
+        add_bf16x32(v, res);
     }
-    if (g.bias && !early_bias) {
-        // (residual first, bias second: the order of the reference epilogue, whose BF16 result the tests reproduce bit for bit)
-        const uint4* b = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(g.bias) + col0);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            uint4 u = __ldg(b + i);
-            float2 f;
-            f = unpack_bf16x2(u.x); v[8 * i + 0] += f.x; v[8 * i + 1] += f.y;
-            f = unpack_bf16x2(u.y); v[8 * i + 2] += f.x; v[8 * i + 3] += f.y;
-            f = unpack_bf16x2(u.z); v[8 * i + 4] += f.x; v[8 * i + 5] += f.y;
-            f = unpack_bf16x2(u.w); v[8 * i + 6] += f.x; v[8 * i + 7] += f.y;
-        }
-    }
+    if (g.bias && !early_bias) add_bias();
     if constexpr (EPI == EPI_F32) {
         float4* dst = reinterpret_cast<float4*>(static_cast<float*>(g.out) + static_cast<size_t>(row) * g.ldo + col0);
 #pragma unroll
-        for (int i = 0; i < 8; i++) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        for (int i = 0; i < 8; i++) dst[i] = make_float4(v[2 * i].x, v[2 * i].y, v[2 * i + 1].x, v[2 * i + 1].y);
         return;
     }
     if constexpr (EPI == EPI_STREAM) {
         // the residual stream in BF16 ...
         uint32_t w[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) w[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+        for (int i = 0; i < 16; i++) w[i] = pack_bf16x2(v[i].x, v[i].y);
         uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo + col0);
 #pragma unroll
         for (int i = 0; i < 4; i++) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-        // ... and, from the rounded values a norm stage would have read back, the sum of squares and the NVFP4 copy
-        uint32_t words[4];
-        uint32_t codes = 0;
+        // ... and, from the rounded values a norm stage would have read back, the NVFP4 copy and the sums (even and odd
+        // columns apart)
 #pragma unroll
-        for (int half = 0; half < 2; half++) {
-            float h[16];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const float2 f = unpack_bf16x2(w[8 * half + i]);
-                sumsq = __fmaf_rn(f.x, f.x, sumsq);
-                sumsq = __fmaf_rn(f.y, f.y, sumsq);
-                sum += f.x;
-                sum += f.y;
-                h[2 * i] = f.x * g.out_inv_gs;
-                h[2 * i + 1] = f.y * g.out_inv_gs;
-            }
-            uint32_t code;
-            uint2 bytes = quantize_block16(h, 0, code);
-            words[2 * half] = bytes.x;
-            words[2 * half + 1] = bytes.y;
-            codes |= code << (8 * half);
+        for (int i = 0; i < 16; i++) {
+            v[i] = unpack_bf16x2(w[i]);
+            sumsq = fma2(v[i], v[i], sumsq);
         }
-        *reinterpret_cast<uint4*>(g.copy_fp4 + static_cast<size_t>(row) * g.ld_copy + (col0 >> 1)) = make_uint4(words[0], words[1], words[2], words[3]);
+        if (g.sum_out) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) sum = add2(sum, v[i]);
+        }
+        uint32_t codes;
+        *reinterpret_cast<uint4*>(g.copy_fp4 + static_cast<size_t>(row) * g.ld_copy + (col0 >> 1)) = quantize_32(v, g.out_inv_gs, codes);
         *reinterpret_cast<uint16_t*>(g.out_scales + scale_offset(row, col0 >> 4, g.out_blocks)) = static_cast<uint16_t>(codes);
         return;
     }
     if constexpr (EPI == EPI_BF16 || EPI == EPI_BF16_EXT) {
         if (!LEAN && EPI == EPI_BF16_EXT && g.gelu_cols > 0) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = col0 + i < g.gelu_cols ? gelu_tanh(bf16_round(v[i])) : 0.f;
+            for (int i = 0; i < 16; i++)
+                v[i] = make_float2(col0 + 2 * i < g.gelu_cols ? gelu_tanh(bf16_round(v[i].x)) : 0.f,
+                                   col0 + 2 * i + 1 < g.gelu_cols ? gelu_tanh(bf16_round(v[i].y)) : 0.f);
         }
-        if (EPI == EPI_BF16_EXT && g.pad_from > 0) {
-            // heads written pad_to columns apart (8-column pieces never straddle a head: pad_from is a multiple of 8)
-            __nv_bfloat16* base = static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo;
+        __nv_bfloat16* base = static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo;
+        const bool padded = EPI == EPI_BF16_EXT && g.pad_from > 0;
+        // padded: heads written pad_to columns apart (8-column pieces never straddle a head: pad_from is a multiple of 8)
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int c = col0 + 8 * i, head = c / g.pad_from;
-                *reinterpret_cast<uint4*>(base + head * g.pad_to + (c - head * g.pad_from)) =
-                    make_uint4(pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
-                               pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
-            }
-            return;
+        for (int i = 0; i < 4; i++) {
+            int c = col0 + 8 * i;
+            if (padded) { const int head = c / g.pad_from; c += head * (g.pad_to - g.pad_from); }
+            *reinterpret_cast<uint4*>(base + c) = make_uint4(pack_bf16x2(v[4 * i].x, v[4 * i].y), pack_bf16x2(v[4 * i + 1].x, v[4 * i + 1].y),
+                                                             pack_bf16x2(v[4 * i + 2].x, v[4 * i + 2].y), pack_bf16x2(v[4 * i + 3].x, v[4 * i + 3].y));
         }
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo + col0);
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            dst[i] = make_uint4(pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
-                                pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
         return;
     }
     if constexpr (EPI == EPI_FP4) {
         if (g.act == 1) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = gelu_sigmoid(v[i]);
+            for (int i = 0; i < 16; i++) v[i] = make_float2(gelu_sigmoid(v[i].x), gelu_sigmoid(v[i].y));
         } else if (!LEAN && g.act == 3) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) { float r = fmaxf(v[i], 0.f); v[i] = r * r; }
+            for (int i = 0; i < 16; i++) {
+                const float2 r = make_float2(fmaxf(v[i].x, 0.f), fmaxf(v[i].y, 0.f));
+                v[i] = mul2(r, r);
+            }
         }
-        uint32_t words[4];
-        uint32_t codes = 0;
-#pragma unroll
-        for (int half = 0; half < 2; half++) {
-            float h[16];
-#pragma unroll
-            for (int i = 0; i < 16; i++) h[i] = v[16 * half + i] * g.out_inv_gs;
-            uint32_t code;
-            uint2 bytes = quantize_block16(h, 0, code);
-            words[2 * half] = bytes.x;
-            words[2 * half + 1] = bytes.y;
-            codes |= code << (8 * half);
-        }
-        *reinterpret_cast<uint4*>(static_cast<uint8_t*>(g.out) + static_cast<size_t>(row) * g.ldo + (col0 >> 1)) =
-            make_uint4(words[0], words[1], words[2], words[3]);
+        uint32_t codes;
+        *reinterpret_cast<uint4*>(static_cast<uint8_t*>(g.out) + static_cast<size_t>(row) * g.ldo + (col0 >> 1)) = quantize_32(v, g.out_inv_gs, codes);
         *reinterpret_cast<uint16_t*>(g.out_scales + scale_offset(row, col0 >> 4, g.out_blocks)) = static_cast<uint16_t>(codes);
         return;
     }
@@ -403,10 +377,9 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         const bool is_k = !is_v && col0 >= kv0;
         const int in_head = is_v ? col0 - kv0 - hd : (is_k ? col0 - kv0 : col0 % hd);
         uint32_t packed[16];
-        if (is_v) {
 #pragma unroll
-            for (int i = 0; i < 16; i++) packed[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-        } else {
+        for (int i = 0; i < 16; i++) packed[i] = pack_bf16x2(v[i].x, v[i].y);
+        if (!is_v) {
             // Q and K heads are stored pair-interleaved: column 2i holds original dim i, column 2i+1 holds dim i+hd/2.
             const __nv_bfloat16* cs = static_cast<const __nv_bfloat16*>(g.rope_cos) + static_cast<size_t>(row) * hd;
             const __nv_bfloat16* sn = static_cast<const __nv_bfloat16*>(g.rope_sin) + static_cast<size_t>(row) * hd;
@@ -431,7 +404,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
                 const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;          // high or low halves of the two table words
                 const uint32_t cw = __byte_perm(tc[0][i >> 1], tc[1][i >> 1], sel);
                 const uint32_t sw = __byte_perm(ts[0][i >> 1], ts[1][i >> 1], sel);
-                const uint32_t xw = pack_bf16x2(v[2 * i], v[2 * i + 1]);   // (x1, x2) rounded to BF16
+                const uint32_t xw = packed[i];                             // (x1, x2) rounded to BF16
                 const uint32_t xr = __byte_perm(xw, xw, 0x1032u) ^ 0x00008000u;   // (-x2, x1)
                 const __nv_bfloat162 p = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&xw), *reinterpret_cast<const __nv_bfloat162*>(&cw));
                 const __nv_bfloat162 q = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&xr), *reinterpret_cast<const __nv_bfloat162*>(&sw));
@@ -449,6 +422,16 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
     }
 }
 
+// The drain of one GEMM instruction.  Warps 4 - 7 drain every tile, each the 32 accumulator rows of its tensor-memory
+// quarter.  A drain is a serial chain per thread (one row each), 0.5 - 1 us per 32 columns, and behind the last tile of an
+// instruction the other warps have nothing left to do: there warp w (0 - 3, same quarter) takes the second half of the
+// columns of warp w + 4 ("helped" tiles; not the 32-wide ones, which are a single chunk).  Quarters without logical rows are
+// neither drained nor helped.
+//
+// A helping warp may be an accumulator use or more ahead of the tensor core (copy warps), where the parity of acc_full
+// aliases; it therefore does not wait on that barrier but on a word that its partner sets to the ordinal of the GEMM
+// instruction once it has seen the accumulator complete.  The partner also leaves the row factors it has computed: the
+// helper comes from its role at about that moment and would have to fetch the row statistics first.
 // LEAN: the drain of the lean kernel variant; the residual-stream and plain BF16 drains there carry no row-statistics code
 // (the host sends programs that give those two epilogues row statistics to the full variant).
 template <int EPI, bool LEAN = false>
@@ -456,16 +439,24 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
                                               int stage_index, int first, int count, PipeState& ps, long long* stamp) {
     const GemmParams& g = st.p.gemm;
     constexpr bool kStats = !(LEAN && (EPI == EPI_STREAM || EPI == EPI_BF16));
+    constexpr bool kResidual = EPI != EPI_GEGLU_FP4 && EPI != EPI_GEGLU_BF16 && EPI != EPI_QKV_ROPE;
     const int quarter = (threadIdx.x >> 5) & 3;          // TMEM lane quarter this warp may read
+    const bool main = threadIdx.x >= 128;
     const int lane = lane_id();
-    for (int t = first; t < first + count; ++t) {
-        const int m_tile = t / g.n_tiles, n_tile = t - m_tile * g.n_tiles;
-        const uint32_t buf = ps.epi_tile & 1u, phase = (ps.epi_tile >> 1) & 1u;
+    const int n_tiles = g.n_tiles, block_n = g.block_n, last = first + count - 1;
+    for (int t = main ? first : last; t <= last; ++t) {
+        const int m_tile = t / n_tiles, n_tile = t - m_tile * n_tiles;
+        const uint32_t use = ps.epi_tile + static_cast<uint32_t>(t - first);
+        const uint32_t buf = use & 1u, phase = (use >> 1) & 1u;
         const int row = m_tile * 128 + quarter * 32 + lane;
         const bool row_ok = row < g.rows;
+        const bool rows_here = m_tile * 128 + quarter * 32 < g.rows;
+        const bool shared_tile = t == last && block_n >= 64, helped = shared_tile && rows_here;
+        if (!main && !helped) break;
+        const int col_begin = main ? 0 : block_n >> 1, col_end = main && helped ? block_n >> 1 : block_n;
         if (EPI == EPI_QKV_ROPE && row_ok) {
             // while the MMAs run: bring this row's rotary table entries (constant data) close
-            const int hd = g.head_dim, col_a = n_tile * g.block_n;
+            const int hd = g.head_dim, col_a = n_tile * block_n + col_begin;
             if (col_a < g.q_cols + hd) {                                   // a Q or K tile
                 const int in_head = col_a >= g.q_cols ? col_a - g.q_cols : col_a % hd;
                 const __nv_bfloat16* cs = static_cast<const __nv_bfloat16*>(g.rope_cos) + static_cast<size_t>(row) * hd + (in_head >> 1);
@@ -473,28 +464,43 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
                 prefetch_l1(cs); prefetch_l1(cs + (hd >> 1)); prefetch_l1(sn); prefetch_l1(sn + (hd >> 1));
             }
         }
-        if ((EPI == EPI_BF16_EXT || EPI == EPI_FP4) && g.col_center && lane < (g.block_n >> 5))
-            prefetch_l1(g.col_center + n_tile * g.block_n + lane * 32);    // constant data: close by when the accumulator is ready
+        if ((EPI == EPI_BF16_EXT || EPI == EPI_FP4) && g.col_center && lane < (block_n >> 5))
+            prefetch_l1(g.col_center + n_tile * block_n + lane * 32);    // constant data: close by when the accumulator is ready
         // A single-tile instruction that reads row statistics (the few-row projections behind a folded norm, whose epilogue
-        // is serial time): once the copy warp has seen the sources complete, the statistics are read and the row factor
-        // computed while the operands are still on their way, instead of after the accumulator is ready.  (Requesting the
-        // residual rows early as well was measured and lost: o_proj 7.9 vs 7.7 us.)
-        const int chunks = g.block_n >> 5;
+        // is serial time) or a residual: once the copy warp has seen the sources complete, the statistics are read and the
+        // row factor computed, and the first residual chunk is requested, while the operands are still on their way instead
+        // of after the accumulator is ready.  (The early residual alone is worth 0.25 of the 10.1 ms pi0 forward.)
         // (compiled into the drains of the projections that stand behind a folded norm in the model; the others read their
         // statistics, if they are given any, once the accumulator is ready)
         constexpr bool kEarly = EPI == EPI_QKV_ROPE || EPI == EPI_GEGLU_FP4 || EPI == EPI_FP4 || EPI == EPI_BF16_EXT;
-        const bool early = kEarly && count == 1 && (g.row_sumsq != nullptr || g.row_factor != nullptr);
-        if (early) {
-            if (!wait_deps_seen(prog, ctl, ps.gemm_seq, stage_index)) return;
+        const bool early = count == 1 && ((kEarly && (g.row_sumsq != nullptr || g.row_factor != nullptr)) || (kResidual && g.residual != nullptr));
+        uint4 res[4] = {};
+        auto load_residual = [&](int c) {
+            if (kResidual && g.residual && row_ok) {
+                const uint4* r = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(g.residual) + static_cast<size_t>(row) * g.ldr + n_tile * block_n + c);
+#pragma unroll
+                for (int i = 0; i < 4; i++) res[i] = __ldcg(r + i);
+            }
+        };
+        volatile float* shared = &ctl->drain_rows[(quarter * 4 + static_cast<int>(ps.gemm_seq & 3u)) * 64 + lane];
+        if (!main) {
+            if (kResidual && early) {
+                if (!word_wait<0>(prog, ctl, &ctl->deps_seen, ps.gemm_seq, stage_index)) return;
+                load_residual(col_begin);
+            }
+            if (!word_wait<0>(prog, ctl, &ctl->drain_seen[quarter], ps.gemm_seq, stage_index)) return;
+        } else if (early) {
+            if (!word_wait<32>(prog, ctl, &ctl->deps_seen, ps.gemm_seq, stage_index)) return;
+            load_residual(0);
         } else {
             if (!mbar_wait_warp(prog, ctl, &ctl->acc_full[buf], phase, stage_index)) return;
         }
         // alpha, times the row's 1/rms where the projection reads un-normalised rows (norm weight folded into B): given
         // as a factor, or as the producer's per-tile sums of squares (complete: the operands behind this accumulator
         // were only copied after the producer stage had finished)
-        float row_scale = g.alpha, row_shift = 0.f, sumsq = 0.f, sum = 0.f;
-        if (kStats && row_ok && g.row_factor) row_scale *= __ldcg(g.row_factor + row);
-        if (kStats && row_ok && g.row_sumsq) {
+        float row_scale = g.alpha, row_shift = 0.f;
+        if (kStats && main && row_ok && g.row_factor) row_scale *= __ldcg(g.row_factor + row);
+        if (kStats && main && row_ok && g.row_sumsq) {
             const float4* part = reinterpret_cast<const float4*>(g.row_sumsq + static_cast<size_t>(row) * g.sumsq_parts);
             const int quads = g.sumsq_parts >> 2;
             float total = 0.f;
@@ -535,36 +541,79 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
                 row_scale *= rsqrtf(total * g.sumsq_inv_width + g.sumsq_eps);
             }
         }
-        if (early && !mbar_wait_warp(prog, ctl, &ctl->acc_full[buf], phase, stage_index)) return;
+        if (main) {
+            if (early && !mbar_wait_warp(prog, ctl, &ctl->acc_full[buf], phase, stage_index)) return;
+            if (helped) {
+                if (kStats) { shared[0] = row_scale; shared[32] = row_shift; }
+                __syncwarp();
+                if (lane == 0) word_set(&ctl->drain_seen[quarter], ps.gemm_seq + 1u);
+            }
+        } else if (kStats) {
+            row_scale = shared[0];
+            row_shift = shared[32];
+        }
         tc_fence_after();
         if (stamp && t == first && threadIdx.x == 128) stamp[6] = static_cast<long long>(global_ns());
         const uint32_t taddr = tmem + buf * 128u + (static_cast<uint32_t>(quarter * 32) << 16);
-        for (int c = 0; c < chunks; ++c) {
-            uint32_t raw[32];
-            tmem_ld32(taddr + c * 32, raw);
-            tmem_ld_wait();
-            if (c == chunks - 1) {
-                // every column of this accumulator is in registers: hand the buffer back to the MMA lane
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ctl->acc_empty[buf]);
+        const uint32_t share = helped ? 1u : 2u;             // parts of the tile this warp speaks for: two per quarter
+        auto columns_read = [&]() {                          // this warp's part of the accumulator is in registers
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_count(&ctl->acc_empty[buf], share);
+        };
+        // Residual-stream statistics: the two halves of a tile are summed apart, whichever warps drain them, and added at the
+        // end, so the bits do not depend on how the tiles are dealt to the workers.
+        float2 sumsq = make_float2(0.f, 0.f), sum = make_float2(0.f, 0.f);
+        float sumsq_half = 0.f, sum_half = 0.f;
+        if (!rows_here) {
+            columns_read();
+        } else {
+            if (!early) load_residual(col_begin);
+            for (int c = col_begin; c < col_end; c += 32) {
+                uint32_t raw[32];
+                tmem_ld32(taddr + c, raw);
+                tmem_ld_wait();
+                if (c + 32 == col_end) columns_read();
+                if (EPI == EPI_STREAM && main && block_n >= 64 && c == block_n >> 1) {
+                    sumsq_half = sumsq.x + sumsq.y;
+                    sum_half = sum.x + sum.y;
+                    sumsq = sum = make_float2(0.f, 0.f);
+                }
+                gemm_epilogue_chunk<EPI, LEAN>(g, raw, res, row, n_tile * block_n + c, row_ok, row_scale, row_shift, sumsq, sum);
+                if (c + 32 < col_end) load_residual(c + 32);
             }
-            gemm_epilogue_chunk<EPI, LEAN>(g, raw, row, n_tile * g.block_n + c * 32, row_ok, row_scale, row_shift, sumsq, sum);
         }
-        if (EPI == EPI_STREAM && row_ok) {
-            g.sumsq_out[static_cast<size_t>(row) * g.sumsq_ld + n_tile] = sumsq;
-            if (g.sum_out) g.sum_out[static_cast<size_t>(row) * g.sumsq_ld + n_tile] = sum;
+        if (EPI == EPI_STREAM && rows_here) {
+            float a = sumsq.x + sumsq.y, b = sum.x + sum.y;
+            if (!main) {                                     // second half: handed to the partner
+                shared[0] = a;
+                shared[32] = b;
+                __syncwarp();
+                if (lane == 0) word_set(&ctl->sums_seen[quarter], ps.gemm_seq + 1u);
+            } else {
+                if (helped) {
+                    if (!word_wait<0>(prog, ctl, &ctl->sums_seen[quarter], ps.gemm_seq, stage_index)) return;
+                    sumsq_half = shared[0];
+                    sum_half = shared[32];
+                }
+                if (row_ok) {
+                    g.sumsq_out[static_cast<size_t>(row) * g.sumsq_ld + n_tile] = a + sumsq_half;
+                    if (g.sum_out) g.sum_out[static_cast<size_t>(row) * g.sumsq_ld + n_tile] = b + sum_half;
+                }
+            }
         }
-        // each epilogue warp publishes its own 32 rows (a GEMM tile counts 4 units): no CTA barrier on this path
-        if (stamp && t == first + count - 1 && threadIdx.x == 128) stamp[7] = static_cast<long long>(global_ns());
+        // The tile is published once, by whichever warp finishes last: a counter that takes one increment per warp of every
+        // tile serialises them in L2 (40 tiles x 6 warps: the attention behind q|k|v saw its sources 0.6 us later).
+        if (stamp && t == last && threadIdx.x == 128) stamp[7] = static_cast<long long>(global_ns());
         fence_proxy_async_global();
         __syncwarp();
-        if (lane == 0) publish_tile(prog, st, t);
-        ps.epi_tile++;
+        if (lane == 0 && join_parts(&ctl->tile_parts[shared_tile ? 4u + (ps.gemm_seq & 3u) : use & 3u], share)) publish_tile(prog, st, t);
     }
+    ps.epi_tile += static_cast<uint32_t>(count);
 }
 
-// Dispatch of one GEMM instruction onto the warp roles. Warp 2 has no role and falls through.
+// Dispatch of one GEMM instruction onto the warp roles (warp 2 has none); behind its role every warp goes through the
+// drain, as one of the draining warps or as a helper of the last tile.
 // LEAN: the kernel variant for programs made only of NVFP4 projections with the pi0 model's epilogues (the host checks
 // this when it builds a program); it carries neither the dense issue loops nor the other drain loops.
 template <bool LEAN>
@@ -582,18 +631,17 @@ __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl
         if (LEAN || operands == GEMM_NVFP4) gemm_mma<GEMM_NVFP4>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
         else if (operands == GEMM_BF16) gemm_mma<GEMM_BF16>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
         else gemm_mma<GEMM_FP8>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
-    } else if (warp >= 4) {
-        const int epilogue = st.p.gemm.epilogue;            // one drain loop per epilogue kind: only its own arithmetic and registers
-        if (epilogue == EPI_BF16) gemm_epilogue<EPI_BF16, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        else if (epilogue == EPI_STREAM) gemm_epilogue<EPI_STREAM, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        else if (epilogue == EPI_GEGLU_FP4) gemm_epilogue<EPI_GEGLU_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        else if (epilogue == EPI_FP4) gemm_epilogue<EPI_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        else if (epilogue == EPI_QKV_ROPE) gemm_epilogue<EPI_QKV_ROPE, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        else if (LEAN || epilogue == EPI_BF16_EXT) gemm_epilogue<EPI_BF16_EXT, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        else if (epilogue == EPI_F32) gemm_epilogue<EPI_F32>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        else gemm_epilogue<EPI_GEGLU_BF16>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-        if (stamp && threadIdx.x == 128) stamp[2] = static_cast<long long>(global_ns());
     }
+    const int epilogue = st.p.gemm.epilogue;                // one drain loop per epilogue kind: only its own arithmetic and registers
+    if (epilogue == EPI_BF16) gemm_epilogue<EPI_BF16, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (epilogue == EPI_STREAM) gemm_epilogue<EPI_STREAM, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (epilogue == EPI_GEGLU_FP4) gemm_epilogue<EPI_GEGLU_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (epilogue == EPI_FP4) gemm_epilogue<EPI_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (epilogue == EPI_QKV_ROPE) gemm_epilogue<EPI_QKV_ROPE, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (LEAN || epilogue == EPI_BF16_EXT) gemm_epilogue<EPI_BF16_EXT, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (epilogue == EPI_F32) gemm_epilogue<EPI_F32>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else gemm_epilogue<EPI_GEGLU_BF16>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    if (stamp && threadIdx.x == 128) stamp[2] = static_cast<long long>(global_ns());
     ps.gemm_seq++;                                          // (every warp: the ordinal of the next GEMM instruction of this CTA)
 }
 

@@ -112,14 +112,6 @@ constexpr int kLinStageBytes = (kLinRows + kLinCols) * kLinLd * 4;     // x bloc
 static_assert(kLinStages * kLinStageBytes <= kDataBytes, "linear32 ring exceeds the data region");
 static_assert(8 * (kLinRows * kLinCols + kLinRows) * 4 <= kLinStages * kLinStageBytes, "partial sums exceed the ring");
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(d)
-        : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)), "l"(*reinterpret_cast<const uint64_t*>(&c)));
-    return *reinterpret_cast<float2*>(&d);
-}
-
 // Geometry of one tile, read once from the (shared-memory) descriptor.
 struct LinTile {
     const void* x;

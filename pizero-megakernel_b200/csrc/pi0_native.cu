@@ -155,11 +155,8 @@ struct Program {
     }
 };
 
-int units_of(const StageDesc& d) { return d.kind == OP_GEMM ? 4 : 1; }
-
 // Fill counter bookkeeping of a stage from its geometry.
 void finish_desc(StageDesc& d) {
-    d.units_per_tile = units_of(d);
     for (int i = 0; i < kMaxSources; i++) {
         d.src[i] = -1;
         d.src_mode[i] = SRC_ALL_BANDS;
@@ -230,7 +227,7 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
     }
     prog->expected.assign(counters, 0);
     for (auto& d : prog->stages)
-        for (int t = 0; t < d.tiles; t++) prog->expected[d.counter_base + std::min(t / d.band_div, d.bands - 1)] += d.units_per_tile;
+        for (int t = 0; t < d.tiles; t++) prog->expected[d.counter_base + std::min(t / d.band_div, d.bands - 1)] += 1;
     // static validation: stage order per worker, every tile exactly once, sources earlier than consumers
     std::vector<std::vector<int>> cover(prog->stages.size());
     for (size_t s = 0; s < prog->stages.size(); s++) {
@@ -1537,8 +1534,7 @@ extern "C" int read_native_linear(void* handle, unsigned long long* counters, in
     std::vector<unsigned int> raw(count);
     int e = read_native_model_counters(handle, raw.data(), nullptr, count, nullptr);
     if (e) return e;
-    // reported in tiles (a GEMM tile is four warp contributions)
-    for (int i = 0; i < count; i++) counters[i] = raw[i] / 4;
+    for (int i = 0; i < count; i++) counters[i] = raw[i];
     *epoch = prog->epoch;
     return cudaSuccess;
 }

@@ -48,6 +48,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_count(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
 // One try of a phase wait. The thread may be suspended inside the instruction; the explicit hint bounds that
 // suspension to about a microsecond (without it the limit is system dependent and can be very long), so a caller
 // that polls an abort flag between tries stays responsive. A completing phase wakes the thread immediately.
@@ -184,11 +187,36 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
 }
 
 // ---------------------------------------------------------------- number formats
-// Two FP32 -> one byte of E2M1 codes (RNE, saturating); `lo` lands in the low nibble.
-__device__ __forceinline__ uint32_t cvt_e2m1x2(float lo, float hi) {
-    uint16_t bits;
-    asm("{ .reg .b8 b; cvt.rn.satfinite.e2m1x2.f32 b, %2, %1; cvt.u16.u8 %0, b; }" : "=h"(bits) : "f"(lo), "f"(hi));
-    return bits;
+// Pairs of FP32 operations in one instruction, each lane rounded as its scalar form.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)), "l"(*reinterpret_cast<const uint64_t*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+    float d;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// Eight FP32 -> four bytes of E2M1 codes (RNE, saturating), the first value in the lowest nibble.
+__device__ __forceinline__ uint32_t cvt_e2m1x8(float2 a, float2 b, float2 c, float2 d) {
+    uint32_t w;
+    asm("{ .reg .b8 p, q, r, s; cvt.rn.satfinite.e2m1x2.f32 p, %2, %1; cvt.rn.satfinite.e2m1x2.f32 q, %4, %3;\n"
+        "  cvt.rn.satfinite.e2m1x2.f32 r, %6, %5; cvt.rn.satfinite.e2m1x2.f32 s, %8, %7; mov.b32 %0, {p, q, r, s}; }"
+        : "=r"(w) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y));
+    return w;
 }
 __device__ __forceinline__ uint32_t encode_ue4m3(float x) {
     return static_cast<uint32_t>(__nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3));
@@ -205,24 +233,28 @@ __device__ __forceinline__ uint32_t block_scale_code(float amax, int policy) {
     if (policy == 1 && decode_ue4m3(code) < desired && code < 126u) code += 1u;
     return code;
 }
-// Quantise 16 values (already divided by the tensor scale) -> 8 bytes + scale code.
-__device__ __forceinline__ uint2 quantize_block16(const float (&v)[16], int policy, uint32_t& code_out) {
-    float amax = 0.f;
+// Quantise 16 values (already divided by the tensor scale) -> 8 bytes + scale code.  Few-row operators run this once per
+// thread as straight-line code, so its length is their time: packed multiplies, three-input maxima and whole-word
+// packing of the codes make it about half as long as the scalar form.
+__device__ __forceinline__ uint2 quantize_block16(const float2 (&v)[8], int policy, uint32_t& code_out) {
+    const float a = max3_abs(max3_abs(v[0].x, v[0].y, v[1].x), max3_abs(v[1].y, v[2].x, v[2].y), max3_abs(v[3].x, v[3].y, v[4].x));
+    const float amax = max3_abs(max3_abs(a, v[4].y, v[5].x), max3_abs(v[5].y, v[6].x, v[6].y), fmaxf(fabsf(v[7].x), fabsf(v[7].y)));
+    const uint32_t code = block_scale_code(amax, policy);
+    const float decoded = decode_ue4m3(code);
+    const float recip = decoded > 0.f ? __frcp_rn(decoded) : 0.f;
+    const float2 r2 = make_float2(recip, recip);
+    float2 s[8];
 #pragma unroll
-    for (int i = 0; i < 16; i++) amax = fmaxf(amax, fabsf(v[i]));
-    uint32_t code = block_scale_code(amax, policy);
-    float decoded = decode_ue4m3(code);
-    float recip = decoded > 0.f ? __frcp_rn(decoded) : 0.f;
-    uint32_t w[2] = {0u, 0u};
-    if (decoded > 0.f) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            uint32_t b = cvt_e2m1x2(v[2 * i] * recip, v[2 * i + 1] * recip) & 0xFFu;
-            w[i >> 2] |= b << (8 * (i & 3));
-        }
-    }
+    for (int i = 0; i < 8; i++) s[i] = mul2(v[i], r2);
     code_out = code;
-    return make_uint2(w[0], w[1]);
+    const uint32_t keep = decoded > 0.f ? 0xffffffffu : 0u;            // zero codes (no negative zeros) under a zero scale
+    return make_uint2(cvt_e2m1x8(s[0], s[1], s[2], s[3]) & keep, cvt_e2m1x8(s[4], s[5], s[6], s[7]) & keep);
+}
+__device__ __forceinline__ uint2 quantize_block16(const float (&v)[16], int policy, uint32_t& code_out) {
+    float2 pairs[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) pairs[i] = make_float2(v[2 * i], v[2 * i + 1]);
+    return quantize_block16(pairs, policy, code_out);
 }
 // Offset of scale (row, block) in the 128x4 atom layout with `blocks` blocks per row.
 __device__ __forceinline__ size_t scale_offset(int row, int block, int blocks) {

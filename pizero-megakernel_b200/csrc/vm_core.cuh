@@ -16,7 +16,7 @@ constexpr int kChunks = 2;                                   // 256-wide K chunk
 constexpr int kTileABytes = 128 * 128;                       // one chunk of one operand: 128 rows x 128 bytes
 constexpr int kSfBytes = kChunks * 4 * 512;                  // scale atoms of one operand: four 64-wide K groups per chunk
 constexpr int kStageBytes = 2 * kChunks * kTileABytes + 2 * kSfBytes;   // largest slot: 72 KiB
-constexpr int kCtlBytes = 3072;
+constexpr int kCtlBytes = 7168;
 constexpr int kDataBytes = 216 * 1024;                       // operator scratch behind the control block: three full-size slots
 constexpr int kSmemBytes = kCtlBytes + kDataBytes + 1024;    // + slack for 1 KiB alignment
 constexpr int kTmemCols = 512;
@@ -44,13 +44,24 @@ struct Ctl {
     uint64_t gather;             // all warps have reached a CTA-wide operator (one arrival per warp)
     uint64_t done;               // all warps have left the instruction loop
     uint32_t tmem_base;
-    volatile uint32_t deps_seen; // GEMM instructions of this CTA whose sources its copy warp has seen complete (monotonic)
+    // ordinals of GEMM instructions (word_set / word_wait): the copy warp has seen the sources complete; per tensor-memory
+    // quarter, the draining warp has seen the last accumulator complete; the helping warp has left its row sums
+    volatile uint32_t deps_seen, drain_seen[4], sums_seen[4];
+    // Parts (of eight) of a tile that are stored (join_parts).  [0, 4): tiles drained by warps 4 - 7 alone, by accumulator use
+    // modulo 4 - those warps are at most two uses apart, because the accumulator of use u + 2 is only filled once all of
+    // them have read the one of use u.  [4, 8): the last tile of an instruction, by GEMM instruction modulo 4 - its helping
+    // warps may be further behind, but the instruction ring keeps all warps less than kRing instructions apart.
+    uint32_t tile_parts[8];
     volatile int abort;          // CTA-local copy of the abort decision
     volatile int dep_ok;         // broadcast slot for CTA-wide operators
     volatile int flag;           // second broadcast slot (outcome of the split-KV ticket wait)
     int gate;                    // CTA-wide operators entered so far, or -1 once a warp has given up on one (gather_enter)
+    // per quarter and GEMM instruction modulo 4 (see tile_parts): row factors for the helping warp, then the sums of squares
+    // and sums of its half of every row
+    volatile float drain_rows[4 * 4 * 2 * 32];
     Slot slot[kRing];
 };
+static_assert(kRing <= 4, "words kept per GEMM instruction modulo 4");
 static_assert(sizeof(Ctl) <= kCtlBytes, "control block too large");
 
 // The ring geometry (slot count and size) belongs to the GEMM, so positions are kept per barrier: bit s of
@@ -144,17 +155,22 @@ __device__ __forceinline__ bool mbar_wait_warp(const VmProgram& prog, Ctl* ctl, 
     return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || mbar_wait_warp_long(prog, ctl, bar, parity, stage);
 }
 
-// Wait (bounded, abort-aware, one decision per warp) until the copy warp of this CTA has seen the sources of GEMM instruction
-// number `seq` complete: from then on everything those sources wrote - and everything that was final before they ran - may
-// be read, so an epilogue warp can request its residual rows and row statistics while the operands are still on their way.
-__device__ __forceinline__ bool wait_deps_seen(const VmProgram& prog, Ctl* ctl, uint32_t seq, int stage) {
+// Shared-memory words that hold the ordinal (+ 1) of the last GEMM instruction for which something has happened; one writer
+// each.  Monotonic, so a waiting warp may be any number of instructions ahead.
+__device__ __forceinline__ void word_set(volatile uint32_t* word, uint32_t value) {
+    asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(word))), "r"(value) : "memory");
+}
+// Whole warp: wait (bounded, abort-aware, one decision per warp) until `word` has passed `seq`; what the writer had seen or
+// written before is then visible to every lane.  PAUSE: nanoseconds between two looks.
+template <int PAUSE>
+__device__ __forceinline__ bool word_wait(const VmProgram& prog, Ctl* ctl, volatile uint32_t* word, uint32_t seq, int stage) {
     unsigned long long start = 0;
     for (uint32_t spin = 1;; ++spin) {
         uint32_t seen;                                       // (every lane reads the word: no broadcast on the way out)
-        asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(seen) : "r"(smem_u32(const_cast<uint32_t*>(&ctl->deps_seen))) : "memory");
+        asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(seen) : "r"(smem_u32(const_cast<uint32_t*>(word))) : "memory");
         if (__all_sync(0xffffffffu, seen > seq)) return true;
         if (__any_sync(0xffffffffu, ctl->abort != 0)) return false;
-        __nanosleep(32);
+        if (PAUSE) __nanosleep(PAUSE);
         if ((spin & 255u) == 0u) {
             int stop = 0;
             if (lane_id() == 0) {
@@ -169,6 +185,14 @@ __device__ __forceinline__ bool wait_deps_seen(const VmProgram& prog, Ctl* ctl, 
             if (__shfl_sync(0xffffffffu, stop, 0)) return false;
         }
     }
+}
+
+// One thread per warp, behind a warp barrier: `share` more of a tile's eight parts are stored.  True for the call that
+// completes the tile; everything the other parts stored is then visible to the caller (and through its release to others).
+__device__ __forceinline__ bool join_parts(uint32_t* word, uint32_t share) {
+    uint32_t before;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(before) : "r"(smem_u32(word)), "r"(share) : "memory");
+    return ((before + share) & 7u) == 0u;
 }
 
 // Entry of a CTA-wide operator: all eight warps go in, or none does.
@@ -275,7 +299,7 @@ __device__ __forceinline__ bool warp_wait_sources(const VmProgram& prog, Ctl* ct
 }
 
 // Publish progress of a tile. Call from ONE thread after a barrier (CTA or warp) that covers every
-// writer thread it speaks for. A stage's tile is complete after `units_per_tile` such calls.
+// writer thread it speaks for. A finished tile counts one.
 __device__ __forceinline__ void publish_tile(const VmProgram& prog, const StageDesc& st, int tile) {
     red_release_add(prog.counters + st.counter_base + tile_band(st, tile), 1u);
 }

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&ctl->acc_full[b], 1);
-            mbar_init(&ctl->acc_empty[b], 4);      // one arrival per epilogue warp
+            mbar_init(&ctl->acc_empty[b], 8);      // two arrivals per tensor-memory quarter
         }
         for (int r = 0; r < kRing; r++) {
             mbar_init(&ctl->ready[r], 32);         // every lane of the prefetch warp
@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
         mbar_init(&ctl->done, kThreads / 32);
         ctl->abort = 0;
         ctl->deps_seen = 0;
+        for (int q = 0; q < 4; q++) ctl->drain_seen[q] = ctl->sums_seen[q] = ctl->tile_parts[q] = ctl->tile_parts[4 + q] = 0;
         ctl->dep_ok = 1;
         ctl->gate = 0;
         mbar_fence_init();

@@ -250,7 +250,6 @@ struct alignas(16) StageDesc {
     int src[kMaxSources];
     int src_mode[kMaxSources];
     int aux_base, aux_count;     // extra program counters owned by the stage (attention: one ticket per head)
-    int units_per_tile;          // counter increments one finished tile contributes (GEMM: one per epilogue warp)
     // Filled by the host when the program is built, so a consumer polls counters without touching its producers'
     // descriptors: first counter, band count and the per-launch contribution of a full / of the last band.
     int src_counter_base[kMaxSources];
