@@ -245,9 +245,9 @@ template <int EPI, bool LEAN = false>
 __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const uint32_t (&raw)[32], const uint4 (&res)[4], int row, int col0,
                                                     bool row_ok, float row_scale, float row_shift, float2& sumsq, float2& sum) {
     float2 v[16];
-    if (!row_ok) return;
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = mul2(make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1])), make_float2(row_scale, row_scale));
+    if (!row_ok) return;
     if constexpr (EPI == EPI_BF16_EXT || EPI == EPI_FP4) {
         if (g.col_center) {
             // folded LayerNorm: subtract the row mean's share, mean * rstd * (sum over K of weight row n)
@@ -444,6 +444,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
     const bool main = threadIdx.x >= 128;
     const int lane = lane_id();
     const int n_tiles = g.n_tiles, block_n = g.block_n, last = first + count - 1;
+    int run = 0;                                         // tiles drained since the last publication
     for (int t = main ? first : last; t <= last; ++t) {
         const int m_tile = t / n_tiles, n_tile = t - m_tile * n_tiles;
         const uint32_t use = ps.epi_tile + static_cast<uint32_t>(t - first);
@@ -602,12 +603,18 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
                 }
             }
         }
-        // The tile is published once, by whichever warp finishes last: a counter that takes one increment per warp of every
-        // tile serialises them in L2 (40 tiles x 6 warps: the attention behind q|k|v saw its sources 0.6 us later).
+        // The tiles of a run - one row band, one instruction - are published together and once, by whichever warp finishes
+        // last.  A counter that takes one increment per warp of every tile serialises them in L2 (40 tiles x 6 warps: the
+        // attention behind q|k|v saw its sources 0.6 us later), and the fences in front of it wait for the stores.
+        run++;
+        if (t != last && (t + 1) / n_tiles == m_tile) continue;
         if (stamp && t == last && threadIdx.x == 128) stamp[7] = static_cast<long long>(global_ns());
         fence_proxy_async_global();
         __syncwarp();
-        if (lane == 0 && join_parts(&ctl->tile_parts[shared_tile ? 4u + (ps.gemm_seq & 3u) : use & 3u], share)) publish_tile(prog, st, t);
+        if (lane == 0 && join_parts(&ctl->tile_parts[shared_tile ? 4u + (ps.gemm_seq & 3u) : ps.epi_run & 3u], share))
+            publish_tile(prog, st, t, static_cast<unsigned int>(main ? run : min(count, t - m_tile * n_tiles + 1)));
+        run = 0;
+        if (!shared_tile) ps.epi_run++;
     }
     ps.epi_tile += static_cast<uint32_t>(count);
 }

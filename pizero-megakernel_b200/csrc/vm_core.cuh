@@ -47,10 +47,10 @@ struct Ctl {
     // ordinals of GEMM instructions (word_set / word_wait): the copy warp has seen the sources complete; per tensor-memory
     // quarter, the draining warp has seen the last accumulator complete; the helping warp has left its row sums
     volatile uint32_t deps_seen, drain_seen[4], sums_seen[4];
-    // Parts (of eight) of a tile that are stored (join_parts).  [0, 4): tiles drained by warps 4 - 7 alone, by accumulator use
-    // modulo 4 - those warps are at most two uses apart, because the accumulator of use u + 2 is only filled once all of
-    // them have read the one of use u.  [4, 8): the last tile of an instruction, by GEMM instruction modulo 4 - its helping
-    // warps may be further behind, but the instruction ring keeps all warps less than kRing instructions apart.
+    // Parts (of eight) of a run of tiles that are stored (join_parts).  [0, 4): runs drained by warps 4 - 7 alone, by their
+    // ordinal modulo 4 - those warps are at most two tiles apart, because the accumulator of use u + 2 is only filled once
+    // all of them have read the one of use u.  [4, 8): runs that end with a helped tile, by GEMM instruction modulo 4 - the
+    // helping warps may be further behind, but the instruction ring keeps all warps less than kRing instructions apart.
     uint32_t tile_parts[8];
     volatile int abort;          // CTA-local copy of the abort decision
     volatile int dep_ok;         // broadcast slot for CTA-wide operators
@@ -73,6 +73,7 @@ struct PipeState {
     uint32_t mma_it = 0;         // K stages consumed by the MMA lane (rotates the scale columns in tensor memory)
     uint32_t mma_tile = 0;       // accumulator tiles produced
     uint32_t epi_tile = 0;       // accumulator tiles drained
+    uint32_t epi_run = 0;        // runs of tiles published by the draining warps alone
     uint32_t gemm_seq = 0;       // GEMM instructions this warp has been through (every warp counts them)
 };
 
@@ -187,8 +188,8 @@ __device__ __forceinline__ bool word_wait(const VmProgram& prog, Ctl* ctl, volat
     }
 }
 
-// One thread per warp, behind a warp barrier: `share` more of a tile's eight parts are stored.  True for the call that
-// completes the tile; everything the other parts stored is then visible to the caller (and through its release to others).
+// One thread per warp, behind a warp barrier: `share` more of the eight parts of a run of tiles are stored.  True for the call
+// that completes the run; everything the other parts stored is then visible to the caller (and through its release to others).
 __device__ __forceinline__ bool join_parts(uint32_t* word, uint32_t share) {
     uint32_t before;
     asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(before) : "r"(smem_u32(word)), "r"(share) : "memory");
@@ -299,9 +300,9 @@ __device__ __forceinline__ bool warp_wait_sources(const VmProgram& prog, Ctl* ct
 }
 
 // Publish progress of a tile. Call from ONE thread after a barrier (CTA or warp) that covers every
-// writer thread it speaks for. A finished tile counts one.
-__device__ __forceinline__ void publish_tile(const VmProgram& prog, const StageDesc& st, int tile) {
-    red_release_add(prog.counters + st.counter_base + tile_band(st, tile), 1u);
+// writer thread it speaks for. A finished tile counts one (`tiles` of one band may be published together).
+__device__ __forceinline__ void publish_tile(const VmProgram& prog, const StageDesc& st, int tile, unsigned int tiles = 1u) {
+    red_release_add(prog.counters + st.counter_base + tile_band(st, tile), tiles);
 }
 
 // CTA-wide operators: warp 0 waits for the bands of the whole tile range, everybody learns the outcome.
