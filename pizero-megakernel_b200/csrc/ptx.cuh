@@ -34,6 +34,9 @@ __device__ __forceinline__ bool elect_one() {
 // Programmatic dependent launch: returns when every grid in front of this one in the stream has completed and its writes
 // are visible.  (Without the launch attribute it returns at once.)
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Once every CTA has said this (or exited), CTAs of the next grid may take up free SMs and prepare; that grid's own
+// grid_dependency_wait still waits for this one's end.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

@@ -88,9 +88,6 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
-    // Up to here nothing that other work on the stream writes was touched: launched with programmatic stream serialisation
-    // (launch_program), this CTA may be set up while the previous kernel's completion is still being processed.
-    grid_dependency_wait();
 
     const int4* stream = prog.code + static_cast<size_t>(blockIdx.x) * prog.length;
     // first instruction of the requested stage range (streams are sorted by stage)
@@ -107,6 +104,10 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
         for (int s = 0; s < kAhead; s++) prefetch_slot(prog, ctl, stream, s, ip0 + s, fetch_instruction(prog, stream, ip0 + s));
         pending = fetch_instruction(prog, stream, ip0 + kAhead);
     }
+    // Up to here only the program itself was read, which no kernel writes: launched with programmatic stream serialisation
+    // (launch_program) this CTA prepares, and fetches its first instructions, while the kernel in front is still finishing.
+    grid_dependency_wait();
+    if (prog.early_dependents) grid_launch_dependents();
 
     PipeState ps;
     uint32_t gathers = 0;        // CTA-wide operators executed so far (phase of the gather barrier)
