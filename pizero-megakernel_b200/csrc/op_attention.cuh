@@ -413,7 +413,7 @@ __device__ __forceinline__ void merge_item(const MergeParams& g, int group, int 
             const float ref = big == -INFINITY ? 0.f : big;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float w = j < g.splits ? exp2f(pair[j].x - ref) : 0.f;          // 0 for a fully masked split
+                const float w = j < g.splits ? exp2_fast(pair[j].x - ref) : 0.f;          // 0 for a fully masked split
                 denom += w * pair[j].y;
                 merge_accumulate(acc, w, x[j]);
             }
@@ -439,7 +439,7 @@ __device__ __forceinline__ void merge_item(const MergeParams& g, int group, int 
             }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float w = s0 + j < g.splits ? exp2f(pair[j].x - ref) : 0.f;     // 0 for a fully masked split
+                const float w = s0 + j < g.splits ? exp2_fast(pair[j].x - ref) : 0.f;     // 0 for a fully masked split
                 denom += w * pair[j].y;
                 merge_accumulate(acc, w, x[j]);
             }
@@ -482,7 +482,7 @@ __device__ __forceinline__ void merge_item_wide(const MergeParams& g, int group,
     float denom = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        const float w = exp2f(pair[j].x - ref);               // 0 for an absent or fully masked split
+        const float w = exp2_fast(pair[j].x - ref);               // 0 for an absent or fully masked split
         denom += w * pair[j].y;
         merge_accumulate(acc, w, x[j]);
     }
@@ -530,42 +530,44 @@ __device__ __forceinline__ void merge_instruction(const VmProgram& prog, Ctl* ct
 // resident on different SMs at the same time) meet on a per-group ticket counter that grows by `splits` per launch; once all partials of
 // the head are published, every tile merges its share of the query rows (row % splits == split), so the merge
 // costs neither a stage of its own nor a serial tail on one SM.
-template <int HDP, bool MASK>
+template <int HDP, bool LEAN, bool MASK, bool TWICE>
 __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& a, int tile, uint8_t* data, uint32_t tmem,
                              uint32_t uses, int stage, long long* stamp, const StageDesc* deps, int dep_first, int dep_count);
 
-// LEAN: kernel variant for programs whose attention stages all run on the tcgen05 tiles (no mma.sync tile code).
+// LEAN: the lean kernel variant (no boolean masks); MMA_SYNC: the variant with the mma.sync tiles.
 // The instruction waits for its sources itself (the instruction loop does not): the tcgen05 tile does so after its
 // index arithmetic, the other tiles up front.
-template <bool LEAN>
+template <bool LEAN, bool MMA_SYNC>
 __device__ __forceinline__ void attn_instruction(const VmProgram& prog, Ctl* ctl, uint8_t* data, uint32_t tmem, uint32_t& tc_tiles,
                                                  const StageDesc& st, int stage_index, int first, int count, long long* stamp) {
     const AttnParams& a = st.p.attn;
-    if (!(LEAN || a.tc) && !cta_wait_sources(prog, ctl, st, stage_index, first, count, stamp)) return;
+    if (MMA_SYNC && !a.tc && !cta_wait_sources(prog, ctl, st, stage_index, first, count, stamp)) return;
     for (int t = first; t < first + count; ++t) {
         long long* stamp_t = t == first ? stamp : nullptr;
         const StageDesc* deps = t == first ? &st : nullptr;
-        if (LEAN || a.tc) {
+        if (!MMA_SYNC || a.tc) {
             bool ok = false;
             if (!LEAN && a.mask) {
                 if constexpr (!LEAN)
-                    ok = a.hd_pad > 128 ? attn_tile_tc<256, true>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count)
-                                        : attn_tile_tc<128, true>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count);
+                    ok = a.hd_pad > 128 ? attn_tile_tc<256, false, true, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count)
+                                        : attn_tile_tc<128, false, true, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count);
             } else {
-                ok = a.hd_pad > 128 ? attn_tile_tc<256, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count)
-                                    : attn_tile_tc<128, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count);
+                // (KV splits of at most 64 queries of 256-wide heads, the action expert's: four threads per row)
+                ok = a.hd_pad > 128 ? (a.q_box <= 64 && a.splits > 1 ? attn_tile_tc<256, LEAN, false, true>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count)
+                                                     : attn_tile_tc<256, LEAN, false, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count))
+                                    : attn_tile_tc<128, LEAN, false, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count);
             }
             tc_tiles++;
             if (!ok) return;                                   // uniform: a wait gave up, the abort flag is set
-        } else if constexpr (!LEAN) {
+        } else if constexpr (MMA_SYNC) {
             if (a.head_dim > 128) attn_tile<256>(a, t, data, stamp_t);
             else attn_tile<80>(a, t, data, stamp_t);
         }
         if (a.splits > 1 && a.fused_merge) {
             const int split = t % a.splits, group = t / a.splits;         // group: one head of one 128-query tile
-            // The barrier orders every thread's partial stores before thread 0's release increment below, which
-            // is cumulative at GPU scope: no per-thread fence is needed.
-            __syncthreads();
+            // A barrier (the tcgen05 tile ends with one) orders every thread's partial stores before thread 0's release
+            // increment below, which is cumulative at GPU scope: no per-thread fence is needed.
+            if (MMA_SYNC && !a.tc) __syncthreads();
             if (threadIdx.x == 0) {
                 const unsigned int target = static_cast<unsigned int>(a.splits) * prog.epoch;
                 red_release_add(a.tickets + group, 1u);

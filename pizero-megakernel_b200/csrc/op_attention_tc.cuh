@@ -6,6 +6,8 @@
 //   S    : tcgen05.mma kind::f16, M 128, N = keys of the tile (<= 256), K = hd -> FP32 in tensor memory columns [0, 256)
 //   P    : every thread owns one query row of one half of the 32-column chunks (tcgen05.ld 32x32b): row maximum, exp2,
 //          row sum in FP32; P is rounded to BF16 and written over Q in the same swizzled K-major layout
+//          (at most 64 queries: the rows are loaded twice, into rows 0 .. 63 and 64 .. 127, so that all eight warps can reach
+//          them in tensor memory; a thread then owns a quarter of the columns, of the scores and of the output)
 //   O    : tcgen05.mma, A = P (K-major), B = V as it lies in memory (hd contiguous: the "MN-major" operand form, one
 //          128-byte row per key) -> FP32 in tensor memory columns [256, 256 + hd)
 //   out  : O / l as BF16 rows, or with KV splits the un-normalised BF16 rows plus (m, l) for the merge
@@ -53,16 +55,23 @@ __device__ __forceinline__ bool cta_wait_phase(const VmProgram& prog, Ctl* ctl, 
 // HDP: elements per head in memory and in the MMAs (128 or 256); a.head_dim: logical width that is stored.
 // `uses` counts the tensor-core attention tiles this CTA has run (phase parity of the four barriers).
 // MASK: the operator's boolean visibility mask is consulted (instantiated for the full kernel variant only).
-template <int HDP, bool MASK = false>
+// TWICE: KV splits of at most 64 queries, loaded twice (see above): the chain of a thread - scores, exponentials, output
+// columns - is what such a tile takes (51 queries, 13 splits of 63 keys inside the model: 11.8 -> 10.8 us).
+// LEAN: of the lean kernel variant, whose 128-element heads are never split.
+// Scores are read from tensor memory again for the exponentials rather than kept in registers: values loaded by tcgen05.ld that
+// live across a barrier or a branch make the compiler spill, and slowed every operator of the kernel by 10 to 20 %.
+template <int HDP, bool LEAN, bool MASK, bool TWICE>
 // deps: when not null, the stage whose sources this call waits for itself (tile range dep_first, dep_count) - after its
 // index arithmetic and just before the first copies, so that the arithmetic is off the dependent path.
 __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& a, int tile, uint8_t* data, uint32_t tmem,
                              uint32_t uses, int stage, long long* stamp, const StageDesc* deps, int dep_first, int dep_count) {
     constexpr int CHUNKS = HDP / 64;
+    constexpr int PARTS = TWICE ? 4 : 2, W = TWICE ? 16 : 32;           // threads per row; score columns a thread takes at a time
     uint8_t* sQ = data;                                  // Q, then P
     uint8_t* sKV = data + kTcQBytes;                     // K, then V
-    float* xm = reinterpret_cast<float*>(data + kTcScratch);           // [2][128] row maxima of the two column halves
-    float* xl = xm + 256;                                               // [2][128] row sums
+    constexpr int ROWS = 256 / PARTS;
+    float* xm = reinterpret_cast<float*>(data + kTcScratch);           // [PARTS][ROWS] row maxima of the column parts
+    float* xl = xm + 256;                                               // [PARTS][ROWS] row sums
 
     const int warp = threadIdx.x >> 5, lane = lane_id();
     const int split = tile % a.splits;
@@ -89,12 +98,13 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
     // ---- Q and K
     if (threadIdx.x == 0) {
         const uint32_t q_bytes = static_cast<uint32_t>(a.q_box) * 128u, k_bytes = static_cast<uint32_t>(a.k_box) * 128u;
-        mbar_expect_tx(bar_qk, CHUNKS * (q_bytes + k_bytes));
+        mbar_expect_tx(bar_qk, CHUNKS * ((TWICE ? 2u : 1u) * q_bytes + k_bytes));
         const int q_row = batch * a.q_batch_rows + q0, k_row = batch * a.kv_batch_rows + k_begin;
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
             tma_load_2d(sQ + c * 16384, a.tmap_q, bar_qk, head * HDP + c * 64, q_row);
             tma_load_2d(sKV + c * k_bytes, a.tmap_k, bar_qk, kvh * HDP + c * 64, k_row);
+            if (TWICE) tma_load_2d(sQ + c * 16384 + 8192, a.tmap_q, bar_qk, head * HDP + c * 64, q_row);
         }
     }
     // ---- S = Q K^T  (only the issuing warp waits for Q and K: nobody else touches them; if its wait gives up, the abort
@@ -128,63 +138,81 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
         for (int c = 0; c < CHUNKS; ++c) tma_load_2d(sKV + c * k_bytes, a.tmap_v, bar_v, kvh * HDP + c * 64, k_row);
     }
 
-    // ---- softmax: thread = query row, the two warp groups take alternate 32-column chunks
-    const int wg = warp >> 2, quarter = warp & 3;
-    const int row = quarter * 32 + lane;                                // query row inside the tile = tensor-memory lane
+    // ---- softmax: thread = query row, the parts take alternate chunks of W columns
+    const int quarter = warp & 3;
+    const int part = TWICE ? (warp >> 2) * 2 + (quarter >> 1) : warp >> 2;
+    const int row = (TWICE ? quarter & 1 : quarter) * 32 + lane;        // query row inside the tile
+    const int warp_rows = q_valid - (row - lane);                       // query rows of this warp (none: nothing to compute)
     const int qrow = q0 + row;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const float sl2 = a.scale * 1.4426950408889634f;
-    const int chunks32 = (n_s + 31) >> 5;
+    const int chunks = (n_s + W - 1) / W;
     const int visible_end = (a.prefix >= 0 && qrow == 0) ? min(keys, a.prefix + 1 - k_begin) : keys;   // keys [0, visible_end) of this tile
-    // bit i of the result: key j * 32 + i of this tile is visible to this thread's query row under the boolean mask
-    auto mask_bits = [&](int j) -> uint32_t {
-        if constexpr (!MASK) return 0xffffffffu;
-        if (qrow >= a.nq) return 0u;
-        const uint8_t* m = a.mask + (static_cast<size_t>(batch) * a.nq + qrow) * a.nk + k_begin + j * 32;
-        uint32_t bits = 0u;
+    uint32_t raw[W];
+    // scores of chunk j, hidden keys at -infinity
+    auto load_scores = [&](int j) {
+        if constexpr (TWICE) tmem_ld16(tmem + lane_addr + j * W, raw);
+        else tmem_ld32(tmem + lane_addr + j * W, raw);
+        uint32_t vis = 0xffffffffu;
+        if constexpr (MASK) {
+            // bit i: key j * W + i of this tile is visible to this thread's query row under the boolean mask
+            vis = 0u;
+            if (qrow < a.nq) {
+                const uint8_t* m = a.mask + (static_cast<size_t>(batch) * a.nq + qrow) * a.nk + k_begin + j * W;
 #pragma unroll 8
-        for (int i = 0; i < 32; i++)
-            if (j * 32 + i < keys && __ldg(m + i)) bits |= 1u << i;
-        return bits;
+                for (int i = 0; i < W; i++)
+                    if (j * W + i < keys && __ldg(m + i)) vis |= 1u << i;
+            }
+        }
+        tmem_ld_wait();
+        const int open = visible_end - j * W;
+        if (MASK || __any_sync(0xffffffffu, open < W)) {
+#pragma unroll
+            for (int i = 0; i < W; i++)
+                if (i >= open || !((vis >> i) & 1u)) raw[i] = 0xff800000u;
+        }
     };
     float m_part = -INFINITY;
-    for (int j = wg; j < chunks32; j += 2) {
-        uint32_t raw[32];
-        tmem_ld32(tmem + lane_addr + j * 32, raw);
-        const uint32_t vis = mask_bits(j);
-        tmem_ld_wait();
+    if (warp_rows > 0) {
+        for (int j = part; j < chunks; j += PARTS) {
+            load_scores(j);
+            float m4[4] = {m_part, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int i = 0; i < 32; i++)
-            if (j * 32 + i < visible_end && ((vis >> i) & 1u)) m_part = fmaxf(m_part, __uint_as_float(raw[i]));
+            for (int i = 0; i < W; i += 8)
+#pragma unroll
+                for (int e = 0; e < 4; e++) m4[e] = max3(m4[e], __uint_as_float(raw[i + 2 * e]), __uint_as_float(raw[i + 2 * e + 1]));
+            m_part = fmaxf(max3(m4[0], m4[1], m4[2]), m4[3]);
+        }
     }
-    xm[wg * 128 + row] = m_part;
+    xm[part * ROWS + row] = m_part;
     __syncthreads();
-    const float m_raw = fmaxf(xm[row], xm[128 + row]);
+    float m_raw = fmaxf(xm[row], xm[ROWS + row]);
+    if (TWICE) m_raw = max3(m_raw, xm[2 * ROWS + row], xm[3 * ROWS + row]);
     const float m_use = m_raw == -INFINITY ? 0.f : m_raw * sl2;
-    float l_part = 0.f;
-    for (int j = wg; j < chunks32; j += 2) {
-        uint32_t raw[32];
-        tmem_ld32(tmem + lane_addr + j * 32, raw);
-        const uint32_t vis = mask_bits(j);
-        tmem_ld_wait();
-        uint32_t packed[16];
+    float2 l_part = make_float2(0.f, 0.f);
+    if (warp_rows > 0) {
+        for (int j = part; j < chunks; j += PARTS) {
+            load_scores(j);
+            uint32_t packed[W / 2];
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int k0 = j * 32 + 2 * i;
-            const float p0 = k0 < visible_end && ((vis >> (2 * i)) & 1u) ? exp2f(__uint_as_float(raw[2 * i]) * sl2 - m_use) : 0.f;
-            const float p1 = k0 + 1 < visible_end && ((vis >> (2 * i + 1)) & 1u) ? exp2f(__uint_as_float(raw[2 * i + 1]) * sl2 - m_use) : 0.f;
-            l_part += p0 + p1;
-            packed[i] = pack2_bf16(p0, p1);
-        }
-        // P chunk of 64 keys = 128 rows x 128 bytes, 16-byte units swizzled with the row (what the K-major descriptor expects)
-        uint8_t* prow = sQ + (j >> 1) * 16384 + row * 128;
+            for (int i = 0; i < W / 2; i++) {
+                const float2 x = fma2(make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1])), make_float2(sl2, sl2), make_float2(-m_use, -m_use));
+                const float2 e = make_float2(exp2_fast(x.x), exp2_fast(x.y));
+                l_part = add2(l_part, e);
+                packed[i] = pack2_bf16(e.x, e.y);
+            }
+            // P chunk of 64 keys = 128 rows x 128 bytes, 16-byte units swizzled with the row (what the K-major descriptor expects)
+            uint8_t* prow = sQ + j * W / 64 * 16384 + row * 128;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int unit = ((j & 1) * 4 + u) ^ (row & 7);
-            *reinterpret_cast<uint4*>(prow + unit * 16) = make_uint4(packed[4 * u], packed[4 * u + 1], packed[4 * u + 2], packed[4 * u + 3]);
+            for (int u = 0; u < W / 8; u++) {
+                const int unit = (j * (W / 8) % 8 + u) ^ (row & 7);
+                const uint4 p4 = make_uint4(packed[4 * u], packed[4 * u + 1], packed[4 * u + 2], packed[4 * u + 3]);
+                *reinterpret_cast<uint4*>(prow + unit * 16) = p4;
+                if (TWICE) *reinterpret_cast<uint4*>(prow + 8192 + unit * 16) = p4;
+            }
         }
     }
-    xl[wg * 128 + row] = l_part;
+    xl[part * ROWS + row] = l_part.x + l_part.y;
     tc_fence_before();
     fence_proxy_async_smem();                            // P (generic stores) must be visible to the tensor core's reads
     __syncthreads();
@@ -212,39 +240,41 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
     tc_fence_after();
     if (stamp && threadIdx.x == 0) stamp[6] = static_cast<long long>(global_ns());
 
-    // ---- output: thread = row, warp group = half of the head's columns
-    const float l_sum = xl[row] + xl[128 + row];
+    // ---- output: thread = row, part = share of the head's columns
+    float l_sum = xl[row] + xl[ROWS + row];
+    if (TWICE) l_sum += xl[2 * ROWS + row] + xl[3 * ROWS + row];
     const bool row_ok = row < q_valid;
-    constexpr int HALF = HDP / 2;
-    const int col_begin = wg * HALF;
-    if (a.splits > 1) {
-        __nv_bfloat16* po = reinterpret_cast<__nv_bfloat16*>(a.partial_o) + (static_cast<size_t>(tile) * kAttnQRows + row) * a.head_dim;
-        for (int c0 = col_begin; c0 < col_begin + HALF; c0 += 32) {
-            uint32_t raw[32];
-            tmem_ld32(tmem + 256u + lane_addr + c0, raw);
-            tmem_ld_wait();
-            if (row_ok) {
+    constexpr int SHARE = HDP / PARTS;
+    const int col_begin = part * SHARE;
+    if (TWICE || (!(LEAN && HDP == 128) && a.splits > 1)) {
+        const size_t ld = static_cast<size_t>(a.head_dim) * 2;
+        uint8_t* po = reinterpret_cast<uint8_t*>(a.partial_o) + (static_cast<size_t>(tile) * kAttnQRows + (row - lane)) * ld;
+        if (warp_rows > 0) {
+            for (int c0 = col_begin; c0 < col_begin + SHARE; c0 += 32) {
+                uint32_t raw[32];
+                tmem_ld32(tmem + 256u + lane_addr + c0, raw);
+                tmem_ld_wait();
+                uint4 p[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (c0 + 8 * u < a.head_dim)
-                        *reinterpret_cast<uint4*>(po + c0 + 8 * u) =
-                            make_uint4(pack2_bf16(__uint_as_float(raw[8 * u]), __uint_as_float(raw[8 * u + 1])),
-                                       pack2_bf16(__uint_as_float(raw[8 * u + 2]), __uint_as_float(raw[8 * u + 3])),
-                                       pack2_bf16(__uint_as_float(raw[8 * u + 4]), __uint_as_float(raw[8 * u + 5])),
-                                       pack2_bf16(__uint_as_float(raw[8 * u + 6]), __uint_as_float(raw[8 * u + 7])));
-                }
+                for (int u = 0; u < 4; u++)
+                    p[u] = make_uint4(pack2_bf16(__uint_as_float(raw[8 * u]), __uint_as_float(raw[8 * u + 1])),
+                                      pack2_bf16(__uint_as_float(raw[8 * u + 2]), __uint_as_float(raw[8 * u + 3])),
+                                      pack2_bf16(__uint_as_float(raw[8 * u + 4]), __uint_as_float(raw[8 * u + 5])),
+                                      pack2_bf16(__uint_as_float(raw[8 * u + 6]), __uint_as_float(raw[8 * u + 7])));
+                // (columns beyond head_dim - padded heads - are not stored: that lane's piece counts as no rows)
+                store_rows64(po + c0 * 2, ld, c0 + 8 * (lane & 3) < a.head_dim ? warp_rows : 0, p);
             }
         }
-        if (wg == 0 && row_ok) {
+        if (part == 0 && row_ok) {
             float* pml = a.partial_ml + (static_cast<size_t>(tile) * kAttnQRows + row) * 2;
             pml[0] = m_raw == -INFINITY ? -INFINITY : m_use;
             pml[1] = l_sum;
         }
-    } else {
+    } else if constexpr (!TWICE) {
         const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
         const size_t grow = static_cast<size_t>(batch) * a.q_batch_rows + q0 + row;
         __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + grow * a.ldo + head * a.head_dim;
-        for (int c0 = col_begin; c0 < col_begin + HALF; c0 += 32) {
+        for (int c0 = col_begin; c0 < col_begin + SHARE; c0 += 32) {
             uint32_t raw[32];
             tmem_ld32(tmem + 256u + lane_addr + c0, raw);
             tmem_ld_wait();

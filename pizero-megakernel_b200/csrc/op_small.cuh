@@ -7,26 +7,64 @@
 
 namespace pi0 {
 
-constexpr int kPatchTokens = 16;      // tokens per tile
-constexpr int kPatchCols = 256;       // output columns per tile (one per thread)
-constexpr int kPatchK = 14 * 14 * 3;  // 588
+// Patch embedding: out[t, n] = sum_k patch[t, k] * W[k, n] + bias[n] + pos[t % 256, n];  k = (dy*14 + dx)*3 + c, images are NHWC.
+//
+// 1 GFLOP in FP32 for three views, and the first stage of the model: nothing else runs beside it.  A tile is 16 tokens (8 when
+// there is only one view, for twice the CTAs) by 384 columns, which gives 144 tiles for the three views of pi0 - one wave.
+// A warp serves 32 columns, 32 + 128 and 32 + 256 for one half of the tokens, so a k costs two broadcast reads of patch
+// values (stored [k][token]), three of weights and twelve packed multiply-adds; the weights come through a six-deep
+// cp.async ring of 14 k each.  (One column per thread with the weights read straight from L2 was bound by the latency of
+// those reads: 157 us for three views, 103 for one.)
+constexpr int kPatchCols = 384;
+constexpr int kPatchK = 14 * 14 * 3;                                   // 588
+constexpr int kPatchStageK = 14;
+constexpr int kPatchStages = 6;
+constexpr int kPatchStageBytes = kPatchStageK * kPatchCols * 4;
+constexpr int kPatchLd = 20;                                           // floats per k of patch values (16 tokens, padded)
+static_assert(kPatchK % kPatchStageK == 0 && kPatchK * kPatchLd * 4 + kPatchStages * kPatchStageBytes <= kDataBytes, "patch tile exceeds the data region");
 
-// out[t, n] = sum_k patch[t, k] * W[k, n] + bias[n] + pos[t % 256, n];  k = (dy*14 + dx)*3 + c, images are NHWC.
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid) {
+    const int bytes = valid ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void patch_issue(const PatchParams& p, float* stage, int k0, int n0) {
+    const float* w = p.weight + static_cast<size_t>(k0) * p.width + n0;
+    if ((p.width & 3) == 0 && (reinterpret_cast<uintptr_t>(p.weight) & 15u) == 0) {
+        for (int i = threadIdx.x; i < kPatchStageK * (kPatchCols / 4); i += kThreads) {
+            const int r = i / (kPatchCols / 4), c = (i - r * (kPatchCols / 4)) * 4;
+            const bool ok = n0 + c < p.width;
+            cp_async16(stage + r * kPatchCols + c, ok ? w + static_cast<size_t>(r) * p.width + c : p.weight, ok);
+        }
+    } else {
+        for (int i = threadIdx.x; i < kPatchStageK * kPatchCols; i += kThreads) {
+            const int r = i / kPatchCols, c = i - r * kPatchCols;
+            const bool ok = n0 + c < p.width;
+            cp_async4(stage + i, ok ? w + static_cast<size_t>(r) * p.width + c : p.weight, ok);
+        }
+    }
+}
+template <int TOKENS>
 __device__ __forceinline__ void patch_tile(const PatchParams& p, const float* images, int tile, uint8_t* data) {
-    float* sp = reinterpret_cast<float*>(data);                    // [16][588]
+    constexpr int kHalf = TOKENS / 2, kPairs = TOKENS / 4;             // tokens / token pairs of one thread
+    float* sp = reinterpret_cast<float*>(data);                        // [588][kPatchLd]
+    float* ring = sp + kPatchK * kPatchLd;                             // [stages][14][384]
     const int ntiles = (p.width + kPatchCols - 1) / kPatchCols;
-    const int tt = tile / ntiles, nt = tile - tt * ntiles;
-    // gather the 16 patches: loads are issued in batches of 8 per thread before any is stored
-    for (int base = 0; base < kPatchTokens * kPatchK; base += kThreads * 8) {
+    const int tt = tile / ntiles, n0 = (tile - tt * ntiles) * kPatchCols;
+    for (int s = 0; s < kPatchStages - 1; ++s) {
+        patch_issue(p, ring + s * (kPatchStageBytes / 4), s * kPatchStageK, n0);
+        cp_async_commit();
+    }
+    // gather the patches: loads are issued in batches of 8 per thread before any is stored
+    for (int base = 0; base < TOKENS * kPatchK; base += kThreads * 8) {
         float v[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const int i = base + j * kThreads + threadIdx.x;
             v[j] = 0.f;
-            if (i < kPatchTokens * kPatchK) {
+            if (i < TOKENS * kPatchK) {
                 const int tok = i / kPatchK, k = i - tok * kPatchK;
                 const int dy = k / 42, rem = k - dy * 42;
-                const int t = tt * kPatchTokens + tok;
+                const int t = tt * TOKENS + tok;
                 const int view = t >> 8, pidx = t & 255, py = pidx >> 4, px = pidx & 15;
                 v[j] = __ldg(images + ((static_cast<size_t>(view) * 224 + py * 14 + dy) * 224 + px * 14) * 3 + rem);
             }
@@ -34,31 +72,61 @@ __device__ __forceinline__ void patch_tile(const PatchParams& p, const float* im
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const int i = base + j * kThreads + threadIdx.x;
-            if (i < kPatchTokens * kPatchK) sp[i] = v[j];
-        }
-    }
-    __syncthreads();
-    const int n = nt * kPatchCols + threadIdx.x;
-    if (n < p.width) {
-        float acc[kPatchTokens];
-#pragma unroll
-        for (int i = 0; i < kPatchTokens; i++) acc[i] = 0.f;
-        for (int k0 = 0; k0 < kPatchK; k0 += 4) {           // 588 = 4 * 147: four weight loads in flight
-            float w[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) w[j] = __ldg(p.weight + static_cast<size_t>(k0 + j) * p.width + n);
-#pragma unroll
-            for (int i = 0; i < kPatchTokens; i++) {
-                const float4 x = *reinterpret_cast<const float4*>(sp + i * kPatchK + k0);
-                acc[i] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], acc[i]))));
+            if (i < TOKENS * kPatchK) {
+                const int tok = i / kPatchK;
+                sp[(i - tok * kPatchK) * kPatchLd + tok] = v[j];
             }
         }
-        const float b = p.bias[n];
+    }
+    const int half = threadIdx.x >> 7, col = threadIdx.x & 127;
+    float2 acc[3][kPairs];
 #pragma unroll
-        for (int i = 0; i < kPatchTokens; i++) {
-            const int t = tt * kPatchTokens + i;
-            const float y = acc[i] + b + p.pos[static_cast<size_t>(t & 255) * p.width + n];
-            static_cast<__nv_bfloat16*>(p.out)[static_cast<size_t>(t) * p.width + n] = __float2bfloat16_rn(y);
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int i = 0; i < kPairs; i++) acc[j][i] = make_float2(0.f, 0.f);
+    constexpr int kSteps = kPatchK / kPatchStageK;
+    for (int s = 0; s < kSteps; ++s) {
+        cp_async_wait<kPatchStages - 2>();
+        __syncthreads();                                               // the stage (and, first, the patches) of every thread; stage s - 1 is free
+        const int next = s + kPatchStages - 1;
+        if (next < kSteps) patch_issue(p, ring + (next % kPatchStages) * (kPatchStageBytes / 4), next * kPatchStageK, n0);
+        cp_async_commit();
+        const float* w = ring + (s % kPatchStages) * (kPatchStageBytes / 4) + col;
+        const float* x = sp + s * kPatchStageK * kPatchLd + half * kHalf;
+#pragma unroll 2
+        for (int k = 0; k < kPatchStageK; ++k) {
+            float2 xp[kPairs];
+#pragma unroll
+            for (int i = 0; i < kPairs; i += 2) {
+                const float4 q = *reinterpret_cast<const float4*>(x + k * kPatchLd + 2 * i);
+                xp[i] = make_float2(q.x, q.y);
+                xp[i + 1] = make_float2(q.z, q.w);
+            }
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const float wk = w[k * kPatchCols + 128 * j];
+#pragma unroll
+                for (int i = 0; i < kPairs; i++) acc[j][i] = fma2(xp[i], make_float2(wk, wk), acc[j][i]);
+            }
+        }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const int n = n0 + col + 128 * j;
+        if (n < p.width) {
+            // (the position rows are read before the first store: the compiler cannot know that they do not overlap the output,
+            // and a load behind every store would be a chain of round trips)
+            const int t0 = tt * TOKENS + half * kHalf;
+            const float b = __ldg(p.bias + n);
+            float pos[kHalf];
+#pragma unroll
+            for (int i = 0; i < kHalf; i++) pos[i] = __ldg(p.pos + static_cast<size_t>((t0 + i) & 255) * p.width + n);
+#pragma unroll
+            for (int i = 0; i < kHalf; i++) {
+                const float y = (i & 1 ? acc[j][i >> 1].y : acc[j][i >> 1].x) + b + pos[i];
+                static_cast<__nv_bfloat16*>(p.out)[static_cast<size_t>(t0 + i) * p.width + n] = __float2bfloat16_rn(y);
+            }
         }
     }
 }
@@ -68,8 +136,9 @@ __device__ __forceinline__ void patch_instruction(const VmProgram& prog, Ctl* ct
     const PatchParams& p = st.p.patch;
     const float* images = p.images ? p.images : prog.in.images;
     for (int t = first; t < first + count; ++t) {
-        patch_tile(p, images, t, data);
-        cta_publish_tile(prog, st, t);
+        if (p.tokens == 16) patch_tile<16>(p, images, t, data);
+        else patch_tile<8>(p, images, t, data);
+        cta_publish_tile(prog, st, t);                                 // (its barrier also frees the buffers for the next tile)
     }
 }
 
@@ -86,7 +155,31 @@ __device__ __forceinline__ void embed_instruction(const VmProgram& prog, Ctl* ct
             tok = tok < 0 ? 0 : (tok >= e.vocab ? e.vocab - 1 : tok);
             const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(e.table) + static_cast<size_t>(tok) * e.width;
             __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(e.out) + static_cast<size_t>(e.row_base + i) * e.width;
-            for (int c = lane; c < e.width; c += 32) dst[c] = __float2bfloat16_rn(__bfloat162float(src[c]) * e.scale);
+            if (e.width % 8 == 0 && ((reinterpret_cast<uintptr_t>(e.table) | reinterpret_cast<uintptr_t>(e.out)) & 15u) == 0) {
+                // 16 bytes per lane and load, eight loads in flight (element by element the row was a chain of 64 round trips:
+                // 32 us for a prompt)
+                const int pieces = e.width >> 3;
+                for (int c0 = lane; c0 < pieces; c0 += 256) {
+                    uint4 u[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (c0 + 32 * j < pieces) u[j] = __ldg(reinterpret_cast<const uint4*>(src) + c0 + 32 * j);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        if (c0 + 32 * j >= pieces) break;
+                        const uint32_t in[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+                        uint32_t w[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&in[q]));
+                            w[q] = pack2_bf16(f.x * e.scale, f.y * e.scale);
+                        }
+                        reinterpret_cast<uint4*>(dst)[c0 + 32 * j] = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                }
+            } else {
+                for (int c = lane; c < e.width; c += 32) dst[c] = __float2bfloat16_rn(__bfloat162float(src[c]) * e.scale);
+            }
         }
         cta_publish_tile(prog, st, t);
     }

@@ -141,6 +141,7 @@ struct Program {
     long long* d_timings = nullptr;
     bool timings_on = false;
     bool lean = false;                 // every stage is one the lean kernel variant runs
+    bool mma_sync = false;             // some attention stage runs on the mma.sync tiles
     bool solo = false;                 // the program of one operator
     int grid = 0;                      // CTAs launched: up to the last worker that has an instruction
     unsigned int epoch = 0;
@@ -202,7 +203,7 @@ bool lean_stage(const StageDesc& d) {
         return g.operands == GEMM_NVFP4 && (g.epilogue == EPI_BF16 || g.epilogue == EPI_STREAM || g.epilogue == EPI_GEGLU_FP4 ||
                                             g.epilogue == EPI_FP4 || g.epilogue == EPI_QKV_ROPE || g.epilogue == EPI_BF16_EXT);
     }
-    if (d.kind == OP_ATTN) return d.p.attn.tc != 0 && !d.p.attn.mask;
+    if (d.kind == OP_ATTN) return d.p.attn.tc != 0 && !d.p.attn.mask && !(d.p.attn.hd_pad == 128 && d.p.attn.splits > 1);
     if (d.kind == OP_NORM) {                                 // the lean norm writes NVFP4 only: no fused residual, inverse scale, other outputs
         const NormParams& n = d.p.norm;
         return n.out && !n.residual && !n.inv_scale && !n.out_fp8 && !n.out_bf16 && !n.out_factor;
@@ -293,12 +294,16 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
         static bool configured[64] = {};
         if (device < 64 && !configured[device]) {
             e = cudaFuncSetAttribute(pi0_vm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             configured[device] = e == cudaSuccess;
         }
         prog->lean = true;
-        for (const auto& d : prog->stages) prog->lean = prog->lean && lean_stage(d);
+        for (const auto& d : prog->stages) {
+            prog->lean = prog->lean && lean_stage(d);
+            prog->mma_sync = prog->mma_sync || (d.kind == OP_ATTN && !d.p.attn.tc);
+        }
     }
     if (e != cudaSuccess) return e;
     *out = prog.release();
@@ -355,7 +360,8 @@ int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begi
     config.numAttrs = 1;
     if (prog->lean && !prog->h_debug && !p.timings) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false>, p);
     if (prog->lean && !prog->h_debug) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true>, p);
-    return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true>, p);
+    if (!prog->mma_sync) return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true, false>, p);
+    return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true, true>, p);
 }
 
 Op* as_op(void* h) {
@@ -1251,11 +1257,12 @@ extern "C" int create_patch_embed(void** handle, const float* images, const floa
     d.kind = OP_PATCH;
     finish_desc(d);
     const int ntiles = (width + kPatchCols - 1) / kPatchCols;
-    d.tiles = views * 256 / kPatchTokens * ntiles;
+    const int tokens = views == 1 ? 8 : 16;
+    d.tiles = views * 256 / tokens * ntiles;
     d.bands = views * 256 / kBandRows;
-    d.band_div = kBandRows / kPatchTokens * ntiles;
+    d.band_div = kBandRows / tokens * ntiles;
     op->cost = 576;
-    d.p.patch = PatchParams{images, weight, bias, pos, out, views, width};
+    d.p.patch = PatchParams{images, weight, bias, pos, out, views, width, tokens};
     *handle = op;
     return cudaSuccess;
 }

@@ -169,7 +169,45 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// 4 x 4 transpose of 16-byte pieces inside every group of four lanes (its own inverse): lane j's piece k <-> lane k's piece j.
+// A drain holds one row per lane; 64 bytes per lane stored row by row touch 32 lines per instruction, and the load / store
+// unit takes one line a cycle (128 x 128 BF16 tiles: 1 us of 3.1 per tile).  Transposed, four lanes cover one row's 64
+// bytes and an instruction eight rows.
+__device__ __forceinline__ void quad_transpose(uint4 (&p)[4]) {
+#pragma unroll
+    for (int bit = 1; bit <= 2; bit <<= 1) {
+        const bool upper = (lane_id() & bit) != 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (i & bit) continue;
+            uint4 &lo = p[i], &hi = p[i + bit];
+            const uint4 send = upper ? lo : hi;
+            const uint4 got = make_uint4(__shfl_xor_sync(0xffffffffu, send.x, bit), __shfl_xor_sync(0xffffffffu, send.y, bit),
+                                         __shfl_xor_sync(0xffffffffu, send.z, bit), __shfl_xor_sync(0xffffffffu, send.w, bit));
+            if (upper) lo = got;
+            else hi = got;
+        }
+    }
+}
+// Whole warp: lane r holds 64 bytes of row r (r < rows) -> rows at `base` + r * ld bytes.
+__device__ __forceinline__ void store_rows64(uint8_t* base, size_t ld, int rows, uint4 (&p)[4]) {
+    quad_transpose(p);
+    const int lane = lane_id(), row0 = lane & ~3;
+    uint8_t* dst = base + static_cast<size_t>(row0) * ld + (lane & 3) * 16;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (row0 + k < rows) *reinterpret_cast<uint4*>(dst + k * ld) = p[k];
+}
 
 // ---------------------------------------------------------------- counters
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
@@ -212,6 +250,17 @@ __device__ __forceinline__ float max3_abs(float a, float b, float c) {
     float d;
     asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// 2^x; results below the normal range become zero
+__device__ __forceinline__ float exp2_fast(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 // Eight FP32 -> four bytes of E2M1 codes (RNE, saturating), the first value in the lowest nibble.
 __device__ __forceinline__ uint32_t cvt_e2m1x8(float2 a, float2 b, float2 c, float2 d) {

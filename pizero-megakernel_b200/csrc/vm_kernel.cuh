@@ -49,7 +49,9 @@ __device__ __forceinline__ bool prefetch_slot(const VmProgram& prog, Ctl* ctl, c
 // lean); LEAN = false runs every operator and option.  Same VM, same protocol; the lean one is simply a smaller kernel.
 // TIMED = false: without the per-instruction time stamps (the lean variant is built both ways, so that a stage profile
 // times the kernel that serves, and serving does not carry the stamp tests: 0.5 % of the pi0 forward).
-template <bool LEAN, bool TIMED = true>
+// MMA_SYNC = false: without the mma.sync attention tiles.  Their 128 accumulators per thread make the compiler spill, and a kernel
+// that spills anywhere was 4 % slower everywhere (BF16 forward 17.7 -> 17.0 ms), so only programs with such tiles carry them.
+template <bool LEAN, bool TIMED = true, bool MMA_SYNC = !LEAN>
 __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_constant__ VmProgram prog) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
             if (st.kind != OP_ATTN && !cta_wait_sources(prog, ctl, st, ins.y, ins.z, ins.w, stamp)) break;
             switch (st.kind) {
                 case OP_NORM: norm_instruction<LEAN>(prog, ctl, data, st, ins.y, ins.z, ins.w); break;
-                case OP_ATTN: attn_instruction<LEAN>(prog, ctl, data, tmem, tc_tiles, st, ins.y, ins.z, ins.w, stamp); break;
+                case OP_ATTN: attn_instruction<LEAN, MMA_SYNC>(prog, ctl, data, tmem, tc_tiles, st, ins.y, ins.z, ins.w, stamp); break;
                 case OP_MERGE: merge_instruction(prog, ctl, st, ins.y, ins.z, ins.w); break;
                 case OP_PATCH: patch_instruction(prog, ctl, data, st, ins.y, ins.z, ins.w); break;
                 case OP_EMBED: embed_instruction(prog, ctl, st, ins.y, ins.z, ins.w); break;

@@ -189,6 +189,7 @@ struct PatchParams {
     const float* pos;            // FP32 [256, width]
     void* out;                   // BF16 [views*256, width]
     int views, width;
+    int tokens;                  // tokens per tile: 16, or 8 with a single view
 };
 
 struct EmbedParams {

@@ -695,6 +695,44 @@ def test_attention_tensor_core_fp4_output(b, nq, nk, h, hd, stored, pitch):
             ResidentAttention(None, q, k, v, head_dim=hd, fp4_output=(data, scales, 0.5), fp4_pitch=72)
 
 
+@pytest.mark.parametrize("views,width", [(1, 1152), (3, 1152), (1, 8), (2, 387), (1, 772)])
+def test_patch_embedding_tiles(views, width):
+    """16- and 8-token tiles, column tiles that end inside a tile, widths that 16-byte copies cannot move.  FP32 sums of 588
+    products in another order than the convolution's differ by about 588 ** 0.5 * 2 ** -24 of their size, BF16 rounding by 2 ** -9."""
+    lib = _native.load()
+    g = torch.Generator(device="cuda").manual_seed(views * 10000 + width)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    images, conv_w = rand(views, 224, 224, 3), rand(width, 3, 14, 14) * 0.05
+    bias, pos = rand(width), rand(256, width)
+    w = conv_w.permute(2, 3, 1, 0).reshape(588, width).contiguous()
+    out = torch.zeros(views * 256, width, dtype=torch.bfloat16, device="cuda")
+    h = C.c_void_p()
+    _native.check(lib.create_patch_embed(C.byref(h), images.data_ptr(), w.data_ptr(), bias.data_ptr(), pos.data_ptr(), out.data_ptr(), views, width, 148), "patch")
+    _native.check(lib.launch_op(h, None), "launch")
+    torch.cuda.synchronize()
+    assert _native.status(lib, h)["code"] == 0
+    lib.destroy_op(h)
+    want = torch.nn.functional.conv2d(images.double().permute(0, 3, 1, 2), conv_w.double(), bias.double(), stride=14).flatten(2).transpose(1, 2) + pos.double()[None]
+    torch.testing.assert_close(out.double(), want.reshape(-1, width), rtol=2.0 ** -8, atol=1e-4)
+
+
+@pytest.mark.parametrize("count,width,offset", [(1, 8, 0), (9, 2048, 0), (3, 20, 0), (5, 72, 1)])
+def test_token_embedding_rows(count, width, offset):
+    """Rows in 16-byte pieces, widths and (offset) table addresses that 16-byte loads cannot read, tokens beyond the vocabulary."""
+    lib = _native.load()
+    g = torch.Generator(device="cuda").manual_seed(count + width)
+    table = torch.randn(11 * width + offset, generator=g, device="cuda").bfloat16()[offset:]
+    tokens = torch.randint(-2, 14, (count,), generator=g, device="cuda")
+    out = torch.zeros(count + 1, width, dtype=torch.bfloat16, device="cuda")
+    h = C.c_void_p()
+    _native.check(lib.create_token_embed(C.byref(h), tokens.data_ptr(), table.data_ptr(), out.data_ptr(), count, width, 1, 11, 3.7, 4), "embed")
+    _native.check(lib.launch_op(h, None), "launch")
+    torch.cuda.synchronize()
+    lib.destroy_op(h)
+    want = (table.view(11, width)[tokens.clamp(0, 10)].float() * np.float32(3.7)).bfloat16()
+    assert torch.equal(out[1:], want) and not out[0].any()
+
+
 def test_small_operators():
     lib = _native.load()
     torch.manual_seed(11)
