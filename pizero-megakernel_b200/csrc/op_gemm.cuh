@@ -247,7 +247,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
     float2 v[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = mul2(make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1])), make_float2(row_scale, row_scale));
-    if (!row_ok) return;
+    constexpr bool kWarpStore = EPI == EPI_BF16 || EPI == EPI_BF16_EXT;      // (the warp stores its rows together)
+    if (!kWarpStore && !row_ok) return;
     if constexpr (EPI == EPI_BF16_EXT || EPI == EPI_FP4) {
         if (g.col_center) {
             // folded LayerNorm: subtract the row mean's share, mean * rstd * (sum over K of weight row n)
@@ -341,16 +342,21 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
                 v[i] = make_float2(col0 + 2 * i < g.gelu_cols ? gelu_tanh(bf16_round(v[i].x)) : 0.f,
                                    col0 + 2 * i + 1 < g.gelu_cols ? gelu_tanh(bf16_round(v[i].y)) : 0.f);
         }
-        __nv_bfloat16* base = static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo;
-        const bool padded = EPI == EPI_BF16_EXT && g.pad_from > 0;
-        // padded: heads written pad_to columns apart (8-column pieces never straddle a head: pad_from is a multiple of 8)
+        uint4 p[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int c = col0 + 8 * i;
-            if (padded) { const int head = c / g.pad_from; c += head * (g.pad_to - g.pad_from); }
-            *reinterpret_cast<uint4*>(base + c) = make_uint4(pack_bf16x2(v[4 * i].x, v[4 * i].y), pack_bf16x2(v[4 * i + 1].x, v[4 * i + 1].y),
-                                                             pack_bf16x2(v[4 * i + 2].x, v[4 * i + 2].y), pack_bf16x2(v[4 * i + 3].x, v[4 * i + 3].y));
-        }
+        for (int i = 0; i < 4; i++)
+            p[i] = make_uint4(pack_bf16x2(v[4 * i].x, v[4 * i].y), pack_bf16x2(v[4 * i + 1].x, v[4 * i + 1].y),
+                              pack_bf16x2(v[4 * i + 2].x, v[4 * i + 2].y), pack_bf16x2(v[4 * i + 3].x, v[4 * i + 3].y));
+        // padded: heads written pad_to columns apart (8-column pieces never straddle a head: pad_from is a multiple of 8); the
+        // lane's piece moves by the gaps in front of it.  Eight rows per store instruction: these drains write wide tiles, whose
+        // stores were a third of their time (768 x 32768 BF16 42.0 -> 38.2 us).  In the residual-stream and q|k|v drains the
+        // transpose costs more than it saves, because the model runs them for few rows, where the chain of a thread counts
+        // (o_proj 5.2 -> 6.1 us).
+        const int lane = lane_id();
+        int gap = 0;
+        if (EPI == EPI_BF16_EXT && g.pad_from > 0) gap = (col0 + (lane & 3) * 8) / g.pad_from * (g.pad_to - g.pad_from);
+        const size_t ld = static_cast<size_t>(g.ldo) * 2;
+        store_rows64(static_cast<uint8_t*>(g.out) + static_cast<size_t>(row - lane) * ld + (col0 + gap) * 2, ld, g.rows - (row - lane), p);
         return;
     }
     if constexpr (EPI == EPI_FP4) {

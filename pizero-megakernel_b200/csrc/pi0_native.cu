@@ -208,6 +208,10 @@ bool lean_stage(const StageDesc& d) {
         const NormParams& n = d.p.norm;
         return n.out && !n.residual && !n.inv_scale && !n.out_fp8 && !n.out_bf16 && !n.out_factor;
     }
+    if (d.kind == OP_LINEAR32) {                             // FP32 rows, or (16-row tiles) BF16 rows with the RMS factor
+        const Linear32Params& l = d.p.lin;
+        return (!l.x_bf16 && !l.rms) || (l.x_bf16 && l.rms && l.row_block == 16);
+    }
     return d.kind != OP_ATTN_PREP && d.kind != OP_SUFFIX && d.kind != OP_PROBE;
 }
 

@@ -156,15 +156,15 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
                     if (np.beta) prefetch_l1(np.beta + i * 32);
                 }
             }
-            // (an attention instruction waits for its sources itself, behind its index arithmetic)
-            if (st.kind != OP_ATTN && !cta_wait_sources(prog, ctl, st, ins.y, ins.z, ins.w, stamp)) break;
+            // (attention and FP32 linears wait for their sources themselves, behind what does not depend on them)
+            if (st.kind != OP_ATTN && st.kind != OP_LINEAR32 && !cta_wait_sources(prog, ctl, st, ins.y, ins.z, ins.w, stamp)) break;
             switch (st.kind) {
                 case OP_NORM: norm_instruction<LEAN>(prog, ctl, data, st, ins.y, ins.z, ins.w); break;
                 case OP_ATTN: attn_instruction<LEAN, MMA_SYNC>(prog, ctl, data, tmem, tc_tiles, st, ins.y, ins.z, ins.w, stamp); break;
                 case OP_MERGE: merge_instruction(prog, ctl, st, ins.y, ins.z, ins.w); break;
                 case OP_PATCH: patch_instruction(prog, ctl, data, st, ins.y, ins.z, ins.w); break;
                 case OP_EMBED: embed_instruction(prog, ctl, st, ins.y, ins.z, ins.w); break;
-                case OP_LINEAR32: linear32_instruction(prog, ctl, data, st, ins.y, ins.z, ins.w, stamp); break;
+                case OP_LINEAR32: linear32_instruction<LEAN>(prog, ctl, data, st, ins.y, ins.z, ins.w, stamp); break;
                 case OP_SUFFIX:
                     if constexpr (!LEAN) suffix_instruction(prog, ctl, st, ins.y, ins.z, ins.w);
                     break;
