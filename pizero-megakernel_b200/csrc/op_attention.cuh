@@ -350,34 +350,31 @@ __device__ void attn_tile(const AttnParams& a, int tile, uint8_t* data, long lon
 constexpr int kMergeRows = 16;
 
 // acc += w * (16 BF16 values of one partial row block)
-__device__ __forceinline__ void merge_accumulate(float (&acc)[16], float w, const uint4 (&x)[2]) {
+__device__ __forceinline__ void merge_accumulate(float2 (&acc)[8], float w, const uint4 (&x)[2]) {
     const uint32_t u[8] = {x[0].x, x[0].y, x[0].z, x[0].w, x[1].x, x[1].y, x[1].z, x[1].w};
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[e]));
-        acc[2 * e] += w * f.x;
-        acc[2 * e + 1] += w * f.y;
-    }
+    for (int e = 0; e < 8; e++) acc[e] = fma2(make_float2(w, w), __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[e])), acc[e]);
 }
 
 // Normalise one (row, 16-column block), round to BF16 and store it (BF16 and / or NVFP4 with its block scale).
-__device__ __forceinline__ void merge_store(const MergeParams& g, int head, int grow, int b, const float (&acc)[16], float denom) {
+__device__ __forceinline__ void merge_store(const MergeParams& g, int head, int grow, int b, const float2 (&acc)[8], float denom) {
     const float inv = denom > 0.f ? 1.f / denom : 0.f;
-    float v[16];
+    uint32_t w[8];                                       // rounded to BF16
 #pragma unroll
-    for (int e = 0; e < 16; e++) v[e] = bf16_round(acc[e] * inv);
+    for (int e = 0; e < 8; e++) {
+        const float2 r = mul2(acc[e], make_float2(inv, inv));
+        w[e] = pack2_bf16(r.x, r.y);
+    }
     const int col = head * g.head_dim + b * 16;
     if (g.out) {
-        uint32_t w[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) w[e] = pack2_bf16(v[2 * e], v[2 * e + 1]);
         uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(grow) * g.ldo + col);
         dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
         dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
     if (g.out_fp4) {
+        float2 v[8];
 #pragma unroll
-        for (int e = 0; e < 16; e++) v[e] *= g.out_inv_gs;
+        for (int e = 0; e < 8; e++) v[e] = mul2(__bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[e])), make_float2(g.out_inv_gs, g.out_inv_gs));
         uint32_t code;
         uint2 bytes = quantize_block16(v, 0, code);
         *reinterpret_cast<uint2*>(g.out_fp4 + static_cast<size_t>(grow) * g.ld_fp4 + (col >> 1)) = bytes;
@@ -392,9 +389,9 @@ __device__ __forceinline__ void merge_item(const MergeParams& g, int group, int 
         const int grow = (group / g.heads) * kAttnQRows + r;          // row in the output
         const float* ml = g.partial_ml + (static_cast<size_t>(group) * g.splits * kAttnQRows + r) * 2;
         const __nv_bfloat16* po = reinterpret_cast<const __nv_bfloat16*>(g.partial_o) + (static_cast<size_t>(group) * g.splits * kAttnQRows + r) * g.head_dim + b * 16;
-        float acc[16];
+        float2 acc[8];
 #pragma unroll
-        for (int e = 0; e < 16; e++) acc[e] = 0.f;
+        for (int e = 0; e < 8; e++) acc[e] = make_float2(0.f, 0.f);
         float denom = 0.f;
         if (g.splits <= 4) {
             // everything the item needs in one batch of independent loads: one round trip to L2 (the reference maximum
@@ -476,9 +473,9 @@ __device__ __forceinline__ void merge_item_wide(const MergeParams& g, int group,
     big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
     big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
     const float ref = big == -INFINITY ? 0.f : big;
-    float acc[16];
+    float2 acc[8];
 #pragma unroll
-    for (int e = 0; e < 16; e++) acc[e] = 0.f;
+    for (int e = 0; e < 8; e++) acc[e] = make_float2(0.f, 0.f);
     float denom = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -490,7 +487,8 @@ __device__ __forceinline__ void merge_item_wide(const MergeParams& g, int group,
     for (int o = 1; o <= 2; o <<= 1) {
         denom += __shfl_xor_sync(0xffffffffu, denom, o);
 #pragma unroll
-        for (int e = 0; e < 16; e++) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+        for (int e = 0; e < 8; e++)
+            acc[e] = add2(acc[e], make_float2(__shfl_xor_sync(0xffffffffu, acc[e].x, o), __shfl_xor_sync(0xffffffffu, acc[e].y, o)));
     }
     if (valid && sub == 0) merge_store(g, head, grow, b, acc, denom);
 }

@@ -112,6 +112,17 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
     constexpr uint64_t kKMajor = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);       // 128-byte swizzle, 8-row groups 1 KiB apart
     const uint32_t q16 = (smem_u32(sQ) & 0x3FFFFu) >> 4, kv16 = (smem_u32(sKV) & 0x3FFFFu) >> 4;
     const uint32_t kchunk16 = static_cast<uint32_t>(a.k_box) * 8u;                                  // one K/V chunk in 16-byte units
+    // V goes behind K where both fit (at most 128 keys) and is requested as soon as the MMAs of S are; otherwise into K's place
+    // once they are complete.  Its copies overlap the softmax.
+    const bool v_apart = 2 * CHUNKS * a.k_box * 128 <= kTcKvBytes;
+    const uint32_t v_offset = v_apart ? static_cast<uint32_t>(CHUNKS * a.k_box) * 128u : 0u;
+    auto load_v = [&]() {
+        const uint32_t k_bytes = static_cast<uint32_t>(a.k_box) * 128u;
+        mbar_expect_tx(bar_v, CHUNKS * k_bytes);
+        const int k_row = batch * a.kv_batch_rows + k_begin;
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) tma_load_2d(sKV + v_offset + c * k_bytes, a.tmap_v, bar_v, kvh * HDP + c * 64, k_row);
+    };
     if (warp == 0 && mbar_wait_warp(prog, ctl, bar_qk, parity, stage)) {
         if (stamp && lane == 0) stamp[4] = static_cast<long long>(global_ns());
         if (elect_one()) {
@@ -123,20 +134,14 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
                            kKMajor | static_cast<uint64_t>(kv16 + c * kchunk16 + 2u * sub), idesc, i != 0 ? 1u : 0u);
             }
             tc_commit(bar_s);
+            if (v_apart) load_v();
         }
         __syncwarp();
     }
     if (!cta_wait_phase(prog, ctl, bar_s, parity, stage)) return false;
     tc_fence_after();
 
-    // ---- V into K's place (its copies overlap the softmax)
-    if (threadIdx.x == 0) {
-        const uint32_t k_bytes = static_cast<uint32_t>(a.k_box) * 128u;
-        mbar_expect_tx(bar_v, CHUNKS * k_bytes);
-        const int k_row = batch * a.kv_batch_rows + k_begin;
-#pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) tma_load_2d(sKV + c * k_bytes, a.tmap_v, bar_v, kvh * HDP + c * 64, k_row);
-    }
+    if (threadIdx.x == 0 && !v_apart) load_v();
 
     // ---- softmax: thread = query row, the parts take alternate chunks of W columns
     const int quarter = warp & 3;
@@ -227,10 +232,11 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
             const uint64_t v_major = (static_cast<uint64_t>(kchunk16) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(HDP >> 3) << 17) | (8u << 24);
             const int steps = n_s >> 4;
+            const uint32_t v16 = kv16 + (v_offset >> 4);
             for (int j = 0; j < steps; ++j) {
                 const uint32_t c = static_cast<uint32_t>(j) >> 2, sub = static_cast<uint32_t>(j) & 3u;
                 tc_mma_f16(tmem + 256u, kKMajor | static_cast<uint64_t>(q16 + c * 1024u + 2u * sub),
-                           v_major | static_cast<uint64_t>(kv16 + static_cast<uint32_t>(j) * 128u), idesc, j != 0 ? 1u : 0u);
+                           v_major | static_cast<uint64_t>(v16 + static_cast<uint32_t>(j) * 128u), idesc, j != 0 ? 1u : 0u);
             }
             tc_commit(bar_o);
         }

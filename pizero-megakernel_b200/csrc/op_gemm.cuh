@@ -44,7 +44,7 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
         // Slots of the previous geometry overlap the new ones at other indices: every copy issued so far must have
         // been read by its MMAs before the first new copy lands (waits for the last release of each slot).
         int alive0 = 1;
-        if (lane == 0)
+        if (lane == 0 && ps.prod_geo != 0)                           // (nothing to wait for in front of the first GEMM)
             for (int s = 0; s < kMaxStagesDense && alive0; ++s)
                 alive0 = mbar_wait(prog, ctl, &ctl->empty[s], ((bits >> s) & 1u) ^ 1u, stage_index) ? 1 : 0;
         alive0 = __shfl_sync(0xffffffffu, alive0, 0);

@@ -122,7 +122,7 @@ class NativePi0:
         return cls(StateDictModel(config or Pi0Config(), state_dict), **kwargs)
 
     def __init__(self, model, *, num_views=3, prompt_len=0, chunk_size=50, flow_steps=10, precision="auto",
-                 library=None, workers=None, partitioned=False, expert_splits=None, prefix_splits=None, expert_block_n=None, expert_dense_block_n=None, vision_block_n=64, fold_layernorms=True,
+                 library=None, workers=None, partitioned=False, expert_splits=None, prefix_splits=None, expert_block_n=None, expert_dense_block_n=None, vision_block_n=None, fold_layernorms=True,
                  rope_inv_freq_dtype=torch.float32, keep_debug_outputs=False, verbose=False, tile_weights=True, schedule="affine",
                  fold_norms=True, attention_path=None, weight_store=None):
         config = getattr(model, "config", None)
@@ -147,7 +147,9 @@ class NativePi0:
         self.partitioned = partitioned
         self.expert_splits = expert_splits
         self.prefix_splits = prefix_splits
-        self.vision_block_n = vision_block_n
+        # output tile width of SigLIP's projections back to the stream (out, fc2; 1152 columns): 64, or 32 for a single view, whose
+        # 36 tiles of 64 would leave three quarters of the SMs idle (one view 5.38 -> 5.34 ms; two views are faster on 64)
+        self.vision_block_n = vision_block_n if vision_block_n is not None else (32 if num_views == 1 else 64)
         self.fold_layernorms = bool(fold_layernorms)
         # output tile widths of the action expert's projections: an int for all four, or a dict per operation.  The default
         # gives the projections with few output columns 32-wide tiles (twice the workers, half the bytes of weight and half
@@ -598,6 +600,10 @@ class NativePi0:
         if self.expert_splits is not None:
             return int(self.expert_splits)
         c = self.config
+        if self.chunk_size + 1 > 64:
+            # two warps per row quarter are busy and the merge of a tile's rows is the longer part: more splits, even if some
+            # tiles share a worker with the projection in front (101 rows: 10.64 -> 10.56 ms with 16 instead of 13)
+            return max(1, min(16, self.workers // c.heads, keys // 32))
         width = self.expert_block_n["qkv"] if isinstance(self.expert_block_n, dict) else self.expert_block_n
         qkv_tiles = -(-(c.heads + 2) * c.head_dim // width)
         return max(1, min(16, (self.workers - qkv_tiles) // c.heads, keys // 32))
