@@ -574,6 +574,21 @@ def test_attention_tensor_core_tiles(b, nq, nk, h, hk, hd, stored, prefix, split
         np.testing.assert_array_equal(other[:, 0], got[:, 0])
 
 
+@pytest.mark.parametrize("b,nq,nk,h,hk,hd,stored,prefix,splits", [
+    (1, 8, 24, 8, 1, 256, 256, None, 1),         # at most 64 queries: every query row lies in the tile twice
+    (1, 63, 128, 2, 1, 256, 256, 100, 1),        # the most keys with V behind K, ...
+    (1, 64, 129, 2, 1, 256, 256, 100, 1),        # ... one more
+    (1, 64, 1000, 8, 1, 256, 256, 900, 16),
+    (1, 65, 1000, 8, 1, 256, 256, 900, 16),      # one query more than fits twice
+    (1, 33, 512, 4, 1, 256, 256, 0, 2),          # 256 keys per tile
+    (2, 64, 200, 4, 4, 72, 128, None, 1),
+    (1, 65, 256, 4, 4, 72, 128, None, 1),
+])
+def test_attention_tiles_of_few_queries(b, nq, nk, h, hk, hd, stored, prefix, splits):
+    """The edges of the tiles for few queries and of the two places of V, under the bars of the other tiles."""
+    test_attention_tensor_core_tiles(b, nq, nk, h, hk, hd, stored, prefix, splits)
+
+
 @pytest.mark.parametrize("b,nq,nk,h,hk,hd,splits,bias,rope,mask,prefix", [
     (2, 100, 180, 4, 2, 64, 1, True, True, False, None),     # the Cosmos head sizes, GQA, biases and rotary tables
     (1, 200, 200, 4, 4, 128, 1, True, True, True, None),
@@ -731,6 +746,69 @@ def test_token_embedding_rows(count, width, offset):
     lib.destroy_op(h)
     want = (table.view(11, width)[tokens.clamp(0, 10)].float() * np.float32(3.7)).bfloat16()
     assert torch.equal(out[1:], want) and not out[0].any()
+
+
+@pytest.mark.parametrize("rows,n,k,flags", [
+    (1, 1, 8, 0), (17, 65, 1032, 0), (50, 1024, 32, 4), (33, 100, 1280, 0), (16, 80, 264, 4),     # FP32 rows
+    (1, 32, 8, 1 | 8), (51, 33, 1288, 1 | 8), (17, 64, 2048, 1 | 8),                                  # BF16 rows, RMS factor
+    (5, 16, 264, 1), (40, 72, 520, 1 | 8), (40, 72, 520, 8),                                          # the other combinations
+])
+def test_fp32_linear_forms(rows, n, k, flags):
+    """The specialised loops of the FP32 linear: row blocks of 16 and 32, columns beyond a multiple of 16, up to eight chunks
+    of K through the ring, the last one partial.  An FP32 sum of k products in any order is within k 2^-24 of the sum
+    of their magnitudes (the RMS factor's sum of squares likewise); the product is compared with FP64 under twice that."""
+    lib = _native.load()
+    torch.manual_seed(rows + n + k + flags)
+    x, w, b = torch.randn(rows, k, device="cuda"), torch.randn(n, k, device="cuda") * 0.1, torch.randn(n, device="cuda")
+    x = x.bfloat16() if flags & 1 else x
+    out = torch.full((rows + 1, n), float("nan"), device="cuda")
+    h = C.c_void_p()
+    _native.check(lib.create_linear32(C.byref(h), x.data_ptr(), w.data_ptr(), b.data_ptr(), None, out.data_ptr(), rows, n, k, k, n,
+                                      flags, 0, 0, 0, 0.0, 1e-6, 64), "lin")
+    try:
+        for _ in range(2):
+            _native.check(lib.launch_op(h, None), "launch")
+        torch.cuda.synchronize()
+    finally:
+        lib.destroy_op(h)
+    xd, wd = x.double(), w.double()
+    factor = torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) if flags & 8 else 1.0
+    want = (xd @ wd.T) * factor + b.double()
+    bound = 2 * (k + 16) * 2.0 ** -24 * ((xd.abs() @ wd.abs().T) * factor + b.double().abs())
+    if flags & 4:
+        want, bound = torch.nn.functional.silu(want), 1.1 * bound + 2.0 ** -20 * want.abs()           # (SiLU's slope is below 1.1)
+    assert bool(((out[:rows].double() - want).abs() <= bound).all())
+    assert bool(out[rows].isnan().all())
+
+
+@pytest.mark.parametrize("m,n,k,rows,block_n", [(256, 512, 192, 129, 128), (128, 256, 64, 1, 64), (128, 256, 448, 33, 32), (384, 768, 256, 321, 128),
+                                               (256, 256, 1152, 255, 64)])
+def test_drains_do_not_depend_on_the_run(m, n, k, rows, block_n):
+    """Instructions of one tile (shared out over eight warps) and runs of several tiles, over the ends of row bands, give
+    the same bits, store the rows that exist and no others, and agree with the FP32 result: a BF16 output is one rounding
+    (2^-8) of sum + bias + residual, a row's NVFP4 blocks those of the same product."""
+    rng = np.random.default_rng(m + n + k)
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    bias, res = bf16(rng.normal(size=n)), bf16(rng.normal(size=(m, n)))
+    kinds = [dict(output_dtype=torch.float32), dict(output_dtype=torch.bfloat16, bias=bias, residual=res),
+             dict(output_dtype=torch.uint8, output_gelu=True, bias=bias), dict(output_dtype=torch.uint8, output_geglu=True)]
+    got = []
+    for kind in kinds:
+        outs = []
+        for workers in (148, 5, 1):
+            with ResidentNVFP4(None, pa, pb, workers=workers, rows=rows, block_n=block_n, **kind) as op:
+                op.output.zero_()
+                y = op.forward()
+                assert op.status()["code"] == 0
+                outs.append((y.cpu(), op.output_scales.cpu() if y.dtype == torch.uint8 else None))
+        for y, sc in outs[1:]:
+            assert torch.equal(y, outs[0][0]) and (sc is None or torch.equal(sc, outs[0][1]))
+        assert not outs[0][0][rows:].any()
+        got.append(outs[0][0])
+    want = got[0].double() + bias.double()[None] + res.double()
+    slack = 2.0 ** -8 * want.abs() + 2.0 ** -22 * (got[0].double().abs() + bias.double().abs()[None] + res.double().abs())
+    assert bool(((got[1].double() - want).abs() <= slack)[:rows].all())
 
 
 def test_small_operators():
