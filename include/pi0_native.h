@@ -265,6 +265,10 @@ int launch_op(void* handle, void* stream);      /* any operator handle, as a one
 int destroy_op(void* handle);
 /* tiles, 128-row bands and K-cost of an operator handle (what the stream compiler needs). */
 int op_geometry(void* handle, int* tiles, int* bands, int* cost);
+/* extension, needs no device: operand ring of a projection (operands 0 NVFP4, 1 BF16, 2 FP8) of `rows` logical rows and
+ * block_n-wide tiles: bytes per slot, slots in flight, and the key a CTA compares to tell whether its ring cursors run on from
+ * the projection before (equal keys imply equal slot sizes and counts). */
+int gemm_ring_geometry(int operands, int rows, int block_n, int* slot_stride, int* ring_stages, unsigned int* key);
 
 /* ------------------------------------------------------------------------------------------------------
  * Whole-model program: one persistent launch over static per-worker instruction streams.

@@ -4,10 +4,12 @@
 // each operand row (64 FP4, 16 BF16 or 32 FP8 elements), so the copy ring and the issue loop are the same code.
 //
 //   warps 0 and 3   : TMA producers - A and B tiles (128 B swizzled rows) and their scale atoms into a ring of slots; the
-//                                     ring is laid out per GEMM: 3 slots of 72 KiB for full NVFP4 tiles, more for narrow ones
+//                                     ring is laid out per GEMM: 3 slots of 72 KiB for full NVFP4 tiles, up to 5 for narrow
+//                                     ones, up to 8 for dense operands (so slots of one size can come in different numbers)
 //   warp 1          : MMA issuer    - one elected thread issues tcgen05.cp (scales smem->TMEM, NVFP4 only) and
 //                                     tcgen05.mma, 32 operand bytes of K each
 //   warps 4..7      : epilogue      - tcgen05.ld of a 128xN FP32 accumulator (one row per thread), fused math, stores
+//   warps 0..3      : second half of the columns of an instruction's last tile, once their roles are done
 //
 // Two TMEM accumulators alternate, so the epilogue of tile t overlaps the MMAs of tile t+1. Pipeline positions live in
 // registers (PipeState) and carry over from one instruction to the next; barriers are never re-initialised.
@@ -40,8 +42,9 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
     const uint32_t ring = static_cast<uint32_t>(g.ring_stages), stride = static_cast<uint32_t>(g.slot_stride);
     const uint32_t off = WEIGHTS ? static_cast<uint32_t>(g.off_b) : 0u, off_sf = static_cast<uint32_t>(WEIGHTS ? g.off_sfb : g.off_sfa);
     const bool scaled = g.operands == GEMM_NVFP4;                    // scale atoms: 512 bytes per MMA group and operand
-    if (ps.prod_geo != stride) {
-        // Slots of the previous geometry overlap the new ones at other indices: every copy issued so far must have
+    const uint32_t geo = ring_key(g.slot_stride, g.ring_stages);
+    if (ps.prod_geo != geo) {
+        // Slots of the previous geometry overlap the new ones at other indices, or are more than the new ring has: every copy issued so far must have
         // been read by its MMAs before the first new copy lands (waits for the last release of each slot).
         int alive0 = 1;
         if (lane == 0 && ps.prod_geo != 0)                           // (nothing to wait for in front of the first GEMM)
@@ -49,7 +52,7 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
                 alive0 = mbar_wait(prog, ctl, &ctl->empty[s], ((bits >> s) & 1u) ^ 1u, stage_index) ? 1 : 0;
         alive0 = __shfl_sync(0xffffffffu, alive0, 0);
         if (!alive0) return;
-        ps.prod_geo = stride;
+        ps.prod_geo = geo;
         slot = 0;
     }
     int current_band = -1;
@@ -122,7 +125,8 @@ __device__ __forceinline__ void gemm_mma(const VmProgram& prog, Ctl* ctl, uint8_
     // (no swizzle, 8-line groups 128 bytes apart)
     constexpr uint64_t kOperandHi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
     constexpr uint64_t kScaleHi = (1ull << 16) | (8ull << 32) | (1ull << 46);
-    if (ps.mma_geo != stride) { ps.mma_geo = stride; ps.mma_slot = 0; }
+    const uint32_t geo = ring_key(g.slot_stride, g.ring_stages);
+    if (ps.mma_geo != geo) { ps.mma_geo = geo; ps.mma_slot = 0; }
     uint32_t slot = uniform_u32(ps.mma_slot), bits = uniform_u32(ps.mma_bits), it = uniform_u32(ps.mma_it), tile_no = uniform_u32(ps.mma_tile);
     const bool leader = elect_one();
     if (leader) {

@@ -411,6 +411,30 @@ size_t operand_row_bytes(int operands, int k) {
     return operands == GEMM_NVFP4 ? static_cast<size_t>(k) / 2 : operands == GEMM_BF16 ? static_cast<size_t>(k) * 2 : static_cast<size_t>(k);
 }
 
+// Rows of A copied per tile.  NVFP4, one row band: the logical rows in whole 8-row swizzle groups (at least 32, so that the 128
+// rows the MMA reads stay inside the slot for every tile width); dense operands: 64 or 128.
+int a_box_rows_of(int operands, int m, int rows) {
+    if (m != 128) return 128;
+    if (operands == GEMM_NVFP4) return std::min(128, std::max(32, (rows + 7) / 8 * 8));
+    return rows <= 64 ? 64 : 128;
+}
+// Operand ring: a slot holds kChunks chunks of the rows that are actually copied (A: a_box_rows, B: block_n) and,
+// for NVFP4, 4 KiB of scale atoms per operand. The MMA always reads 128 rows of A; with fewer copied rows the others are
+// whatever follows in the slot (B, scales) and end in accumulator rows that are never stored, so the read only
+// has to stay inside shared memory, which the slot's own B and scale regions guarantee.
+int ring_layout(GemmParams& g, int operands) {
+    g.off_b = kChunks * 128 * g.a_box_rows;
+    const int sf_bytes = operands == GEMM_NVFP4 ? kSfBytes : 0;
+    g.off_sfa = g.off_b + kChunks * 128 * g.block_n;
+    g.off_sfb = g.off_sfa + sf_bytes;
+    g.slot_stride = g.off_sfb + sf_bytes;
+    g.ring_stages = std::max(kStages, std::min(operands == GEMM_NVFP4 ? kMaxStages : kMaxStagesDense, kDataBytes / g.slot_stride));
+    if (g.slot_stride % 1024 || g.ring_stages * g.slot_stride > kDataBytes ||
+        (kChunks - 1) * 128 * g.a_box_rows + kTileABytes > g.slot_stride)
+        return cudaErrorInvalidValue;
+    return cudaSuccess;
+}
+
 int gemm_refresh(Op* op) {
     GemmParams& g = op->desc.p.gemm;
     CUtensorMap host[2];
@@ -432,19 +456,7 @@ int gemm_refresh(Op* op) {
     if (!g.sum_out || g.sumsq_ld < g.n_tiles) g.sumsq_ld = g.n_tiles;      // statistics rows: one slot per column tile
     g.operands = op->operands;
     g.k_groups = static_cast<int>(row_bytes / 32);
-    // Operand ring: a slot holds kChunks chunks of the rows that are actually copied (A: a_box_rows, B: block_n) and,
-    // for NVFP4, 4 KiB of scale atoms per operand. The MMA always reads 128 rows of A; with fewer copied rows the others are
-    // whatever follows in the slot (B, scales) and end in accumulator rows that are never stored, so the read only
-    // has to stay inside shared memory, which the slot's own B and scale regions guarantee.
-    g.off_b = kChunks * 128 * g.a_box_rows;
-    const int sf_bytes = op->operands == GEMM_NVFP4 ? kSfBytes : 0;
-    g.off_sfa = g.off_b + kChunks * 128 * g.block_n;
-    g.off_sfb = g.off_sfa + sf_bytes;
-    g.slot_stride = g.off_sfb + sf_bytes;
-    g.ring_stages = std::max(kStages, std::min(op->operands == GEMM_NVFP4 ? kMaxStages : kMaxStagesDense, kDataBytes / g.slot_stride));
-    if (g.slot_stride % 1024 || g.ring_stages * g.slot_stride > kDataBytes ||
-        (kChunks - 1) * 128 * g.a_box_rows + kTileABytes > g.slot_stride)
-        return cudaErrorInvalidValue;
+    if ((e = ring_layout(g, op->operands))) return e;
     // tcgen05 instruction descriptor: operand formats at bits 7 and 10 (block-scaled kind: 1 = E2M1; kind::f16: 1 = BF16;
     // kind::f8f6f4: 0 = E4M3), FP32 accumulator (bit 4) for the dense kinds, N / 8 at bit 17, M / 16 at bit 24; both
     // operands K-major.
@@ -680,10 +692,7 @@ extern "C" int configure_resident_fp4_rows(void* handle, int rows) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_GEMM || rows < 1 || rows > op->m) return cudaErrorInvalidValue;
     op->desc.p.gemm.rows = rows;
-    // rows of A copied per tile: the logical rows in whole 8-row swizzle groups (at least 32, so that the 128 rows the MMA
-    // reads stay inside the slot for every tile width)
-    if (op->m == 128 && op->operands == GEMM_NVFP4) op->desc.p.gemm.a_box_rows = std::min(128, std::max(32, (rows + 7) / 8 * 8));
-    else op->desc.p.gemm.a_box_rows = (rows <= 64 && op->m == 128) ? 64 : 128;
+    op->desc.p.gemm.a_box_rows = a_box_rows_of(op->operands, op->m, rows);
     return gemm_refresh(op);
 }
 extern "C" int configure_resident_fp4_weight_layout(void* handle, int tiled) {
@@ -1356,6 +1365,22 @@ extern "C" int op_geometry(void* handle, int* tiles, int* bands, int* cost) {
     if (tiles) *tiles = op->desc.tiles;
     if (bands) *bands = op->desc.bands;
     if (cost) *cost = op->cost;
+    return cudaSuccess;
+}
+
+// extension: the operand ring of a projection (operands: GemmOperands) with one band of `rows` logical rows (more than 128:
+// several bands) and block_n-wide tiles - slot size, slot count and the key under which the kernel's ring cursors run on.
+// Needs no device.
+extern "C" int gemm_ring_geometry(int operands, int rows, int block_n, int* slot_stride, int* ring_stages, unsigned int* key) {
+    if (operands < GEMM_NVFP4 || operands > GEMM_FP8 || rows < 1 || (block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
+    GemmParams g{};
+    g.a_box_rows = a_box_rows_of(operands, rows <= 128 ? 128 : 256, rows);
+    g.block_n = block_n;
+    const int e = ring_layout(g, operands);
+    if (e) return e;
+    if (slot_stride) *slot_stride = g.slot_stride;
+    if (ring_stages) *ring_stages = g.ring_stages;
+    if (key) *key = ring_key(g.slot_stride, g.ring_stages);
     return cudaSuccess;
 }
 

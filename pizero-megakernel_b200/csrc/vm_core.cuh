@@ -65,10 +65,11 @@ static_assert(kRing <= 4, "words kept per GEMM instruction modulo 4");
 static_assert(sizeof(Ctl) <= kCtlBytes, "control block too large");
 
 // The ring geometry (slot count and size) belongs to the GEMM, so positions are kept per barrier: bit s of
-// prod_bits / mma_bits is the parity of the fills / drains slot s has seen. Producer and MMA lane walk the same slot
-// sequence: the cursor continues from one instruction to the next and restarts at 0 when the geometry changes.
+// prod_bits / mma_bits is the parity of the fills / drains slot s has seen. Producers and MMA lane walk the same slot
+// sequence: the cursor continues from one instruction to the next and restarts at 0 when the geometry changes (ring_key:
+// size or count).
 struct PipeState {
-    uint32_t prod_slot = 0, prod_bits = 0, prod_geo = 0;     // TMA lane
+    uint32_t prod_slot = 0, prod_bits = 0, prod_geo = 0;     // TMA lanes (each copy warp its own)
     uint32_t mma_slot = 0, mma_bits = 0, mma_geo = 0;        // MMA lane
     uint32_t mma_it = 0;         // K stages consumed by the MMA lane (rotates the scale columns in tensor memory)
     uint32_t mma_tile = 0;       // accumulator tiles produced

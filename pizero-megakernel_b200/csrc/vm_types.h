@@ -60,7 +60,7 @@ struct GemmParams {
     int block_n;                 // 128 (default), 64 or 32
     int b_tiled;                 // B stored tile-major: block (n_tile, k_stage) is block_n contiguous 128-byte rows
     int a_box_rows;              // rows of A copied per tile: 128, or fewer (a multiple of 8) when there are fewer logical rows
-    int ring_stages;             // operand ring of this GEMM: slots in flight (2..kMaxStages) ...
+    int ring_stages;             // operand ring of this GEMM: slots in flight (kStages..kMaxStagesDense) ...
     int slot_stride;             // ... bytes from one slot to the next (multiple of 1024) ...
     int off_b, off_sfa, off_sfb; // ... and where B, the A scales and the B scales start inside a slot (A starts at 0)
     float alpha;                 // global_scale(A) * global_scale(B)
@@ -107,6 +107,12 @@ struct GemmParams {
     int cache_base;              // first cache row written by this projection
     uint32_t idesc;              // tcgen05 instruction descriptor
 };
+
+// Identity of an operand ring: the ring cursors of a CTA run on from one GEMM to the next only where slot size AND slot count
+// agree (NVFP4 and dense rings of one slot size may differ in depth).  Sizes are multiples of 1024, so the two fit one word; never 0.
+__host__ __device__ inline uint32_t ring_key(int slot_stride, int ring_stages) {
+    return static_cast<uint32_t>(slot_stride) | static_cast<uint32_t>(ring_stages);
+}
 
 struct NormParams {
     const void* in;              // BF16 [rows, width]

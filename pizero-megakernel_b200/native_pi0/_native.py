@@ -103,6 +103,7 @@ _SIGNATURES = {
     "launch_op": [_P, _P],
     "destroy_op": [_P],
     "op_geometry": [_P, C.POINTER(_I), C.POINTER(_I), C.POINTER(_I)],
+    "gemm_ring_geometry": [_I, _I, _I, C.POINTER(_I), C.POINTER(_I), C.POINTER(C.c_uint)],
     "create_native_model": [C.POINTER(_P), _I, _P, _P, _I, _I],
     "launch_native_model": [_P] * 6,
     "launch_native_model_range": [_P] * 6 + [_I] * 3,

@@ -99,6 +99,25 @@ def test_site_precisions(small_model, precision, policy):
         assert nrmse(out, eager) <= 1.3 * max(nrmse(emulation, eager), 0.05)
 
 
+@pytest.mark.parametrize("chunk", [63, 31, 15])
+@pytest.mark.parametrize("precision", [{"*.qkv": "bf16"}, {"expert.*.qkv": "bf16", "expert.*.gate_up": "bf16"}, {"expert.*.down": "bf16"}])
+def test_mixed_formats_whose_ring_slots_have_one_size(small_model, precision, chunk):
+    """With 57 to 64 and with at most 32 expert rows the NVFP4 and the BF16 projections of the expert use operand rings of one
+    slot size and different depths: a worker that goes from one to the other starts the ring again.  Agreement with the
+    oracle emulating the same choice, clean status, and the same bits when launched again and stage by stage."""
+    dims, cfg, sd = small_model
+    x = inputs(1, chunk, 0, dims.vocab)
+    emulation = Pi0Torch(dims, sd, mode="nvfp4", precision=precision).sample_actions(*x)
+    with NativePi0(StateDictModel(cfg, sd), num_views=1, chunk_size=chunk, precision=precision) as engine:
+        out = engine.forward(*x).clone()
+        assert engine.status()["code"] == 0 and engine.precision_policy == "mixed"
+        assert torch.equal(engine.forward(*x), out)
+        for s in range(len(engine.stages)):
+            engine.launch_range(s, s + 1, *x, new_epoch=(s == 0))
+        assert engine.status()["code"] == 0 and torch.equal(engine.output, out)
+    assert nrmse(out, emulation) <= 0.1
+
+
 def test_checkpoint_file_and_calibrated_precisions(small_model, tmp_path):
     """The checkpoint path: a ``model.safetensors`` with OpenPI parameter names is read by ``from_openpi`` (dimensions
     from the tensors) and gives the same bits as the in-memory state dict; a BF16 engine records activation maxima for
