@@ -290,7 +290,9 @@ __device__ __forceinline__ uint32_t block_scale_code(float amax, int policy) {
 // packing of the codes make it about half as long as the scalar form.
 __device__ __forceinline__ uint2 quantize_block16(const float2 (&v)[8], int policy, uint32_t& code_out) {
     const float a = max3_abs(max3_abs(v[0].x, v[0].y, v[1].x), max3_abs(v[1].y, v[2].x, v[2].y), max3_abs(v[3].x, v[3].y, v[4].x));
-    const float amax = max3_abs(max3_abs(a, v[4].y, v[5].x), max3_abs(v[5].y, v[6].x, v[6].y), fmaxf(fabsf(v[7].x), fabsf(v[7].y)));
+    // (the zero costs nothing and keeps the maximum a number: the three-input maxima pass over NaNs, but a block of nothing else
+    // would hand its NaN on to the scale)
+    const float amax = max3_abs(max3_abs(a, v[4].y, v[5].x), max3_abs(v[5].y, v[6].x, v[6].y), max3_abs(v[7].x, v[7].y, 0.f));
     const uint32_t code = block_scale_code(amax, policy);
     const float decoded = decode_ue4m3(code);
     const float recip = decoded > 0.f ? __frcp_rn(decoded) : 0.f;

@@ -811,6 +811,41 @@ def test_drains_do_not_depend_on_the_run(m, n, k, rows, block_n):
     assert bool(((got[1].double() - want).abs() <= slack)[:rows].all())
 
 
+@pytest.mark.parametrize("policy", [0, 1])
+def test_quantiser_passes_over_nans(policy):
+    """The block scale is that of the block's numbers: a block of NaNs alone has scale zero and zero codes, and a NaN among
+    numbers leaves the scale and the codes of its neighbours alone; infinities saturate."""
+    lib = _native.load()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    clean = torch.randn(128, 128, generator=g, device="cuda").bfloat16()
+    x = clean.clone()
+    x[0, :16] = float("nan")
+    x[1, 16:31] = float("nan")
+    x[2, 37] = float("nan")
+    x[3, 48] = float("inf")
+    clean[0, :16] = 0
+    clean[1, 16:31] = 0
+    clean[2, 37] = 0
+
+    def quantise(values):
+        data, scales = torch.zeros(128, 64, dtype=torch.uint8, device="cuda"), torch.zeros(1024, dtype=torch.uint8, device="cuda")
+        _native.check(lib.quantize_nvfp4(values.data_ptr(), data.data_ptr(), scales.data_ptr(), 128, 128, 128, 8, 1.0, policy,
+                                         torch.cuda.current_stream().cuda_stream), "quantise")
+        torch.cuda.synchronize()
+        nibbles = torch.stack((data & 15, data >> 4), -1).view(128, 128)
+        return nibbles.cpu(), torch.from_numpy(unswizzle_scales(scales.cpu().numpy(), 128, 8))
+
+    got, got_scales = quantise(x)
+    want, want_scales = quantise(clean)
+    assert got_scales[0, 0] == 0 and not got[0, :16].any()
+    assert got_scales[3, 3] == 126 and got[3, 48] == 7
+    want_scales[3, 3], want[3, 48:64] = got_scales[3, 3], got[3, 48:64]
+    assert torch.equal(got_scales, want_scales)
+    nans = torch.zeros(128, 128, dtype=torch.bool)
+    nans[1, 16:31] = nans[2, 37] = True
+    assert torch.equal(got[~nans], want[~nans])
+
+
 def test_small_operators():
     lib = _native.load()
     torch.manual_seed(11)
