@@ -99,6 +99,14 @@ class StageOutput:
         self.head = head            # kind "bf16": (head width, pitch) when heads are stored apart with zeros between them
 
 
+OPERATIONS = ("qkv", "o_proj", "gate_up", "down")       # the projections of a Gemma layer
+
+
+def per_operation(width):
+    """Tile widths per operation: a dict as given, an int for all four."""
+    return width if isinstance(width, dict) else dict.fromkeys(OPERATIONS, width)
+
+
 class NativePi0:
     @classmethod
     def from_openpi(cls, checkpoint_path, *, num_views=3, prompt_len=0, chunk_size=50, flow_steps=10,
@@ -627,7 +635,7 @@ class NativePi0:
             _native.check(self.lib.configure_attention_path(handle, int(self.attention_path == "tcgen05")), name)
 
     def _gemma_layer(self, name, site, prefix, i, x_in, x_mid, bufs, *, rows, s_x, extra_sources, cos, sin, cache, cache_base,
-                     attention_rows, mask_prefix, splits, kv_only, block_n, dense_block_n=None, prefix_cache_stage=None,
+                     attention_rows, mask_prefix, splits, kv_only, block_n, dense_block_n=128, prefix_cache_stage=None,
                      streamed_in=None, next_site=None):
         """One Gemma decoder layer.  ``name`` labels the stages (``expert.<step>.<layer>``), ``site`` the weights
         (``expert.<layer>``: one operand format for all Euler steps).
@@ -644,10 +652,9 @@ class NativePi0:
         width = x_in.shape[1]
         H, hd = c.heads, c.head_dim
         a1, a2, a3, a4, qbuf = bufs
-        p_qkv, p_o, p_gu, p_dn = [self.site(f"{site}.{n}") for n in ("qkv", "o_proj", "gate_up", "down")]
-        widths = block_n if isinstance(block_n, dict) else dict.fromkeys(("qkv", "o_proj", "gate_up", "down"), block_n)
-        p_of = dict(zip(("qkv", "o_proj", "gate_up", "down"), (p_qkv, p_o, p_gu, p_dn)))
-        dense_widths = dense_block_n or dict.fromkeys(widths, 128)
+        p_qkv, p_o, p_gu, p_dn = [self.site(f"{site}.{n}") for n in OPERATIONS]
+        widths, dense_widths = per_operation(block_n), per_operation(dense_block_n)
+        p_of = dict(zip(OPERATIONS, (p_qkv, p_o, p_gu, p_dn)))
         tile = lambda op: widths[op] if p_of[op] == "nvfp4" else dense_widths[op]
         sums = lambda key, parts: self.cached((key, x_in.shape[0], parts), lambda: self.tensor((x_in.shape[0], parts), torch.float32))
         gamma1 = lambda: (1.0 + sd[p + "input_layernorm.weight"].float()).contiguous()

@@ -118,6 +118,18 @@ def test_mixed_formats_whose_ring_slots_have_one_size(small_model, precision, ch
     assert nrmse(out, emulation) <= 0.1
 
 
+@pytest.mark.parametrize("width", [128, 64, 32])
+def test_one_width_for_all_dense_projections_of_the_expert(small_model, width):
+    """``expert_dense_block_n`` takes an int for all four projections, as ``expert_block_n`` does; a tile width never changes the
+    sums over K, so the actions keep their bits."""
+    dims, cfg, sd = small_model
+    x = inputs(1, 10, 0, dims.vocab)
+    with NativePi0(StateDictModel(cfg, sd), num_views=1, chunk_size=10, precision="bf16", flow_steps=2) as default, \
+            NativePi0(StateDictModel(cfg, sd), num_views=1, chunk_size=10, precision="bf16", flow_steps=2, expert_dense_block_n=width) as engine:
+        assert torch.equal(engine.forward(*x), default.forward(*x))
+        assert engine.status()["code"] == 0
+
+
 def test_checkpoint_file_and_calibrated_precisions(small_model, tmp_path):
     """The checkpoint path: a ``model.safetensors`` with OpenPI parameter names is read by ``from_openpi`` (dimensions
     from the tensors) and gives the same bits as the in-memory state dict; a BF16 engine records activation maxima for
