@@ -184,8 +184,8 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-# The raw handle of a device's current stream, and the current device, without building stream / device objects; the
-# CPU-only build of PyTorch has neither.
+# The raw handle of a device's current stream, and the current device, without building stream / device objects.  Both names
+# are private: where a build of PyTorch lacks one, launch() goes through the public calls.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _get_device = getattr(torch._C, "_cuda_getDevice", None)
 
@@ -196,10 +196,10 @@ def launch(entry, handle, device, *arguments):
     A small operator takes less time on the GPU than ``torch.cuda.device`` and ``torch.cuda.current_stream`` take on the
     host (together about half of an 8 us call), so the device is only switched when another one is current."""
     index = device.index
-    if _get_device() == index:
+    if _raw_stream is not None and _get_device is not None and _get_device() == index:
         return entry(handle, _raw_stream(index), *arguments)
     with torch.cuda.device(device):
-        return entry(handle, _raw_stream(index), *arguments)
+        return entry(handle, torch.cuda.current_stream(device).cuda_stream, *arguments)
 
 
 def status(lib, handle):

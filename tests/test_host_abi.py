@@ -63,6 +63,34 @@ def test_missing_library_fails_loudly(tmp_path):
         _native.load(tmp_path / "absent.so")
 
 
+@pytest.mark.parametrize("private,device", [((None, None), "cuda:1"), ((lambda i: 77, None), "cuda:1"), ((None, lambda: 1), "cuda:1"),
+                                            ((lambda i: 77, lambda: 0), "cuda:1"), ((lambda i: 77, lambda: 1), "cuda"),
+                                            ((lambda i: 77, lambda: 1), "cuda:1")])
+def test_launch_has_a_way_without_private_names(monkeypatch, private, device):
+    """A launch reaches the library with the current stream of the operator's device, on that device: through PyTorch's private
+    calls where they exist and the device is current, through the public ones otherwise."""
+    from native_pi0 import _native
+    entered = []
+
+    class Guard:
+        def __init__(self, d):
+            entered.append(str(d))
+
+        def __enter__(self):
+            return self
+
+        def __exit__(self, *_):
+            entered.append("left")
+
+    monkeypatch.setattr(_native, "_raw_stream", private[0])
+    monkeypatch.setattr(_native, "_get_device", private[1])
+    monkeypatch.setattr(torch.cuda, "device", Guard)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: type("Stream", (), {"cuda_stream": 77})())
+    assert _native.launch(lambda *a: a, "handle", torch.device(device), 1, 2) == ("handle", 77, 1, 2)
+    direct = None not in private and private[1]() == torch.device(device).index
+    assert entered == ([] if direct else [device, "left"])
+
+
 def test_null_handles_need_no_device(libraries):
     engine, _ = libraries
     for name in ("destroy_resident_fp4", "destroy_norm", "destroy_attention", "destroy_op", "destroy_native_model", "destroy_native_linear"):
