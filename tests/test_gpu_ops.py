@@ -785,8 +785,10 @@ def test_fp32_linear_forms(rows, n, k, flags):
                                                (256, 256, 1152, 255, 64)])
 def test_drains_do_not_depend_on_the_run(m, n, k, rows, block_n):
     """Instructions of one tile (shared out over eight warps) and runs of several tiles, over the ends of row bands, give
-    the same bits, store the rows that exist and no others, and agree with the FP32 result: a BF16 output is one rounding
-    (2^-8) of sum + bias + residual, a row's NVFP4 blocks those of the same product."""
+    the same bits, store the rows that exist and no others, and agree with the FP64 product of the dequantised operands: the FP32
+    output to its summation error (3e-5, as in the other projection tests), a BF16 output is one rounding (2^-8) of
+    sum + bias + residual, and every NVFP4 block is one of the activated product - its scale the E4M3 value nearest to a sixth
+    of the block's maximum, its codes the E2M1 values nearest to the quotients (at most 1/4, or a quarter of the quotient, off)."""
     rng = np.random.default_rng(m + n + k)
     pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
     pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
@@ -809,6 +811,28 @@ def test_drains_do_not_depend_on_the_run(m, n, k, rows, block_n):
     want = got[0].double() + bias.double()[None] + res.double()
     slack = 2.0 ** -8 * want.abs() + 2.0 ** -22 * (got[0].double().abs() + bias.double().abs()[None] + res.double().abs())
     assert bool(((got[1].double() - want).abs() <= slack)[:rows].all())
+    operand = lambda p: torch.from_numpy(oracle.dequantize(p.data, p.scales, p.global_scale, p.logical_shape)).double()     # noqa: E731
+    product = (operand(pa)[:rows] @ operand(pb).T)
+    error = 3e-5 * product.abs() + 1e-5 * product.abs().max()
+    assert bool(((got[0][:rows].double() - product).abs() <= error).all())
+    gate, up = product[:, 0::2], product[:, 1::2]
+    biased = product + bias.double()[None]
+    gelu = torch.nn.functional.gelu
+    activated = [(gelu(biased, approximate="tanh"), 1.13 * error),                                  # (GELU's slope is below 1.13)
+                 (gelu(gate, approximate="tanh") * up, 1.13 * error[:, 0::2] * up.abs() + gelu(gate, approximate="tanh").abs() * error[:, 1::2])]
+    for kind, codes, (value, error) in zip(kinds[2:], got[2:], activated):
+        error = error + 2.0 ** -18 * value.abs()                                                    # (the fast exponential and quotient)
+        width = value.shape[1]
+        with ResidentNVFP4(None, pa, pb, workers=148, rows=rows, block_n=block_n, **kind) as op:
+            assert torch.equal(op.forward().cpu(), codes)
+            scales = torch.from_numpy(unswizzle_scales(op.output_scales.cpu().numpy(), m, width // 16)[:rows].copy()).view(torch.float8_e4m3fn).double()
+        sixth, off = value.abs().view(rows, -1, 16).amax(-1) / 6, error.view(rows, -1, 16).amax(-1)
+        assert bool(((scales - sixth).abs() <= sixth / 16 + 2.0 ** -10 + off).all())                # (2^-10: half the smallest E4M3 step)
+        nibbles = torch.stack((codes[:rows, :width // 2] & 15, codes[:rows, :width // 2] >> 4), -1).view(rows, width).long()
+        table = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6], dtype=torch.float64)
+        step = scales.repeat_interleave(16, 1)
+        decoded = table[nibbles & 7] * torch.where(nibbles > 7, -1.0, 1.0) * step
+        assert bool(((decoded - value).abs() <= torch.maximum(step / 4, torch.where(step > 0, value.abs() / 4, value.abs())) + error).all())
 
 
 @pytest.mark.parametrize("policy", [0, 1])
