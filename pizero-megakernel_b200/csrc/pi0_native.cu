@@ -18,7 +18,6 @@ namespace {
 
 constexpr uint32_t kOpMagic = 0x7069304f;       // "pi0O"
 constexpr uint32_t kProgramMagic = 0x70693050;  // "pi0P"
-constexpr int kEarlyGrid = 148 / 4 + 3;         // CTAs of an operator whose successor may start early (launch_program)
 
 // Current device, checked to be compute capability 10.x. The capability is looked up once per device (one attribute
 // query), so steady-state callers pay only cudaGetDevice.
@@ -143,7 +142,7 @@ struct Program {
     bool timings_on = false;
     bool lean = false;                 // every stage is one the lean kernel variant runs
     bool mma_sync = false;             // some attention stage runs on the mma.sync tiles
-    bool solo = false;                 // the program of one operator
+    bool early = false;                // the program of one operator small enough for its successor to start early (solo_program)
     int grid = 0;                      // CTAs launched: up to the last worker that has an instruction
     unsigned int epoch = 0;
     unsigned long long budget_ns = 2000000000ull;
@@ -344,17 +343,14 @@ int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begi
     p.epoch = prog->epoch;
     p.stage_begin = begin;
     p.stage_end = end;
-    // An operator takes a few microseconds and leaves SMs free: its successor's CTAs may start and wait there.  Only while two
-    // launches fit one CTA per pair of SMs: a larger grid placed around its predecessor shares SM pairs, and their path to
-    // L2, that it would have spread over (768-row FP8 down projection, 96 CTAs: 36.5 instead of 31.6 us).  Whole models keep
-    // their SMs to the end anyway.
-    p.early_dependents = prog->solo && prog->grid <= kEarlyGrid ? 1 : 0;
+    p.early_dependents = prog->early ? 1 : 0;
     p.wait_budget_ns = prog->budget_ns;
     p.in = in;
     p.debug = prog->h_debug;
-    // Programmatic stream serialisation: the CTAs are placed as soon as those of the kernel in front have exited (behind an
-    // operator, as soon as there are free SMs) and wait in the kernel for its completion (grid_dependency_wait).  Ordinary serialisation of back-to-back launches costs
-    // 2 - 4 us on B200, rounded up to multiples of 2.048 us: RMSNorm 51 x 1024 takes 8.2 us per call with it, 5.9 with this.
+    // Programmatic stream serialisation: the CTAs are placed as soon as those of the kernel in front have exited (behind a
+    // small operator, as soon as there are free SMs) and wait in the kernel for its completion (grid_dependency_wait).
+    // Ordinary serialisation of back-to-back launches costs 2 - 4 us on B200, rounded up to multiples of 2.048 us: RMSNorm
+    // 51 x 1024 takes 8.2 us per call with it, 5.9 with this.
     cudaLaunchAttribute serial{};
     serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     serial.val.programmaticStreamSerializationAllowed = 1;
@@ -498,7 +494,18 @@ int solo_program(Op* op) {
     std::vector<int> code = compile_streams(work, op->workers, &length);
     int e = build_program(&op->solo, op->device, stages, code, op->workers, length);
     if (e) return e;
-    op->solo->solo = true;
+    // An operator takes a few microseconds and leaves SMs free: its successor's CTAs may start there and wait.  How large the
+    // successor is, is not known here, and one that fills the rest of the machine is placed worse around its predecessor than
+    // on its own: it shares SM pairs, and their path to L2, that it would have spread over.  The line lies where that begins.
+    // Pairs of launches, early against not: GEMM of 24 / 32 / 37 / 40 / 44 CTAs in front of a BF16 one of 96: -0.36 / -0.19 /
+    // -0.26 / -0.29 / -0.15 us; of 48 / 52 / 64: +0.17 / +0.20 / +0.37; in front of 120 or 128 CTAs -0.2 to 0 up to 44, 0 beyond; in
+    // front of 13 or 40: -0.9 to -1.6 throughout.  One operator behind itself gains 0.4 - 0.8 us up to 74 CTAs and then loses
+    // (FP8 640 / 768 x 2048 x 16384, 80 / 96 CTAs: 31.1 / 31.9 -> 36.0 / 36.5 us).  So: at most three tenths of the SMs (44 of
+    // 148).  Whole models keep their SMs to the end and never let a successor in.
+    int sms = 0;
+    const cudaError_t ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
+    if (ce != cudaSuccess) return ce;
+    op->solo->early = op->solo->grid <= sms * 3 / 10;
     op->solo_dirty = false;
     return cudaSuccess;
 }

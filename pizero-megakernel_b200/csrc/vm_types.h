@@ -304,7 +304,7 @@ struct VmProgram {
     int num_stages, length;
     unsigned int epoch;
     int stage_begin, stage_end;  // execute stages in [begin, end); sources < begin are treated as complete
-    int early_dependents;        // let the next launch of the stream prepare while this one runs (stand-alone operators)
+    int early_dependents;        // let the next launch of the stream prepare while this one runs (small stand-alone operators)
     unsigned long long wait_budget_ns;
     LaunchInputs in;
     int* debug;                  // optional host-mapped progress marks, one word per warp (diagnostics)

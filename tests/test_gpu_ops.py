@@ -835,6 +835,54 @@ def test_drains_do_not_depend_on_the_run(m, n, k, rows, block_n):
         assert bool(((decoded - value).abs() <= torch.maximum(step / 4, torch.where(step > 0, value.abs() / 4, value.abs())) + error).all())
 
 
+@pytest.mark.parametrize("columns", [1024, 5632, 6144])
+def test_launches_that_overlap_keep_the_order_of_the_stream(columns):
+    """Launches prepare while the one in front finishes, behind small operators (8 and 44 CTAs; not 48) on SMs that it leaves
+    free: a consumer still reads what its producer, or a copy or an event of another stream in front of it, wrote, and an input
+    may be overwritten behind the launch that reads it.  Back to back against one at a time."""
+    rng = np.random.default_rng(columns)
+    pa = pack_nvfp4(rng.normal(size=(51, 512)).astype(np.float32), row_alignment=128)
+    p0 = pack_nvfp4(rng.normal(scale=0.05, size=(columns, 512)).astype(np.float32), scale_policy="ceil")
+    p1 = pack_nvfp4(rng.normal(scale=0.05, size=(256, columns)).astype(np.float32), scale_policy="ceil")
+    placeholder = pack_nvfp4(np.zeros((128, columns), np.float32))
+    rows = [torch.randn(51, 1024, device="cuda").bfloat16() for _ in range(8)]
+    source = torch.zeros_like(rows[0])
+    codes = [torch.randint(0, 256, (128, 256), dtype=torch.uint8, device="cuda") for _ in range(8)]
+    other = torch.cuda.Stream()
+    with ResidentNVFP4(None, pa, p0, workers=148, output_dtype=torch.uint8, rows=51) as s0, \
+            ResidentNVFP4(None, placeholder, p1, workers=148, rows=51, activation_buffers=(s0.output, s0.output_scales)) as s1, \
+            ResidentNorm(None, source, kind="rms", precision="fp4", workers=148, row_alignment=128) as norm:
+        def passes(synchronise):
+            kept = []
+            wait = torch.cuda.synchronize if synchronise else lambda: None
+            for i in range(8):
+                source.copy_(rows[i])
+                wait()
+                norm.forward()
+                wait()
+                source.fill_(float("nan"))
+                s0.a[:, :256].copy_(codes[i])
+                wait()
+                s0.forward()
+                wait()
+                s1.forward()
+                wait()
+                other.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(other):
+                    norm_codes = norm.output.clone()
+                    s0.a.zero_()
+                    s1.forward()                                        # (the same operands again, on the other stream)
+                torch.cuda.current_stream().wait_stream(other)
+                kept += [norm_codes, s0.output.clone(), s1.output.clone()]
+                wait()
+            torch.cuda.synchronize()
+            return kept
+
+        one, many = passes(True), passes(False)
+        assert all(torch.equal(a, b) for a, b in zip(one, many))
+        assert all(op.status()["code"] == 0 for op in (s0, s1, norm))
+
+
 @pytest.mark.parametrize("policy", [0, 1])
 def test_quantiser_passes_over_nans(policy):
     """The block scale is that of the block's numbers: a block of NaNs alone has scale zero and zero codes, and a NaN among
