@@ -156,7 +156,9 @@ class NativePi0:
         self.expert_splits = expert_splits
         self.prefix_splits = prefix_splits
         # output tile width of SigLIP's projections back to the stream (out, fc2; 1152 columns): 64, or 32 for a single view, whose
-        # 36 tiles of 64 would leave three quarters of the SMs idle (one view 5.38 -> 5.34 ms; two views are faster on 64)
+        # 36 tiles of 64 would leave three quarters of the SMs idle (one view, 64 -> 32: prompt of 9 tokens 8.17 -> 8.02 ms with a
+        # chunk of 10 and 8.70 -> 8.50 with 50, prompt of 48 8.16 -> 7.95 and 8.65 -> 8.52, no prompt 7.99 -> 8.02 and 8.52 -> 8.50;
+        # two views are faster on 64).  The width is part of how the two weights are packed (see EngineCache).
         self.vision_block_n = vision_block_n if vision_block_n is not None else (32 if num_views == 1 else 64)
         self.fold_layernorms = bool(fold_layernorms)
         # output tile widths of the action expert's projections: an int for all four, or a dict per operation.  The default
@@ -610,7 +612,10 @@ class NativePi0:
         c = self.config
         if self.chunk_size + 1 > 64:
             # two warps per row quarter are busy and the merge of a tile's rows is the longer part: more splits, even if some
-            # tiles share a worker with the projection in front (101 rows: 10.64 -> 10.56 ms with 16 instead of 13)
+            # tiles share a worker with the projection in front.  16 instead of the 13 of the rule below, three views, prompt 48 /
+            # none: 65 rows 10.14 -> 9.94 / 9.79 -> 9.73 ms, 81 rows 10.37 -> 10.28 / 10.05 -> 10.03, 101 rows 10.66 -> 10.57 / 10.32
+            # -> 10.32, 128 rows 11.10 -> 10.87 / 10.72 -> 10.54; two views 9.05 -> 9.14, 9.34 -> 9.38, 9.68 -> 9.68, 10.09 -> 10.03
+            # (a run of one side spreads by up to 0.26).  A single view has too few keys for either.
             return max(1, min(16, self.workers // c.heads, keys // 32))
         width = self.expert_block_n["qkv"] if isinstance(self.expert_block_n, dict) else self.expert_block_n
         qkv_tiles = -(-(c.heads + 2) * c.head_dim // width)
@@ -1005,7 +1010,10 @@ class EngineCache:
 
     A program is compiled for fixed (views, prompt length, chunk size); a deployment that sees a few shapes keeps one
     engine per shape.  The engines share a ``weight_store``, so every weight is packed and resident once (1.46 GB in
-    NVFP4) and an additional shape costs only its activations, KV caches and instruction streams.  At most
+    NVFP4) and an additional shape costs only its activations, KV caches and instruction streams - with one exception:
+    SigLIP's ``out`` and ``fc2`` are packed for the width of the tiles that run them, which is another one for a single
+    view (``vision_block_n``), so a cache that has seen one view and several views holds them twice (NVFP4 130 MB more, BF16
+    340 MB) and packs them at the first request of the second kind; ``vision_block_n=64`` keeps one packing for all.  At most
     ``capacity`` engines stay alive; the least recently used one is closed when another shape arrives.  The state dict
     is kept for building further shapes.
     """

@@ -185,6 +185,21 @@ def test_engine_cache_shares_weights_between_shapes(small_model):
         assert set(cache.engines) == {shapes[0], shapes[2]}
 
 
+@pytest.mark.parametrize("options,extra", [({}, 2), ({"vision_block_n": 64}, 0)])
+def test_engine_cache_of_one_and_three_views(small_model, options, extra):
+    """What a second view count adds to the shared weights: SigLIP's out and fc2, which a single view runs on tiles of another
+    width, or nothing with one width for both."""
+    dims, cfg, sd = small_model
+    x = inputs(1, 7, 3, dims.vocab)
+    with EngineCache(StateDictModel(cfg, sd), **options) as cache:
+        cache.get(3, 3, 7)
+        packed = len(cache.weights)
+        one = cache.get(1, 3, 7)
+        assert len(cache.weights) == packed + extra * cfg.vision_layers
+        with NativePi0(StateDictModel(cfg, sd), num_views=1, prompt_len=3, chunk_size=7, **options) as alone:
+            assert torch.equal(one.forward(*x), alone.forward(*x))
+
+
 def test_norm_stages_instead_of_folded_norms(small_model):
     """``fold_norms=False`` keeps every RMSNorm as a stage of its own (normalised rows are quantised, plain weights):
     more stages, and agreement with the oracle emulating that arithmetic."""
