@@ -251,7 +251,8 @@ int create_token_embed(void** handle, const long long* tokens, const void* table
                        int row_base, int vocab, float scale, int workers);
 /* out[r, n] = f(sum_k x[r + x_row_offset, k] w[n, k]);  flags: 1 x is BF16, 2 out is BF16, 4 SiLU, 8 multiply by
  * rsqrt(mean(x^2)+eps), 16 Euler update out = prev + dt*value.  slot 0: x pointer, 2: launch state, 3: launch
- * noise; prev_slot 3: previous value is the launch noise. */
+ * noise; prev_slot 3: previous value is the launch noise.  In a program w is a constant, like the weights of a projection: it is
+ * read before the stage's sources are waited for. */
 int create_linear32(void** handle, const void* x, const float* w, const float* bias, const float* prev, void* out,
                     int rows, int n, int k, int ldx, int ldo, int flags, int slot, int prev_slot, int x_row_offset,
                     float dt, float eps, int workers);

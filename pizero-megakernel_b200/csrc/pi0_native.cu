@@ -294,6 +294,10 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
     if (e == cudaSuccess) e = cudaMemset(prog->d_counters, 0, sizeof(unsigned int) * std::max(counters, 1));
     if (e == cudaSuccess && counters) e = cudaMemcpy(prog->d_expected, prog->expected.data(), sizeof(unsigned int) * counters, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(prog->d_status, 0, sizeof(VmStatus));
+    // Copies from pageable memory may still be on their way when cudaMemcpy returns, and memsets are asynchronous, on a stream
+    // that the caller's may not be ordered behind.  The first launch reads the program before the kernel in front of it has
+    // finished (grid_dependency_wait), so all of it, and what the operators uploaded when they were created, has to be there now.
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e == cudaSuccess) {
         static bool configured[64] = {};
         if (device < 64 && !configured[device]) {

@@ -883,6 +883,31 @@ def test_launches_that_overlap_keep_the_order_of_the_stream(columns):
         assert all(op.status()["code"] == 0 for op in (s0, s1, norm))
 
 
+def test_first_launches_on_a_stream_of_their_own():
+    """Operators are created and launched at once on a stream that is not ordered behind the default one, behind running small
+    operators whose successors start early: the first launch finds its whole program in place."""
+    rng = np.random.default_rng(8)
+    rows = torch.randn(51, 1024, device="cuda").bfloat16()
+    pa = pack_nvfp4(rng.normal(size=(51, 256)).astype(np.float32), row_alignment=128)
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(512, 256)).astype(np.float32), scale_policy="ceil")
+    with ResidentNorm(None, rows, kind="rms", precision="fp4", workers=148, row_alignment=128) as front, ResidentNVFP4(None, pa, pb, workers=148, rows=51) as op:
+        front.forward()
+        want = op.forward().clone()
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        for _ in range(6):
+            with ResidentNorm(None, rows, kind="rms", precision="fp4", workers=148, row_alignment=128) as front, ResidentNVFP4(None, pa, pb, workers=148, rows=51) as op:
+                stream.synchronize()                                        # (the operands: torch fills them on its own streams)
+                torch.cuda.default_stream().synchronize()
+                front.forward()
+                for _ in range(20):
+                    front.forward()
+                got = op.forward().clone()
+                assert op.status()["code"] == 0 and front.status()["code"] == 0
+                assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("policy", [0, 1])
 def test_quantiser_passes_over_nans(policy):
     """The block scale is that of the block's numbers: a block of NaNs alone has scale zero and zero codes, and a NaN among
