@@ -49,9 +49,9 @@ WORKLOADS = {
     "cfg5": dict(views=3, prompt=16, chunk=63, steps=10, name="configs[4]: pi0 forward, 3 views, 16-token prompt, chunk 63, 10 Euler steps"),
 }
 # Algorithmic work of one forward (GEMM + attention FLOPs) and NVFP4 weight bytes read once.
-# dram_bytes: dram__bytes_read.sum + dram__bytes_write.sum of one launch from an ncu capture of this bench (3.52 GB read: the
+# dram_bytes: dram__bytes_read.sum + dram__bytes_write.sum of one launch from an ncu capture of this bench (3.50 GB read: the
 # 1.29 GB of vision/prefix weights once and the 0.17 GB of expert weights in each of the 10 Euler steps, plus scale atoms and
-# activations that had left L2; 1.02 GB written: activations and split-KV partials leaving the L2 behind the weight stream).
+# activations that had left L2; 1.00 GB written: activations and split-KV partials leaving the L2 behind the weight stream).
 # None: not captured.
 WORK = {"cfg4": dict(gflop=3997.0, weight_mb=1461.0, dram_bytes=4.50e9), "cfg5": dict(gflop=4136.0, weight_mb=1461.0, dram_bytes=None)}
 TRAFFIC_SOURCE = "constant from profiles/pi0_vm_kernel_bench_cfg4_launch_list.md (one ncu capture of this command), not measured in this run"
@@ -348,7 +348,7 @@ def run_engine(args, wl, rank, world):
     if rank == 0 and world == 1 and args.gpu_baselines:
         baselines, eager = gpu_baselines(torch, cfg, sd, wl, dev, args.gpu_baselines.split(","), args.steps)
         accuracy = {"action_nrmse_vs_bf16_eager": float((actions - eager).norm() / eager.norm()),
-                    "note": "random-init weights: W4A4 noise is amplified layer by layer; --precision bf16 gives 0.0023"}
+                    "note": "random-init weights: W4A4 noise is amplified layer by layer; --precision bf16 gives 0.0024"}
         torch.cuda.empty_cache()
     # ---- the replica-sweep shape (16-token prompt, chunk 63) on every rank
     replica = None

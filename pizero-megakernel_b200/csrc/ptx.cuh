@@ -256,7 +256,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-// 2^x; results below the normal range become zero
+// 2^x.  The results of exp2f bit for bit where they are normal numbers (compared for every FP32 x from -150 to 0); smaller ones become
+// zero.  Its callers have subtracted the maximum, so the largest weight is 1 and the loss of another is below 2^-126.
 __device__ __forceinline__ float exp2_fast(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
