@@ -133,6 +133,7 @@ struct Program {
     int workers = 0, length = 0;
     std::vector<StageDesc> stages;
     std::vector<unsigned int> expected;
+    void* d_memory = nullptr;          // one allocation: the five that follow
     StageDesc* d_stages = nullptr;
     int4* d_code = nullptr;
     unsigned int* d_counters = nullptr;
@@ -148,11 +149,7 @@ struct Program {
     unsigned long long budget_ns = 2000000000ull;
     int* h_debug = nullptr;            // host-mapped progress marks (enable_native_model_debug)
     ~Program() {
-        cudaFree(d_stages);
-        cudaFree(d_code);
-        cudaFree(d_counters);
-        cudaFree(d_expected);
-        cudaFree(d_status);
+        cudaFree(d_memory);
         cudaFree(d_timings);
         if (h_debug) cudaFreeHost(h_debug);
     }
@@ -280,23 +277,31 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
         if (polled > 32) return cudaErrorInvalidValue;     // one lane per polled counter
     }
 
-    cudaError_t e = cudaMalloc(&prog->d_stages, sizeof(StageDesc) * prog->stages.size());
-    if (e == cudaSuccess) e = cudaMalloc(&prog->d_code, sizeof(int4) * static_cast<size_t>(workers) * length);
-    if (e == cudaSuccess) e = cudaMalloc(&prog->d_counters, sizeof(unsigned int) * std::max(counters, 1));
-    if (e == cudaSuccess) e = cudaMalloc(&prog->d_expected, sizeof(unsigned int) * std::max(counters, 1));
-    if (e == cudaSuccess) e = cudaMalloc(&prog->d_status, sizeof(VmStatus));
+    // One allocation and one upload for the whole program, counters and status zero.
+    size_t bytes = 0;
+    auto place = [&](size_t n) { const size_t at = bytes; bytes += (n + 511) / 512 * 512; return at; };
+    const size_t stage_bytes = sizeof(StageDesc) * prog->stages.size(), code_bytes = sizeof(int4) * static_cast<size_t>(workers) * length;
+    const size_t at_stages = place(stage_bytes), at_code = place(code_bytes), at_counters = place(sizeof(unsigned int) * std::max(counters, 1));
+    const size_t at_expected = place(sizeof(unsigned int) * std::max(counters, 1)), at_status = place(sizeof(VmStatus));
+    cudaError_t e = cudaMalloc(&prog->d_memory, bytes);
     if (e == cudaSuccess) {
+        uint8_t* base = static_cast<uint8_t*>(prog->d_memory);
+        prog->d_stages = reinterpret_cast<StageDesc*>(base + at_stages);
+        prog->d_code = reinterpret_cast<int4*>(base + at_code);
+        prog->d_counters = reinterpret_cast<unsigned int*>(base + at_counters);
+        prog->d_expected = reinterpret_cast<unsigned int*>(base + at_expected);
+        prog->d_status = reinterpret_cast<VmStatus*>(base + at_status);
         for (auto& d : prog->stages)
             if (d.kind == OP_ATTN && d.aux_count) d.p.attn.tickets = prog->d_counters + d.aux_base;
-        e = cudaMemcpy(prog->d_stages, prog->stages.data(), sizeof(StageDesc) * prog->stages.size(), cudaMemcpyHostToDevice);
+        std::vector<uint8_t> image(bytes, 0);
+        memcpy(image.data() + at_stages, prog->stages.data(), stage_bytes);
+        memcpy(image.data() + at_code, code4.data(), code_bytes);
+        if (counters) memcpy(image.data() + at_expected, prog->expected.data(), sizeof(unsigned int) * counters);
+        e = cudaMemcpy(base, image.data(), bytes, cudaMemcpyHostToDevice);
     }
-    if (e == cudaSuccess) e = cudaMemcpy(prog->d_code, code4.data(), sizeof(int4) * static_cast<size_t>(workers) * length, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(prog->d_counters, 0, sizeof(unsigned int) * std::max(counters, 1));
-    if (e == cudaSuccess && counters) e = cudaMemcpy(prog->d_expected, prog->expected.data(), sizeof(unsigned int) * counters, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(prog->d_status, 0, sizeof(VmStatus));
-    // Copies from pageable memory may still be on their way when cudaMemcpy returns, and memsets are asynchronous, on a stream
-    // that the caller's may not be ordered behind.  The first launch reads the program before the kernel in front of it has
-    // finished (grid_dependency_wait), so all of it, and what the operators uploaded when they were created, has to be there now.
+    // A copy from pageable memory may still be on its way when cudaMemcpy returns, on a stream that the caller's may not be
+    // ordered behind.  The first launch reads the program before the kernel in front of it has finished
+    // (grid_dependency_wait), so all of it, and what the operators uploaded when they were created, has to be there now.
     if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e == cudaSuccess) {
         static bool configured[64] = {};
