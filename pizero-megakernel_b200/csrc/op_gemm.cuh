@@ -32,7 +32,7 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
                                               int stage_index, int first, int count, PipeState& ps, long long* stamp) {
     const GemmParams& g = st.p.gemm;
     const int lane = lane_id();
-    uint32_t slot = ps.prod_slot, bits = ps.prod_bits;
+    uint32_t slot = ps.slot, bits = ps.bits;
     const int k_groups = g.k_groups, n_tiles = g.n_tiles, block_n = g.block_n, b_tiled = g.b_tiled;
     const void* tmap = WEIGHTS ? g.tmap_b : g.tmap_a;
     const uint8_t* scales = WEIGHTS ? g.sfb : g.sfa;
@@ -43,16 +43,16 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
     const uint32_t off = WEIGHTS ? static_cast<uint32_t>(g.off_b) : 0u, off_sf = static_cast<uint32_t>(WEIGHTS ? g.off_sfb : g.off_sfa);
     const bool scaled = g.operands == GEMM_NVFP4;                    // scale atoms: 512 bytes per MMA group and operand
     const uint32_t geo = ring_key(g.slot_stride, g.ring_stages);
-    if (ps.prod_geo != geo) {
+    if (ps.geo != geo) {
         // Slots of the previous geometry overlap the new ones at other indices, or are more than the new ring has: every copy issued so far must have
         // been read by its MMAs before the first new copy lands (waits for the last release of each slot).
         int alive0 = 1;
-        if (lane == 0 && ps.prod_geo != 0)                           // (nothing to wait for in front of the first GEMM)
+        if (lane == 0 && ps.geo != 0)                           // (nothing to wait for in front of the first GEMM)
             for (int s = 0; s < kMaxStagesDense && alive0; ++s)
                 alive0 = mbar_wait(prog, ctl, &ctl->empty[s], ((bits >> s) & 1u) ^ 1u, stage_index) ? 1 : 0;
         alive0 = __shfl_sync(0xffffffffu, alive0, 0);
         if (!alive0) return;
-        ps.prod_geo = geo;
+        ps.geo = geo;
         slot = 0;
     }
     int current_band = -1;
@@ -95,8 +95,8 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
         alive = __shfl_sync(0xffffffffu, alive, 0);
         if (!alive) return;
     }
-    ps.prod_slot = slot;
-    ps.prod_bits = bits;
+    ps.slot = slot;
+    ps.bits = bits;
 }
 
 // Warp 1: one elected thread runs the whole loop - waits, scale copies, MMAs, commits - while the other lanes wait at the
@@ -126,8 +126,8 @@ __device__ __forceinline__ void gemm_mma(const VmProgram& prog, Ctl* ctl, uint8_
     constexpr uint64_t kOperandHi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
     constexpr uint64_t kScaleHi = (1ull << 16) | (8ull << 32) | (1ull << 46);
     const uint32_t geo = ring_key(g.slot_stride, g.ring_stages);
-    if (ps.mma_geo != geo) { ps.mma_geo = geo; ps.mma_slot = 0; }
-    uint32_t slot = uniform_u32(ps.mma_slot), bits = uniform_u32(ps.mma_bits), it = uniform_u32(ps.mma_it), tile_no = uniform_u32(ps.mma_tile);
+    if (ps.geo != geo) { ps.geo = geo; ps.slot = 0; }
+    uint32_t slot = uniform_u32(ps.slot), bits = uniform_u32(ps.bits), it = uniform_u32(ps.it), tile_no = uniform_u32(ps.tile);
     const bool leader = elect_one();
     if (leader) {
         bool landed = false, alive = true;                   // landed: the current slot was seen full by the look-ahead
@@ -193,10 +193,9 @@ __device__ __forceinline__ void gemm_mma(const VmProgram& prog, Ctl* ctl, uint8_
     }
     __syncwarp();
     const int from = __ffs(__ballot_sync(0xffffffffu, leader)) - 1;
-    ps.mma_slot = __shfl_sync(0xffffffffu, slot, from);
-    ps.mma_bits = __shfl_sync(0xffffffffu, bits, from);
-    ps.mma_it = __shfl_sync(0xffffffffu, it, from);
-    ps.mma_tile = __shfl_sync(0xffffffffu, tile_no, from);
+    ps.slot = __shfl_sync(0xffffffffu, slot, from);
+    ps.bits = __shfl_sync(0xffffffffu, bits, from);
+    ps.it = __shfl_sync(0xffffffffu, it, from);
     if (stamp && lane_id() == 0) stamp[5] = static_cast<long long>(global_ns());
 }
 
@@ -241,12 +240,49 @@ __device__ __forceinline__ uint4 quantize_32(const float2 (&v)[16], float inv_gs
     }
     return make_uint4(words[0], words[1], words[2], words[3]);
 }
+// What the drain of one accumulator row needs of the descriptor, in registers and with the row's offsets applied.  The
+// descriptor lies in shared memory, and every asm statement with a memory clobber makes the compiler read a field again: a dozen
+// dependent reads per chunk, from a shared memory that the MMAs keep busy (pi0 forward 9.22 -> 9.06 ms).
+// (Only the fields that an epilogue kind uses exist in its drain.)
+struct DrainRow {
+    uint8_t* out;                // the row of the output (BF16 rows: of the warp's first row, which the warp stores together)
+    const uint8_t* residual;     // the row of the residual, or null
+    const uint8_t* bias;         // BF16 [N] or null
+    const float* center;         // FP32 [N] or null
+    uint8_t* copy;               // EPI_STREAM: the row of the NVFP4 copy
+    uint8_t* scales;             // the row's place in the first scale atom of its row band
+    float inv_gs;
+    int ldo, rows_left;          // BF16 rows: elements per row, rows behind the warp's first one
+    int act, sums;
+};
+// Scale of block `block` of that row (scale_offset, split into a part per row and a part per block).
+__device__ __forceinline__ uint8_t* scale_at(const DrainRow& d, int block) { return d.scales + (block >> 2) * 512 + (block & 3); }
+template <int EPI>
+__device__ __forceinline__ DrainRow drain_row(const GemmParams& g, int row) {
+    DrainRow d = {};
+    const int lane = lane_id();
+    constexpr bool kWarpRows = EPI == EPI_BF16 || EPI == EPI_BF16_EXT;
+    const size_t width = EPI == EPI_F32 ? 4 : EPI == EPI_FP4 || EPI == EPI_GEGLU_FP4 ? 1 : 2;
+    d.ldo = g.ldo;
+    d.out = static_cast<uint8_t*>(g.out) + static_cast<size_t>(kWarpRows ? row - lane : row) * g.ldo * width;
+    d.rows_left = g.rows - (row - lane);
+    if (g.residual) d.residual = static_cast<const uint8_t*>(g.residual) + static_cast<size_t>(row) * g.ldr * 2;
+    d.bias = static_cast<const uint8_t*>(g.bias);
+    d.center = g.col_center;
+    d.inv_gs = g.out_inv_gs;
+    d.act = g.act;
+    d.sums = g.sum_out != nullptr;
+    if (EPI == EPI_STREAM) d.copy = g.copy_fp4 + static_cast<size_t>(row) * g.ld_copy;
+    if (EPI == EPI_STREAM || EPI == EPI_FP4 || EPI == EPI_GEGLU_FP4) d.scales = g.out_scales + scale_offset(row, 0, g.out_blocks);
+    return d;
+}
+
 // One 32-column chunk of one accumulator row (thread == row); `res` holds the residual of the chunk (BF16) if there is one.
 // (Instantiated per epilogue kind: each accumulator drain carries only its own arithmetic and registers.  Values are kept as
 // pairs: the packed FP32 operations shorten the straight-line code that a drain executes once.)
 // LEAN: without the options only the BF16 model uses (rounding before the residual, GELU on BF16 output) and without ReLU^2.
 template <int EPI, bool LEAN = false>
-__device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const uint32_t (&raw)[32], const uint4 (&res)[4], int row, int col0,
+__device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const DrainRow& d, const uint32_t (&raw)[32], const uint4 (&res)[4], int row, int col0,
                                                     bool row_ok, float row_scale, float row_shift, float2& sumsq, float2& sum) {
     float2 v[16];
 #pragma unroll
@@ -254,9 +290,9 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
     constexpr bool kWarpStore = EPI == EPI_BF16 || EPI == EPI_BF16_EXT;      // (the warp stores its rows together)
     if (!kWarpStore && !row_ok) return;
     if constexpr (EPI == EPI_BF16_EXT || EPI == EPI_FP4) {
-        if (g.col_center) {
+        if (d.center) {
             // folded LayerNorm: subtract the row mean's share, mean * rstd * (sum over K of weight row n)
-            const float4* c4 = reinterpret_cast<const float4*>(g.col_center + col0);
+            const float4* c4 = reinterpret_cast<const float4*>(d.center + col0);
             const float2 shift = make_float2(row_shift, row_shift);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -270,12 +306,12 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         // interleaved (gate, up) column pairs -> 16 outputs = one scale block
         float h[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) h[i] = gelu_sigmoid(v[i].x) * v[i].y * g.out_inv_gs;
+        for (int i = 0; i < 16; i++) h[i] = gelu_sigmoid(v[i].x) * v[i].y * d.inv_gs;
         uint32_t code;
         uint2 bytes = quantize_block16(h, 0, code);
         const int out_col = col0 >> 1;
-        *reinterpret_cast<uint2*>(static_cast<uint8_t*>(g.out) + static_cast<size_t>(row) * g.ldo + (out_col >> 1)) = bytes;
-        g.out_scales[scale_offset(row, out_col >> 4, g.out_blocks)] = static_cast<uint8_t>(code);
+        *reinterpret_cast<uint2*>(d.out + (out_col >> 1)) = bytes;
+        *scale_at(d, out_col >> 4) = static_cast<uint8_t>(code);
         return;
     }
     if constexpr (EPI == EPI_GEGLU_BF16) {
@@ -287,7 +323,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
             const float h1 = bf16_round(gelu_tanh(bf16_round(v[2 * i + 1].x))) * bf16_round(v[2 * i + 1].y);
             w[i] = pack_bf16x2(h0, h1);
         }
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo + (col0 >> 1));
+        uint4* dst = reinterpret_cast<uint4*>(d.out + col0);
         dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
         dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
         return;
@@ -295,22 +331,22 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
     // (residual first, bias second: the order of the reference epilogue, whose BF16 result the tests reproduce bit for bit -
     // but a projection that is rounded before the residual is added carries its bias by then)
     auto add_bias = [&]() {
-        const uint4* b = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(g.bias) + col0);
+        const uint4* b = reinterpret_cast<const uint4*>(d.bias + col0 * 2);
         const uint4 u[4] = {__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3)};
         add_bf16x32(v, u);
     };
-    const bool early_bias = !LEAN && EPI == EPI_BF16_EXT && g.bias && g.residual && g.round_before_residual;
+    const bool early_bias = !LEAN && EPI == EPI_BF16_EXT && d.bias && d.residual && g.round_before_residual;
     if (early_bias) add_bias();
-    if (g.residual) {
+    if (d.residual) {
         if (!LEAN && EPI == EPI_BF16_EXT && g.round_before_residual) {
 #pragma unroll
             for (int i = 0; i < 16; i++) v[i] = make_float2(bf16_round(v[i].x), bf16_round(v[i].y));
         }
         add_bf16x32(v, res);
     }
-    if (g.bias && !early_bias) add_bias();
+    if (d.bias && !early_bias) add_bias();
     if constexpr (EPI == EPI_F32) {
-        float4* dst = reinterpret_cast<float4*>(static_cast<float*>(g.out) + static_cast<size_t>(row) * g.ldo + col0);
+        float4* dst = reinterpret_cast<float4*>(d.out + static_cast<size_t>(col0) * 4);
 #pragma unroll
         for (int i = 0; i < 8; i++) dst[i] = make_float4(v[2 * i].x, v[2 * i].y, v[2 * i + 1].x, v[2 * i + 1].y);
         return;
@@ -320,7 +356,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) w[i] = pack_bf16x2(v[i].x, v[i].y);
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo + col0);
+        uint4* dst = reinterpret_cast<uint4*>(d.out + col0 * 2);
 #pragma unroll
         for (int i = 0; i < 4; i++) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
         // ... and, from the rounded values a norm stage would have read back, the NVFP4 copy and the sums (even and odd
@@ -330,13 +366,13 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
             v[i] = unpack_bf16x2(w[i]);
             sumsq = fma2(v[i], v[i], sumsq);
         }
-        if (g.sum_out) {
+        if (d.sums) {
 #pragma unroll
             for (int i = 0; i < 16; i++) sum = add2(sum, v[i]);
         }
         uint32_t codes;
-        *reinterpret_cast<uint4*>(g.copy_fp4 + static_cast<size_t>(row) * g.ld_copy + (col0 >> 1)) = quantize_32(v, g.out_inv_gs, codes);
-        *reinterpret_cast<uint16_t*>(g.out_scales + scale_offset(row, col0 >> 4, g.out_blocks)) = static_cast<uint16_t>(codes);
+        *reinterpret_cast<uint4*>(d.copy + (col0 >> 1)) = quantize_32(v, d.inv_gs, codes);
+        *reinterpret_cast<uint16_t*>(scale_at(d, col0 >> 4)) = static_cast<uint16_t>(codes);
         return;
     }
     if constexpr (EPI == EPI_BF16 || EPI == EPI_BF16_EXT) {
@@ -359,15 +395,14 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         const int lane = lane_id();
         int gap = 0;
         if (EPI == EPI_BF16_EXT && g.pad_from > 0) gap = (col0 + (lane & 3) * 8) / g.pad_from * (g.pad_to - g.pad_from);
-        const size_t ld = static_cast<size_t>(g.ldo) * 2;
-        store_rows64(static_cast<uint8_t*>(g.out) + static_cast<size_t>(row - lane) * ld + (col0 + gap) * 2, ld, g.rows - (row - lane), p);
+        store_rows64(d.out + (col0 + gap) * 2, static_cast<size_t>(d.ldo) * 2, d.rows_left, p);
         return;
     }
     if constexpr (EPI == EPI_FP4) {
-        if (g.act == 1) {
+        if (d.act == 1) {
 #pragma unroll
             for (int i = 0; i < 16; i++) v[i] = make_float2(gelu_sigmoid(v[i].x), gelu_sigmoid(v[i].y));
-        } else if (!LEAN && g.act == 3) {
+        } else if (!LEAN && d.act == 3) {
 #pragma unroll
             for (int i = 0; i < 16; i++) {
                 const float2 r = make_float2(fmaxf(v[i].x, 0.f), fmaxf(v[i].y, 0.f));
@@ -375,8 +410,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
             }
         }
         uint32_t codes;
-        *reinterpret_cast<uint4*>(static_cast<uint8_t*>(g.out) + static_cast<size_t>(row) * g.ldo + (col0 >> 1)) = quantize_32(v, g.out_inv_gs, codes);
-        *reinterpret_cast<uint16_t*>(g.out_scales + scale_offset(row, col0 >> 4, g.out_blocks)) = static_cast<uint16_t>(codes);
+        *reinterpret_cast<uint4*>(d.out + (col0 >> 1)) = quantize_32(v, d.inv_gs, codes);
+        *reinterpret_cast<uint16_t*>(scale_at(d, col0 >> 4)) = static_cast<uint16_t>(codes);
         return;
     }
     // EPI_QKV_ROPE: values are first rounded to BF16 (the projection output), then rotated.
@@ -425,7 +460,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const u
         __nv_bfloat16* dst;
         if (is_v) dst = static_cast<__nv_bfloat16*>(g.cache_v) + static_cast<size_t>(g.cache_base + row) * hd + in_head;
         else if (is_k) dst = static_cast<__nv_bfloat16*>(g.cache_k) + static_cast<size_t>(g.cache_base + row) * hd + in_head;
-        else dst = static_cast<__nv_bfloat16*>(g.out) + static_cast<size_t>(row) * g.ldo + col0;
+        else dst = reinterpret_cast<__nv_bfloat16*>(d.out) + col0;
         uint4* d4 = reinterpret_cast<uint4*>(dst);
 #pragma unroll
         for (int i = 0; i < 4; i++) d4[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
@@ -455,9 +490,11 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
     const int lane = lane_id();
     const int n_tiles = g.n_tiles, block_n = g.block_n, last = first + count - 1;
     int run = 0;                                         // tiles drained since the last publication
+    int known_band = -1;                                 // row band of the tile drained before
+    float row_scale = 1.f, row_shift = 0.f;
     for (int t = main ? first : last; t <= last; ++t) {
         const int m_tile = t / n_tiles, n_tile = t - m_tile * n_tiles;
-        const uint32_t use = ps.epi_tile + static_cast<uint32_t>(t - first);
+        const uint32_t use = ps.tile + static_cast<uint32_t>(t - first);
         const uint32_t buf = use & 1u, phase = (use >> 1) & 1u;
         const int row = m_tile * 128 + quarter * 32 + lane;
         const bool row_ok = row < g.rows;
@@ -477,6 +514,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         }
         if ((EPI == EPI_BF16_EXT || EPI == EPI_FP4) && g.col_center && lane < (block_n >> 5))
             prefetch_l1(g.col_center + n_tile * block_n + lane * 32);    // constant data: close by when the accumulator is ready
+        const DrainRow d = drain_row<EPI>(g, row);
         // A single-tile instruction that reads row statistics (the few-row projections behind a folded norm, whose epilogue
         // is serial time) or a residual: once the copy warp has seen the sources complete, the statistics are read and the
         // row factor computed, and the first residual chunk is requested, while the operands are still on their way instead
@@ -484,11 +522,11 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         // (compiled into the drains of the projections that stand behind a folded norm in the model; the others read their
         // statistics, if they are given any, once the accumulator is ready)
         constexpr bool kEarly = EPI == EPI_QKV_ROPE || EPI == EPI_GEGLU_FP4 || EPI == EPI_FP4 || EPI == EPI_BF16_EXT;
-        const bool early = count == 1 && ((kEarly && (g.row_sumsq != nullptr || g.row_factor != nullptr)) || (kResidual && g.residual != nullptr));
+        const bool early = count == 1 && ((kEarly && (g.row_sumsq != nullptr || g.row_factor != nullptr)) || (kResidual && d.residual != nullptr));
         uint4 res[4] = {};
         auto load_residual = [&](int c) {
-            if (kResidual && g.residual && row_ok) {
-                const uint4* r = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(g.residual) + static_cast<size_t>(row) * g.ldr + n_tile * block_n + c);
+            if (kResidual && d.residual && row_ok) {
+                const uint4* r = reinterpret_cast<const uint4*>(d.residual + (n_tile * block_n + c) * 2);
 #pragma unroll
                 for (int i = 0; i < 4; i++) res[i] = __ldcg(r + i);
             }
@@ -509,9 +547,12 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         // alpha, times the row's 1/rms where the projection reads un-normalised rows (norm weight folded into B): given
         // as a factor, or as the producer's per-tile sums of squares (complete: the operands behind this accumulator
         // were only copied after the producer stage had finished)
-        float row_scale = g.alpha, row_shift = 0.f;
-        if (kStats && main && row_ok && g.row_factor) row_scale *= __ldcg(g.row_factor + row);
-        if (kStats && main && row_ok && g.row_sumsq) {
+        // (once per row band: a worker's next tiles are mostly of the same one, and the statistics are a round trip to L2)
+        const bool factors = m_tile != known_band;
+        known_band = m_tile;
+        if (factors) { row_scale = g.alpha; row_shift = 0.f; }
+        if (kStats && factors && main && row_ok && g.row_factor) row_scale *= __ldcg(g.row_factor + row);
+        if (kStats && factors && main && row_ok && g.row_sumsq) {
             const float4* part = reinterpret_cast<const float4*>(g.row_sumsq + static_cast<size_t>(row) * g.sumsq_parts);
             const int quads = g.sumsq_parts >> 2;
             float total = 0.f;
@@ -590,7 +631,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
                     sum_half = sum.x + sum.y;
                     sumsq = sum = make_float2(0.f, 0.f);
                 }
-                gemm_epilogue_chunk<EPI, LEAN>(g, raw, res, row, n_tile * block_n + c, row_ok, row_scale, row_shift, sumsq, sum);
+                gemm_epilogue_chunk<EPI, LEAN>(g, d, raw, res, row, n_tile * block_n + c, row_ok, row_scale, row_shift, sumsq, sum);
                 if (c + 32 < col_end) load_residual(c + 32);
             }
         }
@@ -621,12 +662,12 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         if (stamp && t == last && threadIdx.x == 128) stamp[7] = static_cast<long long>(global_ns());
         fence_proxy_async_global();
         __syncwarp();
-        if (lane == 0 && join_parts(&ctl->tile_parts[shared_tile ? 4u + (ps.gemm_seq & 3u) : ps.epi_run & 3u], share))
+        if (lane == 0 && join_parts(&ctl->tile_parts[shared_tile ? 4u + (ps.gemm_seq & 3u) : ps.run & 3u], share))
             publish_tile(prog, st, t, static_cast<unsigned int>(main ? run : min(count, t - m_tile * n_tiles + 1)));
         run = 0;
-        if (!shared_tile) ps.epi_run++;
+        if (!shared_tile) ps.run++;
     }
-    ps.epi_tile += static_cast<uint32_t>(count);
+    ps.tile += static_cast<uint32_t>(count);
 }
 
 // Dispatch of one GEMM instruction onto the warp roles (warp 2 has none); behind its role every warp goes through the

@@ -64,17 +64,17 @@ struct Ctl {
 static_assert(kRing <= 4, "words kept per GEMM instruction modulo 4");
 static_assert(sizeof(Ctl) <= kCtlBytes, "control block too large");
 
-// The ring geometry (slot count and size) belongs to the GEMM, so positions are kept per barrier: bit s of
-// prod_bits / mma_bits is the parity of the fills / drains slot s has seen. Producers and MMA lane walk the same slot
+// The ring geometry (slot count and size) belongs to the GEMM, so positions are kept per barrier: bit s of `bits` is the parity of
+// the fills (copy warps) or drains (MMA warp) slot s has seen. Producers and MMA lane walk the same slot
 // sequence: the cursor continues from one instruction to the next and restarts at 0 when the geometry changes (ring_key:
 // size or count).
+// Live across every operator, so each warp keeps no more than its own role needs: the copy warps and the MMA warp use the same
+// three cursor words.
 struct PipeState {
-    uint32_t prod_slot = 0, prod_bits = 0, prod_geo = 0;     // TMA lanes (each copy warp its own)
-    uint32_t mma_slot = 0, mma_bits = 0, mma_geo = 0;        // MMA lane
-    uint32_t mma_it = 0;         // K stages consumed by the MMA lane (rotates the scale columns in tensor memory)
-    uint32_t mma_tile = 0;       // accumulator tiles produced
-    uint32_t epi_tile = 0;       // accumulator tiles drained
-    uint32_t epi_run = 0;        // runs of tiles published by the draining warps alone
+    uint32_t slot = 0, bits = 0, geo = 0;                    // ring cursor of this warp's role
+    uint32_t it = 0;             // K stages consumed by the MMA lane (rotates the scale columns in tensor memory)
+    uint32_t tile = 0;           // accumulator tiles of the GEMM instructions so far (every warp counts them)
+    uint32_t run = 0;            // runs of tiles published by the draining warps alone
     uint32_t gemm_seq = 0;       // GEMM instructions this warp has been through (every warp counts them)
 };
 

@@ -289,6 +289,33 @@ def test_residual_stream_epilogue_and_row_rms_consumer():
                 assert lib.configure_resident_fp4_row_rms(consumer.handle, sumsq.data_ptr(), 6, n, 1e-6) == 1
 
 
+@pytest.mark.parametrize("rows,block_n", [(384, 128), (321, 64), (129, 128)])
+def test_row_factors_over_runs_of_tiles(rows, block_n):
+    """A worker keeps the row factors of a row band over its tiles of that band: runs within a band, over the end of one and
+    over several bands give the bits of one tile per worker, and those are the raw product times rsqrt(mean square + eps)."""
+    lib = _native.load()
+    rng = np.random.default_rng(rows + block_n)
+    m, k, n, parts = 128 * -(-rows // 128), 512, 512, 8
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    sumsq = torch.from_numpy(rng.uniform(0.5, 200.0, size=(m, parts)).astype(np.float32)).cuda()
+    factor = torch.rsqrt(sumsq.double().sum(-1, keepdim=True) / k + 1e-6)
+    for kind in (dict(output_dtype=torch.float32), dict(output_dtype=torch.uint8, output_gelu=True), dict(output_dtype=torch.uint8, output_geglu=True)):
+        outs = []
+        for workers in (148, 4, 2, 1):
+            with ResidentNVFP4(None, pa, pb, workers=workers, rows=rows, block_n=block_n, **kind) as op:
+                raw = op.forward().clone()
+                _native.check(lib.configure_resident_fp4_row_rms(op.handle, sumsq.data_ptr(), parts, k, 1e-6), "row rms")
+                y = op.forward().clone()
+                assert op.status()["code"] == 0
+                outs.append((y, op.output_scales.clone() if y.dtype == torch.uint8 else None))
+                if y.dtype == torch.float32:            # (a sum of 8, a root and two products, each rounded: below 16 units of 2^-24)
+                    want = (raw.double() * factor)[:rows]
+                    assert bool(((y[:rows].double() - want).abs() <= 2.0 ** -20 * want.abs()).all())
+        for y, sc in outs[1:]:
+            assert torch.equal(y, outs[0][0]) and (sc is None or torch.equal(sc, outs[0][1]))
+
+
 def test_folded_layernorm_between_two_projections():
     """LayerNorm folded into the projection that follows: the producer leaves per-tile sums and sums of squares (row
     stride padded to a multiple of 4 slots), the consumer - weight columns times gamma, bias + W beta - turns its
