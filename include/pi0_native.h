@@ -47,6 +47,9 @@ int destroy_resident_fp4(void* handle);
  * Replaces the BF16 path's configure_dense_qkv_rope (native_pi0/dense.cu:231-253). */
 int configure_resident_fp4_qkv_rope(void* handle, void* out_q, int ldq, const void* cos, const void* sin, void* cache_k,
                                     void* cache_v, int q_cols, int head_dim, int cache_base);
+/* extension: the same rotary tables in pair-major order, BF16 entry [head_dim / 2][ld][4] = cos(i), cos(i + head_dim/2), sin(i),
+ * sin(i + head_dim/2) of a row; ld a multiple of 128 that covers the row bands.  Call it behind configure_*_qkv_rope. */
+int configure_qkv_rope_table(void* handle, const void* table, int ld);
 /* extension: residual-stream epilogue.  out BF16 [M, N] = alpha*acc + residual + bias as configure_resident_fp4_bf16;
  * the rounded rows are also quantised, un-normalised, to NVFP4 (copy_fp4 packed [M, N/2], copy_scales swizzled with
  * N/16 blocks per row, tensor scale copy_global_scale), and sumsq FP32 [M, N / tile width] receives, per output tile,

@@ -253,8 +253,8 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
     constexpr int SHARE = HDP / PARTS;
     const int col_begin = part * SHARE;
     if (TWICE || (!(LEAN && HDP == 128) && a.splits > 1)) {
-        const size_t ld = static_cast<size_t>(a.head_dim) * 2;
-        uint8_t* po = reinterpret_cast<uint8_t*>(a.partial_o) + (static_cast<size_t>(tile) * kAttnQRows + (row - lane)) * ld;
+        const int ld = a.head_dim * 2;
+        uint8_t* po = reinterpret_cast<uint8_t*>(a.partial_o) + (static_cast<size_t>(tile) * kAttnQRows + row) * ld;
         if (warp_rows > 0) {
             for (int c0 = col_begin; c0 < col_begin + SHARE; c0 += 32) {
                 uint32_t raw[32];

@@ -245,15 +245,17 @@ __device__ __forceinline__ uint4 quantize_32(const float2 (&v)[16], float inv_gs
 // dependent reads per chunk, from a shared memory that the MMAs keep busy (pi0 forward 9.22 -> 9.06 ms).
 // (Only the fields that an epilogue kind uses exist in its drain.)
 struct DrainRow {
-    uint8_t* out;                // the row of the output (BF16 rows: of the warp's first row, which the warp stores together)
+    uint8_t* out;                // the row of the output
     const uint8_t* residual;     // the row of the residual, or null
     const uint8_t* bias;         // BF16 [N] or null
     const float* center;         // FP32 [N] or null
     uint8_t* copy;               // EPI_STREAM: the row of the NVFP4 copy
     uint8_t* scales;             // the row's place in the first scale atom of its row band
     float inv_gs;
-    int ldo, rows_left;          // BF16 rows: elements per row, rows behind the warp's first one
+    int ldo;                     // BF16 rows: bytes from one row of the output to the next
+    int rows_left;               // rows from the warp's first one on
     int act, sums;
+    bool together;               // EPI_QKV_ROPE: the warp stores its rows together (store_rows64)
 };
 // Scale of block `block` of that row (scale_offset, split into a part per row and a part per block).
 __device__ __forceinline__ uint8_t* scale_at(const DrainRow& d, int block) { return d.scales + (block >> 2) * 512 + (block & 3); }
@@ -261,10 +263,9 @@ template <int EPI>
 __device__ __forceinline__ DrainRow drain_row(const GemmParams& g, int row) {
     DrainRow d = {};
     const int lane = lane_id();
-    constexpr bool kWarpRows = EPI == EPI_BF16 || EPI == EPI_BF16_EXT;
     const size_t width = EPI == EPI_F32 ? 4 : EPI == EPI_FP4 || EPI == EPI_GEGLU_FP4 ? 1 : 2;
-    d.ldo = g.ldo;
-    d.out = static_cast<uint8_t*>(g.out) + static_cast<size_t>(kWarpRows ? row - lane : row) * g.ldo * width;
+    d.ldo = g.ldo * 2;
+    d.out = static_cast<uint8_t*>(g.out) + static_cast<size_t>(row) * g.ldo * width;
     d.rows_left = g.rows - (row - lane);
     if (g.residual) d.residual = static_cast<const uint8_t*>(g.residual) + static_cast<size_t>(row) * g.ldr * 2;
     d.bias = static_cast<const uint8_t*>(g.bias);
@@ -272,6 +273,10 @@ __device__ __forceinline__ DrainRow drain_row(const GemmParams& g, int row) {
     d.inv_gs = g.out_inv_gs;
     d.act = g.act;
     d.sums = g.sum_out != nullptr;
+    // Row by row a store touches 32 lines, and the load / store unit takes one line a cycle: with eight warps at work (several row
+    // bands) a Q | K | V drain waits for it; few rows keep two to four warps busy, and there the transposition only lengthens the
+    // chain of a thread.  With the pair-major table below, q|k|v of the 768-row prefix 12.1 -> 9.4 us.
+    d.together = g.rows > 128;
     if (EPI == EPI_STREAM) d.copy = g.copy_fp4 + static_cast<size_t>(row) * g.ld_copy;
     if (EPI == EPI_STREAM || EPI == EPI_FP4 || EPI == EPI_GEGLU_FP4) d.scales = g.out_scales + scale_offset(row, 0, g.out_blocks);
     return d;
@@ -287,8 +292,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
     float2 v[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = mul2(make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1])), make_float2(row_scale, row_scale));
-    constexpr bool kWarpStore = EPI == EPI_BF16 || EPI == EPI_BF16_EXT;      // (the warp stores its rows together)
-    if (!kWarpStore && !row_ok) return;
+    constexpr bool kWarpStore = EPI == EPI_BF16 || EPI == EPI_BF16_EXT;      // (rows stored together take the whole warp)
+    if (!kWarpStore && !row_ok && !(EPI == EPI_QKV_ROPE && d.together)) return;
     if constexpr (EPI == EPI_BF16_EXT || EPI == EPI_FP4) {
         if (d.center) {
             // folded LayerNorm: subtract the row mean's share, mean * rstd * (sum over K of weight row n)
@@ -395,7 +400,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
         const int lane = lane_id();
         int gap = 0;
         if (EPI == EPI_BF16_EXT && g.pad_from > 0) gap = (col0 + (lane & 3) * 8) / g.pad_from * (g.pad_to - g.pad_from);
-        store_rows64(d.out + (col0 + gap) * 2, static_cast<size_t>(d.ldo) * 2, d.rows_left, p);
+        store_rows64(d.out + (col0 + gap) * 2, d.ldo, d.rows_left, p);
         return;
     }
     if constexpr (EPI == EPI_FP4) {
@@ -425,45 +430,69 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
 #pragma unroll
         for (int i = 0; i < 16; i++) packed[i] = pack_bf16x2(v[i].x, v[i].y);
         if (!is_v) {
-            // Q and K heads are stored pair-interleaved: column 2i holds original dim i, column 2i+1 holds dim i+hd/2.
-            const __nv_bfloat16* cs = static_cast<const __nv_bfloat16*>(g.rope_cos) + static_cast<size_t>(row) * hd;
-            const __nv_bfloat16* sn = static_cast<const __nv_bfloat16*>(g.rope_sin) + static_cast<size_t>(row) * hd;
-            // the 16 pairs of this chunk use table entries [dim0, dim0+16) and [dim0+half, dim0+half+16): 8 vector loads
+            // Q and K heads are stored pair-interleaved: column 2i holds original dim i, column 2i+1 holds dim i+hd/2; the 16 pairs
+            // of this chunk use table entries [dim0, dim0+16) and [dim0+half, dim0+half+16).
             const int dim0 = in_head >> 1;
-            uint32_t tc[2][8], ts[2][8];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const uint4* pc = reinterpret_cast<const uint4*>(cs + dim0 + h * half);
-                const uint4* ps = reinterpret_cast<const uint4*>(sn + dim0 + h * half);
-                const uint4 c0 = __ldg(pc), c1 = __ldg(pc + 1), s0 = __ldg(ps), s1 = __ldg(ps + 1);
-                tc[h][0] = c0.x; tc[h][1] = c0.y; tc[h][2] = c0.z; tc[h][3] = c0.w;
-                tc[h][4] = c1.x; tc[h][5] = c1.y; tc[h][6] = c1.z; tc[h][7] = c1.w;
-                ts[h][0] = s0.x; ts[h][1] = s0.y; ts[h][2] = s0.z; ts[h][3] = s0.w;
-                ts[h][4] = s1.x; ts[h][5] = s1.y; ts[h][6] = s1.z; ts[h][7] = s1.w;
-            }
             // Packed BF16 arithmetic, two lanes = the two members of a rotation pair: with X = (x1, x2), C = (c1, c2),
             // S = (s1, s2) and X' = (-x2, x1) the rotated pair is  bf16(X * C) + bf16(X' * S)  lane by lane - every
             // product rounded to BF16 before the sum, as the reference's rotate-half does.
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;          // high or low halves of the two table words
-                const uint32_t cw = __byte_perm(tc[0][i >> 1], tc[1][i >> 1], sel);
-                const uint32_t sw = __byte_perm(ts[0][i >> 1], ts[1][i >> 1], sel);
-                const uint32_t xw = packed[i];                             // (x1, x2) rounded to BF16
+            auto rotate = [](uint32_t xw, uint32_t cw, uint32_t sw) {      // xw: (x1, x2) rounded to BF16
                 const uint32_t xr = __byte_perm(xw, xw, 0x1032u) ^ 0x00008000u;   // (-x2, x1)
                 const __nv_bfloat162 p = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&xw), *reinterpret_cast<const __nv_bfloat162*>(&cw));
                 const __nv_bfloat162 q = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&xr), *reinterpret_cast<const __nv_bfloat162*>(&sw));
                 const __nv_bfloat162 o = __hadd2_rn(p, q);                  // (_rn: never contracted into a fused multiply-add)
-                packed[i] = *reinterpret_cast<const uint32_t*>(&o);
+                return *reinterpret_cast<const uint32_t*>(&o);
+            };
+            if (LEAN || g.rope_table) {
+                // the lanes' rows of one pair are adjacent: two lines per load (row by row the eight loads of the two tables take 32
+                // lines each, a quarter of the time of a prefix tile)
+                const uint2* t = g.rope_table + static_cast<size_t>(dim0) * g.rope_ld + row;
+                const int ld = g.rope_ld;
+                uint2 cs[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) cs[i] = __ldg(t + static_cast<size_t>(i) * ld);
+#pragma unroll
+                for (int i = 0; i < 16; i++) packed[i] = rotate(packed[i], cs[i].x, cs[i].y);
+            } else if constexpr (!LEAN) {
+                if (row_ok) {
+                    const __nv_bfloat16* cs = static_cast<const __nv_bfloat16*>(g.rope_cos) + static_cast<size_t>(row) * hd;
+                    const __nv_bfloat16* sn = static_cast<const __nv_bfloat16*>(g.rope_sin) + static_cast<size_t>(row) * hd;
+                    uint32_t tc[2][8], ts[2][8];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint4* pc = reinterpret_cast<const uint4*>(cs + dim0 + h * half);
+                        const uint4* ps = reinterpret_cast<const uint4*>(sn + dim0 + h * half);
+                        const uint4 c0 = __ldg(pc), c1 = __ldg(pc + 1), s0 = __ldg(ps), s1 = __ldg(ps + 1);
+                        tc[h][0] = c0.x; tc[h][1] = c0.y; tc[h][2] = c0.z; tc[h][3] = c0.w;
+                        tc[h][4] = c1.x; tc[h][5] = c1.y; tc[h][6] = c1.z; tc[h][7] = c1.w;
+                        ts[h][0] = s0.x; ts[h][1] = s0.y; ts[h][2] = s0.z; ts[h][3] = s0.w;
+                        ts[h][4] = s1.x; ts[h][5] = s1.y; ts[h][6] = s1.z; ts[h][7] = s1.w;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;      // high or low halves of the two table words
+                        packed[i] = rotate(packed[i], __byte_perm(tc[0][i >> 1], tc[1][i >> 1], sel), __byte_perm(ts[0][i >> 1], ts[1][i >> 1], sel));
+                    }
+                }
             }
         }
-        __nv_bfloat16* dst;
-        if (is_v) dst = static_cast<__nv_bfloat16*>(g.cache_v) + static_cast<size_t>(g.cache_base + row) * hd + in_head;
-        else if (is_k) dst = static_cast<__nv_bfloat16*>(g.cache_k) + static_cast<size_t>(g.cache_base + row) * hd + in_head;
-        else dst = reinterpret_cast<__nv_bfloat16*>(d.out) + col0;
-        uint4* d4 = reinterpret_cast<uint4*>(dst);
+        uint8_t* dst;
+        int ld = hd * 2;
+        if (is_v) dst = static_cast<uint8_t*>(g.cache_v) + (static_cast<size_t>(g.cache_base + row) * hd + in_head) * 2;
+        else if (is_k) dst = static_cast<uint8_t*>(g.cache_k) + (static_cast<size_t>(g.cache_base + row) * hd + in_head) * 2;
+        else {
+            dst = d.out + col0 * 2;
+            ld = d.ldo;
+        }
+        uint4 p[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) d4[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+        for (int i = 0; i < 4; i++) p[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+        if (d.together) {
+            store_rows64(dst, ld, d.rows_left, p);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) reinterpret_cast<uint4*>(dst)[i] = p[i];
+        }
     }
 }
 
@@ -502,14 +531,18 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         const bool shared_tile = t == last && block_n >= 64, helped = shared_tile && rows_here;
         if (!main && !helped) break;
         const int col_begin = main ? 0 : block_n >> 1, col_end = main && helped ? block_n >> 1 : block_n;
-        if (EPI == EPI_QKV_ROPE && row_ok) {
-            // while the MMAs run: bring this row's rotary table entries (constant data) close
+        if (EPI == EPI_QKV_ROPE && rows_here) {
+            // while the MMAs run: bring the first chunk's rotary table entries (constant data) close
             const int hd = g.head_dim, col_a = n_tile * block_n + col_begin;
             if (col_a < g.q_cols + hd) {                                   // a Q or K tile
                 const int in_head = col_a >= g.q_cols ? col_a - g.q_cols : col_a % hd;
-                const __nv_bfloat16* cs = static_cast<const __nv_bfloat16*>(g.rope_cos) + static_cast<size_t>(row) * hd + (in_head >> 1);
-                const __nv_bfloat16* sn = static_cast<const __nv_bfloat16*>(g.rope_sin) + static_cast<size_t>(row) * hd + (in_head >> 1);
-                prefetch_l1(cs); prefetch_l1(cs + (hd >> 1)); prefetch_l1(sn); prefetch_l1(sn + (hd >> 1));
+                if (LEAN || g.rope_table) {
+                    prefetch_l1(g.rope_table + static_cast<size_t>((in_head >> 1) + (lane >> 1)) * g.rope_ld + row - lane + (lane & 1) * 16);
+                } else if (!LEAN && row_ok) {
+                    const __nv_bfloat16* cs = static_cast<const __nv_bfloat16*>(g.rope_cos) + static_cast<size_t>(row) * hd + (in_head >> 1);
+                    const __nv_bfloat16* sn = static_cast<const __nv_bfloat16*>(g.rope_sin) + static_cast<size_t>(row) * hd + (in_head >> 1);
+                    prefetch_l1(cs); prefetch_l1(cs + (hd >> 1)); prefetch_l1(sn); prefetch_l1(sn + (hd >> 1));
+                }
             }
         }
         if ((EPI == EPI_BF16_EXT || EPI == EPI_FP4) && g.col_center && lane < (block_n >> 5))
@@ -621,6 +654,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
             columns_read();
         } else {
             if (!early) load_residual(col_begin);
+#pragma unroll 1
             for (int c = col_begin; c < col_end; c += 32) {
                 uint32_t raw[32];
                 tmem_ld32(taddr + c, raw);

@@ -197,6 +197,7 @@ bool lean_stage(const StageDesc& d) {
         const bool stats = g.row_sumsq || g.row_factor;     // (the lean residual-stream and plain BF16 drains read none)
         if (stats && (g.epilogue == EPI_BF16 || g.epilogue == EPI_STREAM)) return false;
         if (g.round_before_residual || g.gelu_cols > 0 || g.act == 3) return false;       // options the lean drains leave out
+        if (g.epilogue == EPI_QKV_ROPE && !g.rope_table) return false;      // (the lean rotary drain reads the pair-major table only)
         return g.operands == GEMM_NVFP4 && (g.epilogue == EPI_BF16 || g.epilogue == EPI_STREAM || g.epilogue == EPI_GEGLU_FP4 ||
                                             g.epilogue == EPI_FP4 || g.epilogue == EPI_QKV_ROPE || g.epilogue == EPI_BF16_EXT);
     }
@@ -631,9 +632,21 @@ extern "C" int configure_resident_fp4_qkv_rope(void* handle, void* out_q, int ld
     g.epilogue = EPI_QKV_ROPE;
     g.bias = nullptr; g.residual = nullptr;
     g.out = out_q; g.ldo = ldq;
-    g.rope_cos = cos; g.rope_sin = sin;
+    g.rope_cos = cos; g.rope_sin = sin; g.rope_table = nullptr;
     g.cache_k = cache_k; g.cache_v = cache_v;
     g.q_cols = q_cols; g.head_dim = head_dim; g.cache_base = cache_base;
+    op->solo_dirty = true;
+    return cudaSuccess;
+}
+// extension: the rotary tables of configure_*_qkv_rope in pair-major order, which a drain reads with adjacent lanes: entry [i][row] is
+// cos[row, i], cos[row, i + head_dim/2], sin[row, i], sin[row, i + head_dim/2] in BF16 (8 bytes), `ld` rows per pair, a multiple of 128
+// that covers the operand's row bands.  Replaces the two tables as the source; to be called behind configure_*_qkv_rope.
+extern "C" int configure_qkv_rope_table(void* handle, const void* table, int ld) {
+    Op* op = as_op(handle);
+    if (!op || op->desc.kind != OP_GEMM || op->desc.p.gemm.epilogue != EPI_QKV_ROPE || !table || ld % 128 || ld < op->m || !aligned16(table))
+        return cudaErrorInvalidValue;
+    op->desc.p.gemm.rope_table = static_cast<const uint2*>(table);
+    op->desc.p.gemm.rope_ld = ld;
     op->solo_dirty = true;
     return cudaSuccess;
 }
@@ -854,7 +867,7 @@ extern "C" int configure_dense_qkv_rope(void* handle, const void* cos, const voi
     if (g.epilogue != EPI_BF16 || g.bias || g.residual || logical_rows > op->m || key_offset + 512 != op->n)
         return cudaErrorInvalidValue;
     g.epilogue = EPI_QKV_ROPE;
-    g.rope_cos = cos; g.rope_sin = sin;
+    g.rope_cos = cos; g.rope_sin = sin; g.rope_table = nullptr;
     g.cache_k = cache_k; g.cache_v = cache_v;
     g.q_cols = key_offset; g.head_dim = 256; g.cache_base = cache_base;
     g.rows = std::min(g.rows, logical_rows);

@@ -184,29 +184,33 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // unit takes one line a cycle (128 x 128 BF16 tiles: 1 us of 3.1 per tile).  Transposed, four lanes cover one row's 64
 // bytes and an instruction eight rows.
 __device__ __forceinline__ void quad_transpose(uint4 (&p)[4]) {
+    const bool odd = (lane_id() & 1) != 0, high = (lane_id() & 2) != 0;
 #pragma unroll
-    for (int bit = 1; bit <= 2; bit <<= 1) {
-        const bool upper = (lane_id() & bit) != 0;
+    for (int w = 0; w < 4; w++) {
+        uint32_t a[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            if (i & bit) continue;
-            uint4 &lo = p[i], &hi = p[i + bit];
-            const uint4 send = upper ? lo : hi;
-            const uint4 got = make_uint4(__shfl_xor_sync(0xffffffffu, send.x, bit), __shfl_xor_sync(0xffffffffu, send.y, bit),
-                                         __shfl_xor_sync(0xffffffffu, send.z, bit), __shfl_xor_sync(0xffffffffu, send.w, bit));
-            if (upper) lo = got;
-            else hi = got;
+        for (int i = 0; i < 4; i++) a[i] = w == 0 ? p[i].x : w == 1 ? p[i].y : w == 2 ? p[i].z : p[i].w;
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? a[i] : a[i + 1], 1);
+            if (odd) a[i] = got; else a[i + 1] = got;
         }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? a[i] : a[i + 2], 2);
+            if (high) a[i] = got; else a[i + 2] = got;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) (w == 0 ? p[i].x : w == 1 ? p[i].y : w == 2 ? p[i].z : p[i].w) = a[i];
     }
 }
-// Whole warp: lane r holds 64 bytes of row r (r < rows) -> rows at `base` + r * ld bytes.
-__device__ __forceinline__ void store_rows64(uint8_t* base, size_t ld, int rows, uint4 (&p)[4]) {
+// Whole warp: lane r holds 64 bytes of row r (r < rows), `own` is where they belong, rows are `ld` bytes apart.
+__device__ __forceinline__ void store_rows64(uint8_t* own, int ld, int rows, uint4 (&p)[4]) {
     quad_transpose(p);
-    const int lane = lane_id(), row0 = lane & ~3;
-    uint8_t* dst = base + static_cast<size_t>(row0) * ld + (lane & 3) * 16;
+    const int lane = lane_id(), mine = lane & 3;
 #pragma unroll
     for (int k = 0; k < 4; k++)
-        if (row0 + k < rows) *reinterpret_cast<uint4*>(dst + k * ld) = p[k];
+        if (lane - mine + k < rows) *reinterpret_cast<uint4*>(own + static_cast<ptrdiff_t>(k - mine) * ld + mine * 16) = p[k];
 }
 
 // ---------------------------------------------------------------- counters

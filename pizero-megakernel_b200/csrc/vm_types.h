@@ -100,6 +100,8 @@ struct GemmParams {
     // EPI_QKV_ROPE
     const void* rope_cos;        // BF16 [rows, head_dim]
     const void* rope_sin;
+    const uint2* rope_table;     // both tables pair by pair, or null: entry [i][row] = cos(i), cos(i + hd/2) | sin(i), sin(i + hd/2), BF16
+    int rope_ld;                 // rows of one pair (whole row bands)
     void* cache_k;               // BF16 [cache_rows, head_dim]
     void* cache_v;
     int q_cols;                  // heads * head_dim (0 when the projection has no Q part)

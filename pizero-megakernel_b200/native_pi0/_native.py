@@ -52,6 +52,7 @@ _SIGNATURES = {
     "configure_resident_fp4_bf16": [_P] * 4,
     "configure_resident_fp4_quantized": [_P] * 5 + [_F, _I],
     "configure_resident_fp4_qkv_rope": [_P, _P, _I, _P, _P, _P, _P, _I, _I, _I],
+    "configure_qkv_rope_table": [_P, _P, _I],
     "configure_resident_fp4_stream": [_P] * 6 + [_F, _P],
     "configure_resident_fp4_row_rms": [_P, _P, _I, _I, _F],
     "configure_resident_fp4_stream_sums": [_P, _P, _I],

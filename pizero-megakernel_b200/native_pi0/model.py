@@ -350,6 +350,7 @@ class NativePi0:
             _native.check(self.lib.configure_resident_fp4_qkv_rope(
                 h, _native.ptr(q), 0 if q is None else q.stride(0), rope["cos"].data_ptr(), rope["sin"].data_ptr(),
                 rope["cache_k"].data_ptr(), rope["cache_v"].data_ptr(), rope["q_cols"], self.config.head_dim, rope["cache_base"]), name)
+            _native.check(self.lib.configure_qkv_rope_table(h, rope["table"].data_ptr(), rope["table"].shape[1]), name)
             hd = self.config.head_dim
             outs = [StageOutput(name + ".k", "k_cache", rope["cache_k"], rows, hd, rope["cache_base"]),
                     StageOutput(name + ".v", "v_cache", rope["cache_v"], rows, hd, rope["cache_base"])]
@@ -452,8 +453,10 @@ class NativePi0:
         sin = torch.zeros_like(cos)
         cos[:rows] = emb.cos().to(torch.bfloat16)
         sin[:rows] = emb.sin().to(torch.bfloat16)
-        self.buffers.extend((cos, sin))
-        return cos, sin
+        # ... and pair by pair, [hd/2, rows_pad, (cos i, cos i + hd/2, sin i, sin i + hd/2)]: what the QKV drain reads
+        table = torch.stack((cos[:, :hd // 2], cos[:, hd // 2:], sin[:, :hd // 2], sin[:, hd // 2:]), dim=-1).permute(1, 0, 2).contiguous()
+        self.buffers.extend((cos, sin, table))
+        return cos, sin, table
 
     def _interleave_heads(self, w):
         """Reorder the rows of a Q or K projection so rotate-half partners (i, i + hd/2) become adjacent."""
@@ -639,7 +642,7 @@ class NativePi0:
         if self.attention_path is not None:
             _native.check(self.lib.configure_attention_path(handle, int(self.attention_path == "tcgen05")), name)
 
-    def _gemma_layer(self, name, site, prefix, i, x_in, x_mid, bufs, *, rows, s_x, extra_sources, cos, sin, cache, cache_base,
+    def _gemma_layer(self, name, site, prefix, i, x_in, x_mid, bufs, *, rows, s_x, extra_sources, rope, cache, cache_base,
                      attention_rows, mask_prefix, splits, kv_only, block_n, dense_block_n=128, prefix_cache_stage=None,
                      streamed_in=None, next_site=None):
         """One Gemma decoder layer.  ``name`` labels the stages (``expert.<step>.<layer>``), ``site`` the weights
@@ -656,6 +659,7 @@ class NativePi0:
         p = f"{prefix}layers.{i}."
         width = x_in.shape[1]
         H, hd = c.heads, c.head_dim
+        cos, sin, table = rope
         a1, a2, a3, a4, qbuf = bufs
         p_qkv, p_o, p_gu, p_dn = [self.site(f"{site}.{n}") for n in OPERATIONS]
         widths, dense_widths = per_operation(block_n), per_operation(dense_block_n)
@@ -680,7 +684,7 @@ class NativePi0:
         wqkv = self.cached(f"{p}qkv.{p_qkv}.{int(fold1 is not None)}.{int(kv_only)}.{tile("qkv")}", make_qkv)
         q_cols, q = (0, None) if kv_only else (H * hd, qbuf)
         s_qkv = self.gemm(f"{name}.qkv", a1, wqkv, rows=rows, sources=[(s_n1, SAME)], block_n=tile("qkv"), row_rms=fold1,
-                          rope=dict(q=q, cos=cos, sin=sin, cache_k=cache[0], cache_v=cache[1], q_cols=q_cols, cache_base=cache_base))
+                          rope=dict(q=q, cos=cos, sin=sin, table=table, cache_k=cache[0], cache_v=cache[1], q_cols=q_cols, cache_base=cache_base))
         if kv_only:
             return s_qkv, s_qkv, None
         attn_out = a2.bf16
@@ -780,7 +784,7 @@ class NativePi0:
             self._own(h)
             extra = [(self.add(3, h, "prefix.embed"), ALL)]
         self.mark("prefix.input", x_a)
-        cos_p, sin_p = self.rope(P, 0)
+        rope_p = self.rope(P, 0)
         self.caches = [(self.tensor((P + S_pad, hd)), self.tensor((P + S_pad, hd))) for _ in range(c.prefix_layers)]
         bufs = (Activation(self, P_pad, c.width), Activation(self, P_pad, H * hd), Activation(self, P_pad, c.width),
                 Activation(self, P_pad, c.mlp), self.tensor((P_pad, H * hd)))
@@ -789,7 +793,7 @@ class NativePi0:
         for i in range(c.prefix_layers):
             s_x, s_kv, streamed = self._gemma_layer(
                 f"prefix.{i}", f"prefix.{i}", LANGUAGE, i, x_a, x_b, bufs, rows=P, s_x=s_x, extra_sources=extra if i == 0 else [],
-                cos=cos_p, sin=sin_p, cache=self.caches[i], cache_base=0, attention_rows=P, mask_prefix=-1,
+                rope=rope_p, cache=self.caches[i], cache_base=0, attention_rows=P, mask_prefix=-1,
                 splits=self._prefix_splits(P), kv_only=(i == c.prefix_layers - 1), block_n=128, streamed_in=streamed,
                 next_site=f"prefix.{i + 1}" if i + 1 < c.prefix_layers else None)
             cache_stage.append(s_kv)
@@ -818,7 +822,7 @@ class NativePi0:
         h1 = self.tensor((self.chunk_size, W), torch.float32)
         actions = self.tensor((self.chunk_size, c.action_dim), torch.float32)
         xe_a, xe_b = self.tensor((S_pad, W)), self.tensor((S_pad, W))
-        cos_s, sin_s = self.rope(S, P)
+        rope_s = self.rope(S, P)
         ebufs = (Activation(self, S_pad, W), Activation(self, S_pad, H * hd), Activation(self, S_pad, W),
                  Activation(self, S_pad, c.expert_mlp), self.tensor((S_pad, H * hd)))
         ebufs[1].bf16 = self.tensor((S_pad, H * hd))
@@ -841,7 +845,7 @@ class NativePi0:
             self.mark(f"expert.{step}.input", xe_a)
             streamed = None
             for i in range(c.expert_layers):
-                s_x, _, streamed = self._expert_layer(step, i, xe_a, xe_b, ebufs, S, P, s_x, cos_s, sin_s, cache_stage[i], streamed)
+                s_x, _, streamed = self._expert_layer(step, i, xe_a, xe_b, ebufs, S, P, s_x, rope_s, cache_stage[i], streamed)
                 self.mark(f"expert.{step}.{i}", xe_a)
             s_prev = self.linear32(f"expert.{step}.euler", xe_a, final_w, final_b, actions, rows=self.chunk_size, sources=[(s_x, ALL)],
                                    ldx=W, x_bf16=True, rms=True, euler=True, prev=None if first else actions,
@@ -872,10 +876,10 @@ class NativePi0:
         if self.verbose:
             print("NativePi0 static program:", self.plan, flush=True)
 
-    def _expert_layer(self, step, i, x_in, x_mid, bufs, S, P, s_x, cos, sin, prefix_cache_stage, streamed):
+    def _expert_layer(self, step, i, x_in, x_mid, bufs, S, P, s_x, rope, prefix_cache_stage, streamed):
         """Every Euler step wires its own stages; the NVFP4 weights are shared through the keyed weight cache."""
         last = i + 1 == self.config.expert_layers
-        return self._gemma_layer(f"expert.{step}.{i}", f"expert.{i}", EXPERT, i, x_in, x_mid, bufs, rows=S, s_x=s_x, extra_sources=[], cos=cos, sin=sin,
+        return self._gemma_layer(f"expert.{step}.{i}", f"expert.{i}", EXPERT, i, x_in, x_mid, bufs, rows=S, s_x=s_x, extra_sources=[], rope=rope,
                                  cache=self.caches[i], cache_base=P, attention_rows=P + S, mask_prefix=P, splits=self._expert_splits(P + S),
                                  kv_only=False, block_n=self.expert_block_n, dense_block_n=self.expert_dense_block_n, prefix_cache_stage=prefix_cache_stage, streamed_in=streamed,
                                  next_site=None if last else f"expert.{i + 1}")

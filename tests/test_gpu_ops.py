@@ -416,6 +416,38 @@ def test_gemm_qkv_rope_epilogue():
     assert (ck[:50] == 7).all() and (ck[50 + rows:] == 7).all() and not qout[rows:].any()
 
 
+@pytest.mark.parametrize("rows,heads,block_n", [(1, 2, 64), (51, 2, 64), (128, 1, 128), (129, 2, 128), (321, 0, 128), (384, 1, 32)])
+def test_qkv_rope_table_in_pair_order(rows, heads, block_n):
+    """The rotary tables pair by pair give the bits of the two tables, for few rows (stored one by one) and for several row bands
+    (stored together), and no row beyond the last is written."""
+    lib = _native.load()
+    rng = np.random.default_rng(rows)
+    m, k, hd = 128 * -(-rows // 128), 256, 256
+    n = (heads + 2) * hd
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    cos, sin = (torch.from_numpy(rng.uniform(-1, 1, size=(m, hd)).astype(np.float32)).bfloat16().cuda() for _ in range(2))
+    half = hd // 2
+    table = torch.stack((cos[:, :half], cos[:, half:], sin[:, :half], sin[:, half:]), -1).permute(1, 0, 2).contiguous()
+    got = []
+    for pairs in (False, True):
+        q = torch.full((m, max(heads, 1) * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        ck, cv = (torch.full((rows + 60, hd), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        with ResidentNVFP4(None, pa, pb, workers=7, output_dtype=torch.bfloat16, rows=rows, block_n=block_n) as op:
+            _native.check(lib.configure_resident_fp4_qkv_rope(op.handle, q.data_ptr() if heads else None, max(heads, 1) * hd, cos.data_ptr(),
+                                                              sin.data_ptr(), ck.data_ptr(), cv.data_ptr(), heads * hd, hd, 50), "rope")
+            if pairs:
+                assert lib.configure_qkv_rope_table(op.handle, table.data_ptr(), m - 128) == 1 and lib.configure_qkv_rope_table(op.handle, None, m) == 1
+                _native.check(lib.configure_qkv_rope_table(op.handle, table.data_ptr(), m), "rope table")
+            op.forward()
+            assert op.status()["code"] == 0
+        for t in (ck, cv):
+            assert (t[:50] == 7).all() and (t[50 + rows:] == 7).all() and not (t[50:50 + rows] == 7).all(1).any()
+        assert (q[rows:] == 7).all() and (heads == 0 or not (q[:rows] == 7).all(1).any())
+        got.append((q, ck, cv))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("rows,width,kind", [(51, 1024, "rms"), (768, 2048, "rms"), (256, 1152, "layer"), (7, 64, "layer")])
 def test_norm_to_nvfp4(rows, width, kind):
     torch.manual_seed(83)
