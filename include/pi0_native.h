@@ -74,13 +74,19 @@ int configure_resident_fp4_stream_sums(void* handle, float* sums, int ld);
 int configure_resident_fp4_row_layernorm(void* handle, const float* sumsq, const float* sums, int parts, int width, float eps,
                                          const float* center);
 /* extension: logical row count (rows >= this are never stored; with at most 64 rows only 64 rows of A are
- * copied per tile) and output tile width: 128, 64, or 32.  With 32-wide NVFP4 tiles the weight scales
+ * copied per tile) and output tile width: 128, 64, 32 or, in NVFP4, 192.  With 32-wide NVFP4 tiles the weight scales
  * given at creation are read in a layout of their own: one 512-byte atom per (32-row tile, group of four 16-element
  * blocks) - [N / 32][K / 64][512] - holding the tile's 32 rows in the first 32-row sub-column of the atom (bytes
  * 16 r + b for row r, block b) and zeros elsewhere, i.e. four times the bytes of the standard layout.  Narrow tiles are
- * for projections of a few rows, whose time is the bytes one SM takes in and the serial epilogue of one tile. */
+ * for projections of a few rows, whose time is the bytes one SM takes in and the serial epilogue of one tile.  192-wide NVFP4
+ * tiles have two such atoms each, [tiles][K / 64][2][512], the tile's 192 rows in order and zeros behind; they are for
+ * projections whose 128-wide tiles are a little more than one per SM, with BF16 or NVFP4 output (no GeGLU, no residual stream) and weights that are not tile-major. */
 int configure_resident_fp4_rows(void* handle, int rows);
 int configure_resident_fp4_tile(void* handle, int block_n);
+/* extension: logical columns of the output (whole 128-column tiles; at most N): the rows of the weight beyond only fill up the last
+ * tile of another width.  The rows of the output are that many columns apart, the bias has that many values.  Behind the epilogue's
+ * own call (BF16 or NVFP4 output, without GeGLU, a residual or padded heads) and before the tile width. */
+int configure_resident_fp4_columns(void* handle, int cols);
 /* extension: tiled = 1 declares that B is stored tile-major (rows of whole 128-byte pieces: K a multiple of 256 in NVFP4,
  * 64 in BF16, 128 in FP8): for every output tile n and every 128-byte piece s of K the block_n x 128 bytes of that block are
  * contiguous, at byte offset ((n * pieces + s) * block_n) * 128; one TMA box is then one contiguous read.  Set the tile

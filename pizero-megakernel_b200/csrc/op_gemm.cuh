@@ -72,22 +72,24 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
         }
         int alive = 1;
         if (lane == 0) {
-            // B scales: the 128-row atom that holds the tile's rows, or - 32-wide tiles - an atom of the tile's own
-            const int sf_tile = !WEIGHTS ? m_tile : block_n == 32 ? n_tile : (n_tile * block_n) >> 7;
+            // B scales: the 128-row atom that holds the tile's rows, or - 32- and 192-wide tiles - an atom or two of the tile's own
+            const bool two = WEIGHTS && block_n > 128;
+            const int sf_tile = !WEIGHTS ? m_tile : block_n == 32 ? n_tile : two ? 2 * n_tile : (n_tile * block_n) >> 7;
+            const uint32_t sf_group = two ? 1024u : 512u;
             const uint8_t* sf = scales + static_cast<size_t>(sf_tile) * k_groups * 512;
             for (int ks = 0; ks < slots; ++ks) {
                 const uint32_t s = slot;
                 if (!mbar_wait(prog, ctl, &ctl->empty[s], ((bits >> s) & 1u) ^ 1u, stage_index)) { alive = 0; break; }
                 uint8_t* base = data + s * stride;
                 uint64_t* bar = &ctl->full[s];
-                const uint32_t sf_bytes = scaled ? static_cast<uint32_t>(min(4 * kChunks, k_groups - ks * 4 * kChunks)) * 512u : 0u;
+                const uint32_t sf_bytes = scaled ? static_cast<uint32_t>(min(4 * kChunks, k_groups - ks * 4 * kChunks)) * sf_group : 0u;
                 // Boxes always deliver kChunks chunks (beyond K the copy engine fills zeros or, inside a padded
                 // allocation, bytes that no MMA reads).  a_box_rows < 128 (few logical rows): only the rows that
                 // exist are copied; the MMA still reads 128 rows, the rest lands in accumulator rows never stored.
                 mbar_expect_tx(bar, bytes + sf_bytes);
                 if (WEIGHTS && b_tiled) tma_load_2d(base + off, tmap, bar, 0, (n_tile * chunks + ks * kChunks) * block_n);
                 else tma_load_3d(base + off, tmap, bar, 0, WEIGHTS ? n_tile * block_n : m_tile * 128, ks * kChunks);
-                if (scaled) bulk_load(base + off_sf, sf + static_cast<size_t>(ks) * (4 * kChunks * 512), sf_bytes, bar);
+                if (scaled) bulk_load(base + off_sf, sf + static_cast<size_t>(ks) * (4 * kChunks) * sf_group, sf_bytes, bar);
                 bits ^= 1u << s;
                 slot = s + 1 == ring ? 0u : s + 1;
             }
@@ -99,6 +101,49 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
     ps.bits = bits;
 }
 
+// The issuing thread's loop for NVFP4 tiles of 192 columns.  Such a tile takes both accumulator buffers (two uses) from column 0 on and
+// has two atoms of B scales per group, so the scale columns of a slot are A's four of every group (eight apart) and behind them B's
+// eight, two slots in turn.  It is the one tile of its instruction as a rule; the loop of the other widths stays free of it (with
+// the place of the scale columns as a variable, or both widths from one template, a slot takes 40 - 100 ns longer).
+__device__ __forceinline__ void gemm_mma_wide(const VmProgram& prog, Ctl* ctl, const GemmParams& g, uint32_t data16, uint32_t tmem, int stage_index,
+                                              int count, uint32_t& slot, uint32_t& bits, uint32_t& it, uint32_t& tile_no, long long* stamp) {
+    constexpr uint64_t kOperandHi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+    constexpr uint64_t kScaleHi = (1ull << 16) | (8ull << 32) | (1ull << 46);
+    const int k_groups = g.k_groups, slots = (k_groups + 4 * kChunks - 1) / (4 * kChunks);
+    const uint32_t a_chunk16 = static_cast<uint32_t>(g.a_box_rows) * 8u, b_chunk16 = static_cast<uint32_t>(g.block_n) * 8u;
+    for (int t = 0; t < count; ++t) {
+        for (uint32_t u = 0; u < 2; ++u)
+            if (!mbar_wait(prog, ctl, &ctl->acc_empty[(tile_no + u) & 1u], (((tile_no + u) >> 1) & 1u) ^ 1u, stage_index)) return;
+        tc_fence_after();
+        for (int ks = 0; ks < slots; ++ks) {
+            if (!mbar_wait(prog, ctl, &ctl->full[slot], (bits >> slot) & 1u, stage_index)) return;
+            if (stamp && t == 0 && ks == 0) stamp[4] = static_cast<long long>(global_ns());
+            const uint32_t a16 = data16 + (slot * static_cast<uint32_t>(g.slot_stride) >> 4), b16 = a16 + (static_cast<uint32_t>(g.off_b) >> 4);
+            const uint32_t sfa16 = a16 + (static_cast<uint32_t>(g.off_sfa) >> 4), sfb16 = a16 + (static_cast<uint32_t>(g.off_sfb) >> 4);
+            const uint32_t groups = static_cast<uint32_t>(min(4 * kChunks, k_groups - ks * 4 * kChunks));
+            const uint32_t sfa = tmem + kSfCol0 + (it & 1u) * 128u, sfb = sfa + 64u;
+            for (uint32_t gi = 0; gi < groups; ++gi) {
+                tc_copy_sf(sfa + gi * 8, kScaleHi | static_cast<uint64_t>(sfa16 + gi * 32));
+                tc_copy_sf(sfb + gi * 8, kScaleHi | static_cast<uint64_t>(sfb16 + gi * 64));
+                tc_copy_sf(sfb + gi * 8 + 4, kScaleHi | static_cast<uint64_t>(sfb16 + gi * 64 + 32));
+            }
+            for (uint32_t gi = 0; gi < groups; ++gi) {
+                const uint32_t chunk = gi >> 2, sub = gi & 3u;
+                tc_mma_nvfp4(tmem, kOperandHi | static_cast<uint64_t>(a16 + chunk * a_chunk16 + 2u * sub),
+                             kOperandHi | static_cast<uint64_t>(b16 + chunk * b_chunk16 + 2u * sub), g.idesc, sfa + gi * 8, sfb + gi * 8,
+                             static_cast<uint32_t>(ks != 0 || gi != 0));
+            }
+            tc_commit(&ctl->empty[slot]);
+            bits ^= 1u << slot;
+            slot = slot + 1 == static_cast<uint32_t>(g.ring_stages) ? 0u : slot + 1;
+            it++;
+        }
+        tc_commit(&ctl->acc_full[0]);
+        tc_commit(&ctl->acc_full[1]);
+        tile_no += 2;
+    }
+}
+
 // Warp 1: one elected thread runs the whole loop - waits, scale copies, MMAs, commits - while the other lanes wait at the
 // end.  The queue in front of the tensor core holds only about two MMAs, so whatever the issuing thread does between two
 // slots is idle tensor time: with a warp-wide barrier vote and an election per slot a slot of eight MMAs cost 690 (BF16,
@@ -106,7 +151,7 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
 // tested (without blocking) half-way through the current one, and a slot that has landed by then costs no wait at all.
 // The operand arithmetic starts from values broadcast over the warp, so that descriptors stay in uniform registers.
 // (One instantiation per operand format, so each issue loop carries only its own instructions.)
-template <int OPERANDS>
+template <int OPERANDS, bool WIDE>
 __device__ __forceinline__ void gemm_mma(const VmProgram& prog, Ctl* ctl, uint8_t* data, uint32_t tmem_in, const StageDesc& st,
                                          int stage_index, int first_in, int count_in, PipeState& ps, long long* stamp) {
     const GemmParams& g = st.p.gemm;
@@ -129,7 +174,9 @@ __device__ __forceinline__ void gemm_mma(const VmProgram& prog, Ctl* ctl, uint8_
     if (ps.geo != geo) { ps.geo = geo; ps.slot = 0; }
     uint32_t slot = uniform_u32(ps.slot), bits = uniform_u32(ps.bits), it = uniform_u32(ps.it), tile_no = uniform_u32(ps.tile);
     const bool leader = elect_one();
-    if (leader) {
+    if (WIDE && __builtin_expect(block_n > 128, 0)) {
+        if (leader) gemm_mma_wide(prog, ctl, g, data16, tmem, stage_index, count, slot, bits, it, tile_no, stamp);
+    } else if (leader) {
         bool landed = false, alive = true;                   // landed: the current slot was seen full by the look-ahead
         for (int t = first; alive && t < first + count; ++t) {
             const int n_tile = t % n_tiles;
@@ -508,7 +555,9 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
 // helper comes from its role at about that moment and would have to fetch the row statistics first.
 // LEAN: the drain of the lean kernel variant; the residual-stream and plain BF16 drains there carry no row-statistics code
 // (the host sends programs that give those two epilogues row statistics to the full variant).
-template <int EPI, bool LEAN = false>
+// WIDE: NVFP4 tiles of 192 columns, which take two accumulator uses and may end beyond the logical columns.  An instantiation of its
+// own: with both in one drain the others' take 0.1 us longer (one view 5.21 -> 5.31 ms, BF16 16.16 -> 16.51).
+template <int EPI, bool LEAN = false, bool WIDE = false>
 __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, uint32_t tmem, const StageDesc& st,
                                               int stage_index, int first, int count, PipeState& ps, long long* stamp) {
     const GemmParams& g = st.p.gemm;
@@ -518,19 +567,22 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
     const bool main = threadIdx.x >= 128;
     const int lane = lane_id();
     const int n_tiles = g.n_tiles, block_n = g.block_n, last = first + count - 1;
+    constexpr int kUses = WIDE ? 2 : 1;                  // accumulator uses of a tile
     int run = 0;                                         // tiles drained since the last publication
     int known_band = -1;                                 // row band of the tile drained before
     float row_scale = 1.f, row_shift = 0.f;
     for (int t = main ? first : last; t <= last; ++t) {
         const int m_tile = t / n_tiles, n_tile = t - m_tile * n_tiles;
-        const uint32_t use = ps.tile + static_cast<uint32_t>(t - first);
+        const uint32_t use = ps.tile + static_cast<uint32_t>((t - first) * kUses);
         const uint32_t buf = use & 1u, phase = (use >> 1) & 1u;
         const int row = m_tile * 128 + quarter * 32 + lane;
         const bool row_ok = row < g.rows;
         const bool rows_here = m_tile * 128 + quarter * 32 < g.rows;
         const bool shared_tile = t == last && block_n >= 64, helped = shared_tile && rows_here;
         if (!main && !helped) break;
-        const int col_begin = main ? 0 : block_n >> 1, col_end = main && helped ? block_n >> 1 : block_n;
+        const int col_begin = main ? 0 : block_n >> 1;
+        int col_end = main && helped ? block_n >> 1 : block_n;
+        if constexpr (WIDE) col_end = min(col_end, g.cols - n_tile * block_n);      // (logical columns are multiples of 32)
         if (EPI == EPI_QKV_ROPE && rows_here) {
             // while the MMAs run: bring the first chunk's rotary table entries (constant data) close
             const int hd = g.head_dim, col_a = n_tile * block_n + col_begin;
@@ -639,18 +691,19 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         }
         tc_fence_after();
         if (stamp && t == first && threadIdx.x == 128) stamp[6] = static_cast<long long>(global_ns());
-        const uint32_t taddr = tmem + buf * 128u + (static_cast<uint32_t>(quarter * 32) << 16);
+        const uint32_t taddr = tmem + (WIDE ? 0u : buf * 128u) + (static_cast<uint32_t>(quarter * 32) << 16);
         const uint32_t share = helped ? 1u : 2u;             // parts of the tile this warp speaks for: two per quarter
         auto columns_read = [&]() {                          // this warp's part of the accumulator is in registers
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_count(&ctl->acc_empty[buf], share);
+            if (WIDE && lane == 0) mbar_arrive_count(&ctl->acc_empty[buf ^ 1u], share);
         };
         // Residual-stream statistics: the two halves of a tile are summed apart, whichever warps drain them, and added at the
         // end, so the bits do not depend on how the tiles are dealt to the workers.
         float2 sumsq = make_float2(0.f, 0.f), sum = make_float2(0.f, 0.f);
         float sumsq_half = 0.f, sum_half = 0.f;
-        if (!rows_here) {
+        if (!rows_here || (WIDE && col_begin >= col_end)) {
             columns_read();
         } else {
             if (!early) load_residual(col_begin);
@@ -701,14 +754,16 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         run = 0;
         if (!shared_tile) ps.run++;
     }
-    ps.tile += static_cast<uint32_t>(count);
+    ps.tile += static_cast<uint32_t>(count * kUses);
 }
 
 // Dispatch of one GEMM instruction onto the warp roles (warp 2 has none); behind its role every warp goes through the
 // drain, as one of the draining warps or as a helper of the last tile.
 // LEAN: the kernel variant for programs made only of NVFP4 projections with the pi0 model's epilogues (the host checks
 // this when it builds a program); it carries neither the dense issue loops nor the other drain loops.
-template <bool LEAN>
+// WIDE: with the forms for 192-wide NVFP4 tiles.  The variant that BF16 models and most operators launch goes without (BF16 forward
+// 16.14 ms, 16.70 with them): programs that need both run the one with everything.
+template <bool LEAN, bool WIDE>
 __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl, uint8_t* data, uint32_t tmem,
                                                  const StageDesc& st, int stage_index, int first, int count,
                                                  PipeState& ps, long long* stamp) {
@@ -720,12 +775,15 @@ __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl
         gemm_producer<true>(prog, ctl, data, st, stage_index, first, count, ps, nullptr);
     } else if (warp == 1) {
         const int operands = st.p.gemm.operands;
-        if (LEAN || operands == GEMM_NVFP4) gemm_mma<GEMM_NVFP4>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
-        else if (operands == GEMM_BF16) gemm_mma<GEMM_BF16>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
-        else gemm_mma<GEMM_FP8>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
+        if (LEAN || operands == GEMM_NVFP4) gemm_mma<GEMM_NVFP4, WIDE>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
+        else if (operands == GEMM_BF16) gemm_mma<GEMM_BF16, false>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
+        else gemm_mma<GEMM_FP8, false>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
     }
     const int epilogue = st.p.gemm.epilogue;                // one drain loop per epilogue kind: only its own arithmetic and registers
-    if (epilogue == EPI_BF16) gemm_epilogue<EPI_BF16, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    if (WIDE && __builtin_expect(st.p.gemm.block_n > 128, 0)) {
+        if (epilogue == EPI_FP4) gemm_epilogue<EPI_FP4, LEAN, WIDE>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+        else gemm_epilogue<EPI_BF16_EXT, LEAN, WIDE>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    } else if (epilogue == EPI_BF16) gemm_epilogue<EPI_BF16, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_STREAM) gemm_epilogue<EPI_STREAM, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_GEGLU_FP4) gemm_epilogue<EPI_GEGLU_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_FP4) gemm_epilogue<EPI_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);

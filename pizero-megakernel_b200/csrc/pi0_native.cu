@@ -143,6 +143,7 @@ struct Program {
     bool timings_on = false;
     bool lean = false;                 // every stage is one the lean kernel variant runs
     bool mma_sync = false;             // some attention stage runs on the mma.sync tiles
+    bool wide = false;                   // a projection has 192-wide tiles
     bool early = false;                // the program of one operator small enough for its successor to start early (solo_program)
     int grid = 0;                      // CTAs launched: up to the last worker that has an instruction
     unsigned int epoch = 0;
@@ -317,6 +318,7 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
         for (const auto& d : prog->stages) {
             prog->lean = prog->lean && lean_stage(d);
             prog->mma_sync = prog->mma_sync || (d.kind == OP_ATTN && !d.p.attn.tc);
+            prog->wide = prog->wide || (d.kind == OP_GEMM && d.p.gemm.block_n > 128);
         }
     }
     if (e != cudaSuccess) return e;
@@ -373,7 +375,7 @@ int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begi
     config.numAttrs = 1;
     if (prog->lean && !prog->h_debug && !p.timings) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false>, p);
     if (prog->lean && !prog->h_debug) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true>, p);
-    if (!prog->mma_sync) return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true, false>, p);
+    if (!prog->mma_sync && !prog->wide) return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true, false>, p);
     return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true, true>, p);
 }
 
@@ -430,11 +432,12 @@ int a_box_rows_of(int operands, int m, int rows) {
 // has to stay inside shared memory, which the slot's own B and scale regions guarantee.
 int ring_layout(GemmParams& g, int operands) {
     g.off_b = kChunks * 128 * g.a_box_rows;
-    const int sf_bytes = operands == GEMM_NVFP4 ? kSfBytes : 0;
+    const int sf_bytes = operands == GEMM_NVFP4 ? kSfBytes : 0, sfb_bytes = g.block_n > 128 ? 2 * sf_bytes : sf_bytes;
+    const int fewest = g.block_n > 128 ? 2 : kStages;       // (192-wide tiles: slots of up to 92 KiB)
     g.off_sfa = g.off_b + kChunks * 128 * g.block_n;
     g.off_sfb = g.off_sfa + sf_bytes;
-    g.slot_stride = g.off_sfb + sf_bytes;
-    g.ring_stages = std::max(kStages, std::min(operands == GEMM_NVFP4 ? kMaxStages : kMaxStagesDense, kDataBytes / g.slot_stride));
+    g.slot_stride = g.off_sfb + sfb_bytes;
+    g.ring_stages = std::max(fewest, std::min(operands == GEMM_NVFP4 ? kMaxStages : kMaxStagesDense, kDataBytes / g.slot_stride));
     if (g.slot_stride % 1024 || g.ring_stages * g.slot_stride > kDataBytes ||
         (kChunks - 1) * 128 * g.a_box_rows + kTileABytes > g.slot_stride)
         return cudaErrorInvalidValue;
@@ -445,6 +448,8 @@ int gemm_refresh(Op* op) {
     GemmParams& g = op->desc.p.gemm;
     CUtensorMap host[2];
     const size_t row_bytes = operand_row_bytes(op->operands, op->k);
+    const int n_tiles = (g.cols + g.block_n - 1) / g.block_n;
+    if (n_tiles * g.block_n > op->n) return cudaErrorInvalidValue;        // (the weight has rows for whole tiles)
     int e = encode_operand(&host[0], op->a, op->m, row_bytes, g.a_box_rows);
     if (!e) e = g.b_tiled ? encode_tiled(&host[1], op->b, op->n * static_cast<int>(row_bytes / 128), kChunks * g.block_n)
                           : encode_operand(&host[1], op->b, op->n, row_bytes, g.block_n);
@@ -458,7 +463,7 @@ int gemm_refresh(Op* op) {
     g.tmap_a = op->maps;
     g.tmap_b = op->maps + 1;
     g.m_tiles = op->m / 128;
-    g.n_tiles = op->n / g.block_n;
+    g.n_tiles = n_tiles;
     if (!g.sum_out || g.sumsq_ld < g.n_tiles) g.sumsq_ld = g.n_tiles;      // statistics rows: one slot per column tile
     g.operands = op->operands;
     g.k_groups = static_cast<int>(row_bytes / 32);
@@ -575,6 +580,7 @@ extern "C" int create_resident_fp4(void** handle, const void* a, const void* b, 
     g.sfa = static_cast<const uint8_t*>(sfa);
     g.sfb = static_cast<const uint8_t*>(sfb);
     g.block_n = 128;
+    g.cols = n;
     g.a_box_rows = 128;
     g.alpha = alpha;
     g.epilogue = EPI_F32;
@@ -726,15 +732,35 @@ extern "C" int configure_resident_fp4_rows(void* handle, int rows) {
 }
 extern "C" int configure_resident_fp4_weight_layout(void* handle, int tiled) {
     Op* op = as_op(handle);
-    if (!op || op->desc.kind != OP_GEMM || (tiled != 0 && tiled != 1) || (tiled && operand_row_bytes(op->operands, op->k) % 128))
+    if (!op || op->desc.kind != OP_GEMM || (tiled != 0 && tiled != 1) || (tiled && operand_row_bytes(op->operands, op->k) % 128) ||
+        (tiled && op->desc.p.gemm.block_n > 128))              // (a box has at most 256 rows)
         return cudaErrorInvalidValue;
     op->desc.p.gemm.b_tiled = tiled;
     return gemm_refresh(op);
 }
 extern "C" int configure_resident_fp4_tile(void* handle, int block_n) {
     Op* op = as_op(handle);
-    if (!op || op->desc.kind != OP_GEMM || (block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
-    op->desc.p.gemm.block_n = block_n;
+    if (!op || op->desc.kind != OP_GEMM || (block_n != 192 && block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
+    GemmParams& g = op->desc.p.gemm;
+    if (block_n == 192) {                                    // (the two epilogues whose drains have a form for such tiles)
+        if (g.epilogue == EPI_BF16) g.epilogue = EPI_BF16_EXT;
+        if (op->operands != GEMM_NVFP4 || g.b_tiled || (g.epilogue != EPI_FP4 && g.epilogue != EPI_BF16_EXT) || (g.cols + 191) / 192 * 192 > op->n)
+            return cudaErrorInvalidValue;
+    }
+    g.block_n = block_n;
+    return gemm_refresh(op);
+}
+// extension: logical columns of the output, whole 128-column tiles and not more than N: the weight's rows beyond only fill up the
+// last tile of another width.  Neither results nor bias exist for them, and the rows of the output are that many columns apart.
+// Behind the epilogue's own call (BF16 or NVFP4 output, without GeGLU, a residual or padded heads) and before the tile width.
+extern "C" int configure_resident_fp4_columns(void* handle, int cols) {
+    Op* op = as_op(handle);
+    if (!op || op->desc.kind != OP_GEMM || cols < 128 || cols % 128 || cols > op->n) return cudaErrorInvalidValue;
+    GemmParams& g = op->desc.p.gemm;
+    if ((g.epilogue != EPI_FP4 && g.epilogue != EPI_BF16 && g.epilogue != EPI_BF16_EXT) || g.residual || g.pad_from || g.block_n > 128) return cudaErrorInvalidValue;
+    g.cols = cols;
+    g.ldo = g.epilogue == EPI_FP4 ? cols / 2 : cols;
+    if (g.epilogue == EPI_FP4) g.out_blocks = cols / 16;
     return gemm_refresh(op);
 }
 extern "C" int resident_fp4_resources(void* handle, int* values, int count) {
@@ -778,6 +804,7 @@ extern "C" int create_dense(void** handle, const void* a, const void* b, void* o
     finish_desc(d);
     GemmParams& g = d.p.gemm;
     g.block_n = 128;
+    g.cols = n;
     g.a_box_rows = 128;
     g.alpha = alpha;
     g.epilogue = bf16 ? EPI_BF16 : EPI_F32;
@@ -1401,7 +1428,7 @@ extern "C" int op_geometry(void* handle, int* tiles, int* bands, int* cost) {
 // several bands) and block_n-wide tiles - slot size, slot count and the key under which the kernel's ring cursors run on.
 // Needs no device.
 extern "C" int gemm_ring_geometry(int operands, int rows, int block_n, int* slot_stride, int* ring_stages, unsigned int* key) {
-    if (operands < GEMM_NVFP4 || operands > GEMM_FP8 || rows < 1 || (block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
+    if (operands < GEMM_NVFP4 || operands > GEMM_FP8 || rows < 1 || (block_n != 128 && block_n != 64 && block_n != 32 && (block_n != 192 || operands != GEMM_NVFP4))) return cudaErrorInvalidValue;
     GemmParams g{};
     g.a_box_rows = a_box_rows_of(operands, rows <= 128 ? 128 : 256, rows);
     g.block_n = block_n;

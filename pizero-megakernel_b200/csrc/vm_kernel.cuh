@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
         if (stamp && threadIdx.x == 0) stamp[0] = static_cast<long long>(global_ns());
         if (st.kind == OP_GEMM) {
             if constexpr (!LEAN) mark(prog, 800000 + ins.y);
-            gemm_instruction<LEAN>(prog, ctl, data, tmem, st, ins.y, ins.z, ins.w, ps, stamp);
+            gemm_instruction<LEAN, LEAN || MMA_SYNC>(prog, ctl, data, tmem, st, ins.y, ins.z, ins.w, ps, stamp);
             // one decision per warp: the lanes with a role return later than the others and must not leave alone
             if (__any_sync(0xffffffffu, ctl->abort != 0)) break;
         } else {

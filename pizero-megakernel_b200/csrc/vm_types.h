@@ -57,7 +57,8 @@ struct GemmParams {
     int operands;                // GemmOperands
     int m_tiles, n_tiles;        // 128-row x block_n-column output tiles
     int k_groups;                // row_bytes / 32: one MMA each (64 FP4, 16 BF16 or 32 FP8 elements of K)
-    int block_n;                 // 128 (default), 64 or 32
+    int block_n;                 // 128 (default), 64 or 32, NVFP4 also 192 (such a tile takes both accumulator buffers: two accumulator uses)
+    int cols;                    // logical columns of the output (<= N; only 192-wide tiles may end beyond them)
     int b_tiled;                 // B stored tile-major: block (n_tile, k_stage) is block_n contiguous 128-byte rows
     int a_box_rows;              // rows of A copied per tile: 128, or fewer (a multiple of 8) when there are fewer logical rows
     int ring_stages;             // operand ring of this GEMM: slots in flight (kStages..kMaxStagesDense) ...

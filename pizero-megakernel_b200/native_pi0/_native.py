@@ -59,6 +59,7 @@ _SIGNATURES = {
     "configure_resident_fp4_row_layernorm": [_P, _P, _P, _I, _I, _F, _P],
     "configure_resident_fp4_rows": [_P, _I],
     "configure_resident_fp4_tile": [_P, _I],
+    "configure_resident_fp4_columns": [_P, _I],
     "configure_resident_fp4_weight_layout": [_P, _I],
     "resident_fp4_resources": [_P, C.POINTER(_I), _I],
     "destroy_resident_fp4": [_P],

@@ -238,14 +238,26 @@ class NativePi0:
             store[key] = make()
         return store[key]
 
-    def weight(self, w, *, rows_to=128, block_n=128, precision="nvfp4", row_sums=False):
+    def tile_width(self, bands, w):
+        """Output tile width of a wide projection with ``bands`` row bands: 192 where that makes one tile per SM out of a few more than
+        one 128-wide tile.  A second round of tiles costs as much as the first, half as many columns more cost their copies and a third
+        of the drain (three views: SigLIP's q|k|v 162 tiles -> 108, 12.3 -> 9.3 us; fc1 204 -> 138, 15.8 -> 11.6).  NVFP4 weights with
+        scales for such tiles only (``wide_scales``), and only while every site is NVFP4: the kernel variant of other programs is the faster
+        without such tiles."""
+        rounds = lambda width: -(-bands * -(-w.logical_rows // width) // self.workers)
+        uniform = self.default_precision == "nvfp4" and all(v == "nvfp4" for _, v in self.precision_map)
+        return 192 if uniform and getattr(w, "wide_scales", None) is not None and rounds(192) == 1 and rounds(128) > 1 else 128
+
+    def weight(self, w, *, block_n=128, precision="nvfp4", row_sums=False, wide=False):
         """BF16/FP32 [N, K] -> the site's operand format on the device: NVFP4 (ceil block scales, tensor scale
         amax/(6*448)) or zero-padded BF16.
+
+        ``wide``: rows for whole 192-wide tiles too and, where the codes are not tile-major, their scales for those (``tile_width``).
 
         When K is a multiple of 256 the packed NVFP4 codes are re-laid tile-major for ``block_n``-wide output tiles
         (``Fp4Matrix.tiled = block_n``): every TMA box of the weight operand is then one contiguous read."""
         n, k = w.shape
-        np_, kp = padded(n, rows_to), padded(k, 64)
+        np_, kp = padded(n, 384 if wide else 128), padded(k, 64)      # whole tiles and whole scale atoms
         src = torch.zeros((np_, kp), device=self.device, dtype=torch.bfloat16)
         src[:n, :k] = w.to(torch.bfloat16)
         if precision == "bf16":
@@ -266,6 +278,9 @@ class NativePi0:
         if block_n == 32:
             from native_pi0.primitives import narrow_tile_scales
             m.scales = narrow_tile_scales(m.scales, np_, kp // 16)     # an atom of scales per 32-row tile
+        if wide and kp % 256:
+            from native_pi0.primitives import wide_tile_scales
+            m.wide_scales = wide_tile_scales(m.scales, np_, kp // 16)  # the same scales, two atoms per 192-row tile
         m.scale_tile = block_n if block_n == 32 else 128
         m.tiled = 0
         if self.tile_weights and kp % 256 == 0 and np_ % block_n == 0:
@@ -341,7 +356,7 @@ class NativePi0:
                                                 m, n, k, self.workers, 0, 1, 1.0), name)
         else:
             _native.check(self.lib.create_resident_fp4(C.byref(h), src.data.data_ptr(), w.data.data_ptr(), src.scales.data_ptr(),
-                                                       w.scales.data_ptr(), placeholder.data_ptr(), m, n, k, self.workers,
+                                                       (w.wide_scales if block_n == 192 else w.scales).data_ptr(), placeholder.data_ptr(), m, n, k, self.workers,
                                                        float(np.float32(src.global_scale) * np.float32(w.global_scale))), name)
         self._own(h)
         cols = getattr(w, "logical_rows", n)
@@ -387,6 +402,8 @@ class NativePi0:
             if head_pad is not None:
                 _native.check(self.lib.configure_dense_head_pad(h, head_pad[0], head_pad[1], out.stride(0)), name)
             outs = [StageOutput(name, "bf16", out, rows, cols, head=head_pad)]
+        if out_act is not None and activation != 2 and out_act.width < n:       # (the weight is padded to whole tiles of either width)
+            _native.check(self.lib.configure_resident_fp4_columns(h, out_act.width), name)
         if row_rms is not None:
             sumsq, parts, width, eps = row_rms
             _native.check(self.lib.configure_resident_fp4_row_rms(h, sumsq.data_ptr(), parts, width, float(eps)), name)
@@ -531,10 +548,10 @@ class NativePi0:
             w_qkv_raw = lambda: torch.cat([sd[p + f"self_attn.{n}_proj.weight"] for n in "qkv"])
             b_qkv_raw = torch.cat([sd[p + f"self_attn.{n}_proj.bias"] for n in "qkv"])
             if fold1:
-                wqkv = self.cached(p + "qkv.nvfp4.ln", lambda: self.weight(folded(w_qkv_raw(), b_qkv_raw, g1, b1)[0], row_sums=True))
+                wqkv = self.cached(p + "qkv.nvfp4.ln", lambda: self.weight(folded(w_qkv_raw(), b_qkv_raw, g1, b1)[0], wide=True, row_sums=True))
                 bqkv = folded(w_qkv_raw(), b_qkv_raw, g1, b1)[1]
             else:
-                wqkv = self.cached(p + "qkv." + p_qkv, lambda: self.weight(w_qkv_raw(), precision=p_qkv))
+                wqkv = self.cached(p + "qkv." + p_qkv, lambda: self.weight(w_qkv_raw(), precision=p_qkv, wide=p_qkv == "nvfp4"))
                 bqkv = b_qkv_raw.to(torch.bfloat16).contiguous()
             quant_in_tile = padded_heads and p_out == "nvfp4"
             if quant_in_tile:
@@ -543,10 +560,10 @@ class NativePi0:
                 wo = self.cached(f"{p}out.{p_out}.{narrow(p_out)}", lambda: self.weight(sd[p + "self_attn.out_proj.weight"], block_n=narrow(p_out), precision=p_out))
             bo = sd[p + "self_attn.out_proj.bias"].to(torch.bfloat16).contiguous()
             if fold2:
-                w1 = self.cached(p + "fc1.nvfp4.ln", lambda: self.weight(folded(sd[p + "mlp.fc1.weight"], sd[p + "mlp.fc1.bias"], g2, b2)[0], row_sums=True))
+                w1 = self.cached(p + "fc1.nvfp4.ln", lambda: self.weight(folded(sd[p + "mlp.fc1.weight"], sd[p + "mlp.fc1.bias"], g2, b2)[0], wide=True, row_sums=True))
                 bias1 = folded(sd[p + "mlp.fc1.weight"], sd[p + "mlp.fc1.bias"], g2, b2, mlp_pad)[1]
             else:
-                w1 = self.cached(p + "fc1." + p_fc1, lambda: self.weight(sd[p + "mlp.fc1.weight"], precision=p_fc1))
+                w1 = self.cached(p + "fc1." + p_fc1, lambda: self.weight(sd[p + "mlp.fc1.weight"], precision=p_fc1, wide=p_fc1 == "nvfp4"))
                 bias1 = torch.zeros(mlp_pad, device=self.device, dtype=torch.bfloat16)
                 bias1[:c.vision_mlp] = sd[p + "mlp.fc1.bias"].to(torch.bfloat16)
             w2 = self.cached(f"{p}fc2.{p_fc2}.{narrow(p_fc2)}", lambda: self.weight(sd[p + "mlp.fc2.weight"], block_n=narrow(p_fc2), precision=p_fc2))
@@ -559,7 +576,7 @@ class NativePi0:
                 s_ln, ln1 = self.norm(f"vision.{i}.ln1", xa, a_ln.only(p_qkv), rows=M, sources=[(s_x, SAME)], kind="layer", gamma=g1,
                                       beta=b1, eps=c.ln_eps), None
             s_qkv = self.gemm(f"vision.{i}.qkv", a_ln, wqkv, rows=M, sources=[(s_ln, SAME)], out=buf, bias=bqkv,
-                              head_pad=(hd, pitch) if padded_heads else None, row_ln=ln1)
+                              head_pad=(hd, pitch) if padded_heads else None, block_n=self.tile_width(2 * V, wqkv), row_ln=ln1)
             h = C.c_void_p()
             q, k, v = buf[:, :WP], buf[:, WP:2 * WP], buf[:, 2 * WP:]
             _native.check(lib.create_attention(C.byref(h), q.data_ptr(), k.data_ptr(), v.data_ptr(), None, None, None, None, None,
@@ -589,7 +606,7 @@ class NativePi0:
                 s_ln2, ln2 = self.norm(f"vision.{i}.ln2", xb, a_ln2.only(p_fc1), rows=M, sources=[(s_o, SAME)], kind="layer", gamma=g2,
                                        beta=b2, eps=c.ln_eps), None
             s_fc1 = self.gemm(f"vision.{i}.fc1", a_ln2, w1, rows=M, sources=[(s_ln2, SAME)], out_act=a_h.require(p_fc2), out_precision=p_fc2,
-                              bias=bias1, activation=1, act_cols=c.vision_mlp, row_ln=ln2)
+                              bias=bias1, activation=1, act_cols=c.vision_mlp, block_n=self.tile_width(2 * V, w1), row_ln=ln2)
             s_x = self.gemm(f"vision.{i}.fc2", a_h, w2, rows=M, sources=[(s_fc1, SAME)], out=xa, bias=bias2, residual=xb,
                             block_n=narrow(p_fc2),
                             stream=(a_ln.require("nvfp4"), stats("vision.sumsq1"), stats("vision.sum1")) if fold1_next else None)

@@ -68,6 +68,16 @@ def narrow_tile_scales(swizzled, rows, blocks):
     return narrow.reshape(-1)
 
 
+def wide_tile_scales(swizzled, rows, blocks):
+    """Weight scales for 192-wide output tiles: from the standard layout (as in ``narrow_tile_scales``; ``rows`` a multiple of 128) to
+    two atoms per (192-row tile, group of four blocks) with the tile's rows in order and zeros behind; whole tiles only."""
+    atoms, groups, tiles = rows // 128, blocks // 4, rows // 192
+    pieces = swizzled.view(atoms, groups, 32, 4, 4).permute(0, 3, 1, 2, 4).reshape(atoms * 4, groups, 32, 4)[:tiles * 6]   # [32-row piece, group, row, block]
+    wide = torch.zeros((tiles, 8, groups, 32, 4), dtype=torch.uint8, device=swizzled.device)
+    wide[:, :6] = pieces.view(tiles, 6, groups, 32, 4)
+    return wide.view(tiles, 2, 4, groups, 32, 4).permute(0, 3, 1, 4, 2, 5).reshape(-1)
+
+
 class ResidentNVFP4:
     def __init__(self, library, activation, weight, *, workers=16, device="cuda",
                  output_dtype=torch.float32, bias=None, residual=None,
@@ -93,6 +103,10 @@ class ResidentNVFP4:
                 if k % 64:
                     raise ValueError("32-wide tiles need K to be a multiple of 64")
                 self.sb = narrow_tile_scales(self.sb, n, k // 16)
+            elif block_n == 192:
+                if k % 64 or n % 192:
+                    raise ValueError("192-wide tiles need K to be a multiple of 64 and N of 192")
+                self.sb = wide_tile_scales(self.sb, n, k // 16)
             if kind == "fp4":
                 self.output = packed_tma_buffer((m, self.output_width // 2), device=self.device)
                 atoms = ((m + 127) // 128) * ((self.output_width // 16 + 3) // 4)

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 from native_pi0 import _native
 from native_pi0.attention import ResidentAttention
 from native_pi0.normalization import ResidentNorm
-from native_pi0.primitives import ResidentNVFP4
+from native_pi0.primitives import ResidentNVFP4, wide_tile_scales
 from native_pi0.quantization import PackedNVFP4, interleave_gate_up, pack_nvfp4, swizzle_scales, unswizzle_scales
 from oracle import nvfp4 as oracle
 from oracle import ops as oracle_ops
@@ -414,6 +414,94 @@ def test_gemm_qkv_rope_epilogue():
     got_v = cv[50:50 + rows].float().cpu().numpy()
     assert relrms(got_v, y[:, (heads + 1) * hd:].float().numpy()) < 4e-3
     assert (ck[:50] == 7).all() and (ck[50 + rows:] == 7).all() and not qout[rows:].any()
+
+
+@pytest.mark.parametrize("m,k,rows", [(128, 64, 1), (256, 1152, 200), (384, 768, 384)])
+def test_wide_tiles_give_the_bits_of_narrow_ones(m, k, rows):
+    """192-wide tiles under every epilogue, one and several per worker, against 128-wide ones: the sums over K are the same.
+    With fewer logical columns than the weight has rows the last tile is cut, and nothing beyond is stored."""
+    from native_pi0.dense import ResidentDense
+    lib = _native.load()
+    rng = np.random.default_rng(m + k)
+    n = 768
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    bias = bf16(rng.normal(size=n))
+    res = bf16(rng.normal(size=(m, n)))
+    for kind in (dict(output_dtype=torch.bfloat16, bias=bias), dict(output_dtype=torch.bfloat16, residual=res), dict(output_dtype=torch.uint8),
+                 dict(output_dtype=torch.uint8, output_gelu=True, bias=bias)):
+        outs = []
+        for block_n, workers in ((128, 148), (192, 148), (192, 3), (192, 1)):
+            with ResidentNVFP4(None, pa, pb, workers=workers, rows=rows, block_n=block_n, **kind) as op:
+                op.output.zero_()
+                y = op.forward().clone()
+                assert op.status()["code"] == 0
+                outs.append((y, op.output_scales.clone() if y.dtype == torch.uint8 else None))
+        for y, sc in outs[1:]:
+            assert torch.equal(y, outs[0][0]) and (sc is None or torch.equal(sc, outs[0][1]))
+    cols = 640                                              # three whole tiles and a third of one
+    with ResidentNVFP4(None, pa, pb, workers=148, rows=rows, output_dtype=torch.uint8, output_gelu=True, bias=bias) as whole:
+        codes = whole.forward()
+        scales = unswizzle_scales(whole.output_scales.cpu().numpy(), m, n // 16)
+        cols = 640                                          # three whole tiles and a third of one
+        sb = wide_tile_scales(whole.sb, n, k // 16)
+        for block_n in (192, 128):
+            out = torch.full((m * n // 2,), 0xee, dtype=torch.uint8, device="cuda")
+            out_scales = torch.zeros(m * n // 16, dtype=torch.uint8, device="cuda")
+            handle = C.c_void_p()
+            _native.check(lib.create_resident_fp4(C.byref(handle), whole.a.data_ptr(), whole.b.data_ptr(), whole.sa.data_ptr(),
+                                                  (sb if block_n == 192 else whole.sb).data_ptr(), out.data_ptr(), m, n, k, 5,
+                                                  float(whole.activation_global_scale * whole.weight_global_scale)), "create")
+            _native.check(lib.configure_resident_fp4_quantized(handle, whole.bias.data_ptr(), None, out.data_ptr(), out_scales.data_ptr(), 1.0, 1), "quantized")
+            _native.check(lib.configure_resident_fp4_rows(handle, rows), "rows")
+            for bad in (0, 96, n + 128):
+                assert lib.configure_resident_fp4_columns(handle, bad) == 1
+            _native.check(lib.configure_resident_fp4_columns(handle, cols), "columns")
+            _native.check(lib.configure_resident_fp4_tile(handle, block_n), "tile")
+            _native.check(lib.launch_resident_fp4(handle, torch.cuda.current_stream().cuda_stream), "launch")
+            torch.cuda.synchronize()
+            assert torch.equal(out[:rows * cols // 2].view(rows, cols // 2), codes[:rows, :cols // 2]) and (out[rows * cols // 2:] == 0xee).all()
+            got = unswizzle_scales(out_scales[:m * cols // 16].cpu().numpy(), m, cols // 16)
+            np.testing.assert_array_equal(got[:rows], scales[:rows, :cols // 16])
+            _native.check(lib.destroy_resident_fp4(handle), "destroy")
+        for bad in (96, 256):
+            assert lib.configure_resident_fp4_tile(whole.handle, bad) == 1
+    with pytest.raises(RuntimeError):                       # FP32 rows have no form of the drain for such tiles
+        ResidentNVFP4(None, pa, pb, block_n=192)
+    with ResidentDense(None, torch.zeros(8, 64).bfloat16(), torch.zeros(768, 64).bfloat16()) as dense:
+        assert lib.configure_resident_fp4_tile(dense.handle, 192) == 1
+
+
+def test_tile_widths_mixed_on_one_worker():
+    """Projections that use the accumulator buffers differently (tiles of up to 128 columns one each, NVFP4 tiles of 192 both) one
+    after the other on the same workers, from odd and from even uses."""
+    from native_pi0.dense import ResidentDense
+    from native_pi0.linear import NativeStageProgram
+    lib = _native.load()
+    rng = np.random.default_rng(5)
+    m, n, k = 256, 768, 512
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    a, b = (torch.from_numpy(rng.normal(size=s).astype(np.float32)).cuda().bfloat16() for s in ((m, k), (n, k)))
+    ops, want = [], []
+    for block_n, dense in ((128, False), (64, True), (64, False), (192, False), (128, True), (192, False), (192, False), (64, True), (64, False)) * 2:
+        if dense:
+            op = ResidentDense(None, a, b, output_dtype=torch.float32, workers=148)
+            _native.check(lib.configure_resident_fp4_tile(op.handle, block_n), "tile")
+        else:
+            op = ResidentNVFP4(None, pa, pb, workers=148, output_dtype=torch.bfloat16, block_n=block_n)
+        want.append(op.forward().clone())
+        ops.append(op)
+    assert all(torch.equal(w, want[0 if w.dtype == torch.bfloat16 else 1]) for w in want)
+    for workers in (5, 3, 1):
+        for op in ops:
+            op.output.zero_()
+        with NativeStageProgram(None, [(op, []) for op in ops], workers=workers) as program:
+            program.forward()
+            assert program.status()["code"] == 0
+        assert all(torch.equal(op.output, w) for op, w in zip(ops, want))
+    for op in ops:
+        op.close()
 
 
 @pytest.mark.parametrize("rows,heads,block_n", [(1, 2, 64), (51, 2, 64), (128, 1, 128), (129, 2, 128), (321, 0, 128), (384, 1, 32)])

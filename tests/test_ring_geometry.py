@@ -60,3 +60,33 @@ def test_cursors_stay_inside_the_ring_of_a_mixed_expert(ring, actions, dense):
             for _ in range(count * slots):
                 assert cursor < stages, (worker, stage, op)
                 cursor = 0 if cursor + 1 == stages else cursor + 1
+
+
+def test_wide_tiles_have_rings_that_fit(ring):
+    """192-wide NVFP4 tiles: slots that fit, and a key that no other ring shares."""
+    for rows in (1, 64, 65, 128, 768):
+        stride, stages, key = ring(NVFP4, rows, 192)
+        assert 2 <= stages <= 5 and stages * stride <= DATA_BYTES and stride % 1024 == 0
+        for operands in (NVFP4, BF16, FP8):
+            for other in (1, 64, 65, 128, 768):
+                for width in (128, 64, 32):
+                    assert ring(operands, other, width)[2] != key or ring(operands, other, width)[:2] == (stride, stages)
+
+
+@pytest.mark.parametrize("rows,blocks", [(384, 4), (768, 72), (4608, 8)])
+def test_scales_of_wide_tiles(rows, blocks):
+    """Row r of 192-wide tile t, block b, lies where two standard atoms of 128 rows hold it; the rest is zero."""
+    import numpy as np
+    import torch
+    from native_pi0.primitives import wide_tile_scales
+    from native_pi0.quantization import scale_offsets
+    standard = torch.from_numpy(np.random.default_rng(rows).integers(1, 255, size=rows * blocks, dtype=np.uint8))
+    wide = wide_tile_scales(standard, rows, blocks).numpy()
+    matrix = standard.numpy()[scale_offsets(rows, blocks)].reshape(rows, blocks)
+    assert wide.size == rows // 192 * (blocks // 4) * 1024
+    r, b = np.meshgrid(np.arange(rows), np.arange(blocks), indexing="ij")
+    inside = r % 192
+    where = ((r // 192 * (blocks // 4) + b // 4) * 2 + inside // 128) * 512 + inside % 32 * 16 + inside % 128 // 32 * 4 + b % 4
+    np.testing.assert_array_equal(wide[where], matrix)
+    wide[where] = 0
+    assert not wide.any()
