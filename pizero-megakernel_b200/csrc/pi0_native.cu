@@ -113,7 +113,9 @@ struct Op {
     const void *a = nullptr, *b = nullptr;
     int m = 0, n = 0, k = 0;
     int operands = GEMM_NVFP4;
-    CUtensorMap* maps = nullptr;       // device: [0] = A, [1] = B
+    CUtensorMap* maps = nullptr;       // device: [0] = A, [1] = B, [2] = B with boxes of the stand-alone launch's tile width
+    int solo_width = 0;                // that width
+    bool tile_given = false;           // the caller has chosen a tile width
     // attention bookkeeping
     Op* merge = nullptr;               // owned merge stage (splits > 1)
     uint16_t* partial_o = nullptr;
@@ -444,39 +446,66 @@ int ring_layout(GemmParams& g, int operands) {
     return cudaSuccess;
 }
 
+// Everything of a GEMM stage that follows from its tile width.
+int gemm_tiles(StageDesc& d, int operands, int m, int block_n) {
+    GemmParams& g = d.p.gemm;
+    g.block_n = block_n;
+    g.m_tiles = m / 128;
+    g.n_tiles = (g.cols + block_n - 1) / block_n;
+    if (int e = ring_layout(g, operands)) return e;
+    // tcgen05 instruction descriptor: operand formats at bits 7 and 10 (block-scaled kind: 1 = E2M1; kind::f16: 1 = BF16;
+    // kind::f8f6f4: 0 = E4M3), FP32 accumulator (bit 4) for the dense kinds, N / 8 at bit 17, M / 16 at bit 24; both
+    // operands K-major.
+    const uint32_t fmt = operands == GEMM_FP8 ? 0u : 1u;
+    const uint32_t acc_f32 = operands == GEMM_NVFP4 ? 0u : (1u << 4);
+    g.idesc = acc_f32 | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(block_n >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
+    d.tiles = g.m_tiles * g.n_tiles;
+    d.bands = g.m_tiles;
+    d.band_div = g.n_tiles;
+    return cudaSuccess;
+}
+
+// Tile width of a dense projection that is launched by itself and has not been given one (in a program of several stages it keeps 128).
+// Such a launch is paid by the operand rows that an SM takes in, A's and the tile's own for every tile it gets, and every width
+// gives the same sums over K.  The estimate picks the fastest width in all that were measured (us back to back, 128 / 64 / 32 columns):
+// BF16 333 x 1000 x 1152 9.3 / 8.7 / 8.1, 20 x 4352 x 4352 25.5 / 20.6 / 17.5, 768 x 1152 x 4352 25.2 / 19.8 / 24.0, 500 x 1700 x 1000 9.7 /
+// 9.1 / 10.3, 820 x 2048 x 2048 16.6 / 19.0 / 23.4; FP8 50 x 500 x 4352 11.8 / 9.9 / 8.7, 768 x 2048 x 4096 16.5 / 18.7 / 20.5.
+int solo_tile_width(const Op* op) {
+    const GemmParams& g = op->desc.p.gemm;
+    if (op->operands == GEMM_NVFP4 || op->tile_given || g.b_tiled || g.epilogue == EPI_STREAM) return g.block_n;
+    int best = 128, least = 0;
+    for (const int width : {128, 64, 32}) {
+        const int tiles = op->m / 128 * ((g.cols + width - 1) / width);
+        const int rows = (tiles + op->workers - 1) / op->workers * (g.a_box_rows + width);
+        if (!least || rows < least) { best = width; least = rows; }
+    }
+    return best;
+}
+
 int gemm_refresh(Op* op) {
     GemmParams& g = op->desc.p.gemm;
-    CUtensorMap host[2];
+    CUtensorMap host[3];
     const size_t row_bytes = operand_row_bytes(op->operands, op->k);
-    const int n_tiles = (g.cols + g.block_n - 1) / g.block_n;
-    if (n_tiles * g.block_n > op->n) return cudaErrorInvalidValue;        // (the weight has rows for whole tiles)
+    if ((g.cols + g.block_n - 1) / g.block_n * g.block_n > op->n) return cudaErrorInvalidValue;        // (the weight has rows for whole tiles)
     int e = encode_operand(&host[0], op->a, op->m, row_bytes, g.a_box_rows);
     if (!e) e = g.b_tiled ? encode_tiled(&host[1], op->b, op->n * static_cast<int>(row_bytes / 128), kChunks * g.block_n)
                           : encode_operand(&host[1], op->b, op->n, row_bytes, g.block_n);
+    op->solo_width = solo_tile_width(op);
+    host[2] = host[1];
+    if (!e && op->solo_width != g.block_n) e = encode_operand(&host[2], op->b, op->n, row_bytes, op->solo_width);
     if (e) return e;
     if (!op->maps) {
-        cudaError_t ce = cudaMalloc(&op->maps, 2 * sizeof(CUtensorMap));
+        cudaError_t ce = cudaMalloc(&op->maps, 3 * sizeof(CUtensorMap));
         if (ce != cudaSuccess) return ce;
     }
     cudaError_t ce = cudaMemcpy(op->maps, host, sizeof(host), cudaMemcpyHostToDevice);
     if (ce != cudaSuccess) return ce;
     g.tmap_a = op->maps;
     g.tmap_b = op->maps + 1;
-    g.m_tiles = op->m / 128;
-    g.n_tiles = n_tiles;
-    if (!g.sum_out || g.sumsq_ld < g.n_tiles) g.sumsq_ld = g.n_tiles;      // statistics rows: one slot per column tile
     g.operands = op->operands;
     g.k_groups = static_cast<int>(row_bytes / 32);
-    if ((e = ring_layout(g, op->operands))) return e;
-    // tcgen05 instruction descriptor: operand formats at bits 7 and 10 (block-scaled kind: 1 = E2M1; kind::f16: 1 = BF16;
-    // kind::f8f6f4: 0 = E4M3), FP32 accumulator (bit 4) for the dense kinds, N / 8 at bit 17, M / 16 at bit 24; both
-    // operands K-major.
-    const uint32_t fmt = op->operands == GEMM_FP8 ? 0u : 1u;
-    const uint32_t acc_f32 = op->operands == GEMM_NVFP4 ? 0u : (1u << 4);
-    g.idesc = acc_f32 | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(g.block_n >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
-    op->desc.tiles = g.m_tiles * g.n_tiles;
-    op->desc.bands = g.m_tiles;
-    op->desc.band_div = g.n_tiles;
+    if ((e = gemm_tiles(op->desc, op->operands, op->m, g.block_n))) return e;
+    if (!g.sum_out || g.sumsq_ld < g.n_tiles) g.sumsq_ld = g.n_tiles;      // statistics rows: one slot per column tile
     op->cost = op->k;
     op->solo_dirty = true;
     return cudaSuccess;
@@ -496,8 +525,15 @@ int solo_program(Op* op) {
         self.src[0] = 0;
         self.src_mode[0] = SRC_ALL_BANDS;
     }
+    if (self.kind == OP_GEMM) {
+        const int width = solo_tile_width(op);             // (not the one encoded: the epilogue has been changed since)
+        if (width == op->solo_width && width != self.p.gemm.block_n) {
+            if (int e = gemm_tiles(self, op->operands, op->m, width)) return e;
+            self.p.gemm.tmap_b = op->maps + 2;
+        }
+    }
     stages.push_back(self);
-    work.push_back({op->desc.tiles, op->cost});
+    work.push_back({self.tiles, op->cost});
     if (op->merge && !op->desc.p.attn.fused_merge) {
         StageDesc m = op->merge->desc;
         m.src[0] = static_cast<int>(stages.size()) - 1;
@@ -748,6 +784,7 @@ extern "C" int configure_resident_fp4_tile(void* handle, int block_n) {
             return cudaErrorInvalidValue;
     }
     g.block_n = block_n;
+    op->tile_given = true;
     return gemm_refresh(op);
 }
 // extension: logical columns of the output, whole 128-column tiles and not more than N: the weight's rows beyond only fill up the
@@ -927,6 +964,7 @@ extern "C" int configure_dense_tile(void* handle, int block_n) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_GEMM || op->operands == GEMM_NVFP4 || (block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
     op->desc.p.gemm.block_n = block_n;
+    op->tile_given = true;
     return gemm_refresh(op);
 }
 

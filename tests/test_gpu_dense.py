@@ -9,6 +9,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from native_pi0 import _native
 from native_pi0.dense import ResidentDense, head_order
 from native_pi0.linear import NativeStageProgram
 from oracle import ops as oracle_ops
@@ -194,3 +195,29 @@ def test_two_dense_stages_in_one_launch():
             got = program.forward()
             assert program.status()["code"] == 0
             assert torch.equal(got[:m, :n1], want)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 100, 504), (64, 640, 520), (65, 96, 1000), (333, 1000, 1152), (500, 1700, 512), (768, 1152, 640), (300, 4400, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float8_e4m3fn])
+def test_stand_alone_tile_width_gives_the_same_bits(m, n, k, dtype):
+    """A dense projection launched by itself picks its tile width; with a width given, or as a stage of a program, the result is the
+    same bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")          # noqa: E731
+    a, b, bias, res = randn(m, k).to(dtype), randn(n, k).to(dtype), randn(n), randn(m, n)
+    for kind in (dict(output_dtype=torch.float32), dict(bias=bias, residual=res)):
+        with ResidentDense(None, a, b, alpha=0.05, **kind) as op:
+            want = op.forward().clone()
+            assert op.status()["code"] == 0
+            exact = 0.05 * a.double() @ b.double().T
+            if kind.get("output_dtype") == torch.float32:                  # (products and sums in FP32: 2^-24 per addition of K terms)
+                bound = 2.0 ** -22 * (k ** 0.5) * (0.05 * a.double().abs() @ b.double().abs().T)
+                assert bool(((want.double() - exact).abs() <= bound).all())
+            with NativeStageProgram(None, [(op, [])]) as program:
+                op.output.zero_()
+                program.forward()
+                assert program.status()["code"] == 0 and torch.equal(op.logical_output, want)
+            for width in (128, 64, 32):
+                _native.check(_native.load().configure_dense_tile(op.handle, width), "tile")
+                op.output.zero_()
+                assert torch.equal(op.forward(), want)
