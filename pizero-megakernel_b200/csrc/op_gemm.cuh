@@ -761,8 +761,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
 // drain, as one of the draining warps or as a helper of the last tile.
 // LEAN: the kernel variant for programs made only of NVFP4 projections with the pi0 model's epilogues (the host checks
 // this when it builds a program); it carries neither the dense issue loops nor the other drain loops.
-// WIDE: with the forms for 192-wide NVFP4 tiles.  The variant that BF16 models and most operators launch goes without (BF16 forward
-// 16.14 ms, 16.70 with them): programs that need both run the one with everything.
+// WIDE: with the forms for 192-wide NVFP4 tiles.
 template <bool LEAN, bool WIDE>
 __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl, uint8_t* data, uint32_t tmem,
                                                  const StageDesc& st, int stage_index, int first, int count,

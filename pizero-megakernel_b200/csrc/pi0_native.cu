@@ -314,6 +314,8 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             configured[device] = e == cudaSuccess;
         }
         prog->lean = true;
@@ -375,8 +377,10 @@ int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begi
     config.stream = stream;
     config.attrs = &serial;
     config.numAttrs = 1;
-    if (prog->lean && !prog->h_debug && !p.timings) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false>, p);
-    if (prog->lean && !prog->h_debug) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true>, p);
+    if (prog->lean && !prog->h_debug) {
+        if (prog->wide) return p.timings ? cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true, false, true>, p) : cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false, false, true>, p);
+        return p.timings ? cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true>, p) : cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false>, p);
+    }
     if (!prog->mma_sync && !prog->wide) return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true, false>, p);
     return cudaLaunchKernelEx(&config, pi0_vm_kernel<false, true, true>, p);
 }

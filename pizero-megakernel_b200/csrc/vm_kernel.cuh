@@ -52,7 +52,9 @@ __device__ __forceinline__ bool prefetch_slot(const VmProgram& prog, Ctl* ctl, c
 // MMA_SYNC = false: without the mma.sync attention tiles.  Their 128 accumulators per thread make the compiler spill, and the kernel
 // that spills there is slower everywhere (the same program on both: BF16 forward 17.34 and 16.17 ms, expert in BF16 13.88 and 12.80,
 // BF16 333 x 1000 x 1152 11.2 and 9.5 us, FP8 768 x 2048 x 16384 32.7 and 31.3), so only programs with such tiles carry them.
-template <bool LEAN, bool TIMED = true, bool MMA_SYNC = !LEAN>
+// WIDE = true: with the forms for 192-wide NVFP4 tiles, which three-view models run; the smaller kernel without them is faster for everything
+// else (one view 5.26 -> 5.23 ms, BF16 forward 16.70 -> 16.14, q|k|v of 51 rows 5.84 -> 5.75 us).
+template <bool LEAN, bool TIMED = true, bool MMA_SYNC = !LEAN, bool WIDE = MMA_SYNC>
 __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_constant__ VmProgram prog) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
         if (stamp && threadIdx.x == 0) stamp[0] = static_cast<long long>(global_ns());
         if (st.kind == OP_GEMM) {
             if constexpr (!LEAN) mark(prog, 800000 + ins.y);
-            gemm_instruction<LEAN, LEAN || MMA_SYNC>(prog, ctl, data, tmem, st, ins.y, ins.z, ins.w, ps, stamp);
+            gemm_instruction<LEAN, WIDE>(prog, ctl, data, tmem, st, ins.y, ins.z, ins.w, ps, stamp);
             // one decision per warp: the lanes with a role return later than the others and must not leave alone
             if (__any_sync(0xffffffffu, ctl->abort != 0)) break;
         } else {
