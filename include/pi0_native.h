@@ -80,12 +80,14 @@ int configure_resident_fp4_row_layernorm(void* handle, const float* sumsq, const
  * 16 r + b for row r, block b) and zeros elsewhere, i.e. four times the bytes of the standard layout.  Narrow tiles are
  * for projections of a few rows, whose time is the bytes one SM takes in and the serial epilogue of one tile.  192-wide NVFP4
  * tiles have two such atoms each, [tiles][K / 64][2][512], the tile's 192 rows in order and zeros behind; they are for
- * projections whose 128-wide tiles are a little more than one per SM, with BF16 or NVFP4 output (no GeGLU, no residual stream) and weights that are not tile-major. */
+ * projections whose 128-wide tiles are a little more than one per SM, with BF16 or NVFP4 output (no GeGLU, no residual stream, no
+ * fused q|k|v) and weights that are not tile-major.  Whichever of the calls comes last and does not go with the others returns
+ * cudaErrorInvalidValue and changes nothing. */
 int configure_resident_fp4_rows(void* handle, int rows);
 int configure_resident_fp4_tile(void* handle, int block_n);
 /* extension: logical columns of the output (whole 128-column tiles; at most N): the rows of the weight beyond only fill up the last
- * tile of another width.  The rows of the output are that many columns apart, the bias has that many values.  Behind the epilogue's
- * own call (BF16 or NVFP4 output, without GeGLU, a residual or padded heads) and before the tile width. */
+ * tile of another width.  The rows of the output are that many columns apart, the bias has that many values.  For BF16 or NVFP4
+ * output without GeGLU, a residual or padded heads, chosen before or afterwards; before a tile width of 192. */
 int configure_resident_fp4_columns(void* handle, int cols);
 /* extension: tiled = 1 declares that B is stored tile-major (rows of whole 128-byte pieces: K a multiple of 256 in NVFP4,
  * 64 in BF16, 128 in FP8): for every output tile n and every 128-byte piece s of K the block_n x 128 bytes of that block are

@@ -198,7 +198,7 @@ bool lean_stage(const StageDesc& d) {
     if (d.kind == OP_GEMM) {
         const GemmParams& g = d.p.gemm;
         const bool stats = g.row_sumsq || g.row_factor;     // (the lean residual-stream and plain BF16 drains read none)
-        if (stats && (g.epilogue == EPI_BF16 || g.epilogue == EPI_STREAM)) return false;
+        if (stats && (g.epilogue == EPI_STREAM || (g.epilogue == EPI_BF16 && g.block_n <= 128))) return false;     // (192: the extended drain)
         if (g.round_before_residual || g.gelu_cols > 0 || g.act == 3) return false;       // options the lean drains leave out
         if (g.epilogue == EPI_QKV_ROPE && !g.rope_table) return false;      // (the lean rotary drain reads the pair-major table only)
         return g.operands == GEMM_NVFP4 && (g.epilogue == EPI_BF16 || g.epilogue == EPI_STREAM || g.epilogue == EPI_GEGLU_FP4 ||
@@ -490,13 +490,13 @@ int gemm_refresh(Op* op) {
     GemmParams& g = op->desc.p.gemm;
     CUtensorMap host[3];
     const size_t row_bytes = operand_row_bytes(op->operands, op->k);
-    if ((g.cols + g.block_n - 1) / g.block_n * g.block_n > op->n) return cudaErrorInvalidValue;        // (the weight has rows for whole tiles)
-    int e = encode_operand(&host[0], op->a, op->m, row_bytes, g.a_box_rows);
+    int e = gemm_tiles(op->desc, op->operands, op->m, g.block_n);
+    if (!e) e = encode_operand(&host[0], op->a, op->m, row_bytes, g.a_box_rows);
     if (!e) e = g.b_tiled ? encode_tiled(&host[1], op->b, op->n * static_cast<int>(row_bytes / 128), kChunks * g.block_n)
                           : encode_operand(&host[1], op->b, op->n, row_bytes, g.block_n);
-    op->solo_width = solo_tile_width(op);
+    const int solo_width = solo_tile_width(op);
     host[2] = host[1];
-    if (!e && op->solo_width != g.block_n) e = encode_operand(&host[2], op->b, op->n, row_bytes, op->solo_width);
+    if (!e && solo_width != g.block_n) e = encode_operand(&host[2], op->b, op->n, row_bytes, solo_width);
     if (e) return e;
     if (!op->maps) {
         cudaError_t ce = cudaMalloc(&op->maps, 3 * sizeof(CUtensorMap));
@@ -508,9 +508,37 @@ int gemm_refresh(Op* op) {
     g.tmap_b = op->maps + 1;
     g.operands = op->operands;
     g.k_groups = static_cast<int>(row_bytes / 32);
-    if ((e = gemm_tiles(op->desc, op->operands, op->m, g.block_n))) return e;
+    op->solo_width = solo_width;
     if (!g.sum_out || g.sumsq_ld < g.n_tiles) g.sumsq_ld = g.n_tiles;      // statistics rows: one slot per column tile
     op->cost = op->k;
+    op->solo_dirty = true;
+    return cudaSuccess;
+}
+
+// Whether the parts of a GEMM stage go together: there are drains of 192-wide tiles for BF16 and NVFP4 rows only, and one that has no
+// form for its tiles would store another layout than the destination's.  Fewer logical columns than the weight has rows are for
+// the same outputs, without a residual or padded heads.
+bool gemm_parts_fit(const Op* op) {
+    const GemmParams& g = op->desc.p.gemm;
+    const bool plain_rows = g.epilogue == EPI_BF16 || g.epilogue == EPI_BF16_EXT || g.epilogue == EPI_FP4;
+    if (g.block_n > 128 && (op->operands != GEMM_NVFP4 || g.b_tiled || !plain_rows)) return false;   // (tile-major: a box has at most 256 rows)
+    if (g.cols < op->n && (!plain_rows || g.residual || (g.epilogue == EPI_BF16_EXT && g.pad_from))) return false;
+    return (g.cols + g.block_n - 1) / g.block_n * g.block_n <= op->n;                                // (the weight has rows for whole tiles)
+}
+
+// Every call that changes an epilogue, a tile width, logical rows or columns or the weight's layout goes through here, so that they go
+// together whatever the order of the calls.  A refused change leaves the operator as it was.  `refresh`: the tensor maps or tiles follow from it.
+template <typename Change>
+int gemm_configure(Op* op, bool refresh, Change change) {
+    const StageDesc before = op->desc;
+    const bool tile_given = op->tile_given;
+    change(op->desc.p.gemm);
+    const int e = !gemm_parts_fit(op) ? static_cast<int>(cudaErrorInvalidValue) : refresh ? gemm_refresh(op) : static_cast<int>(cudaSuccess);
+    if (e) {
+        op->desc = before;
+        op->tile_given = tile_given;
+        return e;
+    }
     op->solo_dirty = true;
     return cudaSuccess;
 }
@@ -641,13 +669,12 @@ extern "C" int launch_resident_fp4(void* handle, void* stream) {
 extern "C" int configure_resident_fp4_bf16(void* handle, const void* bias, const void* residual, void* out) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_GEMM || !out) return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    g.epilogue = EPI_BF16;
-    g.round_before_residual = 0; g.gelu_cols = 0; g.pad_from = 0; g.pad_to = 0;
-    g.bias = bias; g.residual = residual; g.ldr = op->n;
-    g.out = out; g.ldo = op->n;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_BF16;
+        g.round_before_residual = 0; g.gelu_cols = 0; g.pad_from = 0; g.pad_to = 0;
+        g.bias = bias; g.residual = residual; g.ldr = op->n;
+        g.out = out; g.ldo = g.cols;
+    });
 }
 extern "C" int configure_resident_fp4_quantized(void* handle, const void* bias, const void* residual, void* out, void* scales,
                                                 float global_scale, int activation) {
@@ -655,18 +682,17 @@ extern "C" int configure_resident_fp4_quantized(void* handle, const void* bias, 
     if (!op || op->desc.kind != OP_GEMM || !out || !scales || !std::isfinite(global_scale) || global_scale <= 0 ||
         activation < 0 || activation > 3)
         return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
     if (activation == 2 && (bias || residual || op->n % 256)) return cudaErrorInvalidValue;
-    const int width = activation == 2 ? op->n / 2 : op->n;
-    g.epilogue = activation == 2 ? EPI_GEGLU_FP4 : EPI_FP4;
-    g.act = activation == 2 ? 0 : activation;
-    g.bias = bias; g.residual = residual; g.ldr = op->n;
-    g.out = out; g.ldo = width / 2;
-    g.out_scales = static_cast<uint8_t*>(scales);
-    g.out_blocks = width / 16;
-    g.out_inv_gs = 1.f / global_scale;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        const int width = activation == 2 ? op->n / 2 : g.cols;
+        g.epilogue = activation == 2 ? EPI_GEGLU_FP4 : EPI_FP4;
+        g.act = activation == 2 ? 0 : activation;
+        g.bias = bias; g.residual = residual; g.ldr = op->n;
+        g.out = out; g.ldo = width / 2;
+        g.out_scales = static_cast<uint8_t*>(scales);
+        g.out_blocks = width / 16;
+        g.out_inv_gs = 1.f / global_scale;
+    });
 }
 extern "C" int configure_resident_fp4_qkv_rope(void* handle, void* out_q, int ldq, const void* cos, const void* sin,
                                                void* cache_k, void* cache_v, int q_cols, int head_dim, int cache_base) {
@@ -674,15 +700,14 @@ extern "C" int configure_resident_fp4_qkv_rope(void* handle, void* out_q, int ld
     if (!op || op->desc.kind != OP_GEMM || !cos || !sin || !cache_k || !cache_v || head_dim < 32 || head_dim % 32 ||
         q_cols < 0 || q_cols % head_dim || q_cols + 2 * head_dim != op->n || (q_cols && !out_q) || cache_base < 0)
         return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    g.epilogue = EPI_QKV_ROPE;
-    g.bias = nullptr; g.residual = nullptr;
-    g.out = out_q; g.ldo = ldq;
-    g.rope_cos = cos; g.rope_sin = sin; g.rope_table = nullptr;
-    g.cache_k = cache_k; g.cache_v = cache_v;
-    g.q_cols = q_cols; g.head_dim = head_dim; g.cache_base = cache_base;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_QKV_ROPE;
+        g.bias = nullptr; g.residual = nullptr;
+        g.out = out_q; g.ldo = ldq;
+        g.rope_cos = cos; g.rope_sin = sin; g.rope_table = nullptr;
+        g.cache_k = cache_k; g.cache_v = cache_v;
+        g.q_cols = q_cols; g.head_dim = head_dim; g.cache_base = cache_base;
+    });
 }
 // extension: the rotary tables of configure_*_qkv_rope in pair-major order, which a drain reads with adjacent lanes: entry [i][row] is
 // cos[row, i], cos[row, i + head_dim/2], sin[row, i], sin[row, i + head_dim/2] in BF16 (8 bytes), `ld` rows per pair, a multiple of 128
@@ -704,20 +729,19 @@ extern "C" int configure_resident_fp4_stream(void* handle, const void* bias, con
     if (!op || op->desc.kind != OP_GEMM || !out || !copy_fp4 || !copy_scales || !sumsq || !std::isfinite(copy_global_scale) ||
         copy_global_scale <= 0 || !aligned16(out) || !aligned16(copy_fp4) || !aligned16(bias) || !aligned16(residual) || !aligned16(sumsq))
         return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    g.epilogue = EPI_STREAM;
-    g.round_before_residual = 0; g.gelu_cols = 0;
-    g.bias = bias; g.residual = residual; g.ldr = op->n;
-    g.out = out; g.ldo = op->n;
-    g.copy_fp4 = static_cast<uint8_t*>(copy_fp4); g.ld_copy = op->n / 2;
-    g.out_scales = static_cast<uint8_t*>(copy_scales);
-    g.out_blocks = op->n / 16;
-    g.out_inv_gs = 1.f / copy_global_scale;
-    g.sumsq_out = sumsq;
-    g.sum_out = nullptr;
-    g.sumsq_ld = op->n / g.block_n;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_STREAM;
+        g.round_before_residual = 0; g.gelu_cols = 0;
+        g.bias = bias; g.residual = residual; g.ldr = op->n;
+        g.out = out; g.ldo = op->n;
+        g.copy_fp4 = static_cast<uint8_t*>(copy_fp4); g.ld_copy = op->n / 2;
+        g.out_scales = static_cast<uint8_t*>(copy_scales);
+        g.out_blocks = op->n / 16;
+        g.out_inv_gs = 1.f / copy_global_scale;
+        g.sumsq_out = sumsq;
+        g.sum_out = nullptr;
+        g.sumsq_ld = op->n / g.block_n;
+    });
 }
 // extension: a residual-stream projection also leaves the per-tile SUMS of its rounded rows (for a LayerNorm folded into
 // the projection that follows), and the row stride of both statistics arrays becomes ld floats (>= N / tile width, a multiple
@@ -766,43 +790,39 @@ extern "C" int configure_resident_fp4_row_layernorm(void* handle, const float* s
 extern "C" int configure_resident_fp4_rows(void* handle, int rows) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_GEMM || rows < 1 || rows > op->m) return cudaErrorInvalidValue;
-    op->desc.p.gemm.rows = rows;
-    op->desc.p.gemm.a_box_rows = a_box_rows_of(op->operands, op->m, rows);
-    return gemm_refresh(op);
+    return gemm_configure(op, true, [&](GemmParams& g) {
+        g.rows = rows;
+        g.a_box_rows = a_box_rows_of(op->operands, op->m, rows);
+    });
 }
 extern "C" int configure_resident_fp4_weight_layout(void* handle, int tiled) {
     Op* op = as_op(handle);
-    if (!op || op->desc.kind != OP_GEMM || (tiled != 0 && tiled != 1) || (tiled && operand_row_bytes(op->operands, op->k) % 128) ||
-        (tiled && op->desc.p.gemm.block_n > 128))              // (a box has at most 256 rows)
+    if (!op || op->desc.kind != OP_GEMM || (tiled != 0 && tiled != 1) || (tiled && operand_row_bytes(op->operands, op->k) % 128))
         return cudaErrorInvalidValue;
-    op->desc.p.gemm.b_tiled = tiled;
-    return gemm_refresh(op);
+    return gemm_configure(op, true, [&](GemmParams& g) { g.b_tiled = tiled; });
 }
 extern "C" int configure_resident_fp4_tile(void* handle, int block_n) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_GEMM || (block_n != 192 && block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    if (block_n == 192) {                                    // (the two epilogues whose drains have a form for such tiles)
-        if (g.epilogue == EPI_BF16) g.epilogue = EPI_BF16_EXT;
-        if (op->operands != GEMM_NVFP4 || g.b_tiled || (g.epilogue != EPI_FP4 && g.epilogue != EPI_BF16_EXT) || (g.cols + 191) / 192 * 192 > op->n)
-            return cudaErrorInvalidValue;
-    }
-    g.block_n = block_n;
-    op->tile_given = true;
-    return gemm_refresh(op);
+    return gemm_configure(op, true, [&](GemmParams& g) {
+        g.block_n = block_n;
+        op->tile_given = true;
+    });
 }
 // extension: logical columns of the output, whole 128-column tiles and not more than N: the weight's rows beyond only fill up the
-// last tile of another width.  Neither results nor bias exist for them, and the rows of the output are that many columns apart.
-// Behind the epilogue's own call (BF16 or NVFP4 output, without GeGLU, a residual or padded heads) and before the tile width.
+// last tile of another width.  Neither results nor bias exist for them, and the rows of the output are that many columns apart, also of
+// an epilogue that is set afterwards.  For BF16 or NVFP4 output without GeGLU, a residual or padded heads; before a tile width of 192.
 extern "C" int configure_resident_fp4_columns(void* handle, int cols) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_GEMM || cols < 128 || cols % 128 || cols > op->n) return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    if ((g.epilogue != EPI_FP4 && g.epilogue != EPI_BF16 && g.epilogue != EPI_BF16_EXT) || g.residual || g.pad_from || g.block_n > 128) return cudaErrorInvalidValue;
-    g.cols = cols;
-    g.ldo = g.epilogue == EPI_FP4 ? cols / 2 : cols;
-    if (g.epilogue == EPI_FP4) g.out_blocks = cols / 16;
-    return gemm_refresh(op);
+    const GemmParams& now = op->desc.p.gemm;
+    if ((now.epilogue != EPI_FP4 && now.epilogue != EPI_BF16 && now.epilogue != EPI_BF16_EXT) || now.residual || now.pad_from || now.block_n > 128)
+        return cudaErrorInvalidValue;
+    return gemm_configure(op, true, [&](GemmParams& g) {
+        g.cols = cols;
+        g.ldo = g.epilogue == EPI_FP4 ? cols / 2 : cols;
+        if (g.epilogue == EPI_FP4) g.out_blocks = cols / 16;
+    });
 }
 extern "C" int resident_fp4_resources(void* handle, int* values, int count) {
     Op* op = as_op(handle);
@@ -881,32 +901,32 @@ extern "C" int configure_dense_round_before_residual(void* handle) {
     Op* op = dense_bf16(handle);
     const bool plain = op && (op->desc.p.gemm.epilogue == EPI_BF16 || op->desc.p.gemm.epilogue == EPI_BF16_EXT);
     if (!plain || !op->desc.p.gemm.residual) return cudaErrorInvalidValue;
-    op->desc.p.gemm.epilogue = EPI_BF16_EXT;
-    op->desc.p.gemm.round_before_residual = 1;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_BF16_EXT;
+        g.round_before_residual = 1;
+    });
 }
 extern "C" int configure_dense_geglu(void* handle, void* compact_output) {
     Op* op = dense_bf16(handle);
     if (!op || !compact_output || !aligned16(compact_output)) return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    if (g.epilogue != EPI_BF16 || g.bias || g.residual || op->n % 256) return cudaErrorInvalidValue;
-    g.epilogue = EPI_GEGLU_BF16;
-    g.out = compact_output;
-    g.ldo = op->n / 2;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    const GemmParams& now = op->desc.p.gemm;
+    if (now.epilogue != EPI_BF16 || now.bias || now.residual || op->n % 256) return cudaErrorInvalidValue;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_GEGLU_BF16;
+        g.out = compact_output;
+        g.ldo = op->n / 2;
+    });
 }
 extern "C" int configure_dense_gelu(void* handle, int logical_columns) {
     Op* op = dense_bf16(handle);
     if (!op) return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    if ((g.epilogue != EPI_BF16 && g.epilogue != EPI_BF16_EXT) || g.residual || logical_columns < 1 || logical_columns > op->n)
+    const GemmParams& now = op->desc.p.gemm;
+    if ((now.epilogue != EPI_BF16 && now.epilogue != EPI_BF16_EXT) || now.residual || logical_columns < 1 || logical_columns > op->n)
         return cudaErrorInvalidValue;
-    g.epilogue = EPI_BF16_EXT;
-    g.gelu_cols = logical_columns;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_BF16_EXT;
+        g.gelu_cols = logical_columns;
+    });
 }
 extern "C" int configure_dense_rms_factor(void* handle, const float* factors) {
     Op* op = dense_bf16(handle);
@@ -920,10 +940,10 @@ extern "C" int configure_dense_rms_factor(void* handle, const float* factors) {
 extern "C" int configure_dense_skinny(void* handle) {
     Op* op = dense_bf16(handle);
     if (!op || op->m != 128) return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    g.a_box_rows = 64;                      // only 64 rows of A are copied per tile ...
-    g.rows = std::min(g.rows, 64);          // ... and only those rows are ever stored
-    return gemm_refresh(op);
+    return gemm_configure(op, true, [&](GemmParams& g) {
+        g.a_box_rows = 64;                      // only 64 rows of A are copied per tile ...
+        g.rows = std::min(g.rows, 64);          // ... and only those rows are ever stored
+    });
 }
 extern "C" int configure_dense_qkv_rope(void* handle, const void* cos, const void* sin, void* cache_k, void* cache_v,
                                         int logical_rows, int key_offset, int cache_base) {
@@ -931,30 +951,30 @@ extern "C" int configure_dense_qkv_rope(void* handle, const void* cos, const voi
     if (!op || !cos || !sin || !cache_k || !cache_v || logical_rows < 1 || key_offset < 0 || key_offset % 256 || cache_base < 0 ||
         !aligned16(cos) || !aligned16(sin) || !aligned16(cache_k) || !aligned16(cache_v))
         return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    if (g.epilogue != EPI_BF16 || g.bias || g.residual || logical_rows > op->m || key_offset + 512 != op->n)
+    const GemmParams& now = op->desc.p.gemm;
+    if (now.epilogue != EPI_BF16 || now.bias || now.residual || logical_rows > op->m || key_offset + 512 != op->n)
         return cudaErrorInvalidValue;
-    g.epilogue = EPI_QKV_ROPE;
-    g.rope_cos = cos; g.rope_sin = sin; g.rope_table = nullptr;
-    g.cache_k = cache_k; g.cache_v = cache_v;
-    g.q_cols = key_offset; g.head_dim = 256; g.cache_base = cache_base;
-    g.rows = std::min(g.rows, logical_rows);
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_QKV_ROPE;
+        g.rope_cos = cos; g.rope_sin = sin; g.rope_table = nullptr;
+        g.cache_k = cache_k; g.cache_v = cache_v;
+        g.q_cols = key_offset; g.head_dim = 256; g.cache_base = cache_base;
+        g.rows = std::min(g.rows, logical_rows);
+    });
 }
 // extension: store the BF16 output with every group of `from` columns (a head) starting `to` columns after the previous
 // one, in rows of `ld` elements; the columns between the heads are not written (keep them zero).  No residual.
 extern "C" int configure_dense_head_pad(void* handle, int from, int to, int ld) {
     Op* op = dense_bf16(handle);
     if (!op) return cudaErrorInvalidValue;
-    GemmParams& g = op->desc.p.gemm;
-    if ((g.epilogue != EPI_BF16 && g.epilogue != EPI_BF16_EXT) || g.residual || from < 8 || from % 8 || to < from || to % 8 ||
+    const GemmParams& now = op->desc.p.gemm;
+    if ((now.epilogue != EPI_BF16 && now.epilogue != EPI_BF16_EXT) || now.residual || from < 8 || from % 8 || to < from || to % 8 ||
         ld < (op->n + from - 1) / from * to || ld % 8)
         return cudaErrorInvalidValue;
-    g.epilogue = EPI_BF16_EXT;
-    g.pad_from = from; g.pad_to = to; g.ldo = ld;
-    op->solo_dirty = true;
-    return cudaSuccess;
+    return gemm_configure(op, false, [&](GemmParams& g) {
+        g.epilogue = EPI_BF16_EXT;
+        g.pad_from = from; g.pad_to = to; g.ldo = ld;
+    });
 }
 // extension: logical rows (as configure_resident_fp4_rows) and output tile width of a dense projection.
 extern "C" int configure_dense_rows(void* handle, int rows) {
@@ -967,9 +987,10 @@ extern "C" int configure_dense_rows(void* handle, int rows) {
 extern "C" int configure_dense_tile(void* handle, int block_n) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_GEMM || op->operands == GEMM_NVFP4 || (block_n != 128 && block_n != 64 && block_n != 32)) return cudaErrorInvalidValue;
-    op->desc.p.gemm.block_n = block_n;
-    op->tile_given = true;
-    return gemm_refresh(op);
+    return gemm_configure(op, true, [&](GemmParams& g) {
+        g.block_n = block_n;
+        op->tile_given = true;
+    });
 }
 
 // =====================================================================================================

@@ -472,6 +472,72 @@ def test_wide_tiles_give_the_bits_of_narrow_ones(m, k, rows):
         assert lib.configure_resident_fp4_tile(dense.handle, 192) == 1
 
 
+def test_epilogues_behind_a_width_or_columns_that_they_do_not_go_with():
+    """An epilogue without a drain for 192-wide tiles, or for fewer columns than the weight has rows, is refused when it comes behind
+    them too, and a refused call leaves the operator as it was.  (Nothing that is refused is launched.)"""
+    from native_pi0.dense import ResidentDense
+    lib = _native.load()
+    rng = np.random.default_rng(11)
+    m, n, k, cols = 128, 768, 256, 640
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    out, other, res = (torch.zeros(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    codes, scales, sums = (torch.zeros(m * n, dtype=torch.uint8, device="cuda") for _ in range(3))
+    tables = torch.zeros(4, m, 256, dtype=torch.bfloat16, device="cuda")
+
+    def refused(h, plain):
+        """Each epilogue without such a form; ``plain`` puts the BF16 rows back behind the one that starts from them."""
+        assert lib.configure_resident_fp4_quantized(h, None, None, codes.data_ptr(), scales.data_ptr(), 1.0, 2) == 1
+        assert lib.configure_resident_fp4_stream(h, None, None, other.data_ptr(), codes.data_ptr(), scales.data_ptr(), 1.0, sums.data_ptr()) == 1
+        assert lib.configure_resident_fp4_qkv_rope(h, other.data_ptr(), n, *[t.data_ptr() for t in tables], 256, 256, 0) == 1
+        plain()
+        assert lib.configure_dense_geglu(h, other.data_ptr()) == 1
+        assert lib.configure_dense_qkv_rope(h, *[t.data_ptr() for t in tables], m, 256, 0) == 1
+
+    with ResidentNVFP4(None, pa, pb, workers=148, output_dtype=torch.bfloat16, block_n=192) as op:
+        want = op.forward().clone()
+        refused(op.handle, lambda: _native.check(lib.configure_resident_fp4_bf16(op.handle, None, None, op.output.data_ptr()), "bf16"))
+        assert lib.configure_resident_fp4_weight_layout(op.handle, 1) == 1
+        op.output.zero_()
+        assert torch.equal(op.forward(), want) and op.status()["code"] == 0
+
+    with ResidentNVFP4(None, pa, pb, workers=148, output_dtype=torch.bfloat16) as op:
+        # columns, then epilogues: BF16 and NVFP4 rows keep them, the others (and residuals, padded heads) are refused
+        bf16_rows = lambda: _native.check(lib.configure_resident_fp4_bf16(op.handle, None, None, out.data_ptr()), "bf16")      # noqa: E731
+        bf16_rows()
+        _native.check(lib.configure_resident_fp4_columns(op.handle, cols), "columns")
+        refused(op.handle, bf16_rows)
+        assert lib.configure_resident_fp4_bf16(op.handle, None, res.data_ptr(), other.data_ptr()) == 1
+        assert lib.configure_resident_fp4_quantized(op.handle, None, res.data_ptr(), codes.data_ptr(), scales.data_ptr(), 1.0, 0) == 1
+        assert lib.configure_dense_head_pad(op.handle, 256, 256, n) == 1
+        op.forward()
+        assert torch.equal(out.view(-1)[:m * cols].view(m, cols), want[:, :cols]) and not out.view(-1)[m * cols:].any()
+        _native.check(lib.configure_resident_fp4_quantized(op.handle, None, None, codes.data_ptr(), scales.data_ptr(), 1.0, 0), "quantized")
+        op.forward()
+        torch.cuda.synchronize()
+        with ResidentNVFP4(None, pa, pb, workers=148, output_dtype=torch.uint8) as whole:
+            assert torch.equal(codes[:m * cols // 2].view(m, cols // 2), whole.forward()[:, :cols // 2]) and not codes[m * cols // 2:].any()
+            np.testing.assert_array_equal(unswizzle_scales(scales[:m * cols // 16].cpu().numpy(), m, cols // 16),
+                                          unswizzle_scales(whole.output_scales.cpu().numpy(), m, n // 16)[:, :cols // 16])
+        _native.check(lib.configure_resident_fp4_columns(op.handle, n), "columns")
+        # a width that goes back to 128 leaves the plain rows, from which GeGLU starts
+        bf16_rows()
+        _native.check(lib.configure_resident_fp4_tile(op.handle, 192), "tile")
+        _native.check(lib.configure_resident_fp4_tile(op.handle, 128), "tile")
+        _native.check(lib.configure_dense_geglu(op.handle, other.data_ptr()), "GeGLU")
+
+    a, b = (torch.from_numpy(rng.normal(size=s).astype(np.float32)).bfloat16().cuda() for s in ((m, k), (n, k)))
+    geglu, fresh_geglu = (torch.zeros(m, n // 2, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    with ResidentDense(None, a, b) as dense, ResidentDense(None, a, b, geglu_output=fresh_geglu) as fresh:
+        want = dense.forward().clone()
+        assert lib.configure_resident_fp4_tile(dense.handle, 192) == 1
+        assert torch.equal(dense.forward(), want)
+        _native.check(lib.configure_dense_geglu(dense.handle, geglu.data_ptr()), "GeGLU")      # (from plain BF16 rows only)
+        dense.forward()
+        fresh.forward()
+        assert torch.equal(geglu, fresh_geglu) and geglu.any()
+
+
 def test_tile_widths_mixed_on_one_worker():
     """Projections that use the accumulator buffers differently (tiles of up to 128 columns one each, NVFP4 tiles of 192 both) one
     after the other on the same workers, from odd and from even uses."""
