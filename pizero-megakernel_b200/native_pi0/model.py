@@ -241,23 +241,38 @@ class NativePi0:
     def tile_width(self, bands, w):
         """Output tile width of a wide projection with ``bands`` row bands: 192 where that makes one tile per SM out of a few more than
         one 128-wide tile.  A second round of tiles costs as much as the first, half as many columns more cost their copies and a third
-        of the drain (three views: SigLIP's q|k|v 162 tiles -> 108, 12.3 -> 9.3 us; fc1 204 -> 138, 15.8 -> 11.6).  NVFP4 weights with
-        scales for such tiles only (``wide_scales``), and only while every site is NVFP4: the kernel variant of other programs is the faster
+        of the drain (three views: SigLIP's q|k|v 162 tiles -> 108, 12.3 -> 9.3 us; fc1 204 -> 138, 15.8 -> 11.6).  NVFP4 weights
+        packed for such tiles only (``wide``), and only while every site is NVFP4: the kernel variant of other programs is the faster
         without such tiles."""
         rounds = lambda width: -(-bands * -(-w.logical_rows // width) // self.workers)
         uniform = self.default_precision == "nvfp4" and all(v == "nvfp4" for _, v in self.precision_map)
-        return 192 if uniform and getattr(w, "wide_scales", None) is not None and rounds(192) == 1 and rounds(128) > 1 else 128
+        return 192 if uniform and getattr(w, "wide", False) and rounds(192) == 1 and rounds(128) > 1 else 128
+
+    def wide_scales(self, w):
+        """The scales of ``w`` for 192-wide tiles (a third more bytes than the others): made for the first engine that reads them, kept with
+        the weight for the others of its store.  Engines of one or two views and of mixed formats never ask for them."""
+        scales = w.wide_scales
+        if scales is None:
+            from native_pi0.primitives import wide_tile_scales
+            scales = wide_tile_scales(w.scales, w.rows_pad, w.k // 16)
+            torch.cuda.current_stream(self.device).synchronize()
+            w.wide_scales = scales
+        self.buffers.append(scales)
+        return scales
 
     def weight(self, w, *, block_n=128, precision="nvfp4", row_sums=False, wide=False):
         """BF16/FP32 [N, K] -> the site's operand format on the device: NVFP4 (ceil block scales, tensor scale
         amax/(6*448)) or zero-padded BF16.
 
-        ``wide``: rows for whole 192-wide tiles too and, where the codes are not tile-major, their scales for those (``tile_width``).
+        ``wide``: rows for whole 192-wide tiles too, where the codes are not tile-major (``tile_width``, ``wide_scales``): one packing for
+        every view count, 6 % more rows of fc1.
 
         When K is a multiple of 256 the packed NVFP4 codes are re-laid tile-major for ``block_n``-wide output tiles
         (``Fp4Matrix.tiled = block_n``): every TMA box of the weight operand is then one contiguous read."""
         n, k = w.shape
-        np_, kp = padded(n, 384 if wide else 128), padded(k, 64)      # whole tiles and whole scale atoms
+        kp = padded(k, 64)
+        wide = wide and kp % 256 != 0
+        np_ = padded(n, 384 if wide else 128)                         # whole tiles and whole scale atoms
         src = torch.zeros((np_, kp), device=self.device, dtype=torch.bfloat16)
         src[:n, :k] = w.to(torch.bfloat16)
         if precision == "bf16":
@@ -278,9 +293,7 @@ class NativePi0:
         if block_n == 32:
             from native_pi0.primitives import narrow_tile_scales
             m.scales = narrow_tile_scales(m.scales, np_, kp // 16)     # an atom of scales per 32-row tile
-        if wide and kp % 256:
-            from native_pi0.primitives import wide_tile_scales
-            m.wide_scales = wide_tile_scales(m.scales, np_, kp // 16)  # the same scales, two atoms per 192-row tile
+        m.wide, m.wide_scales = wide, None
         m.scale_tile = block_n if block_n == 32 else 128
         m.tiled = 0
         if self.tile_weights and kp % 256 == 0 and np_ % block_n == 0:
@@ -356,7 +369,7 @@ class NativePi0:
                                                 m, n, k, self.workers, 0, 1, 1.0), name)
         else:
             _native.check(self.lib.create_resident_fp4(C.byref(h), src.data.data_ptr(), w.data.data_ptr(), src.scales.data_ptr(),
-                                                       (w.wide_scales if block_n == 192 else w.scales).data_ptr(), placeholder.data_ptr(), m, n, k, self.workers,
+                                                       (self.wide_scales(w) if block_n == 192 else w.scales).data_ptr(), placeholder.data_ptr(), m, n, k, self.workers,
                                                        float(np.float32(src.global_scale) * np.float32(w.global_scale))), name)
         self._own(h)
         cols = getattr(w, "logical_rows", n)

@@ -200,6 +200,34 @@ def test_engine_cache_of_one_and_three_views(small_model, options, extra):
             assert torch.equal(one.forward(*x), alone.forward(*x))
 
 
+@pytest.mark.parametrize("views,workers,precision,wide", [(3, 148, "nvfp4", {"qkv", "fc1"}), (3, 120, "nvfp4", {"qkv"}), (2, 148, "nvfp4", set()), (1, 148, "nvfp4", set()),
+                                                          (3, 148, {"expert.*.down": "bf16"}, set())])
+def test_wide_tiles_of_the_vision_tower(small_model, views, workers, precision, wide):
+    """SigLIP's q|k|v (3456 columns) and fc1 (4304, stored as 4352) run on 192-wide tiles where those are one round of the workers and 128-wide ones are
+    not, and only in engines of one format; actions have the bits of 128-wide tiles, and no other engine keeps scales for them."""
+    class Narrow(NativePi0):
+        def tile_width(self, bands, w):
+            return 128
+    dims, cfg, sd = small_model
+    x = inputs(views, 7, 3, dims.vocab)
+    outs = []
+    for kind in (NativePi0, Narrow):
+        store = {}
+        with kind(StateDictModel(cfg, sd), num_views=views, prompt_len=3, chunk_size=7, workers=workers, precision=precision, weight_store=store) as engine:
+            chosen = set()
+            for name, columns in (("qkv", 3456), ("fc1", 4352)):
+                tiles = engine.stage_tiles[engine.stage_names.index(f"vision.0.{name}")]
+                assert tiles in (2 * views * -(-columns // 192), 2 * views * (columns // 128))
+                if tiles == 2 * views * -(-columns // 192):
+                    chosen.add(name)
+            assert chosen == (wide if kind is NativePi0 else set())
+            scales = sum(getattr(w, "wide_scales", None) is not None for w in store.values())
+            assert scales == len(chosen) * cfg.vision_layers
+            outs.append(engine.forward(*x).clone())
+            assert engine.status()["code"] == 0
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_norm_stages_instead_of_folded_norms(small_model):
     """``fold_norms=False`` keeps every RMSNorm as a stage of its own (normalised rows are quantised, plain weights):
     more stages, and agreement with the oracle emulating that arithmetic."""
