@@ -418,7 +418,7 @@ def test_gemm_qkv_rope_epilogue():
 
 @pytest.mark.parametrize("m,k,rows", [(128, 64, 1), (256, 1152, 200), (384, 768, 384)])
 def test_wide_tiles_give_the_bits_of_narrow_ones(m, k, rows):
-    """192-wide tiles under every epilogue, one and several per worker, against 128-wide ones: the sums over K are the same.
+    """192-wide tiles with bias, residual, NVFP4 output and GELU, one and several per worker, against 128-wide ones: the sums over K are the same.
     With fewer logical columns than the weight has rows the last tile is cut, and nothing beyond is stored."""
     from native_pi0.dense import ResidentDense
     lib = _native.load()
@@ -439,7 +439,6 @@ def test_wide_tiles_give_the_bits_of_narrow_ones(m, k, rows):
                 outs.append((y, op.output_scales.clone() if y.dtype == torch.uint8 else None))
         for y, sc in outs[1:]:
             assert torch.equal(y, outs[0][0]) and (sc is None or torch.equal(sc, outs[0][1]))
-    cols = 640                                              # three whole tiles and a third of one
     with ResidentNVFP4(None, pa, pb, workers=148, rows=rows, output_dtype=torch.uint8, output_gelu=True, bias=bias) as whole:
         codes = whole.forward()
         scales = unswizzle_scales(whole.output_scales.cpu().numpy(), m, n // 16)
@@ -470,6 +469,52 @@ def test_wide_tiles_give_the_bits_of_narrow_ones(m, k, rows):
         ResidentNVFP4(None, pa, pb, block_n=192)
     with ResidentDense(None, torch.zeros(8, 64).bfloat16(), torch.zeros(768, 64).bfloat16()) as dense:
         assert lib.configure_resident_fp4_tile(dense.handle, 192) == 1
+
+
+@pytest.mark.parametrize("m,rows,k", [(128, 1, 64), (256, 200, 320), (768, 768, 1152)])
+@pytest.mark.parametrize("form", ["heads", "gelu", "rows"])
+def test_wide_tiles_behind_a_folded_layernorm(form, m, rows, k):
+    """What SigLIP runs on 192-wide tiles - q|k|v with heads stored apart, fc1 cut at its logical columns, both behind a folded
+    LayerNorm - and BF16 rows that are cut, against 128-wide ones, one and several tiles per worker: the same bits, nothing elsewhere."""
+    lib = _native.load()
+    rng = np.random.default_rng(m + k)
+    n, heads, pitch, parts = 1152, 16, 128, 20
+    cols = n if form == "heads" else 1024                  # six 192-wide tiles, or five and a third
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    bias = bf16(rng.normal(size=n))
+    center, sums = (torch.from_numpy(rng.normal(size=s).astype(np.float32)).cuda() for s in ((n,), (m, parts)))
+    sumsq = torch.from_numpy(rng.uniform(20, 90, size=(m, parts)).astype(np.float32)).cuda()
+    got = []
+    for block_n, workers in ((128, 148), (192, 148), (192, 3), (192, 1)):
+        out = torch.full((m * heads * pitch,), 7.0, dtype=torch.bfloat16, device="cuda")
+        codes = torch.full((m * n // 2,), 0xee, dtype=torch.uint8, device="cuda")
+        scales = torch.zeros(m * n // 16, dtype=torch.uint8, device="cuda")
+        with ResidentNVFP4(None, pa, pb, workers=workers, rows=rows, output_dtype=torch.bfloat16, bias=bias, block_n=block_n) as op:
+            _native.check(lib.configure_resident_fp4_tile(op.handle, 128), "tile")
+            if form == "gelu":
+                _native.check(lib.configure_resident_fp4_quantized(op.handle, op.bias.data_ptr(), None, codes.data_ptr(), scales.data_ptr(), 1.0, 1), "quantized")
+            else:
+                _native.check(lib.configure_resident_fp4_bf16(op.handle, op.bias.data_ptr(), None, out.data_ptr()), "bf16")
+            if form == "heads":
+                _native.check(lib.configure_dense_head_pad(op.handle, n // heads, pitch, heads * pitch), "heads")
+            else:
+                _native.check(lib.configure_resident_fp4_columns(op.handle, cols), "columns")
+            _native.check(lib.configure_resident_fp4_tile(op.handle, block_n), "tile")
+            _native.check(lib.configure_resident_fp4_row_layernorm(op.handle, sumsq.data_ptr(), sums.data_ptr(), parts, 1152, 1e-6, center.data_ptr()), "layernorm")
+            op.forward()
+            assert op.status()["code"] == 0
+        got.append((out, codes, scales))
+    for again in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(again, got[0]))
+    out, codes, scales = got[0]
+    if form == "gelu":
+        assert (codes[:rows * cols // 2] != 0xee).any() and (codes[rows * cols // 2:] == 0xee).all() and (out == 7).all()
+    elif form == "heads":
+        view = out.view(m, heads, pitch)
+        assert (view[:, :, n // heads:] == 7).all() and (view[rows:] == 7).all() and not (view[:rows, :, :n // heads] == 7).all(-1).any()
+    else:
+        assert (out[rows * cols:] == 7).all() and not (out[:rows * cols].view(rows, cols) == 7).all(-1).any()
 
 
 def test_epilogues_behind_a_width_or_columns_that_they_do_not_go_with():
