@@ -48,7 +48,8 @@ int destroy_resident_fp4(void* handle);
 int configure_resident_fp4_qkv_rope(void* handle, void* out_q, int ldq, const void* cos, const void* sin, void* cache_k,
                                     void* cache_v, int q_cols, int head_dim, int cache_base);
 /* extension: the same rotary tables in pair-major order, BF16 entry [head_dim / 2][ld][4] = cos(i), cos(i + head_dim/2), sin(i),
- * sin(i + head_dim/2) of a row; ld a multiple of 128 that covers the row bands.  Call it behind configure_*_qkv_rope. */
+ * sin(i + head_dim/2) of a row; ld a multiple of 128 that covers the row bands.  Call it behind configure_*_qkv_rope.  A load then covers two lines instead of 32
+ * (768 rows: 9.8 us against 12.1 - 13.0). */
 int configure_qkv_rope_table(void* handle, const void* table, int ld);
 /* extension: residual-stream epilogue.  out BF16 [M, N] = alpha*acc + residual + bias as configure_resident_fp4_bf16;
  * the rounded rows are also quantised, un-normalised, to NVFP4 (copy_fp4 packed [M, N/2], copy_scales swizzled with

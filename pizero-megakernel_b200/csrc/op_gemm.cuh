@@ -554,7 +554,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
 // instruction once it has seen the accumulator complete.  The partner also leaves the row factors it has computed: the
 // helper comes from its role at about that moment and would have to fetch the row statistics first.
 // LEAN: the drain of the lean kernel variant; the residual-stream and plain BF16 drains there carry no row-statistics code
-// (the host sends programs that give those two epilogues row statistics to the full variant).
+// (the host sends programs that give those two epilogues row statistics to the full variant), and that of q|k|v reads the pair-major
+// rotary table only.
 // WIDE: NVFP4 tiles of 192 columns, which take two accumulator uses and may end beyond the logical columns.  An instantiation of its
 // own: with both in one drain the others' take 0.1 us longer (one view 5.21 -> 5.31 ms, BF16 16.16 -> 16.51).
 template <int EPI, bool LEAN = false, bool WIDE = false>
@@ -761,8 +762,8 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
 // drain, as one of the draining warps or as a helper of the last tile.
 // LEAN: the kernel variant for programs made only of NVFP4 projections with the pi0 model's epilogues (the host checks
 // this when it builds a program); it carries neither the dense issue loops nor the other drain loops.
-// WIDE: with the forms for 192-wide NVFP4 tiles.
-template <bool LEAN, bool WIDE>
+// WIDE: with the forms for 192-wide NVFP4 tiles.  ROTARY_ROWS: with those for rotary tables row by row.
+template <bool LEAN, bool WIDE, bool ROTARY_ROWS>
 __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl, uint8_t* data, uint32_t tmem,
                                                  const StageDesc& st, int stage_index, int first, int count,
                                                  PipeState& ps, long long* stamp) {
@@ -786,7 +787,7 @@ __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl
     else if (epilogue == EPI_STREAM) gemm_epilogue<EPI_STREAM, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_GEGLU_FP4) gemm_epilogue<EPI_GEGLU_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_FP4) gemm_epilogue<EPI_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
-    else if (epilogue == EPI_QKV_ROPE) gemm_epilogue<EPI_QKV_ROPE, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (epilogue == EPI_QKV_ROPE) gemm_epilogue<EPI_QKV_ROPE, LEAN && !ROTARY_ROWS>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (LEAN || epilogue == EPI_BF16_EXT) gemm_epilogue<EPI_BF16_EXT, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_F32) gemm_epilogue<EPI_F32>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else gemm_epilogue<EPI_GEGLU_BF16>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);

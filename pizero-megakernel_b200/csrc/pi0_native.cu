@@ -145,7 +145,8 @@ struct Program {
     bool timings_on = false;
     bool lean = false;                 // every stage is one the lean kernel variant runs
     bool mma_sync = false;             // some attention stage runs on the mma.sync tiles
-    bool wide = false;                   // a projection has 192-wide tiles
+    bool wide = false;                 // a projection has 192-wide tiles
+    bool rotary_rows = false;          // a q|k|v projection has no pair-major rotary table
     bool early = false;                // the program of one operator small enough for its successor to start early (solo_program)
     int grid = 0;                      // CTAs launched: up to the last worker that has an instruction
     unsigned int epoch = 0;
@@ -200,7 +201,6 @@ bool lean_stage(const StageDesc& d) {
         const bool stats = g.row_sumsq || g.row_factor;     // (the lean residual-stream and plain BF16 drains read none)
         if (stats && (g.epilogue == EPI_STREAM || (g.epilogue == EPI_BF16 && g.block_n <= 128))) return false;     // (192: the extended drain)
         if (g.round_before_residual || g.gelu_cols > 0 || g.act == 3) return false;       // options the lean drains leave out
-        if (g.epilogue == EPI_QKV_ROPE && !g.rope_table) return false;      // (the lean rotary drain reads the pair-major table only)
         return g.operands == GEMM_NVFP4 && (g.epilogue == EPI_BF16 || g.epilogue == EPI_STREAM || g.epilogue == EPI_GEGLU_FP4 ||
                                             g.epilogue == EPI_FP4 || g.epilogue == EPI_QKV_ROPE || g.epilogue == EPI_BF16_EXT);
     }
@@ -215,6 +215,10 @@ bool lean_stage(const StageDesc& d) {
     }
     return d.kind != OP_ATTN_PREP && d.kind != OP_SUFFIX && d.kind != OP_PROBE;
 }
+
+// Whether a launch goes to a lean variant: progress marks are written by the full ones only, and the one with row-major rotary tables has
+// no time stamps.
+bool lean_launch(const Program* prog) { return prog->lean && !prog->h_debug && !(prog->rotary_rows && prog->timings_on); }
 
 // Build a program from stage descriptors (sources already set) and compact int4 instructions.
 int build_program(Program** out, int device, const std::vector<StageDesc>& stages_in, const std::vector<int>& code4,
@@ -315,6 +319,7 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, false, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(pi0_vm_kernel<true, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
             configured[device] = e == cudaSuccess;
         }
@@ -323,7 +328,9 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
             prog->lean = prog->lean && lean_stage(d);
             prog->mma_sync = prog->mma_sync || (d.kind == OP_ATTN && !d.p.attn.tc);
             prog->wide = prog->wide || (d.kind == OP_GEMM && d.p.gemm.block_n > 128);
+            prog->rotary_rows = prog->rotary_rows || (d.kind == OP_GEMM && d.p.gemm.epilogue == EPI_QKV_ROPE && !d.p.gemm.rope_table);
         }
+        if (prog->rotary_rows && prog->wide) prog->lean = false;        // (no lean variant has both)
     }
     if (e != cudaSuccess) return e;
     *out = prog.release();
@@ -377,7 +384,8 @@ int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begi
     config.stream = stream;
     config.attrs = &serial;
     config.numAttrs = 1;
-    if (prog->lean && !prog->h_debug) {
+    if (lean_launch(prog)) {
+        if (prog->rotary_rows) return cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false, false, false, true>, p);
         if (prog->wide) return p.timings ? cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true, false, true>, p) : cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false, false, true>, p);
         return p.timings ? cudaLaunchKernelEx(&config, pi0_vm_kernel<true, true>, p) : cudaLaunchKernelEx(&config, pi0_vm_kernel<true, false>, p);
     }
@@ -1626,7 +1634,7 @@ extern "C" int read_native_model_counters(void* handle, unsigned int* counts, un
 extern "C" int native_model_kernel_variant(void* handle, int* lean) {
     Program* prog = as_program(handle);
     if (!prog || !lean) return cudaErrorInvalidValue;
-    *lean = (prog->lean && !prog->h_debug) ? 1 : 0;             // (progress marks are written by the full variant only)
+    *lean = lean_launch(prog) ? 1 : 0;
     return cudaSuccess;
 }
 extern "C" int enable_native_model_debug(void* handle, int enable) {

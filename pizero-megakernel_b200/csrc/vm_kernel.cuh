@@ -54,7 +54,11 @@ __device__ __forceinline__ bool prefetch_slot(const VmProgram& prog, Ctl* ctl, c
 // BF16 333 x 1000 x 1152 11.2 and 9.5 us, FP8 768 x 2048 x 16384 32.7 and 31.3), so only programs with such tiles carry them.
 // WIDE = true: with the forms for 192-wide NVFP4 tiles, which three-view models run; the smaller kernel without them is faster for everything
 // else (one view 5.26 -> 5.23 ms, BF16 forward 16.70 -> 16.14, q|k|v of 51 rows 5.84 -> 5.75 us).
-template <bool LEAN, bool TIMED = true, bool MMA_SYNC = !LEAN, bool WIDE = MMA_SYNC>
+// ROTARY_ROWS = true: q|k|v drains that read their rotary tables row by row, for programs without the pair-major table
+// (configure_qkv_rope_table).  In the lean variants that serve the model that code costs 1 % of a forward it is not part of (three views 8.92 -> 9.03
+// ms, one view 5.20 -> 5.25); a variant of its own keeps such programs lean (q|k|v of 51 rows, row-major tables: 6.50 us here, 7.50 in the
+// variant with every operator; of 768 rows 12.4 and 13.5).
+template <bool LEAN, bool TIMED = true, bool MMA_SYNC = !LEAN, bool WIDE = MMA_SYNC, bool ROTARY_ROWS = !LEAN>
 __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_constant__ VmProgram prog) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(kThreads, 1) pi0_vm_kernel(const __grid_consta
         if (stamp && threadIdx.x == 0) stamp[0] = static_cast<long long>(global_ns());
         if (st.kind == OP_GEMM) {
             if constexpr (!LEAN) mark(prog, 800000 + ins.y);
-            gemm_instruction<LEAN, WIDE>(prog, ctl, data, tmem, st, ins.y, ins.z, ins.w, ps, stamp);
+            gemm_instruction<LEAN, WIDE, ROTARY_ROWS>(prog, ctl, data, tmem, st, ins.y, ins.z, ins.w, ps, stamp);
             // one decision per warp: the lanes with a role return later than the others and must not leave alone
             if (__any_sync(0xffffffffu, ctl->abort != 0)) break;
         } else {

@@ -647,6 +647,46 @@ def test_qkv_rope_table_in_pair_order(rows, heads, block_n):
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("rows,block_n", [(51, 64), (200, 128)])
+def test_programs_with_row_major_rotary_tables_stay_lean(rows, block_n):
+    """The lean kernel runs q|k|v with either order of the rotary tables; with time stamps, or 192-wide tiles in the same program, row-major
+    ones take the variant with everything.  All of them give the same bits."""
+    from native_pi0.linear import NativeStageProgram
+    lib = _native.load()
+    rng = np.random.default_rng(rows)
+    m, k, hd, n = 128 * -(-rows // 128), 256, 256, 768
+    pa = pack_nvfp4(rng.normal(size=(m, k)).astype(np.float32))
+    pb = pack_nvfp4(rng.normal(scale=0.05, size=(n, k)).astype(np.float32), scale_policy="ceil")
+    cos, sin = (torch.from_numpy(rng.uniform(-1, 1, size=(m, hd)).astype(np.float32)).bfloat16().cuda() for _ in range(2))
+    half = hd // 2
+    table = torch.stack((cos[:, :half], cos[:, half:], sin[:, :half], sin[:, half:]), -1).permute(1, 0, 2).contiguous()
+    q, ck, cv = (torch.zeros(m, hd, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    got = []
+
+    def launch(run):
+        for t in (q, ck, cv):
+            t.zero_()
+        run()
+        got.append([t.clone() for t in (q, ck, cv)])
+
+    with (ResidentNVFP4(None, pa, pb, workers=148, output_dtype=torch.bfloat16, rows=rows, block_n=block_n) as op,
+          ResidentNVFP4(None, pa, pb, workers=148, output_dtype=torch.bfloat16, rows=rows, block_n=192) as wide):
+        for pairs in (False, True):
+            _native.check(lib.configure_resident_fp4_qkv_rope(op.handle, q.data_ptr(), hd, cos.data_ptr(), sin.data_ptr(), ck.data_ptr(), cv.data_ptr(), hd, hd, 0), "rope")
+            if pairs:
+                _native.check(lib.configure_qkv_rope_table(op.handle, table.data_ptr(), m), "rope table")
+            launch(op.forward)
+            for others, timed, lean in (([], 0, 1), ([], 1, int(pairs)), ([(wide, [])], 0, int(pairs))):
+                with NativeStageProgram(None, others + [(op, [])]) as program:
+                    _native.check(lib.enable_native_model_timings(program.handle, timed), "timings")
+                    value = C.c_int(-1)
+                    _native.check(lib.native_model_kernel_variant(program.handle, C.byref(value)), "variant")
+                    assert value.value == lean, (pairs, timed, len(others))
+                    launch(program.forward)
+                    assert program.status()["code"] == 0
+    assert got[0][0].any() and all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other))
+
+
 @pytest.mark.parametrize("rows,width,kind", [(51, 1024, "rms"), (768, 2048, "rms"), (256, 1152, "layer"), (7, 64, "layer")])
 def test_norm_to_nvfp4(rows, width, kind):
     torch.manual_seed(83)
