@@ -27,7 +27,10 @@ namespace pi0 {
 // MMAs that read it.
 // The loop works on register copies of the descriptor: that lies in shared memory, and every asm statement with a memory
 // clobber would make the compiler read it again.
-template <bool WEIGHTS>
+// WIDE: also the two scale atoms per group of 192-wide tiles.  With that choice in its loop the copy warp of a few-row projection is later
+// (q|k|v of 51 rows 5.65 -> 5.76 us), so the lean variant without such tiles goes without; the ones with every operator keep
+// it, where nothing was gained (BF16 forward 16.13 ms without, 16.08 with).
+template <bool WEIGHTS, bool WIDE>
 __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, uint8_t* data, const StageDesc& st,
                                               int stage_index, int first, int count, PipeState& ps, long long* stamp) {
     const GemmParams& g = st.p.gemm;
@@ -73,7 +76,7 @@ __device__ __forceinline__ void gemm_producer(const VmProgram& prog, Ctl* ctl, u
         int alive = 1;
         if (lane == 0) {
             // B scales: the 128-row atom that holds the tile's rows, or - 32- and 192-wide tiles - an atom or two of the tile's own
-            const bool two = WEIGHTS && block_n > 128;
+            const bool two = WIDE && WEIGHTS && block_n > 128;
             const int sf_tile = !WEIGHTS ? m_tile : block_n == 32 ? n_tile : two ? 2 * n_tile : (n_tile * block_n) >> 7;
             const uint32_t sf_group = two ? 1024u : 512u;
             const uint8_t* sf = scales + static_cast<size_t>(sf_tile) * k_groups * 512;
@@ -769,10 +772,10 @@ __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl
                                                  PipeState& ps, long long* stamp) {
     const int warp = threadIdx.x >> 5;
     if (warp == 0) {
-        gemm_producer<false>(prog, ctl, data, st, stage_index, first, count, ps, stamp);
+        gemm_producer<false, WIDE || !LEAN>(prog, ctl, data, st, stage_index, first, count, ps, stamp);
         if (stamp && threadIdx.x == 0) stamp[3] = static_cast<long long>(global_ns());
     } else if (warp == 3) {
-        gemm_producer<true>(prog, ctl, data, st, stage_index, first, count, ps, nullptr);
+        gemm_producer<true, WIDE || !LEAN>(prog, ctl, data, st, stage_index, first, count, ps, nullptr);
     } else if (warp == 1) {
         const int operands = st.p.gemm.operands;
         if (LEAN || operands == GEMM_NVFP4) gemm_mma<GEMM_NVFP4, WIDE>(prog, ctl, data, tmem, st, stage_index, first, count, ps, stamp);
