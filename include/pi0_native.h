@@ -137,7 +137,8 @@ int configure_dense_qkv_rope(void* handle, const void* cos, const void* sin, voi
 int configure_dense_head_pad(void* handle, int from, int to, int ld);
 /* extension: logical row count and output tile width (128, 64 or 32) of a dense projection.  The NVFP4 GEMM's
  * configure_resident_fp4_{bf16, quantized, qkv_rope, rows, tile, weight_layout} calls accept dense handles too (a dense
- * projection may emit NVFP4 for an NVFP4 consumer). */
+ * projection may emit NVFP4 for an NVFP4 consumer).  A width that has been given stays: one that never was is chosen by size where
+ * the projection is launched by itself, and 128 in a program of several stages. */
 int configure_dense_rows(void* handle, int rows);
 int configure_dense_tile(void* handle, int block_n);
 

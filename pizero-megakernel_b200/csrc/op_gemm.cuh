@@ -4,14 +4,14 @@
 // each operand row (64 FP4, 16 BF16 or 32 FP8 elements), so the copy ring and the issue loop are the same code.
 //
 //   warps 0 and 3   : TMA producers - A and B tiles (128 B swizzled rows) and their scale atoms into a ring of slots; the
-//                                     ring is laid out per GEMM: 3 slots of 72 KiB for full NVFP4 tiles, up to 5 for narrow
+//                                     ring is laid out per GEMM: 3 slots of 72 KiB for 128-wide NVFP4 tiles, up to 5 for narrow
 //                                     ones, up to 8 for dense operands (so slots of one size can come in different numbers)
 //   warp 1          : MMA issuer    - one elected thread issues tcgen05.cp (scales smem->TMEM, NVFP4 only) and
 //                                     tcgen05.mma, 32 operand bytes of K each
 //   warps 4..7      : epilogue      - tcgen05.ld of a 128xN FP32 accumulator (one row per thread), fused math, stores
 //   warps 0..3      : second half of the columns of an instruction's last tile, once their roles are done
 //
-// Two TMEM accumulators alternate, so the epilogue of tile t overlaps the MMAs of tile t+1. Pipeline positions live in
+// Two TMEM accumulators alternate, so the epilogue of tile t overlaps the MMAs of tile t+1 (192-wide tiles take both). Pipeline positions live in
 // registers (PipeState) and carry over from one instruction to the next; barriers are never re-initialised.
 #pragma once
 #include "vm_core.cuh"
@@ -444,8 +444,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
                               pack_bf16x2(v[4 * i + 2].x, v[4 * i + 2].y), pack_bf16x2(v[4 * i + 3].x, v[4 * i + 3].y));
         // padded: heads written pad_to columns apart (8-column pieces never straddle a head: pad_from is a multiple of 8); the
         // lane's piece moves by the gaps in front of it.  Eight rows per store instruction: these drains write wide tiles, whose
-        // stores were a third of their time (768 x 32768 BF16 42.0 -> 38.2 us).  In the residual-stream and q|k|v drains the
-        // transpose costs more than it saves, because the model runs them for few rows, where the chain of a thread counts
+        // stores were a third of their time (768 x 32768 BF16 42.0 -> 38.2 us).  In the residual-stream drain, and in q|k|v's of a
+        // single row band, the transpose costs more than it saves: few warps are at work there, and the chain of a thread counts
         // (o_proj 5.2 -> 6.1 us).
         const int lane = lane_id();
         int gap = 0;

@@ -447,7 +447,7 @@ int a_box_rows_of(int operands, int m, int rows) {
 int ring_layout(GemmParams& g, int operands) {
     g.off_b = kChunks * 128 * g.a_box_rows;
     const int sf_bytes = operands == GEMM_NVFP4 ? kSfBytes : 0, sfb_bytes = g.block_n > 128 ? 2 * sf_bytes : sf_bytes;
-    const int fewest = g.block_n > 128 ? 2 : kStages;       // (192-wide tiles: slots of up to 92 KiB)
+    const int fewest = g.block_n > 128 ? kStagesWide : kStages;
     g.off_sfa = g.off_b + kChunks * 128 * g.block_n;
     g.off_sfb = g.off_sfa + sf_bytes;
     g.slot_stride = g.off_sfb + sfb_bytes;
@@ -479,9 +479,11 @@ int gemm_tiles(StageDesc& d, int operands, int m, int block_n) {
 
 // Tile width of a dense projection that is launched by itself and has not been given one (in a program of several stages it keeps 128).
 // Such a launch is paid by the operand rows that an SM takes in, A's and the tile's own for every tile it gets, and every width
-// gives the same sums over K.  The estimate picks the fastest width in all that were measured (us back to back, 128 / 64 / 32 columns):
-// BF16 333 x 1000 x 1152 9.3 / 8.7 / 8.1, 20 x 4352 x 4352 25.5 / 20.6 / 17.5, 768 x 1152 x 4352 25.2 / 19.8 / 24.0, 500 x 1700 x 1000 9.7 /
-// 9.1 / 10.3, 820 x 2048 x 2048 16.6 / 19.0 / 23.4; FP8 50 x 500 x 4352 11.8 / 9.9 / 8.7, 768 x 2048 x 4096 16.5 / 18.7 / 20.5.
+// gives the same sums over K.  In 24 shapes of 1 to 820 rows, 100 to 4400 columns and K of 504 to 4400 the estimate picks the fastest
+// width (to 2 %) back to back, and behind a flushed L2 too (us, 128 / 64 / 32 columns; flushed, launch and event included, in brackets):
+// BF16 333 x 1000 x 1152 9.4 / 8.7 / 8.2 (17.2 / 15.4 / 14.3), 20 x 4352 x 4352 18.0 / 14.5 / 14.3 (33.7 / 27.6 / 24.6), 768 x 1152 x 4352 19.0 /
+// 15.7 / 21.5 (30.7 / 25.5 / 29.7), 820 x 4400 x 4400 40.0 / 50.1 / 68.0 (54.2 / 65.5 / 80.9), 10 x 100 x 504 6.9 / 5.9 / 5.7 (14.3 / 12.5 / 12.3);
+// FP8 50 x 500 x 4352 11.8 / 10.0 / 8.7 (20.5 / 18.4 / 16.4), 768 x 2048 x 4096 13.3 / 16.2 / 18.1 (22.5 / 24.6 / 26.6).
 int solo_tile_width(const Op* op) {
     const GemmParams& g = op->desc.p.gemm;
     if (op->operands == GEMM_NVFP4 || op->tile_given || g.b_tiled || g.epilogue == EPI_STREAM) return g.block_n;

@@ -7,24 +7,26 @@ namespace pi0 {
 
 // GEMM pipeline: a ring of slots, each holding kChunks consecutive 256-wide K chunks of A and B plus their scale
 // atoms. One slot is filled by four copies (A, B, SFA, SFB). The ring is laid out per GEMM by the host (slot size from
-// the rows that are really copied, as many slots as fit): kStages slots of kStageBytes for full tiles, up to
-// kMaxStages for the narrowest ones.
-constexpr int kStages = 3;                                   // slots in flight with full-size tiles (128 rows of A and of B)
+// the rows that are really copied, as many slots as fit): kStages slots of kStageBytes for 128 x 128 tiles, kStagesWide of
+// kStageBytesWide for 192-wide NVFP4 ones, up to kMaxStages or kMaxStagesDense for the narrowest ones.
+constexpr int kStages = 3;                                   // slots in flight with 128-wide tiles (128 rows of A and of B)
+constexpr int kStagesWide = 2;                               // ... with 192-wide NVFP4 tiles
 constexpr int kMaxStages = 5;                                // slots in flight with the narrowest NVFP4 tiles (64 rows of each) ...
 constexpr int kMaxStagesDense = 8;                           // ... and BF16 / FP8 tiles, whose slots cover less of K and carry no scales
 constexpr int kChunks = 2;                                   // 256-wide K chunks per slot
 constexpr int kTileABytes = 128 * 128;                       // one chunk of one operand: 128 rows x 128 bytes
 constexpr int kSfBytes = kChunks * 4 * 512;                  // scale atoms of one operand: four 64-wide K groups per chunk
-constexpr int kStageBytes = 2 * kChunks * kTileABytes + 2 * kSfBytes;   // largest slot: 72 KiB
+constexpr int kStageBytes = 2 * kChunks * kTileABytes + 2 * kSfBytes;   // 72 KiB
+constexpr int kStageBytesWide = kChunks * (kTileABytes + 192 * 128) + 3 * kSfBytes;   // largest slot, two scale atoms of B per group: 92 KiB
 constexpr int kCtlBytes = 7168;
-constexpr int kDataBytes = 216 * 1024;                       // operator scratch behind the control block: three full-size slots
+constexpr int kDataBytes = 216 * 1024;                       // operator scratch behind the control block: three 128-wide slots or two 192-wide ones
 constexpr int kSmemBytes = kCtlBytes + kDataBytes + 1024;    // + slack for 1 KiB alignment
 constexpr int kTmemCols = 512;
 constexpr int kSfCol0 = 256;                                 // accumulators use columns [0,256)
 constexpr int kRing = 4;                                     // instruction slots resident in shared memory
 constexpr int kAhead = 2;                                    // the prefetch warp runs this many instructions ahead
 constexpr int kPrefetchWarp = 2;
-static_assert(kStages * kStageBytes <= kDataBytes, "GEMM ring exceeds the data region");
+static_assert(kStages * kStageBytes <= kDataBytes && kStagesWide * kStageBytesWide <= kDataBytes, "GEMM ring exceeds the data region");
 static_assert(sizeof(StageDesc) % 16 == 0, "descriptors are copied in 16-byte pieces");
 
 // One decoded instruction: the stream entry and a private copy of its stage descriptor.

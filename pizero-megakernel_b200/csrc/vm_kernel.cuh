@@ -53,7 +53,7 @@ __device__ __forceinline__ bool prefetch_slot(const VmProgram& prog, Ctl* ctl, c
 // that spills there is slower everywhere (the same program on both: BF16 forward 17.34 and 16.17 ms, expert in BF16 13.88 and 12.80,
 // BF16 333 x 1000 x 1152 11.2 and 9.5 us, FP8 768 x 2048 x 16384 32.7 and 31.3), so only programs with such tiles carry them.
 // WIDE = true: with the forms for 192-wide NVFP4 tiles, which three-view models run; the smaller kernel without them is faster for everything
-// else (one view 5.26 -> 5.23 ms, BF16 forward 16.70 -> 16.14, q|k|v of 51 rows 5.84 -> 5.75 us).
+// else (the same programs with and without: one view 5.26 and 5.20 ms, BF16 forward 16.64 and 16.08, q|k|v of 51 rows 6.05 and 5.74 us).
 // ROTARY_ROWS = true: q|k|v drains that read their rotary tables row by row, for programs without the pair-major table
 // (configure_qkv_rope_table).  In the lean variants that serve the model that code costs 1 % of a forward it is not part of (three views 8.92 -> 9.03
 // ms, one view 5.20 -> 5.25); a variant of its own keeps such programs lean (q|k|v of 51 rows, row-major tables: 6.50 us here, 7.50 in the

@@ -61,7 +61,7 @@ struct GemmParams {
     int cols;                    // logical columns of the output (<= N; only 192-wide tiles may end beyond them)
     int b_tiled;                 // B stored tile-major: block (n_tile, k_stage) is block_n contiguous 128-byte rows
     int a_box_rows;              // rows of A copied per tile: 128, or fewer (a multiple of 8) when there are fewer logical rows
-    int ring_stages;             // operand ring of this GEMM: slots in flight (kStages..kMaxStagesDense) ...
+    int ring_stages;             // operand ring of this GEMM: slots in flight (kStagesWide..kMaxStagesDense) ...
     int slot_stride;             // ... bytes from one slot to the next (multiple of 1024) ...
     int off_b, off_sfa, off_sfb; // ... and where B, the A scales and the B scales start inside a slot (A starts at 0)
     float alpha;                 // global_scale(A) * global_scale(B)
