@@ -528,14 +528,15 @@ __device__ __forceinline__ void merge_instruction(const VmProgram& prog, Ctl* ct
 // resident on different SMs at the same time) meet on a per-group ticket counter that grows by `splits` per launch; once all partials of
 // the head are published, every tile merges its share of the query rows (row % splits == split), so the merge
 // costs neither a stage of its own nor a serial tail on one SM.
-template <int HDP, bool LEAN, bool MASK, bool TWICE>
+template <int HDP, bool LEAN, bool MASK, bool TWICE, bool PIECES = false>
 __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& a, int tile, uint8_t* data, uint32_t tmem,
                              uint32_t uses, int stage, long long* stamp, const StageDesc* deps, int dep_first, int dep_count);
 
-// LEAN: the lean kernel variant (no boolean masks); MMA_SYNC: the variant with the mma.sync tiles.
+// LEAN: the lean kernel variant (no boolean masks); MMA_SYNC: the variant with the mma.sync tiles; PIECES: how its partial rows are
+// transposed (quad_transpose).
 // The instruction waits for its sources itself (the instruction loop does not): the tcgen05 tile does so after its
 // index arithmetic, the other tiles up front.
-template <bool LEAN, bool MMA_SYNC>
+template <bool LEAN, bool MMA_SYNC, bool PIECES>
 __device__ __forceinline__ void attn_instruction(const VmProgram& prog, Ctl* ctl, uint8_t* data, uint32_t tmem, uint32_t& tc_tiles,
                                                  const StageDesc& st, int stage_index, int first, int count, long long* stamp) {
     const AttnParams& a = st.p.attn;
@@ -551,8 +552,8 @@ __device__ __forceinline__ void attn_instruction(const VmProgram& prog, Ctl* ctl
                                         : attn_tile_tc<128, false, true, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count);
             } else {
                 // (KV splits of at most 64 queries of 256-wide heads, the action expert's: four threads per row)
-                ok = a.hd_pad > 128 ? (a.q_box <= 64 && a.splits > 1 ? attn_tile_tc<256, LEAN, false, true>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count)
-                                                     : attn_tile_tc<256, LEAN, false, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count))
+                ok = a.hd_pad > 128 ? (a.q_box <= 64 && a.splits > 1 ? attn_tile_tc<256, LEAN, false, true, PIECES>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count)
+                                                     : attn_tile_tc<256, LEAN, false, false, PIECES>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count))
                                     : attn_tile_tc<128, LEAN, false, false>(prog, ctl, a, t, data, tmem, tc_tiles, stage_index, stamp_t, deps, first, count);
             }
             tc_tiles++;

@@ -60,7 +60,7 @@ __device__ __forceinline__ bool cta_wait_phase(const VmProgram& prog, Ctl* ctl, 
 // LEAN: of the lean kernel variant, whose 128-element heads are never split.
 // Scores are read from tensor memory again for the exponentials rather than kept in registers: values loaded by tcgen05.ld that
 // live across a barrier or a branch make the compiler spill, which slows every operator of the kernel (forward 9.6 -> 10.3 ms and more).
-template <int HDP, bool LEAN, bool MASK, bool TWICE>
+template <int HDP, bool LEAN, bool MASK, bool TWICE, bool PIECES>
 // deps: when not null, the stage whose sources this call waits for itself (tile range dep_first, dep_count) - after its
 // index arithmetic and just before the first copies, so that the arithmetic is off the dependent path.
 __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& a, int tile, uint8_t* data, uint32_t tmem,
@@ -268,7 +268,7 @@ __device__ bool attn_tile_tc(const VmProgram& prog, Ctl* ctl, const AttnParams& 
                                       pack2_bf16(__uint_as_float(raw[8 * u + 4]), __uint_as_float(raw[8 * u + 5])),
                                       pack2_bf16(__uint_as_float(raw[8 * u + 6]), __uint_as_float(raw[8 * u + 7])));
                 // (columns beyond head_dim - padded heads - are not stored: that lane's piece counts as no rows)
-                store_rows64(po + c0 * 2, ld, c0 + 8 * (lane & 3) < a.head_dim ? warp_rows : 0, p);
+                store_rows64<PIECES>(po + c0 * 2, ld, c0 + 8 * (lane & 3) < a.head_dim ? warp_rows : 0, p);
             }
         }
         if (part == 0 && row_ok) {
