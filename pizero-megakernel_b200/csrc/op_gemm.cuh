@@ -309,7 +309,7 @@ struct DrainRow {
 };
 // Scale of block `block` of that row (scale_offset, split into a part per row and a part per block).
 __device__ __forceinline__ uint8_t* scale_at(const DrainRow& d, int block) { return d.scales + (block >> 2) * 512 + (block & 3); }
-template <int EPI>
+template <int EPI, bool LEAN>
 __device__ __forceinline__ DrainRow drain_row(const GemmParams& g, int row) {
     DrainRow d = {};
     const int lane = lane_id();
@@ -317,8 +317,9 @@ __device__ __forceinline__ DrainRow drain_row(const GemmParams& g, int row) {
     d.ldo = g.ldo * 2;
     d.out = static_cast<uint8_t*>(g.out) + static_cast<size_t>(row) * g.ldo * width;
     d.rows_left = g.rows - (row - lane);
-    if (g.residual) d.residual = static_cast<const uint8_t*>(g.residual) + static_cast<size_t>(row) * g.ldr * 2;
-    d.bias = static_cast<const uint8_t*>(g.bias);
+    constexpr bool kPlain = EPI == EPI_F32 && LEAN;              // (nothing is added)
+    if (!kPlain && g.residual) d.residual = static_cast<const uint8_t*>(g.residual) + static_cast<size_t>(row) * g.ldr * 2;
+    if (!kPlain) d.bias = static_cast<const uint8_t*>(g.bias);
     d.center = g.col_center;
     d.inv_gs = g.out_inv_gs;
     d.act = g.act;
@@ -558,7 +559,8 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
 // helper comes from its role at about that moment and would have to fetch the row statistics first.
 // LEAN: the drain of the lean kernel variant; the residual-stream and plain BF16 drains there carry no row-statistics code
 // (the host sends programs that give those two epilogues row statistics to the full variant), and that of q|k|v reads the pair-major
-// rotary table only.
+// rotary table only.  Of FP32 rows (in the full variants): without bias, residual and row factors kept over tiles, for raw NVFP4 products; with
+// them in one drain such products took longer (3 x 8192 x 1024 7.26 us, 6.6 here, 700 x 4352 x 1152 16.6 and 16.2; dense ones did not).
 // WIDE: NVFP4 tiles of 192 columns, which take two accumulator uses and may end beyond the logical columns.  An instantiation of its
 // own: with both in one drain the others' take 0.1 us longer (one view 5.21 -> 5.31 ms, BF16 16.16 -> 16.51).
 template <int EPI, bool LEAN = false, bool WIDE = false>
@@ -566,7 +568,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
                                               int stage_index, int first, int count, PipeState& ps, long long* stamp) {
     const GemmParams& g = st.p.gemm;
     constexpr bool kStats = !(LEAN && (EPI == EPI_STREAM || EPI == EPI_BF16));
-    constexpr bool kResidual = EPI != EPI_GEGLU_FP4 && EPI != EPI_GEGLU_BF16 && EPI != EPI_QKV_ROPE;
+    constexpr bool kResidual = EPI != EPI_GEGLU_FP4 && EPI != EPI_GEGLU_BF16 && EPI != EPI_QKV_ROPE && !(EPI == EPI_F32 && LEAN);
     const int quarter = (threadIdx.x >> 5) & 3;          // TMEM lane quarter this warp may read
     const bool main = threadIdx.x >= 128;
     const int lane = lane_id();
@@ -603,7 +605,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         }
         if ((EPI == EPI_BF16_EXT || EPI == EPI_FP4) && g.col_center && lane < (block_n >> 5))
             prefetch_l1(g.col_center + n_tile * block_n + lane * 32);    // constant data: close by when the accumulator is ready
-        const DrainRow d = drain_row<EPI>(g, row);
+        const DrainRow d = drain_row<EPI, LEAN>(g, row);
         // A single-tile instruction that reads row statistics (the few-row projections behind a folded norm, whose epilogue
         // is serial time) or a residual: once the copy warp has seen the sources complete, the statistics are read and the
         // row factor computed, and the first residual chunk is requested, while the operands are still on their way instead
@@ -637,7 +639,7 @@ __device__ __forceinline__ void gemm_epilogue(const VmProgram& prog, Ctl* ctl, u
         // as a factor, or as the producer's per-tile sums of squares (complete: the operands behind this accumulator
         // were only copied after the producer stage had finished)
         // (once per row band: a worker's next tiles are mostly of the same one, and the statistics are a round trip to L2)
-        const bool factors = m_tile != known_band;
+        const bool factors = (EPI == EPI_F32 && LEAN) || m_tile != known_band;
         known_band = m_tile;
         if (factors) { row_scale = g.alpha; row_shift = 0.f; }
         if (kStats && factors && main && row_ok && g.row_factor) row_scale *= __ldcg(g.row_factor + row);
@@ -792,6 +794,8 @@ __device__ __forceinline__ void gemm_instruction(const VmProgram& prog, Ctl* ctl
     else if (epilogue == EPI_FP4) gemm_epilogue<EPI_FP4, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_QKV_ROPE) gemm_epilogue<EPI_QKV_ROPE, LEAN && !ROTARY_ROWS>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (LEAN || epilogue == EPI_BF16_EXT) gemm_epilogue<EPI_BF16_EXT, LEAN>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
+    else if (epilogue == EPI_F32 && st.p.gemm.operands == GEMM_NVFP4 && !st.p.gemm.bias && !st.p.gemm.residual)
+        gemm_epilogue<EPI_F32, true>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else if (epilogue == EPI_F32) gemm_epilogue<EPI_F32>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     else gemm_epilogue<EPI_GEGLU_BF16>(prog, ctl, tmem, st, stage_index, first, count, ps, stamp);
     if (stamp && threadIdx.x == 128) stamp[2] = static_cast<long long>(global_ns());
