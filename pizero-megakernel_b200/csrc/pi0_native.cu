@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/pi0_native.h"
+#include "solo.h"
 #include "vm_kernel.cuh"
 
 namespace pi0 {
@@ -103,6 +104,13 @@ int encode_bf16_rows(CUtensorMap* map, const void* base, size_t rows, int ld, in
 
 struct Program;
 
+// Stand-alone launch through a kernel of its own (solo.h), made together with the stand-alone program.
+struct SoloRoute {
+    enum { NORM } kind;
+    SoloNorm norm{};
+    int grid = 0, groups = 1;
+};
+
 struct Op {
     uint32_t magic = kOpMagic;
     int device = 0;
@@ -127,6 +135,7 @@ struct Op {
     void* prep_scratch = nullptr;      // its padded BF16 copies of Q, K and V
     Program* solo = nullptr;           // lazily built one/two-stage program for stand-alone launches
     bool solo_dirty = true;
+    std::unique_ptr<SoloRoute> route;  // how such a launch runs instead, where the operator has a kernel of its own (status, counters and epoch stay the program's)
 };
 
 struct Program {
@@ -337,7 +346,8 @@ int build_program(Program** out, int device, const std::vector<StageDesc>& stage
     return cudaSuccess;
 }
 
-int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begin, int end, bool new_epoch) {
+// What every launch of a program, or in the place of one, begins with.
+int begin_launch(Program* prog, cudaStream_t stream, bool new_epoch) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
@@ -354,6 +364,11 @@ int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begi
         }
         prog->epoch++;
     }
+    return cudaSuccess;
+}
+
+int launch_program(Program* prog, cudaStream_t stream, LaunchInputs in, int begin, int end, bool new_epoch) {
+    if (int e = begin_launch(prog, stream, new_epoch)) return e;
     VmProgram p{};
     p.stages = prog->d_stages;
     p.code = prog->d_code;
@@ -553,6 +568,37 @@ int gemm_configure(Op* op, bool refresh, Change change) {
     return cudaSuccess;
 }
 
+// The kernel of its own that a stand-alone launch of `op` takes, if there is one.  Its finished tiles are counted where the program's
+// would be, so the counters of the handle keep their meaning (expected: per launch and row band).
+int solo_route(Op* op) {
+    op->route.reset();
+    auto route = std::make_unique<SoloRoute>();
+    Program* prog = op->solo;
+    const StageDesc& d = op->desc;
+    std::vector<unsigned int> expected(prog->expected.size(), 0);
+    if (d.kind == OP_NORM) {
+        route->kind = SoloRoute::NORM;
+        route->norm.n = d.p.norm;
+        // four rows (256 threads) per CTA, eight where that would be more than one round of them
+        const int rows = d.p.norm.rows;
+        route->groups = (rows + kNormPairRows - 1) / kNormPairRows <= op->workers ? 1 : 2;
+        const int per = kNormPairRows * route->groups, blocks = (rows + per - 1) / per;
+        route->grid = std::min(blocks, op->workers);
+        for (int b = 0; b < blocks; b++) expected[b * per / kBandRows]++;
+        SoloGuard& guard = route->norm.guard;
+        guard = {prog->d_status, prog->budget_ns, prog->d_counters, 1};
+    } else {
+        return cudaSuccess;
+    }
+    prog->expected = expected;
+    op->route = std::move(route);
+    return cudaSuccess;
+}
+cudaError_t launch_route(const Op* op, cudaStream_t stream) {
+    const SoloRoute& r = *op->route;
+    return launch_solo_norm(r.norm, r.grid, r.groups, stream);
+}
+
 // Stand-alone program of one operator (plus its merge stage when the attention is split).
 int solo_program(Op* op) {
     if (op->solo && !op->solo_dirty) return cudaSuccess;
@@ -599,6 +645,7 @@ int solo_program(Op* op) {
     const cudaError_t ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
     if (ce != cudaSuccess) return ce;
     op->solo->early = op->solo->grid <= sms * 3 / 10;
+    if (int re = solo_route(op)) return re;
     op->solo_dirty = false;
     return cudaSuccess;
 }
@@ -613,6 +660,10 @@ int launch_solo(void* handle, void* stream) {
         if (device != op->device) return cudaErrorInvalidDevice;
         int e = solo_program(op);
         if (e) return e;
+    }
+    if (op->route) {
+        if (int e = begin_launch(op->solo, static_cast<cudaStream_t>(stream), true)) return e;
+        return launch_route(op, static_cast<cudaStream_t>(stream));
     }
     return launch_program(op->solo, static_cast<cudaStream_t>(stream), LaunchInputs{}, 0, static_cast<int>(op->solo->stages.size()), true);
 }

@@ -91,7 +91,7 @@ __device__ __forceinline__ void mark(const VmProgram& prog, int code) {
 }
 
 // (out of line: it runs once, when a launch gives up, and its stores need not sit in every wait loop)
-__device__ __noinline__ void report(const VmProgram& prog, int code, int stage, int band, unsigned int observed,
+static __device__ __noinline__ void report(const VmProgram& prog, int code, int stage, int band, unsigned int observed,
                                        unsigned int expected) {
     VmStatus* s = prog.status;
     if (atomicCAS(&s->abort, 0, 1) == 0) {
@@ -108,7 +108,7 @@ __device__ __noinline__ void report(const VmProgram& prog, int code, int stage, 
 // Wait on an mbarrier phase with a time budget. Returns false when the budget expires or the
 // program has been aborted; the caller leaves its loop.  The first try suspends for up to about a microsecond, which
 // covers nearly every wait of a running pipeline; the loop behind it is out of line, so that the pipeline loops stay short.
-__device__ __noinline__ bool mbar_wait_long(const VmProgram& prog, Ctl* ctl, uint64_t* bar, uint32_t parity, int stage) {
+static __device__ __noinline__ bool mbar_wait_long(const VmProgram& prog, Ctl* ctl, uint64_t* bar, uint32_t parity, int stage) {
     // Reading the global timer costs about a microsecond, so the clock is only consulted once a wait has
     // already lasted for several tries (the budget counts from that first reading).
     unsigned long long start = 0;
@@ -135,7 +135,7 @@ __device__ __forceinline__ bool mbar_wait(const VmProgram& prog, Ctl* ctl, uint6
 // vote, and every lane has observed the completed phase when the call returns.  Only lane 0 keeps the time budget; its
 // verdict is broadcast, so a time-out can never split the warp in front of a warp-collective instruction.
 // (A version in which lane 0 waited alone and the others adopted its result measured 3 % slower on the pi0 forward.)
-__device__ __noinline__ bool mbar_wait_warp_long(const VmProgram& prog, Ctl* ctl, uint64_t* bar, uint32_t parity, int stage) {
+static __device__ __noinline__ bool mbar_wait_warp_long(const VmProgram& prog, Ctl* ctl, uint64_t* bar, uint32_t parity, int stage) {
     unsigned long long start = 0;
     for (uint32_t spin = 1;; ++spin) {
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;   // each try suspends for at most ~1 us

@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import subprocess
+import tempfile
 from pathlib import Path
 
 import torch
@@ -18,20 +19,24 @@ LIBRARY = HERE / "libpi0_native.so"
 TRACE_LIBRARY = HERE / "libpi0_trace.so"
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "--expt-relaxed-constexpr", "-shared", "-Xcompiler", "-fPIC"]
+              "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC"]
+UNITS = ("pi0_native.cu", "solo_norm.cu")
 
 
 def build(force=False, verbose=False):
     """Compile the CUDA extension in-tree (cross-compiles without a GPU)."""
     nvcc = os.environ.get("NVCC", "nvcc")
-    sources = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h"))
-    newest = max(p.stat().st_mtime for p in sources)
+    units = [CSRC / name for name in UNITS]
+    newest = max(p.stat().st_mtime for p in [*units, *CSRC.glob("*.cuh"), *CSRC.glob("*.h"), *HERE.parent.parent.glob("include/*.h")])
     if force or not LIBRARY.exists() or LIBRARY.stat().st_mtime < newest:
-        cmd = [nvcc, *NVCC_FLAGS, "-o", str(LIBRARY), str(CSRC / "pi0_native.cu")]
-        if verbose:
-            cmd.insert(1, "-Xptxas")
-            cmd.insert(2, "-v")
-        subprocess.run(cmd, check=True)
+        with tempfile.TemporaryDirectory() as folder:                       # units side by side, then one link
+            objects = [str(Path(folder) / (unit.stem + ".o")) for unit in units]
+            verbosity = ["-Xptxas", "-v"] if verbose else []
+            compilers = [subprocess.Popen([nvcc, *NVCC_FLAGS, *verbosity, "-c", "-o", out, str(unit)]) for unit, out in zip(units, objects)]
+            codes = [c.wait() for c in compilers]
+            if any(codes):
+                raise subprocess.CalledProcessError(max(codes, key=abs), [nvcc, "-c", *map(str, units)])
+            subprocess.run([nvcc, *NVCC_FLAGS, "-shared", "-o", str(LIBRARY), *objects], check=True)
     trace_src = CSRC / "launch_trace.cpp"
     if trace_src.exists() and (force or not TRACE_LIBRARY.exists() or TRACE_LIBRARY.stat().st_mtime < trace_src.stat().st_mtime):
         cuda_home = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
