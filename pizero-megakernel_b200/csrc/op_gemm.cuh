@@ -337,14 +337,15 @@ __device__ __forceinline__ DrainRow drain_row(const GemmParams& g, int row) {
 // (Instantiated per epilogue kind: each accumulator drain carries only its own arithmetic and registers.  Values are kept as
 // pairs: the packed FP32 operations shorten the straight-line code that a drain executes once.)
 // LEAN: without the options only the BF16 model uses (rounding before the residual, GELU on BF16 output) and without ReLU^2.
-template <int EPI, bool LEAN = false>
+// TOGETHER: FP32 rows are stored by the whole warp (store_rows64); every lane of the warp calls.
+template <int EPI, bool LEAN = false, bool TOGETHER = false>
 __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const DrainRow& d, const uint32_t (&raw)[32], const uint4 (&res)[4], int row, int col0,
                                                     bool row_ok, float row_scale, float row_shift, float2& sumsq, float2& sum) {
     float2 v[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = mul2(make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1])), make_float2(row_scale, row_scale));
     constexpr bool kWarpStore = EPI == EPI_BF16 || EPI == EPI_BF16_EXT;      // (rows stored together take the whole warp)
-    if (!kWarpStore && !row_ok && !(EPI == EPI_QKV_ROPE && d.together)) return;
+    if (!kWarpStore && !row_ok && !(EPI == EPI_QKV_ROPE && d.together) && !(EPI == EPI_F32 && TOGETHER)) return;
     if constexpr (EPI == EPI_BF16_EXT || EPI == EPI_FP4) {
         if (d.center) {
             // folded LayerNorm: subtract the row mean's share, mean * rstd * (sum over K of weight row n)
@@ -401,6 +402,19 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& g, const D
         add_bf16x32(v, res);
     }
     if (d.bias && !early_bias) add_bias();
+    if constexpr (EPI == EPI_F32 && TOGETHER) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint4 p[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 a = v[8 * h + 2 * i], b = v[8 * h + 2 * i + 1];
+                p[i] = make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
+            }
+            store_rows64(d.out + static_cast<size_t>(col0 + 16 * h) * 4, g.ldo * 4, d.rows_left, p);
+        }
+        return;
+    }
     if constexpr (EPI == EPI_F32) {
         float4* dst = reinterpret_cast<float4*>(d.out + static_cast<size_t>(col0) * 4);
 #pragma unroll

@@ -106,8 +106,9 @@ struct Program;
 
 // Stand-alone launch through a kernel of its own (solo.h), made together with the stand-alone program.
 struct SoloRoute {
-    enum { NORM } kind;
+    enum { NORM, GEMM } kind;
     SoloNorm norm{};
+    SoloGemmPlan gemm{};
     int grid = 0, groups = 1;
 };
 
@@ -570,7 +571,7 @@ int gemm_configure(Op* op, bool refresh, Change change) {
 
 // The kernel of its own that a stand-alone launch of `op` takes, if there is one.  Its finished tiles are counted where the program's
 // would be, so the counters of the handle keep their meaning (expected: per launch and row band).
-int solo_route(Op* op) {
+int solo_route(Op* op, int sms) {
     op->route.reset();
     auto route = std::make_unique<SoloRoute>();
     Program* prog = op->solo;
@@ -587,6 +588,17 @@ int solo_route(Op* op) {
         for (int b = 0; b < blocks; b++) expected[b * per / kBandRows]++;
         SoloGuard& guard = route->norm.guard;
         guard = {prog->d_status, prog->budget_ns, prog->d_counters, 1};
+    } else if (d.kind == OP_GEMM) {
+        route->kind = SoloRoute::GEMM;
+        const SoloGemmRequest request{&d.p.gemm, op->a, op->b, op->m, op->n, op->k, op->operands, op->workers};
+        SoloGemmPlan& plan = route->gemm;
+        cudaError_t e = plan_solo_gemm(request, &plan);
+        if (e == cudaErrorNotSupported) return cudaSuccess;
+        if (e != cudaSuccess) return e;
+        SoloGemm& p = plan.args;
+        route->grid = plan.grid;
+        for (int row = 0; row < d.p.gemm.rows; row += p.tile_rows) expected[row / kBandRows] += p.n_tiles;
+        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, plan.grid <= sms * 3 / 10 ? 1 : 0};
     } else {
         return cudaSuccess;
     }
@@ -596,7 +608,9 @@ int solo_route(Op* op) {
 }
 cudaError_t launch_route(const Op* op, cudaStream_t stream) {
     const SoloRoute& r = *op->route;
-    return launch_solo_norm(r.norm, r.grid, r.groups, stream);
+    if (r.kind == SoloRoute::NORM) return launch_solo_norm(r.norm, r.grid, r.groups, stream);
+    return op->operands == GEMM_NVFP4 ? launch_solo_gemm_nvfp4(r.gemm.args, r.gemm.cg, r.grid, r.gemm.smem, stream)
+                                      : launch_solo_gemm_dense(r.gemm.args, r.gemm.cg, r.grid, r.gemm.smem, stream);
 }
 
 // Stand-alone program of one operator (plus its merge stage when the attention is split).
@@ -645,7 +659,7 @@ int solo_program(Op* op) {
     const cudaError_t ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
     if (ce != cudaSuccess) return ce;
     op->solo->early = op->solo->grid <= sms * 3 / 10;
-    if (int re = solo_route(op)) return re;
+    if (int re = solo_route(op, sms)) return re;
     op->solo_dirty = false;
     return cudaSuccess;
 }

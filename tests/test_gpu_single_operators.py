@@ -1,13 +1,22 @@
 """Operators that are launched by themselves have kernels of their own (``csrc/solo.h``).  They are held to the stage of a program with the
 same handle - bit for bit where both add up in one order - and otherwise to 64-bit arithmetic, at the edges of their tiles and of the
 rules that choose them."""
+import numpy as np
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
+from native_pi0.dense import ResidentDense
 from native_pi0.linear import NativeStageProgram
 from native_pi0.normalization import ResidentNorm
+from native_pi0.primitives import ResidentNVFP4
+from native_pi0.quantization import PackedNVFP4
+
+
+def codes(rng, rows, k, scale):
+    return PackedNVFP4(rng.integers(0, 256, size=(rows, k // 2), dtype=np.uint8), rng.integers(40, 61, size=(rows, k // 16), dtype=np.uint8),
+                       np.float32(scale), (rows, k))
 
 
 def outputs(op):
@@ -31,6 +40,63 @@ def alone_and_as_a_stage(op):
         assert status["code"] == 0 and status["epoch"] == launch + 1
         for got, w in zip(outputs(op), want):
             assert torch.equal(got, w)
+
+
+@pytest.mark.parametrize("rows,n,k,block_n,tiled", [
+    (1, 128, 64, 128, False),            # a single K group, one tile
+    (51, 2560, 1024, 64, True),
+    (51, 640, 320, 32, False),           # 32-wide tiles with scales of their own, half-filled last slot
+    (129, 384, 1152, 128, False),        # one row in the second band
+    (256, 16384, 1024, 128, True),       # pairs of CTAs: 192-wide tiles over blocks of 128 rows, the last one cut
+    (640, 8256 // 128 * 128, 1088, 128, False),      # odd number of row bands, K not in whole slots
+    (300, 16384, 512, 64, True),         # blocks of 64 rows
+])
+@pytest.mark.parametrize("out,act", [("f32", "none"), ("bf16", "none"), ("fp4", "none"), ("fp4", "gelu"), ("fp4", "geglu"), ("fp4", "relu2")])
+def test_nvfp4_projection(rows, n, k, block_n, tiled, out, act):
+    if act == "geglu" and n % 256:
+        pytest.skip("GeGLU takes whole pairs of 128 columns")
+    rng, m = np.random.default_rng(rows + n + k), -(-rows // 128) * 128
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    added = out != "f32" and act != "geglu"
+    with ResidentNVFP4(None, codes(rng, m, k, 1.0), codes(rng, n, k, 0.01), workers=148, rows=rows, block_n=block_n, tiled_weight=tiled,
+                       output_dtype={"f32": torch.float32, "bf16": torch.bfloat16, "fp4": torch.uint8}[out], output_gelu=act == "gelu",
+                       output_geglu=act == "geglu", output_relu2=act == "relu2",
+                       bias=torch.randn(n, generator=g, device="cuda") if added else None,
+                       residual=torch.randn(m, n, generator=g, device="cuda") if added else None) as op:
+        alone_and_as_a_stage(op)
+
+
+@pytest.mark.parametrize("workers", [1, 3, 148])
+@pytest.mark.parametrize("rows,n,k", [(1, 104, 504), (65, 1000, 1152), (333, 1000, 1152), (820, 4400, 1088), (256, 9000, 640)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float8_e4m3fn])
+def test_dense_projection(rows, n, k, dtype, workers):
+    g = torch.Generator(device="cuda").manual_seed(rows + n + k)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")          # noqa: E731
+    for kind in (dict(output_dtype=torch.float32), dict(output_dtype=torch.float32, bias=randn(n), residual=randn(rows, n)), dict(bias=randn(n), residual=randn(rows, n))):
+        with ResidentDense(None, randn(rows, k).to(dtype), randn(n, k).to(dtype), alpha=0.05, workers=workers, **kind) as op:
+            alone_and_as_a_stage(op)
+
+
+@pytest.mark.parametrize("rows,n,k,dtype", [(768, 2048, 16384, torch.float8_e4m3fn), (513, 1930, 8192, torch.float8_e4m3fn), (300, 1200, 8192, torch.bfloat16)])
+def test_dense_projection_over_a_long_k(rows, n, k, dtype):
+    """K split over the pairs of a cluster: sums of parts, repeated bit for bit and no further from 64 bits than one sum over all of K."""
+    g = torch.Generator(device="cuda").manual_seed(k + n)
+    a, b = torch.randn(rows, k, generator=g, device="cuda").to(dtype), torch.randn(n, k, generator=g, device="cuda").to(dtype)
+    with ResidentDense(None, a, b, output_dtype=torch.float32, workers=148) as op:
+        exact = a.double() @ b.double().T
+        bound = 2.0 ** -22 * k ** 0.5 * (a.double().abs() @ b.double().abs().T)              # (FP32 sums of K terms)
+        with NativeStageProgram(None, [(op, [])]) as program:
+            program.forward()
+            single = float((op.logical_output.double() - exact).norm())
+        want = op.forward().clone()
+        assert op.status()["code"] == 0 and bool(((want.double() - exact).abs() <= bound).all())
+        assert float((want.double() - exact).norm()) <= 1.02 * single
+        for _ in range(3):
+            op.output.fill_(float("nan"))
+            assert torch.equal(op.forward(), want)
+    bias, residual = torch.randn(n, generator=g, device="cuda"), torch.randn(rows, n, generator=g, device="cuda").bfloat16()
+    with ResidentDense(None, a, b, bias=bias, residual=residual, workers=148) as op:
+        assert torch.equal(op.forward(), (want + residual.float() + bias.bfloat16().float()).bfloat16())
 
 
 @pytest.mark.parametrize("rows,width", [(1, 16), (51, 1024), (592, 2048), (593, 1168), (2000, 64)])
