@@ -106,10 +106,12 @@ struct Program;
 
 // Stand-alone launch through a kernel of its own (solo.h), made together with the stand-alone program.
 struct SoloRoute {
-    enum { NORM, GEMM } kind;
+    enum { NORM, GEMM, ATTENTION } kind;
     SoloNorm norm{};
     SoloGemmPlan gemm{};
+    SoloAttnPlan attention{};
     int grid = 0, groups = 1;
+    std::vector<int> band_tiles;       // attention: row tiles per 128-query band
 };
 
 struct Op {
@@ -599,6 +601,23 @@ int solo_route(Op* op, int sms) {
         route->grid = plan.grid;
         for (int row = 0; row < d.p.gemm.rows; row += p.tile_rows) expected[row / kBandRows] += p.n_tiles;
         p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, plan.grid <= sms * 3 / 10 ? 1 : 0};
+    } else if (d.kind == OP_ATTN && !op->prep) {
+        route->kind = SoloRoute::ATTENTION;
+        SoloAttnPlan& plan = route->attention;
+        cudaError_t e = plan_solo_attention(d.p.attn, op->partial_o, op->partial_bytes / (kAttnQRows * 256 * sizeof(uint16_t)), op->workers, sms, &plan);
+        if (e == cudaErrorNotSupported) return cudaSuccess;
+        if (e != cudaSuccess) return e;
+        SoloAttn& p = plan.args;
+        route->grid = plan.grid;
+        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, plan.grid <= sms * 3 / 10 ? 1 : 0};
+        route->band_tiles.assign(d.bands, 0);
+        for (int t = 0; t < plan.row_tiles; t++) {
+            const int band = t * 128 / p.heads / 128;
+            route->band_tiles[band]++;
+            expected[band] += p.splits;
+        }
+        p.partial_ml = op->partial_ml;
+        p.tickets = prog->d_counters + prog->stages[0].aux_base;
     } else {
         return cudaSuccess;
     }
@@ -607,7 +626,12 @@ int solo_route(Op* op, int sms) {
     return cudaSuccess;
 }
 cudaError_t launch_route(const Op* op, cudaStream_t stream) {
-    const SoloRoute& r = *op->route;
+    SoloRoute& r = *op->route;
+    if (r.kind == SoloRoute::ATTENTION) {
+        SoloAttn& p = r.attention.args;
+        p.target = op->solo->epoch * static_cast<unsigned int>(p.splits) * 4u;
+        return launch_solo_attention(p, r.grid, r.attention.smem, stream);
+    }
     if (r.kind == SoloRoute::NORM) return launch_solo_norm(r.norm, r.grid, r.groups, stream);
     return op->operands == GEMM_NVFP4 ? launch_solo_gemm_nvfp4(r.gemm.args, r.gemm.cg, r.grid, r.gemm.smem, stream)
                                       : launch_solo_gemm_dense(r.gemm.args, r.gemm.cg, r.grid, r.gemm.smem, stream);
@@ -634,6 +658,8 @@ int solo_program(Op* op) {
             self.p.gemm.tmap_b = op->maps + 2;
         }
     }
+    // (tickets of the split attention's own kernel; a program's stage has them only with the merge inside)
+    if (self.kind == OP_ATTN && self.p.attn.splits > 1) self.aux_count = self.p.attn.heads * self.bands;
     stages.push_back(self);
     work.push_back({self.tiles, op->cost});
     if (op->merge && !op->desc.p.attn.fused_merge) {
@@ -1289,9 +1315,11 @@ extern "C" int configure_attention_splits(void* handle, int splits) {
     float* partial_ml = nullptr;
     const int groups = a.heads * ((a.nq + kAttnQRows - 1) / kAttnQRows);          // heads x 128-query tiles
     const size_t tasks = static_cast<size_t>(groups) * splits;
+    // (the kernel of its own that a stand-alone launch may take has splits of its own: one round of SMs at most)
+    const size_t room = a.kv_heads == 1 && a.head_dim == 256 ? std::max<size_t>(tasks, sm_count(op->device)) : tasks;
     if (splits > 1) {
-        cudaError_t e = cudaMalloc(&partial_o, tasks * kAttnQRows * a.head_dim * sizeof(uint16_t));
-        if (e == cudaSuccess) e = cudaMalloc(&partial_ml, tasks * kAttnQRows * 2 * sizeof(float));
+        cudaError_t e = cudaMalloc(&partial_o, room * kAttnQRows * a.head_dim * sizeof(uint16_t));
+        if (e == cudaSuccess) e = cudaMalloc(&partial_ml, room * kAttnQRows * 2 * sizeof(float));
         if (e != cudaSuccess) {
             cudaFree(partial_o);
             cudaFree(partial_ml);
@@ -1303,8 +1331,8 @@ extern "C" int configure_attention_splits(void* handle, int splits) {
     cudaFree(op->partial_ml);
     op->partial_o = partial_o;
     op->partial_ml = partial_ml;
-    op->partial_bytes = splits > 1 ? tasks * kAttnQRows * a.head_dim * sizeof(uint16_t) : 0;
-    op->stat_bytes = splits > 1 ? tasks * kAttnQRows * 2 * sizeof(float) : 0;
+    op->partial_bytes = splits > 1 ? room * kAttnQRows * a.head_dim * sizeof(uint16_t) : 0;
+    op->stat_bytes = splits > 1 ? room * kAttnQRows * 2 * sizeof(float) : 0;
     a.splits = splits;
     a.fused_merge = 0;
     a.partial_o = partial_o;
@@ -1363,7 +1391,12 @@ extern "C" int attention_split_diagnostics(void* handle, unsigned long long* cou
     std::vector<unsigned int> raw(op->solo->expected.size());
     e = cudaMemcpy(raw.data(), op->solo->d_counters, raw.size() * sizeof(unsigned int), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return e;
-    if (a.fused_merge && d.aux_count == groups) {
+    if (op->route) {
+        // the kernel of its own: arrivals of the row tiles that hold the band's rows, in units of the configured splits
+        const int own = op->route->attention.args.splits;
+        for (int g = 0; g < groups; g++)
+            counts[g] = static_cast<unsigned long long>(raw[d.counter_base + g / a.heads]) * a.splits / static_cast<unsigned int>(op->route->band_tiles[g / a.heads] * own);
+    } else if (a.fused_merge && d.aux_count == groups) {
         for (int g = 0; g < groups; g++) counts[g] = raw[d.aux_base + g];
     } else {
         // one counter per 128-query tile: heads * splits tiles each, every head of the tile has the same share

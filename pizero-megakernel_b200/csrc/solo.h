@@ -45,6 +45,32 @@ struct alignas(64) SoloGemm {
     int sf_col, sf_mask, tmem_cols;  // first scale column, slots whose scales alternate (mask), columns allocated
 };
 
+struct alignas(64) SoloAttn {
+    CUtensorMap map_q, map_k, map_v;     // BF16 rows with boxes of 64 columns
+    CUtensorMap map_out;         // rows of the output, or of the partial rows
+    SoloGuard guard;
+    void* out;                   // BF16 [rows, 256]
+    uint16_t* partial_o;         // BF16 bits [row tile][split][128][256]
+    float* partial_ml;           // FP32 [row tile][split][128][2]
+    unsigned int* tickets;       // program counters: 64-column pieces (4 a CTA) whose partial rows are out, per row tile, over all launches ...
+    unsigned int target;         // ... and how many that will be after this one
+    int rows, heads;             // rows = queries x heads
+    int keys, splits, per, cols; // keys of a split, score columns computed for them (a multiple of 16, at most 272)
+    int box_rows, boxes;         // rows of K / V per copy, copies per 64-column piece
+    int items;                   // row tiles x splits
+    int off_k, off_v, ctl_offset;    // shared memory: Q and P at 0, K, V
+    int prefix;
+    float scale;
+};
+struct SoloAttnPlan {
+    SoloAttn args;
+    int grid, row_tiles;
+    size_t smem;
+};
+// `room`: items for which `partial_o` has partial rows.
+cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t room, int workers, int sms, SoloAttnPlan* plan);
+cudaError_t launch_solo_attention(const SoloAttn& p, int grid, size_t smem, cudaStream_t stream);
+
 // What a GEMM handle asks for; tile geometry and ring of `g` are the persistent kernel's and are not read.
 struct SoloGemmRequest {
     const GemmParams* g;
@@ -76,6 +102,8 @@ int solo_gemm_clusters(int ctas);
 constexpr int kSoloChunks1 = 2, kSoloChunks2 = 1;    // 128-byte chunks of K per slot: tiles of one CTA, of a pair
 constexpr int kSoloMaxSlots = 8;
 constexpr int kSoloCtlBytes = 1024;
+constexpr int kSoloMaxSmem = 227 * 1024;
+constexpr int kSoloAttnCtl = 5120;                   // barriers, exchange of the softmax
 constexpr int kSoloDataBytes = 225 * 1024;
 
 }  // namespace pi0

@@ -160,4 +160,62 @@ cudaError_t plan_solo_gemm(const SoloGemmRequest& r, SoloGemmPlan* plan) {
     return e;
 }
 
+cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t room, int workers, int sms, SoloAttnPlan* plan) {
+    if (!a.tc || a.mask || a.out_fp4 || !a.out || a.batches != 1 || a.kv_heads != 1 || a.head_dim != 256 || a.hd_pad != 256 || a.ldq != a.heads * 256 ||
+        a.ldo != a.heads * 256)
+        return cudaErrorNotSupported;
+    memset(plan, 0, sizeof(*plan));
+    SoloAttn& p = plan->args;
+    p.rows = a.nq * a.heads;
+    const int row_tiles = (p.rows + 127) / 128;
+    // KV splits of the kernel's own, the same whatever the number of workers (the order of the sums hangs on them).  The estimate (us): rounds of
+    // SMs, the keys of a tile, and the meeting of the splits - the partial rows of all CTAs through L2, then the rows that a warp merges one
+    // batch of loads after another.  It picks the fastest of 41 shapes tried, or one within 2 % (9 - 101 queries over 300 - 920 keys: 8 - 13 splits,
+    // 9.0 - 10.4 us; 256 rows unsplit 9.6, with 4 splits 10.4; 300 rows in 4 splits 10.7, in 2 12.6, in 7 11.9; 784 rows in 3 15.3, in 4 23).
+    const int most = a.splits == 1 ? 1 : static_cast<int>(room / row_tiles);
+    int best = 0;
+    double least = 0;
+    for (int s = 1; s <= 64 && s <= a.nk; s++) {
+        const int per = (a.nk + s - 1) / s, cols = (per + 15) / 16 * 16;
+        if (cols > 272 || (s - 1) * per >= a.nk || s > most) continue;
+        const int rounds = (row_tiles * s + sms - 1) / sms, rows = (128 + s - 1) / s, at_once = s <= 4 ? 48 : 16;
+        double t = rounds * (4.0 + cols * 0.022);
+        if (s > 1) t += 4.2 + 0.9 * ((rows + at_once - 1) / at_once - 1) + 0.9 * row_tiles * s / sms + 0.3 * std::max(0, s - 12);
+        if (best == 0 || t < least) { best = s; least = t; }
+    }
+    if (!best) return cudaErrorNotSupported;
+    p.splits = best;
+    p.per = (a.nk + best - 1) / best;
+    p.cols = (p.per + 15) / 16 * 16;
+    p.boxes = p.cols > 256 ? 2 : 1;
+    p.box_rows = p.cols / p.boxes;
+    p.keys = a.nk;
+    p.heads = a.heads;
+    p.items = row_tiles * best;
+    p.prefix = a.prefix;
+    p.scale = a.scale;
+    p.out = a.out;
+    p.partial_o = partial_o;
+    plan->row_tiles = row_tiles;
+    plan->grid = std::min(p.items, std::min(workers, sms));
+    const int first = std::max(4 * 16384, (p.cols + 63) / 64 * 16384), kv = 4 * p.cols * 128;     // Q, later P; K or V
+    p.off_k = first;
+    const bool apart = first + 2 * kv + kSoloAttnCtl + 1024 <= kSoloMaxSmem;
+    p.off_v = apart ? first + kv : first;
+    p.ctl_offset = p.off_v + kv;
+    plan->smem = p.ctl_offset + kSoloAttnCtl + 1024;
+    if (plan->smem > static_cast<size_t>(kSoloMaxSmem)) return cudaErrorNotSupported;
+    const cuuint64_t q_dims[2] = {256u, static_cast<cuuint64_t>(p.rows)}, q_strides[1] = {512u};
+    const cuuint32_t q_box[2] = {64u, 128u};
+    const cuuint64_t kv_dims[2] = {256u, static_cast<cuuint64_t>(a.kv_batch_rows)}, kv_strides[1] = {static_cast<cuuint64_t>(a.ldkv) * 2u};
+    const cuuint32_t kv_box[2] = {64u, static_cast<cuuint32_t>(p.box_rows)};
+    cudaError_t e = encode(&p.map_q, a.q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q_dims, q_strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (e == cudaSuccess) e = encode(&p.map_k, a.k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (e == cudaSuccess) e = encode(&p.map_v, a.v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    const cuuint64_t out_dims[2] = {256u, static_cast<cuuint64_t>(best > 1 ? p.items * 128 : p.rows)};
+    if (e == cudaSuccess)
+        e = encode(&p.map_out, best > 1 ? static_cast<const void*>(partial_o) : a.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, out_dims, q_strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    return e;
+}
+
 }  // namespace pi0

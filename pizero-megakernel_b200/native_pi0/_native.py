@@ -20,7 +20,7 @@ TRACE_LIBRARY = HERE / "libpi0_trace.so"
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC"]
-UNITS = ("pi0_native.cu", "solo_plan.cpp", "solo_norm.cu", "solo_gemm_nvfp4.cu", "solo_gemm_dense.cu")
+UNITS = ("pi0_native.cu", "solo_plan.cpp", "solo_norm.cu", "solo_gemm_nvfp4.cu", "solo_gemm_dense.cu", "solo_attention.cu")
 
 
 def build(force=False, verbose=False):

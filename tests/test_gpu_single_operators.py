@@ -7,6 +7,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from native_pi0.attention import ResidentAttention
 from native_pi0.dense import ResidentDense
 from native_pi0.linear import NativeStageProgram
 from native_pi0.normalization import ResidentNorm
@@ -97,6 +98,36 @@ def test_dense_projection_over_a_long_k(rows, n, k, dtype):
     bias, residual = torch.randn(n, generator=g, device="cuda"), torch.randn(rows, n, generator=g, device="cuda").bfloat16()
     with ResidentDense(None, a, b, bias=bias, residual=residual, workers=148) as op:
         assert torch.equal(op.forward(), (want + residual.float() + bias.bfloat16().float()).bfloat16())
+
+
+@pytest.mark.parametrize("nq,nk,heads,prefix,splits,workers", [
+    (1, 1, 1, None, 1, 148), (1, 16, 8, None, 1, 148), (16, 17, 8, 3, 1, 148),                # one row; whole and ragged pieces of 16 keys
+    (17, 256, 8, None, 1, 2), (300, 256, 3, 100, 1, 148),                                     # heads that do not divide the 128 rows of a tile
+    (784, 784, 8, None, 4, 148), (700, 816, 8, None, 4, 148), (769, 819, 8, 0, 4, 40),        # up to 272 keys a tile; several tiles per CTA
+    (51, 819, 8, 768, 13, 148), (51, 819, 8, 768, 13, 3), (101, 920, 8, 819, 13, 148), (2, 2000, 8, 1500, 32, 148),
+])
+def test_attention_of_heads_with_one_kv_head(nq, nk, heads, prefix, splits, workers):
+    g = torch.Generator(device="cuda").manual_seed(nq + nk)
+    make = lambda n, h: torch.randn(1, n, h, 256, generator=g, device="cuda").bfloat16()      # noqa: E731
+    q, k, v = make(nq, heads), make(nk, 1), make(nk, 1)
+    scores = torch.einsum("qhd,kd->hqk", q[0].double(), k[0, :, 0].double()) / 16
+    if prefix is not None:
+        scores[:, 0, prefix + 1:] = -torch.inf
+    want = torch.einsum("hqk,kd->qhd", scores.softmax(-1), v[0, :, 0].double())
+    with ResidentAttention(None, q, k, v, workers=workers, prefix=prefix, splits=splits, head_dim=256, path="tcgen05") as op:
+        for launch in range(3):
+            op.output.fill_(float("nan"))
+            if splits > 1:
+                op.poison_partials()
+            got = op.forward().reshape(nq, heads, 256).clone()
+            assert op.status()["code"] == 0
+            assert float((got.double() - want).norm() / want.norm()) <= 6e-3                  # (probabilities and rows in BF16)
+            if launch:
+                assert torch.equal(got, first)
+            first = got
+        if splits > 1:
+            state = op.read_split_counts()
+            assert state["epoch"] == 3 and all(c == 3 * splits for c in state["counts"])
 
 
 @pytest.mark.parametrize("rows,width", [(1, 16), (51, 1024), (592, 2048), (593, 1168), (2000, 64)])
