@@ -611,7 +611,8 @@ int solo_route(Op* op, int sms) {
         route->grid = plan.grid;
         p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, plan.grid <= sms * 3 / 10 ? 1 : 0};
         route->band_tiles.assign(d.bands, 0);
-        for (int t = 0; t < plan.row_tiles; t++) {
+        if (p.head_dim != 256) std::fill(expected.begin(), expected.begin() + d.bands, static_cast<unsigned int>(p.heads));
+        for (int t = 0; p.head_dim == 256 && t < plan.row_tiles; t++) {
             const int band = t * 128 / p.heads / 128;
             route->band_tiles[band]++;
             expected[band] += p.splits;

@@ -46,7 +46,7 @@ struct alignas(64) SoloGemm {
 };
 
 struct alignas(64) SoloAttn {
-    CUtensorMap map_q, map_k, map_v;     // BF16 rows with boxes of 64 columns
+    CUtensorMap map_q, map_k, map_v;     // BF16 [image][row][columns] with boxes of 64 columns
     CUtensorMap map_out;         // rows of the output, or of the partial rows
     SoloGuard guard;
     void* out;                   // BF16 [rows, 256]
@@ -54,7 +54,8 @@ struct alignas(64) SoloAttn {
     float* partial_ml;           // FP32 [row tile][split][128][2]
     unsigned int* tickets;       // program counters: 64-column pieces (4 a CTA) whose partial rows are out, per row tile, over all launches ...
     unsigned int target;         // ... and how many that will be after this one
-    int rows, heads;             // rows = queries x heads
+    int rows, heads;             // rows of Q that tiles are cut from: queries x heads, or the queries of an image (heads apart)
+    int head_dim, group, query_tiles;    // heads apart: logical columns of a head, query heads per KV head, tiles per image
     int keys, splits, per, cols; // keys of a split, score columns computed for them (a multiple of 16, at most 272)
     int box_rows, boxes;         // rows of K / V per copy, copies per 64-column piece
     int items;                   // row tiles x splits

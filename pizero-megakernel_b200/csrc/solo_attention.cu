@@ -1,11 +1,14 @@
-// Attention launched by itself, for query heads that share one KV head of 256 (Gemma): softmax(scale * Q K^T + suffix mask) V.
+// Attention launched by itself: softmax(scale * Q K^T + suffix mask) V.
 //
-// With one KV head the rows (query, head) all read the same keys, and they lie one behind another in memory: Q is one matrix of
+// PIECES = 4: query heads that share one KV head of 256 (Gemma).  With one KV head the rows (query, head) all read the same keys, and they lie one behind another in memory: Q is one matrix of
 // queries x heads rows of 256, cut into tiles of 128 rows whatever the number of queries is.  A work item is one such tile against one range of
 // keys (KV split); 784 queries of 8 heads are 49 tiles x 3 ranges, one round of an SM each, where tiles per head (7 x 8, the last of each
 // with 16 rows) x 4 ranges are 224.
+// PIECES = 2: heads of at most 128, stored 128 apart (SigLIP), with at most 256 keys: an item is 128 queries of one head of one image, no splits.
 //
-//   warp 0       copies: Q and K in four pieces of 64 columns, V in four (behind K, or in K's place once the scores are complete)
+// Three images of 256 queries, 16 heads: 7.4 us (as a program of one stage 10.8), one image of 200 6.7 (9.7).
+//
+//   warp 0       copies: Q and K in pieces of 64 columns, V likewise (behind K, or in K's place once the scores are complete)
 //   warp 1       tensor memory; S = Q K^T piece by piece as they land, O = P V
 //   warps 2-17   four threads per row: row maximum, exponentials, P in BF16 over Q, then a quarter of O's columns each
 //
@@ -56,6 +59,22 @@ __device__ __forceinline__ uint4 pack_row(const float2 (&acc)[4]) {
     return make_uint4(pack2_bf16(acc[0].x, acc[0].y), pack2_bf16(acc[1].x, acc[1].y), pack2_bf16(acc[2].x, acc[2].y), pack2_bf16(acc[3].x, acc[3].y));
 }
 
+// Where a work item begins: its rows of Q, its keys, the columns of its heads.
+struct AttnItem {
+    int row0, key0, q_column, kv_column, batch, head;
+};
+template <int PIECES>
+__device__ __forceinline__ AttnItem attn_item(const SoloAttn& p, int item) {
+    if constexpr (PIECES == 4) {
+        const int row_tile = item / p.splits;
+        return {row_tile * 128, (item - row_tile * p.splits) * p.per, 0, 0, 0, 0};
+    } else {
+        const int tile = item / p.heads, head = item - tile * p.heads, batch = tile / p.query_tiles;
+        return {(tile - batch * p.query_tiles) * 128, 0, head * 128, head / p.group * 128, batch, head};
+    }
+}
+
+template <int PIECES>
 __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(const __grid_constant__ SoloAttn p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -63,14 +82,14 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
     SoloAttnCtl* ctl = reinterpret_cast<SoloAttnCtl*>(base + p.ctl_offset);
     const int warp = threadIdx.x >> 5, lane = lane_id();
     if (threadIdx.x == 0) {
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < PIECES; c++) {
             mbar_init(&ctl->k[c], 1);
             mbar_init(&ctl->v[c], 1);
         }
         mbar_init(&ctl->s, 1);
         mbar_init(&ctl->o, 1);
         mbar_init(&ctl->p, 16);
-        mbar_init(&ctl->free, 4);
+        mbar_init(&ctl->free, PIECES == 4 ? 4 : 1);
         ctl->abort = 0;
         mbar_fence_init();
         prefetch_tmap(&p.map_q);
@@ -95,24 +114,24 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
             const int boxes = p.boxes, box_rows = p.box_rows;
             uint32_t n = 0;
             bool alive = true;
-            auto load = [&](const void* map, uint8_t* to, uint64_t* bar, int c, int key) {
-                for (int b = 0; b < boxes; ++b) tma_load_2d(to + static_cast<uint32_t>(c) * slab + static_cast<uint32_t>(b) * box, map, bar, c * 64, key + b * box_rows);
+            auto load = [&](const void* map, uint8_t* to, uint64_t* bar, int c, int column, int key, int batch) {
+                for (int b = 0; b < boxes; ++b) tma_load_3d(to + static_cast<uint32_t>(c) * slab + static_cast<uint32_t>(b) * box, map, bar, column + c * 64, key + b * box_rows, batch);
             };
             grid_dependency_wait();
             for (int item = blockIdx.x; alive && item < items; item += gridDim.x, ++n) {
-                const int row_tile = item / splits, key = (item - row_tile * splits) * per;
+                const AttnItem at = attn_item<PIECES>(p, item);
                 if (n > 0 && !solo_wait(w, &ctl->free, (n - 1) & 1u)) break;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < PIECES; ++c) {
                     mbar_expect_tx(&ctl->k[c], 16384u + slab);
-                    tma_load_2d(data + c * 16384, &p.map_q, &ctl->k[c], c * 64, row_tile * 128);
-                    load(&p.map_k, sk, &ctl->k[c], c, key);
+                    tma_load_3d(data + c * 16384, &p.map_q, &ctl->k[c], at.q_column + c * 64, at.row0, at.batch);
+                    load(&p.map_k, sk, &ctl->k[c], c, at.kv_column, at.key0, at.batch);
                 }
                 if (!v_apart && !solo_wait(w, &ctl->s, n & 1u)) break;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < PIECES; ++c) {
                     mbar_expect_tx(&ctl->v[c], slab);
-                    load(&p.map_v, sv, &ctl->v[c], c, key);
+                    load(&p.map_v, sv, &ctl->v[c], c, at.kv_column, at.key0, at.batch);
                 }
             }
         }
@@ -123,13 +142,13 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
             constexpr uint64_t kKMajor = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
             constexpr uint32_t kBf16 = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
             const uint32_t n1 = static_cast<uint32_t>(min(cols, 256)), n2 = static_cast<uint32_t>(cols) - n1;
-            const uint32_t idesc1 = kBf16 | ((n1 >> 3) << 17), idesc2 = kBf16 | ((n2 >> 3) << 17), idesc_o = kBf16 | (1u << 16) | ((256u >> 3) << 17);
+            const uint32_t idesc1 = kBf16 | ((n1 >> 3) << 17), idesc2 = kBf16 | ((n2 >> 3) << 17), idesc_o = kBf16 | (1u << 16) | ((PIECES * 64u >> 3) << 17);
             const int steps = cols >> 4;
             uint32_t n = 0;
             bool alive = true;
             for (int item = blockIdx.x; alive && item < items; item += gridDim.x, ++n) {
 #pragma unroll 1
-                for (uint32_t c = 0; alive && c < 4; ++c) {
+                for (uint32_t c = 0; alive && c < PIECES; ++c) {
                     if (!solo_wait(w, &ctl->k[c], n & 1u)) { alive = false; break; }
                     tc_fence_after();
 #pragma unroll
@@ -144,7 +163,7 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                 tc_commit(&ctl->s);
                 if (!solo_wait(w, &ctl->p, n & 1u)) break;
                 tc_fence_after();
-                for (uint32_t c = 0; alive && c < 4; ++c) alive = solo_wait(w, &ctl->v[c], n & 1u);
+                for (uint32_t c = 0; alive && c < PIECES; ++c) alive = solo_wait(w, &ctl->v[c], n & 1u);
                 if (!alive) break;
                 tc_fence_after();
                 // B = V with the columns of the head contiguous: pieces of 64 columns one slab apart, one 128-byte row per key, groups of 8 keys 1 KiB apart
@@ -168,10 +187,11 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
         grid_dependency_wait();
         if (p.guard.early) grid_launch_dependents();
         for (int item = blockIdx.x; item < items; item += gridDim.x, ++n) {
-            const int row_tile = item / splits, k_begin = (item - row_tile * splits) * per;
+            const AttnItem at = attn_item<PIECES>(p, item);
+            const int row_tile = item / splits, k_begin = at.key0;
             const int keys = max(min(p.keys - k_begin, per), 0);
-            const int global_row = row_tile * 128 + row, warp_rows = p.rows - (global_row - lane);
-            const int visible = p.prefix >= 0 && global_row < p.heads ? min(keys, p.prefix + 1 - k_begin) : keys;     // (the heads of query 0)
+            const int tile_row = at.row0 + row, warp_rows = p.rows - (tile_row - lane);
+            const int visible = p.prefix >= 0 && tile_row < (PIECES == 4 ? p.heads : 1) ? min(keys, p.prefix + 1 - k_begin) : keys;     // (query 0)
             alive = alive && solo_wait_warp(w, &ctl->s, n & 1u);
             tc_fence_after();
             uint32_t raw[16];
@@ -230,46 +250,61 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
             const float l_sum = (ctl->xl[0][row] + ctl->xl[1][row]) + (ctl->xl[2][row] + ctl->xl[3][row]);
             const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
             const float2 ml = make_float2(m_raw == -INFINITY ? -INFINITY : m_use, l_sum);
-            if (splits > 1 && share == 3 && warp_rows > 0) {
+            if (PIECES == 4 && splits > 1 && share == 3 && warp_rows > 0) {
                 reinterpret_cast<float2*>(p.partial_ml)[static_cast<size_t>(item) * 128 + row] = ml;
                 __threadfence();                             // (most of a microsecond, which the MMAs of O cover)
             }
             alive = alive && solo_wait_warp(w, &ctl->o, n & 1u);
             tc_fence_after();
             // 64 columns of O as BF16 over P, whose MMAs are done, in the layout of a swizzled copy
-            uint8_t* piece = data + share * 16384;
             const float f = splits > 1 ? 1.f : inv;
+            uint8_t* piece = PIECES == 4 ? data + share * 16384 + row * 128 : data + row * p.head_dim * 2;     // (PIECES = 2: rows of the head's columns)
             if (alive) {
 #pragma unroll 1
-                for (int j = 0; j < 4; ++j) {
-                    tmem_ld16(lane_addr + 256u + share * 64 + j * 16, raw);
+                for (int j = 0; j < PIECES; ++j) {
+                    const int column = share * (PIECES * 16) + j * 16;
+                    tmem_ld16(lane_addr + 256u + column, raw);
                     tmem_ld_wait();
                     uint32_t packed[8];
 #pragma unroll
                     for (int i = 0; i < 8; i++) packed[i] = pack2_bf16(__uint_as_float(raw[2 * i]) * f, __uint_as_float(raw[2 * i + 1]) * f);
 #pragma unroll
-                    for (int u = 0; u < 2; u++)
-                        *reinterpret_cast<uint4*>(piece + row * 128 + ((j * 2 + u) ^ (row & 7)) * 16) = make_uint4(packed[4 * u], packed[4 * u + 1], packed[4 * u + 2], packed[4 * u + 3]);
+                    for (int u = 0; u < 2; u++) {
+                        const uint4 unit = make_uint4(packed[4 * u], packed[4 * u + 1], packed[4 * u + 2], packed[4 * u + 3]);
+                        if constexpr (PIECES == 4) *reinterpret_cast<uint4*>(piece + ((j * 2 + u) ^ (row & 7)) * 16) = unit;
+                        else if (column + u * 8 < p.head_dim) *reinterpret_cast<uint4*>(piece + (column + u * 8) * 2) = unit;
+                    }
                 }
             }
             tc_fence_before();
             fence_proxy_async_smem();
-            named_barrier(6 + share, 128);                   // the piece is complete
-            if (quarter == 0 && lane == 0) {
-                // rows beyond the last one are left out by the copy engine
-                if (alive) {
-                    tma_store_2d(&p.map_out, piece, share * 64, splits > 1 ? item * 128 : row_tile * 128);
-                    bulk_store_wait();
+            if constexpr (PIECES == 4) {
+                named_barrier(6 + share, 128);               // the piece is complete
+                if (quarter == 0 && lane == 0) {
+                    // rows beyond the last one are left out by the copy engine
+                    if (alive) {
+                        tma_store_2d(&p.map_out, data + share * 16384, share * 64, splits > 1 ? item * 128 : at.row0);
+                        bulk_store_wait();
+                    }
+                    if (splits > 1) red_release_add(p.tickets + row_tile, 1u);
+                    mbar_arrive(&ctl->free);
                 }
-                if (splits > 1) red_release_add(p.tickets + row_tile, 1u);
-                mbar_arrive(&ctl->free);
+            } else {
+                named_barrier(6, 512);
+                if (warp == 2 && lane == 0) {
+                    if (alive) {
+                        tma_store_3d(&p.map_out, data, at.head * p.head_dim, at.row0, at.batch);
+                        bulk_store_wait();
+                    }
+                    mbar_arrive(&ctl->free);
+                }
             }
             named_barrier(5, 512);                           // (xm and xl are free for the next item)
             if (warp == 2 && lane == 0) {
-                atomicAdd(p.guard.counters + static_cast<unsigned>(row_tile) * 128u / static_cast<unsigned>(p.heads) / 128u, 1u);
+                atomicAdd(p.guard.counters + (PIECES == 4 ? static_cast<unsigned>(row_tile) * 128u / static_cast<unsigned>(p.heads) / 128u : static_cast<unsigned>(item / p.heads)), 1u);
             }
         }
-        if (splits > 1) {
+        if (PIECES == 4 && splits > 1) {
             // A CTA merges a share of the rows of its tiles.  All CTAs of the grid are resident, and none waits before
             // its own partial rows are out.
             for (int item = blockIdx.x; item < items; item += gridDim.x) {
@@ -343,13 +378,16 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
     if (warp == 1) tmem_dealloc_cg<1>(tmem, 512);
 }
 
-cudaError_t launch_solo_attention(const SoloAttn& p, int grid, size_t smem, cudaStream_t stream) {
+namespace {
+template <int PIECES>
+cudaError_t launch_form(const SoloAttn& p, int grid, size_t smem, cudaStream_t stream) {
     static bool configured[64] = {};
+    const auto kernel = pi0_attention_kernel<PIECES>;
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     if (device >= 64 || !configured[device]) {
-        e = cudaFuncSetAttribute(pi0_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloMaxSmem);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloMaxSmem);
         if (e != cudaSuccess) return e;
         if (device < 64) configured[device] = true;
     }
@@ -363,7 +401,12 @@ cudaError_t launch_solo_attention(const SoloAttn& p, int grid, size_t smem, cuda
     config.stream = stream;
     config.attrs = &serial;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, pi0_attention_kernel, p);
+    return cudaLaunchKernelEx(&config, kernel, p);
+}
+}  // namespace
+
+cudaError_t launch_solo_attention(const SoloAttn& p, int grid, size_t smem, cudaStream_t stream) {
+    return p.head_dim == 256 ? launch_form<4>(p, grid, smem, stream) : launch_form<2>(p, grid, smem, stream);
 }
 
 }  // namespace pi0

@@ -161,12 +161,16 @@ cudaError_t plan_solo_gemm(const SoloGemmRequest& r, SoloGemmPlan* plan) {
 }
 
 cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t room, int workers, int sms, SoloAttnPlan* plan) {
-    if (!a.tc || a.mask || a.out_fp4 || !a.out || a.batches != 1 || a.kv_heads != 1 || a.head_dim != 256 || a.hd_pad != 256 || a.ldq != a.heads * 256 ||
-        a.ldo != a.heads * 256)
-        return cudaErrorNotSupported;
+    const bool shared_kv = a.batches == 1 && a.kv_heads == 1 && a.head_dim == 256 && a.hd_pad == 256 && a.ldq == a.heads * 256 && a.ldo == a.heads * 256;
+    const bool apart_heads = a.hd_pad == 128 && a.splits == 1;
+    if (!a.tc || a.mask || a.out_fp4 || !a.out || !(shared_kv || apart_heads)) return cudaErrorNotSupported;
     memset(plan, 0, sizeof(*plan));
     SoloAttn& p = plan->args;
-    p.rows = a.nq * a.heads;
+    p.rows = shared_kv ? a.nq * a.heads : a.nq;
+    p.head_dim = a.head_dim;
+    p.group = a.heads / a.kv_heads;
+    p.query_tiles = (a.nq + 127) / 128;
+    const int pieces = a.hd_pad / 64;
     const int row_tiles = (p.rows + 127) / 128;
     // KV splits of the kernel's own, the same whatever the number of workers (the order of the sums hangs on them).  The estimate (us): rounds of
     // SMs, the keys of a tile, and the meeting of the splits - the partial rows of all CTAs through L2, then the rows that a warp merges one
@@ -177,7 +181,7 @@ cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t
     double least = 0;
     for (int s = 1; s <= 64 && s <= a.nk; s++) {
         const int per = (a.nk + s - 1) / s, cols = (per + 15) / 16 * 16;
-        if (cols > 272 || (s - 1) * per >= a.nk || s > most) continue;
+        if (cols > (shared_kv ? 272 : 256) || (s - 1) * per >= a.nk || s > most) continue;
         const int rounds = (row_tiles * s + sms - 1) / sms, rows = (128 + s - 1) / s, at_once = s <= 4 ? 48 : 16;
         double t = rounds * (4.0 + cols * 0.022);
         if (s > 1) t += 4.2 + 0.9 * ((rows + at_once - 1) / at_once - 1) + 0.9 * row_tiles * s / sms + 0.3 * std::max(0, s - 12);
@@ -191,31 +195,39 @@ cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t
     p.box_rows = p.cols / p.boxes;
     p.keys = a.nk;
     p.heads = a.heads;
-    p.items = row_tiles * best;
+    p.items = shared_kv ? row_tiles * best : a.batches * p.query_tiles * a.heads;
     p.prefix = a.prefix;
     p.scale = a.scale;
     p.out = a.out;
     p.partial_o = partial_o;
     plan->row_tiles = row_tiles;
     plan->grid = std::min(p.items, std::min(workers, sms));
-    const int first = std::max(4 * 16384, (p.cols + 63) / 64 * 16384), kv = 4 * p.cols * 128;     // Q, later P; K or V
+    const int first = std::max(pieces, (p.cols + 63) / 64) * 16384, kv = pieces * p.cols * 128;     // Q, later P and the output; K or V
     p.off_k = first;
     const bool apart = first + 2 * kv + kSoloAttnCtl + 1024 <= kSoloMaxSmem;
     p.off_v = apart ? first + kv : first;
     p.ctl_offset = p.off_v + kv;
     plan->smem = p.ctl_offset + kSoloAttnCtl + 1024;
     if (plan->smem > static_cast<size_t>(kSoloMaxSmem)) return cudaErrorNotSupported;
-    const cuuint64_t q_dims[2] = {256u, static_cast<cuuint64_t>(p.rows)}, q_strides[1] = {512u};
-    const cuuint32_t q_box[2] = {64u, 128u};
-    const cuuint64_t kv_dims[2] = {256u, static_cast<cuuint64_t>(a.kv_batch_rows)}, kv_strides[1] = {static_cast<cuuint64_t>(a.ldkv) * 2u};
-    const cuuint32_t kv_box[2] = {64u, static_cast<cuuint32_t>(p.box_rows)};
-    cudaError_t e = encode(&p.map_q, a.q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q_dims, q_strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (e == cudaSuccess) e = encode(&p.map_k, a.k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (e == cudaSuccess) e = encode(&p.map_v, a.v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
-    const cuuint64_t out_dims[2] = {256u, static_cast<cuuint64_t>(best > 1 ? p.items * 128 : p.rows)};
-    if (e == cudaSuccess)
-        e = encode(&p.map_out, best > 1 ? static_cast<const void*>(partial_o) : a.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, out_dims, q_strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
-    return e;
+    const cuuint64_t images = static_cast<cuuint64_t>(a.batches), out_bytes = static_cast<cuuint64_t>(a.ldo) * 2u;
+    const cuuint64_t q_width = shared_kv ? 256u : static_cast<cuuint64_t>(a.heads) * 128u, q_ld = shared_kv ? 512u : static_cast<cuuint64_t>(a.ldq) * 2u;
+    const cuuint64_t q_dims[3] = {q_width, static_cast<cuuint64_t>(p.rows), images}, q_strides[2] = {q_ld, q_ld * static_cast<cuuint64_t>(shared_kv ? p.rows : a.q_batch_rows)};
+    const cuuint32_t q_box[3] = {64u, 128u, 1u};
+    const cuuint64_t kv_ld = static_cast<cuuint64_t>(a.ldkv) * 2u;
+    const cuuint64_t kv_dims[3] = {static_cast<cuuint64_t>(a.kv_heads * a.hd_pad), static_cast<cuuint64_t>(a.kv_batch_rows), images}, kv_strides[2] = {kv_ld, kv_ld * static_cast<cuuint64_t>(a.kv_batch_rows)};
+    const cuuint32_t kv_box[3] = {64u, static_cast<cuuint32_t>(p.box_rows), 1u};
+    cudaError_t e = encode(&p.map_q, a.q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, q_dims, q_strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (e == cudaSuccess) e = encode(&p.map_k, a.k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (e == cudaSuccess) e = encode(&p.map_v, a.v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (e != cudaSuccess) return e;
+    if (shared_kv) {
+        const cuuint64_t dims[2] = {256u, static_cast<cuuint64_t>(best > 1 ? p.items * 128 : p.rows)}, strides[1] = {512u};
+        return encode(&p.map_out, best > 1 ? static_cast<const void*>(partial_o) : a.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
+    }
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(a.heads * a.head_dim), static_cast<cuuint64_t>(a.nq), images};
+    const cuuint64_t strides[2] = {out_bytes, out_bytes * static_cast<cuuint64_t>(a.q_batch_rows)};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(a.head_dim), 128u, 1u};
+    return encode(&p.map_out, a.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 }  // namespace pi0

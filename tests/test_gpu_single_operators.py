@@ -130,6 +130,28 @@ def test_attention_of_heads_with_one_kv_head(nq, nk, heads, prefix, splits, work
             assert state["epoch"] == 3 and all(c == 3 * splits for c in state["counts"])
 
 
+@pytest.mark.parametrize("batches,nq,nk,heads,kv_heads,head_dim,prefix,workers", [
+    (1, 1, 1, 1, 1, 72, None, 148), (1, 16, 17, 2, 2, 72, 3, 148),                            # one row; ragged pieces of 16 keys
+    (3, 256, 256, 16, 16, 72, None, 148), (2, 129, 240, 16, 16, 72, None, 148),               # one row in an image's second tile
+    (3, 200, 196, 4, 2, 72, None, 5), (1, 130, 256, 3, 1, 72, 0, 148),                        # several tiles per CTA; query heads that share KV heads
+])
+def test_attention_of_heads_stored_128_apart(batches, nq, nk, heads, kv_heads, head_dim, prefix, workers):
+    g = torch.Generator(device="cuda").manual_seed(nq + nk)
+    make = lambda n, h: torch.nn.functional.pad(torch.randn(batches, n, h, head_dim, generator=g, device="cuda"), (0, 128 - head_dim)).bfloat16()      # noqa: E731
+    q, k, v = make(nq, heads), make(nk, kv_heads), make(nk, kv_heads)
+    kd, vd = (t[..., :head_dim].double().repeat_interleave(heads // kv_heads, 2) for t in (k, v))
+    scores = torch.einsum("bqhd,bkhd->bhqk", q[..., :head_dim].double(), kd) * head_dim ** -0.5
+    if prefix is not None:
+        scores[:, :, 0, prefix + 1:] = -torch.inf
+    want = torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1), vd)
+    with ResidentAttention(None, q, k, v, workers=workers, prefix=prefix, head_dim=head_dim, path="tcgen05") as op:
+        for _ in range(3):
+            op.output.fill_(float("nan"))
+            got = op.forward().reshape(want.shape).double()
+            assert op.status()["code"] == 0
+            assert float((got - want).norm() / want.norm()) <= 6e-3
+
+
 @pytest.mark.parametrize("rows,width", [(1, 16), (51, 1024), (592, 2048), (593, 1168), (2000, 64)])
 def test_norm(rows, width):
     g = torch.Generator(device="cuda").manual_seed(rows + width)
