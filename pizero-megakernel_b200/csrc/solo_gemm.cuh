@@ -5,7 +5,7 @@
 //           rows of B, and the tensor cores of both read both halves of B: an SM takes in (128 + bn / 2) rows per 128 x bn of output
 //           instead of (128 + bn).
 //
-//   warp 0      copies of A                        warps 3, 2  copies of B, of the scales
+//   warp 0      copies of A and its scales         warps 3, 2  copies of B, of its scales
 //   warp 1      tensor memory; scale copies and MMAs (in the pair's first CTA)
 //   warps 4 ..  drain: warp w the 32 rows of quarter w & 3 and a share of the columns
 //
@@ -99,30 +99,41 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
             uint32_t slot = 0, phase = 1;
             bool alive = true;
             if (warp == 0) {
-                const uint32_t bytes = static_cast<uint32_t>(p.a_rows) * 128u * kC * CG;
-                const void* map = &p.map_a;
+                const uint32_t bytes = static_cast<uint32_t>(p.a_rows) * 128u * kC, off_sf = static_cast<uint32_t>(p.off_sfa);
+                const void *map = &p.map_a, *map_sf = &p.map_sfa;
+                const uint8_t* scales = g.sfa;
                 grid_dependency_wait();
                 for (int tile = unit; alive && tile < items; tile += units) {
                     const int m0 = (tile % m_tiles * CG + static_cast<int>(rank)) * tile_rows;
+                    int atom = (m0 >> 7) * k_groups + ks_begin * 4 * kC, left = k_groups - ks_begin * 4 * kC;
 #pragma unroll 1
                     for (int ks = ks_begin; ks < ks_end; ++ks) {
                         if (!solo_wait(w, &ctl->empty[slot], phase)) { alive = false; break; }
-                        if (leader) mbar_expect_tx(&ctl->full[slot], bytes);
-                        tma_load_3d_cg<CG>(data + slot * stride, map, full0 + slot * 8u, 0, m0, ks * kC);
+                        // (pairs bring whole groups of scale atoms by tensor map: beyond the last one the copy engine fills zeros)
+                        const uint32_t sf = !kScaled ? 0u : 512u * (CG == 2 ? 4u * kC : static_cast<uint32_t>(min(4 * kC, left)));
+                        if (leader) mbar_expect_tx(&ctl->full[slot], (bytes + sf) * CG);
+                        uint8_t* dst = data + slot * stride;
+                        tma_load_3d_cg<CG>(dst, map, full0 + slot * 8u, 0, m0, ks * kC);
+                        if (kScaled) {
+                            if (CG == 2) tma_load_2d_cg<CG>(dst + off_sf, map_sf, full0 + slot * 8u, 0, atom);
+                            else bulk_load(dst + off_sf, scales + static_cast<size_t>(atom) * 512, sf, &ctl->full[slot]);
+                            atom += 4 * kC;
+                            left -= 4 * kC;
+                        }
                         if (++slot == stages) { slot = 0; phase ^= 1u; }
                     }
                 }
             } else {
                 // B: at most four copies per chunk, two of them by each thread
-                const uint32_t off_b = static_cast<uint32_t>(p.off_b), off_sfa = static_cast<uint32_t>(p.off_sfa), off_sfb = static_cast<uint32_t>(p.off_sfb);
+                const uint32_t off_b = static_cast<uint32_t>(p.off_b), off_sfb = static_cast<uint32_t>(p.off_sfb);
                 const int block = p.b_block, boxes = p.b_boxes, box_rows = p.b_rows, per_tile = p.sfb_per_tile, atoms = p.sfb_atoms;
                 const int box0 = warp == 3 ? 0 : 2, mine = warp == 3 ? min(boxes, 2) : max(boxes - 2, 0);
                 const uint32_t box_bytes = static_cast<uint32_t>(box_rows) * 128u * kC * static_cast<uint32_t>(mine);
-                const void *map = &p.map_b, *map_sfa = &p.map_sfa, *map_sfb = &p.map_sfb;
-                const uint8_t *sfa = g.sfa, *sfb = g.sfb;
+                const void *map = &p.map_b, *map_sfb = &p.map_sfb;
+                const uint8_t* sfb = g.sfb;
                 grid_dependency_wait();
                 for (int tile = unit; alive && tile < items; tile += units) {
-                    const int n_tile = tile / m_tiles, n0 = n_tile * bn, m0 = ((tile - n_tile * m_tiles) * CG + static_cast<int>(rank)) * tile_rows;
+                    const int n_tile = tile / m_tiles, n0 = n_tile * bn;
                     int at[2], blk[2];                                        // where a copy begins inside its block of rows, and which block that is
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
@@ -130,15 +141,15 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                         blk[b] = r / block;
                         at[b] = r - blk[b] * block;
                     }
-                    const int a_atom = m0 >> 7, b_atom = per_tile ? n_tile : n0 >> 7;
+                    const int b_atom = per_tile ? n_tile : n0 >> 7;
+                    int atom = b_atom * k_groups + ks_begin * 4 * kC, left = k_groups - ks_begin * 4 * kC;
 #pragma unroll 1
                     for (int ks = ks_begin; ks < ks_end; ++ks) {
                         if (!solo_wait(w, &ctl->empty[slot], phase)) { alive = false; break; }
                         uint8_t* dst = data + slot * stride;
                         const uint32_t bar = full0 + slot * 8u;
-                        // (pairs bring whole groups of atoms by tensor map: beyond the last one the copy engine fills zeros)
-                        const uint32_t sf = !kScaled || warp == 3 ? 0u : 512u * (CG == 2 ? 4u * kC : static_cast<uint32_t>(min(4 * kC, k_groups - ks * 4 * kC)));
-                        if (leader) mbar_expect_tx(&ctl->full[slot], (box_bytes + sf * static_cast<uint32_t>(1 + atoms)) * CG);
+                        const uint32_t sf = !kScaled || warp == 3 ? 0u : 512u * (CG == 2 ? 4u * kC : static_cast<uint32_t>(min(4 * kC, left)));
+                        if (leader) mbar_expect_tx(&ctl->full[slot], (box_bytes + sf * static_cast<uint32_t>(atoms)) * CG);
                         if (boxes == 1) {
                             if (mine) tma_load_4d_cg<CG>(dst + off_b, map, bar, 0, at[0], ks * kC, blk[0]);
                         } else {
@@ -149,13 +160,10 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                                     if (b < mine) tma_load_4d_cg<CG>(dst + off_b + (c * boxes + box0 + b) * box_rows * 128, map, bar, 0, at[b], ks * kC + c, blk[b]);
                         }
                         if (kScaled && warp == 2) {
-                            if (CG == 2) {
-                                tma_load_2d_cg<CG>(dst + off_sfa, map_sfa, bar, 0, a_atom * k_groups + ks * 4 * kC);
-                                tma_load_3d_cg<CG>(dst + off_sfb, map_sfb, bar, 0, ks * 4 * kC, b_atom);
-                            } else {
-                                bulk_load(dst + off_sfa, sfa + static_cast<size_t>(a_atom * k_groups + ks * 4 * kC) * 512, sf, &ctl->full[slot]);
-                                bulk_load(dst + off_sfb, sfb + static_cast<size_t>(b_atom * k_groups + ks * 4 * kC) * 512, sf, &ctl->full[slot]);
-                            }
+                            if (CG == 2) tma_load_3d_cg<CG>(dst + off_sfb, map_sfb, bar, 0, ks * 4 * kC, b_atom);
+                            else bulk_load(dst + off_sfb, sfb + static_cast<size_t>(atom) * 512, sf, &ctl->full[slot]);
+                            atom += 4 * kC;
+                            left -= 4 * kC;
                         }
                         if (++slot == stages) { slot = 0; phase ^= 1u; }
                     }
@@ -169,13 +177,14 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
             constexpr uint64_t kOperandHi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
             constexpr uint64_t kScaleHi = (1ull << 16) | (8ull << 32) | (1ull << 46);
             const uint32_t a_chunk16 = static_cast<uint32_t>(p.a_rows) * 8u, b_chunk16 = static_cast<uint32_t>(p.bn / CG) * 8u;
-            const uint32_t sfb_groups = static_cast<uint32_t>(p.sfb_atoms) * 4u, sf_slot = 4u * kC * (4u + sfb_groups);
+            const bool two_atoms = CG == 2 && p.sfb_atoms == 2;               // (tiles of more than 128 columns)
+            const uint32_t sfb_groups = two_atoms ? 8u : 4u, sf_slot = 4u * kC * (4u + sfb_groups);
             const uint32_t stages = static_cast<uint32_t>(p.stages), stride16 = static_cast<uint32_t>(p.stride) >> 4, off_b16 = static_cast<uint32_t>(p.off_b) >> 4;
             const uint32_t off_sfa16 = static_cast<uint32_t>(p.off_sfa) >> 4, off_sfb16 = static_cast<uint32_t>(p.off_sfb) >> 4;
             const uint32_t sf_col = tmem_u + static_cast<uint32_t>(p.sf_col), sf_mask = static_cast<uint32_t>(p.sf_mask), idesc = g.idesc;
             const uint32_t acc_stride = static_cast<uint32_t>(p.acc_stride);
             const int k_groups = g.k_groups, bn = p.bn;
-            const bool per_tile = p.sfb_per_tile != 0, two_atoms = p.sfb_atoms == 2, two_bufs = p.acc_bufs == 2;
+            const bool per_tile = p.sfb_per_tile != 0, two_bufs = p.acc_bufs == 2;
             const uint16_t both = static_cast<uint16_t>(3u << pair_u);
             uint32_t slot = 0, phase = 0, use = 0, it = 0;
             bool alive = true, landed = false;                                // landed: the slot was seen full half-way through the one before
@@ -188,16 +197,15 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
 #pragma unroll 1
                 for (int ks = ks_begin; ks < ks_end; ++ks) {
                     if (!landed && !solo_wait(w, &ctl->full[slot], phase)) { alive = false; break; }
-                    tc_fence_after();
                     const uint32_t next = slot + 1 == stages ? 0u : slot + 1, next_phase = next == 0 ? phase ^ 1u : phase;
                     const uint32_t a16 = data16 + slot * stride16, b16 = a16 + off_b16;
                     const uint32_t groups = static_cast<uint32_t>(min(4 * kC, k_groups - ks * 4 * kC));
                     const uint32_t sfa = sf_col + (it & sf_mask) * sf_slot, sfb = sfa + 16u * kC;
                     const uint32_t sfa16 = a16 + off_sfa16, sfb16 = a16 + off_sfb16;
-                    auto copy_scales = [&](uint32_t gi) {
+                    auto copy_scales = [&](uint32_t gi, bool two) {
                         tc_copy_sf_cg<CG>(sfa + gi * 4, kScaleHi | static_cast<uint64_t>(sfa16 + gi * 32));
-                        tc_copy_sf_cg<CG>(sfb + gi * sfb_groups, kScaleHi | static_cast<uint64_t>(sfb16 + gi * 32));
-                        if (two_atoms) tc_copy_sf_cg<CG>(sfb + gi * 8 + 4, kScaleHi | static_cast<uint64_t>(sfb16 + 4 * kC * 32 + gi * 32));
+                        tc_copy_sf_cg<CG>(sfb + gi * (two ? 8u : 4u), kScaleHi | static_cast<uint64_t>(sfb16 + gi * 32));
+                        if (two) tc_copy_sf_cg<CG>(sfb + gi * 8 + 4, kScaleHi | static_cast<uint64_t>(sfb16 + 4 * kC * 32 + gi * 32));
                     };
                     auto issue = [&](uint32_t gi, uint32_t acc) {
                         const uint32_t chunk = gi >> 2, k32 = gi & 3u;
@@ -207,9 +215,15 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                         else tc_mma_dense_cg<CG, OPERANDS == GEMM_FP8>(d, da, db, idesc, acc);
                     };
                     if (groups == 4u * kC) {
+                        // (all scale copies in front of the MMAs: alternating costs the tensor pipe)
                         if constexpr (kScaled) {
+                            if (two_atoms) {
 #pragma unroll
-                            for (uint32_t gi = 0; gi < 4u * kC; ++gi) copy_scales(gi);
+                                for (uint32_t gi = 0; gi < 4u * kC; ++gi) copy_scales(gi, true);
+                            } else {
+#pragma unroll
+                                for (uint32_t gi = 0; gi < 4u * kC; ++gi) copy_scales(gi, false);
+                            }
                         }
 #pragma unroll
                         for (uint32_t gi = 0; gi < 4u * kC; ++gi) {
@@ -220,7 +234,7 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                         landed = false;
 #pragma unroll 1
                         for (uint32_t gi = 0; gi < groups; ++gi) {
-                            if constexpr (kScaled) copy_scales(gi);
+                            if constexpr (kScaled) copy_scales(gi, two_atoms);
                             issue(gi, static_cast<uint32_t>(ks != ks_begin || gi != 0));
                         }
                     }
