@@ -171,21 +171,22 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
             }
         }
     } else if (warp == 1) {
-        // (values broadcast over the warp stay in uniform registers, which the tcgen05 instructions want)
-        const uint32_t tmem_u = uniform_u32(tmem), data16 = uniform_u32((smem_u32(data) & 0x3FFFFu) >> 4), pair_u = uniform_u32(first_rank);
+        // (values broadcast over the whole warp, in front of the election, stay in uniform registers, which the tcgen05 instructions want)
+        constexpr uint64_t kOperandHi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+        constexpr uint64_t kScaleHi = (1ull << 16) | (8ull << 32) | (1ull << 46);
+        const bool two_atoms = CG == 2 && uniform_i32(p.sfb_atoms) == 2;      // (tiles of more than 128 columns)
+        const uint32_t tmem_u = uniform_u32(tmem), data16 = uniform_u32((smem_u32(data) & 0x3FFFFu) >> 4);
+        const uint32_t a_chunk16 = uniform_u32(static_cast<uint32_t>(p.a_rows)) * 8u, b_chunk16 = uniform_u32(static_cast<uint32_t>(p.bn / CG)) * 8u;
+        const uint32_t sfb_groups = two_atoms ? 8u : 4u, sf_slot = 4u * kC * (4u + sfb_groups);
+        const uint32_t stages = uniform_u32(static_cast<uint32_t>(p.stages)), stride16 = uniform_u32(static_cast<uint32_t>(p.stride)) >> 4;
+        const uint32_t off_b16 = uniform_u32(static_cast<uint32_t>(p.off_b)) >> 4, off_sfa16 = uniform_u32(static_cast<uint32_t>(p.off_sfa)) >> 4,
+                       off_sfb16 = uniform_u32(static_cast<uint32_t>(p.off_sfb)) >> 4;
+        const uint32_t sf_col = tmem_u + uniform_u32(static_cast<uint32_t>(p.sf_col)), sf_mask = uniform_u32(static_cast<uint32_t>(p.sf_mask)), idesc = uniform_u32(g.idesc);
+        const uint32_t acc_stride = uniform_u32(static_cast<uint32_t>(p.acc_stride));
+        const int k_groups = uniform_i32(g.k_groups), bn = uniform_i32(p.bn), ks_first = uniform_i32(ks_begin), ks_last = uniform_i32(ks_end);
+        const bool per_tile = p.sfb_per_tile != 0, two_bufs = uniform_i32(p.acc_bufs) == 2;
+        const uint16_t both = static_cast<uint16_t>(3u << uniform_u32(first_rank));
         if (leader && elect_one()) {
-            constexpr uint64_t kOperandHi = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-            constexpr uint64_t kScaleHi = (1ull << 16) | (8ull << 32) | (1ull << 46);
-            const uint32_t a_chunk16 = static_cast<uint32_t>(p.a_rows) * 8u, b_chunk16 = static_cast<uint32_t>(p.bn / CG) * 8u;
-            const bool two_atoms = CG == 2 && p.sfb_atoms == 2;               // (tiles of more than 128 columns)
-            const uint32_t sfb_groups = two_atoms ? 8u : 4u, sf_slot = 4u * kC * (4u + sfb_groups);
-            const uint32_t stages = static_cast<uint32_t>(p.stages), stride16 = static_cast<uint32_t>(p.stride) >> 4, off_b16 = static_cast<uint32_t>(p.off_b) >> 4;
-            const uint32_t off_sfa16 = static_cast<uint32_t>(p.off_sfa) >> 4, off_sfb16 = static_cast<uint32_t>(p.off_sfb) >> 4;
-            const uint32_t sf_col = tmem_u + static_cast<uint32_t>(p.sf_col), sf_mask = static_cast<uint32_t>(p.sf_mask), idesc = g.idesc;
-            const uint32_t acc_stride = static_cast<uint32_t>(p.acc_stride);
-            const int k_groups = g.k_groups, bn = p.bn;
-            const bool per_tile = p.sfb_per_tile != 0, two_bufs = p.acc_bufs == 2;
-            const uint16_t both = static_cast<uint16_t>(3u << pair_u);
             uint32_t slot = 0, phase = 0, use = 0, it = 0;
             bool alive = true, landed = false;                                // landed: the slot was seen full half-way through the one before
             for (int tile = unit; alive && tile < items; tile += units) {
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                 const uint32_t d = tmem_u + buf * acc_stride;
                 const uint32_t sub = per_tile ? 0u : static_cast<uint32_t>((tile / m_tiles * bn) & 127) >> 5;    // (even: tiles are multiples of 64 columns)
 #pragma unroll 1
-                for (int ks = ks_begin; ks < ks_end; ++ks) {
+                for (int ks = ks_first; ks < ks_last; ++ks) {
                     if (!landed && !solo_wait(w, &ctl->full[slot], phase)) { alive = false; break; }
                     const uint32_t next = slot + 1 == stages ? 0u : slot + 1, next_phase = next == 0 ? phase ^ 1u : phase;
                     const uint32_t a16 = data16 + slot * stride16, b16 = a16 + off_b16;
@@ -228,14 +229,14 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
 #pragma unroll
                         for (uint32_t gi = 0; gi < 4u * kC; ++gi) {
                             if (gi == 2u * kC) landed = mbar_test_wait(&ctl->full[next], next_phase);
-                            issue(gi, gi != 0 ? 1u : static_cast<uint32_t>(ks != ks_begin));
+                            issue(gi, gi != 0 ? 1u : static_cast<uint32_t>(ks != ks_first));
                         }
                     } else {
                         landed = false;
 #pragma unroll 1
                         for (uint32_t gi = 0; gi < groups; ++gi) {
                             if constexpr (kScaled) copy_scales(gi, two_atoms);
-                            issue(gi, static_cast<uint32_t>(ks != ks_begin || gi != 0));
+                            issue(gi, static_cast<uint32_t>(ks != ks_first || gi != 0));
                         }
                     }
                     tc_commit_cg<CG>(&ctl->empty[slot], both);

@@ -36,10 +36,10 @@ struct Shape {
     int cg, bn, tile_rows, splits;
 };
 
-// Estimated microseconds of a launch in this shape: rounds of the slowest of copies (what an SM takes in, at its own rate or at its share of
-// what all of them draw from L2 together), MMAs and drain.  Fitted to 70 projections of 1 to 820 rows (NVFP4, BF16 and FP8, all widths of
-// the model and odd ones) in up to ten shapes each, 3.6 - 60 us: the estimate is within 9 %, and its choice 0.01 % slower than the fastest
-// shape on average, 1 % at most.
+// Estimated microseconds of a launch in this shape: the longest of what one SM takes in, what all of them draw from L2 together, MMAs and drains,
+// and the last drain.  Rates and cycles per MMA group as measured on single shapes; on 70 projections of 1 to 820 rows (NVFP4, BF16 and FP8, all
+// widths of the model and odd ones) in up to ten shapes each, 3.6 - 60 us, the choice is 0.1 % slower than the fastest shape on average, 7 % at
+// most.
 double estimate(const SoloGemmRequest& r, const Shape& s, int chunks, int a_rows) {
     const GemmParams& g = *r.g;
     const bool scaled = r.operands == GEMM_NVFP4;
@@ -47,13 +47,13 @@ double estimate(const SoloGemmRequest& r, const Shape& s, int chunks, int a_rows
     const int ctas = s.cg * s.splits, items = row_tiles * col_tiles, units = std::min(r.workers / ctas, solo_gemm_clusters(ctas)), rounds = (items + units - 1) / units;
     const double k_chunks = static_cast<double>(chunks) / s.splits;
     const double rows = a_rows + static_cast<double>(s.bn) / s.cg + (scaled ? (128.0 + (s.bn + 127) / 128 * 128) / 8 : 0.0);
-    const double rate = std::min(162e3, 12.7e6 / (std::min(units, items) * ctas));              // bytes per microsecond and SM
-    const double copy = rows * 128.0 * k_chunks / rate;
-    const double group = scaled ? (s.cg == 1 ? 68 + 0.22 * s.bn : 86 + 0.05 * s.bn) : s.cg == 1 ? std::max(19.0, 0.24 * s.bn) : std::max(47.0, 0.5 * s.bn);
-    const double mma = k_chunks * 4.0 * group / 1.9e3;
+    const double bytes = rows * 128.0 * k_chunks;                                            // of one CTA and tile
+    const double copy = std::max(rounds * bytes / 150e3, items * ctas * bytes / 14.6e6);
+    const double group = scaled ? (s.cg == 1 ? std::max(40.0, 0.8 * s.bn) : 96 + 0.04 * s.bn) : s.cg == 1 ? 45 + 0.2 * s.bn : std::max(43.0, 0.29 * s.bn);
+    const double mma = rounds * k_chunks * 4.0 * group / 1.9e3;
     const int shares = solo_drain_warps(r.operands, g.epilogue) / 4;
-    const double drain = (s.bn / 32 + shares - 1) / shares * (g.epilogue == EPI_F32 ? 0.42 : 0.58);
-    return 3.6 + (s.cg == 2 ? 1.9 : 0.0) + (s.splits > 1 ? 1.5 : 0.0) + rounds * std::max({copy, mma, rounds > 1 ? drain : 0.0}) + drain;
+    const double drain = (s.bn / 32 + shares - 1) / shares * (g.epilogue == EPI_F32 ? 0.44 : 0.55);
+    return 3.4 + (s.cg == 2 ? 2.0 : 0.0) + (s.splits > 1 ? 1.5 : 0.0) + 0.1 * rounds + std::max({copy, mma, rounds > 1 ? rounds * drain : 0.0}) + drain;
 }
 
 }  // namespace
@@ -65,6 +65,9 @@ cudaError_t plan_solo_gemm(const SoloGemmRequest& r, SoloGemmPlan* plan) {
     if (!plain || g.row_factor || g.row_sumsq || g.round_before_residual || g.gelu_cols > 0 || g.pad_from > 0 || g.col_center || g.cols != r.n || g.block_n > 128)
         return cudaErrorNotSupported;
     if (scaled && g.epilogue == EPI_F32 && (g.bias || g.residual)) return cudaErrorNotSupported;
+    // Few rows over a long K are one tile per CTA whose MMAs are all there is: the persistent kernel's issue loop is as fast, its first operands
+    // earlier (51 x 2048 x 16384 14.3 us, 15.3 here; 51 x 1152 x 4352 7.35 and 6.8).
+    if (scaled && r.m == 128 && r.k >= 12288) return cudaErrorNotSupported;
     const size_t row_bytes = scaled ? static_cast<size_t>(r.k) / 2 : r.operands == GEMM_BF16 ? static_cast<size_t>(r.k) * 2 : static_cast<size_t>(r.k);
     const int chunks = static_cast<int>((row_bytes + 127) / 128), k_groups = static_cast<int>(row_bytes / 32);
     const int few = std::min(128, std::max(scaled ? 32 : 64, (g.rows + 7) / 8 * 8));          // rows copied when there is one row band
