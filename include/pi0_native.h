@@ -137,8 +137,9 @@ int configure_dense_qkv_rope(void* handle, const void* cos, const void* sin, voi
 int configure_dense_head_pad(void* handle, int from, int to, int ld);
 /* extension: logical row count and output tile width (128, 64 or 32) of a dense projection.  The NVFP4 GEMM's
  * configure_resident_fp4_{bf16, quantized, qkv_rope, rows, tile, weight_layout} calls accept dense handles too (a dense
- * projection may emit NVFP4 for an NVFP4 consumer).  A width that has been given stays: one that never was is chosen by size where
- * the projection is launched by itself, and 128 in a program of several stages. */
+ * projection may emit NVFP4 for an NVFP4 consumer).  The width is that of the stage in a program (128 if never given) and of tile-major
+ * weights; a projection that is launched by itself chooses its own tiles by size.  Every width gives the same bits; a K of 4096 bytes or
+ * more per part may be summed in parts where the launch has SMs to spare, with FP32 sums added in order. */
 int configure_dense_rows(void* handle, int rows);
 int configure_dense_tile(void* handle, int block_n);
 
@@ -230,7 +231,7 @@ int attention_merge_handle(void* handle, void** merge);
  * that a launch which read a partial it had not written itself would produce NaNs.  attention_split_diagnostics
  * returns, per (128-query tile, head) group, how many split tiles have arrived over all stand-alone launches so
  * far (capacity >= number of groups) and the launch count `epoch`; every count equals splits * epoch after a clean
- * launch. */
+ * launch.  (A stand-alone launch may cut the keys into splits of its own: its arrivals are given in units of the configured ones.) */
 int attention_poison_partials(void* handle, void* stream);
 int attention_split_diagnostics(void* handle, unsigned long long* counts, int capacity, unsigned int* epoch);
 
