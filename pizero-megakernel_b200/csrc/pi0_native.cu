@@ -571,6 +571,11 @@ int gemm_configure(Op* op, bool refresh, Change change) {
     return cudaSuccess;
 }
 
+// Whether a launch of `grid` CTAs lets its successor's start while it runs: see solo_program for the small ones.  One that takes the whole
+// chip can let it in, too: the successor's CTAs find no other place than the SM of one that has ended, and prepare there while the last ones
+// run (gate/up of 768 rows, 148 CTAs: 34.3 -> 33.5 us; attention of 784 rows, 147: the same).
+int lets_successor_in(int grid, int sms) { return grid <= sms * 3 / 10 || grid >= sms - 8 ? 1 : 0; }
+
 // The kernel of its own that a stand-alone launch of `op` takes, if there is one.  Its finished tiles are counted where the program's
 // would be, so the counters of the handle keep their meaning (expected: per launch and row band).
 int solo_route(Op* op, int sms) {
@@ -600,7 +605,7 @@ int solo_route(Op* op, int sms) {
         SoloGemm& p = plan.args;
         route->grid = plan.grid;
         for (int row = 0; row < d.p.gemm.rows; row += p.tile_rows) expected[row / kBandRows] += p.n_tiles;
-        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, plan.grid <= sms * 3 / 10 ? 1 : 0};
+        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, lets_successor_in(plan.grid, sms)};
     } else if (d.kind == OP_ATTN && !op->prep) {
         route->kind = SoloRoute::ATTENTION;
         SoloAttnPlan& plan = route->attention;
@@ -609,7 +614,7 @@ int solo_route(Op* op, int sms) {
         if (e != cudaSuccess) return e;
         SoloAttn& p = plan.args;
         route->grid = plan.grid;
-        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, plan.grid <= sms * 3 / 10 ? 1 : 0};
+        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, lets_successor_in(plan.grid, sms)};
         route->band_tiles.assign(d.bands, 0);
         if (p.head_dim != 256) std::fill(expected.begin(), expected.begin() + d.bands, static_cast<unsigned int>(p.heads));
         for (int t = 0; p.head_dim == 256 && t < plan.row_tiles; t++) {

@@ -14,7 +14,7 @@
 // What bounds it: with few rows the chain copies - MMAs - drain (expert q|k|v of 51 rows: 1.2 us to the first operands, 0.8 for its MMAs, 0.7 for
 // the drain, 1.3 to the next launch: 4.0 us; as a stage of the persistent kernel 5.6); with many the operands that all SMs together draw from
 // L2, 13 - 16 TB/s (gate/up of 768 rows: 282 MB in tiles of pairs, 453 MB in 128 x 128 ones), and under sustained load the power limit.  Measured
-// with other operands on every launch, in turn with the stage of the persistent kernel: gate/up + GeGLU 768 x 32768 x 2048 34.3 us (43.9), BF16
+// with other operands on every launch, in turn with the stage of the persistent kernel: gate/up + GeGLU 768 x 32768 x 2048 33.5 us (43.6), BF16
 // 333 x 1000 x 1152 6.4 (8.2), FP8 768 x 2048 x 16384 34.7 (42.7; without the split of K 34.2 - 43 by tile).
 //
 // CTAs stay for several tiles; where tensor memory holds two accumulators, the drain of one tile overlaps the MMAs of the next.
