@@ -231,7 +231,7 @@ int attention_merge_handle(void* handle, void** merge);
  * that a launch which read a partial it had not written itself would produce NaNs.  attention_split_diagnostics
  * returns, per (128-query tile, head) group, how many split tiles have arrived over all stand-alone launches so
  * far (capacity >= number of groups) and the launch count `epoch`; every count equals splits * epoch after a clean
- * launch.  (A stand-alone launch may cut the keys into splits of its own: its arrivals are given in units of the configured ones.) */
+ * launch. */
 int attention_poison_partials(void* handle, void* stream);
 int attention_split_diagnostics(void* handle, unsigned long long* counts, int capacity, unsigned int* epoch);
 

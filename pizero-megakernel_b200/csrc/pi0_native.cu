@@ -609,7 +609,7 @@ int solo_route(Op* op, int sms) {
     } else if (d.kind == OP_ATTN && !op->prep) {
         route->kind = SoloRoute::ATTENTION;
         SoloAttnPlan& plan = route->attention;
-        cudaError_t e = plan_solo_attention(d.p.attn, op->partial_o, op->partial_bytes / (kAttnQRows * 256 * sizeof(uint16_t)), op->workers, sms, &plan);
+        cudaError_t e = plan_solo_attention(d.p.attn, op->workers, sms, &plan);
         if (e == cudaErrorNotSupported) return cudaSuccess;
         if (e != cudaSuccess) return e;
         SoloAttn& p = plan.args;
@@ -622,7 +622,6 @@ int solo_route(Op* op, int sms) {
             route->band_tiles[band]++;
             expected[band] += p.splits;
         }
-        p.partial_ml = op->partial_ml;
         p.tickets = prog->d_counters + prog->stages[0].aux_base;
     } else {
         return cudaSuccess;
@@ -1398,10 +1397,8 @@ extern "C" int attention_split_diagnostics(void* handle, unsigned long long* cou
     e = cudaMemcpy(raw.data(), op->solo->d_counters, raw.size() * sizeof(unsigned int), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return e;
     if (op->route) {
-        // the kernel of its own: arrivals of the row tiles that hold the band's rows, in units of the configured splits
-        const int own = op->route->attention.args.splits;
-        for (int g = 0; g < groups; g++)
-            counts[g] = static_cast<unsigned long long>(raw[d.counter_base + g / a.heads]) * a.splits / static_cast<unsigned int>(op->route->band_tiles[g / a.heads] * own);
+        // the kernel of its own: every row tile that begins in the band has the same share
+        for (int g = 0; g < groups; g++) counts[g] = raw[d.counter_base + g / a.heads] / static_cast<unsigned int>(op->route->band_tiles[g / a.heads]);
     } else if (a.fused_merge && d.aux_count == groups) {
         for (int g = 0; g < groups; g++) counts[g] = raw[d.aux_base + g];
     } else {

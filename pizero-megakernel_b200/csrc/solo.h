@@ -56,8 +56,7 @@ struct alignas(64) SoloAttn {
     unsigned int target;         // ... and how many that will be after this one
     int rows, heads;             // rows of Q that tiles are cut from: queries x heads, or the queries of an image (heads apart)
     int head_dim, group, query_tiles;    // heads apart: logical columns of a head, query heads per KV head, tiles per image
-    int keys, splits, per, cols; // keys of a split, score columns computed for them (a multiple of 16, at most 272)
-    int box_rows, boxes;         // rows of K / V per copy, copies per 64-column piece
+    int keys, splits, per, cols; // keys of a split, score columns computed for them (a multiple of 16, at most 256)
     int items;                   // row tiles x splits
     int off_k, off_v, ctl_offset;    // shared memory: Q and P at 0, K, V
     int prefix;
@@ -68,8 +67,7 @@ struct SoloAttnPlan {
     int grid, row_tiles;
     size_t smem;
 };
-// `room`: items for which `partial_o` has partial rows.
-cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t room, int workers, int sms, SoloAttnPlan* plan);
+cudaError_t plan_solo_attention(const AttnParams& a, int workers, int sms, SoloAttnPlan* plan);
 cudaError_t launch_solo_attention(const SoloAttn& p, int grid, size_t smem, cudaStream_t stream);
 
 // What a GEMM handle asks for; tile geometry and ring of `g` are the persistent kernel's and are not read.

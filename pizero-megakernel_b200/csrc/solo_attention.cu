@@ -2,8 +2,7 @@
 //
 // PIECES = 4: query heads that share one KV head of 256 (Gemma).  With one KV head the rows (query, head) all read the same keys, and they lie one behind another in memory: Q is one matrix of
 // queries x heads rows of 256, cut into tiles of 128 rows whatever the number of queries is.  A work item is one such tile against one range of
-// keys (KV split); 784 queries of 8 heads are 49 tiles x 3 ranges, one round of an SM each, where tiles per head (7 x 8, the last of each
-// with 16 rows) x 4 ranges are 224.
+// keys (KV split); 784 queries of 8 heads in 4 ranges are 196 items, where tiles per head (7 x 8, the last of each with 16 rows) are 224.
 // PIECES = 2: heads of at most 128, stored 128 apart (SigLIP), with at most 256 keys: an item is 128 queries of one head of one image, no splits.
 //
 // Three images of 256 queries, 16 heads: 7.4 us (as a program of one stage 10.8), one image of 200 6.7 (9.7).
@@ -13,11 +12,12 @@
 //   warps 2-17   four threads per row: row maximum, exponentials, P in BF16 over Q, then a quarter of O's columns each
 //
 // What bounds it: a chain of copies, scores, softmax, MMAs, one trip to L2 with the partial rows and one back (51 queries over 819 keys, 13 splits:
-// scores complete 1.6 us after the release, O 3.2, partial rows out and counted 5.9, merged 8.7, next launch released 10.3; the tiles per
-// head of a program's stage 12.0); with 262 keys a tile 35,000 exponentials per SM besides (784 queries: 15.2 us, tiles per head 29).  The
+// scores complete 1.6 us after the release, O 3.2, partial rows out and counted 5.9, merged 8.7, next launch released 10.0; the tiles per
+// head of a program's stage 12.2); with 196 keys a tile 25,000 exponentials per SM and item besides, and where there are more items than SMs
+// the second one's copies wait for the first one's output (784 queries: 23.7 us, tiles per head 29.5; 623 in 3 ranges, one round, 13.4 and 17.1).  The
 // splits of a tile as a cluster that exchanges its rows through shared memory, by stores or by copies, were no faster (10.8).
 //
-// S takes up to 272 columns of tensor memory and O those from 256 on: O is begun when every score has been read.  Ranges of keys meet as
+// S takes up to 256 columns of tensor memory and O those from 256 on.  Ranges of keys, those that the operator was given, meet as
 // un-normalised BF16 rows with their maximum and sum (as in op_attention_tc.cuh): when all of a tile's ranges have arrived, each of their
 // CTAs merges a share of the rows.
 #include "op_attention.cuh"
@@ -110,13 +110,8 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
 
     if (warp == 0) {
         if (lane == 0) {
-            const uint32_t box = static_cast<uint32_t>(p.box_rows) * 128u;
-            const int boxes = p.boxes, box_rows = p.box_rows;
             uint32_t n = 0;
             bool alive = true;
-            auto load = [&](const void* map, uint8_t* to, uint64_t* bar, int c, int column, int key, int batch) {
-                for (int b = 0; b < boxes; ++b) tma_load_3d(to + static_cast<uint32_t>(c) * slab + static_cast<uint32_t>(b) * box, map, bar, column + c * 64, key + b * box_rows, batch);
-            };
             grid_dependency_wait();
             for (int item = blockIdx.x; alive && item < items; item += gridDim.x, ++n) {
                 const AttnItem at = attn_item<PIECES>(p, item);
@@ -125,13 +120,13 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                 for (int c = 0; c < PIECES; ++c) {
                     mbar_expect_tx(&ctl->k[c], 16384u + slab);
                     tma_load_3d(data + c * 16384, &p.map_q, &ctl->k[c], at.q_column + c * 64, at.row0, at.batch);
-                    load(&p.map_k, sk, &ctl->k[c], c, at.kv_column, at.key0, at.batch);
+                    tma_load_3d(sk + static_cast<uint32_t>(c) * slab, &p.map_k, &ctl->k[c], at.kv_column + c * 64, at.key0, at.batch);
                 }
                 if (!v_apart && !solo_wait(w, &ctl->s, n & 1u)) break;
 #pragma unroll
                 for (int c = 0; c < PIECES; ++c) {
                     mbar_expect_tx(&ctl->v[c], slab);
-                    load(&p.map_v, sv, &ctl->v[c], c, at.kv_column, at.key0, at.batch);
+                    tma_load_3d(sv + static_cast<uint32_t>(c) * slab, &p.map_v, &ctl->v[c], at.kv_column + c * 64, at.key0, at.batch);
                 }
             }
         }
@@ -141,8 +136,7 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
         if (elect_one()) {
             constexpr uint64_t kKMajor = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
             constexpr uint32_t kBf16 = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
-            const uint32_t n1 = static_cast<uint32_t>(min(cols, 256)), n2 = static_cast<uint32_t>(cols) - n1;
-            const uint32_t idesc1 = kBf16 | ((n1 >> 3) << 17), idesc2 = kBf16 | ((n2 >> 3) << 17), idesc_o = kBf16 | (1u << 16) | ((PIECES * 64u >> 3) << 17);
+            const uint32_t idesc_s = kBf16 | ((static_cast<uint32_t>(cols) >> 3) << 17), idesc_o = kBf16 | (1u << 16) | ((PIECES * 64u >> 3) << 17);
             const int steps = cols >> 4;
             uint32_t n = 0;
             bool alive = true;
@@ -153,10 +147,8 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                     tc_fence_after();
 #pragma unroll
                     for (uint32_t i = 0; i < 4; ++i) {
-                        const uint64_t a = kKMajor | static_cast<uint64_t>(q16 + c * 1024u + 2u * i);
-                        const uint32_t b = k16 + c * slab16 + 2u * i, acc = (c | i) != 0u ? 1u : 0u;
-                        tc_mma_f16(tmem_u, a, kKMajor | static_cast<uint64_t>(b), idesc1, acc);
-                        if (n2) tc_mma_f16(tmem_u + 256u, a, kKMajor | static_cast<uint64_t>(b + 2048u), idesc2, acc);     // (256 rows on)
+                        tc_mma_f16(tmem_u, kKMajor | static_cast<uint64_t>(q16 + c * 1024u + 2u * i), kKMajor | static_cast<uint64_t>(k16 + c * slab16 + 2u * i), idesc_s,
+                                   (c | i) != 0u ? 1u : 0u);
                     }
                 }
                 if (!alive) break;

@@ -164,7 +164,7 @@ cudaError_t plan_solo_gemm(const SoloGemmRequest& r, SoloGemmPlan* plan) {
     return e;
 }
 
-cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t room, int workers, int sms, SoloAttnPlan* plan) {
+cudaError_t plan_solo_attention(const AttnParams& a, int workers, int sms, SoloAttnPlan* plan) {
     const bool shared_kv = a.batches == 1 && a.kv_heads == 1 && a.head_dim == 256 && a.hd_pad == 256 && a.ldq == a.heads * 256 && a.ldo == a.heads * 256;
     const bool apart_heads = a.hd_pad == 128 && a.splits == 1;
     if (!a.tc || a.mask || a.out_fp4 || !a.out || !(shared_kv || apart_heads)) return cudaErrorNotSupported;
@@ -176,34 +176,20 @@ cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t
     p.query_tiles = (a.nq + 127) / 128;
     const int pieces = a.hd_pad / 64;
     const int row_tiles = (p.rows + 127) / 128;
-    // KV splits of the kernel's own, the same whatever the number of workers (the order of the sums hangs on them).  The estimate (us): rounds of
-    // SMs, the keys of a tile, and the meeting of the splits - the partial rows of all CTAs through L2, then the rows that a warp merges one
-    // batch of loads after another.  It picks the fastest of 41 shapes tried, or one within 2 % (9 - 101 queries over 300 - 920 keys: 8 - 13 splits,
-    // 9.0 - 10.4 us; 256 rows unsplit 9.6, with 4 splits 10.4; 300 rows in 4 splits 10.7, in 2 12.6, in 7 11.9; 784 rows in 3 15.3, in 4 23).
-    const int most = a.splits == 1 ? 1 : static_cast<int>(room / row_tiles);
-    int best = 0;
-    double least = 0;
-    for (int s = 1; s <= 64 && s <= a.nk; s++) {
-        const int per = (a.nk + s - 1) / s, cols = (per + 15) / 16 * 16;
-        if (cols > (shared_kv ? 272 : 256) || (s - 1) * per >= a.nk || s > most) continue;
-        const int rounds = (row_tiles * s + sms - 1) / sms, rows = (128 + s - 1) / s, at_once = s <= 4 ? 48 : 16;
-        double t = rounds * (4.0 + cols * 0.022);
-        if (s > 1) t += 4.2 + 0.9 * ((rows + at_once - 1) / at_once - 1) + 0.9 * row_tiles * s / sms + 0.3 * std::max(0, s - 12);
-        if (best == 0 || t < least) { best = s; least = t; }
-    }
-    if (!best) return cudaErrorNotSupported;
-    p.splits = best;
-    p.per = (a.nk + best - 1) / best;
-    p.cols = (p.per + 15) / 16 * 16;
-    p.boxes = p.cols > 256 ? 2 : 1;
-    p.box_rows = p.cols / p.boxes;
+    // The ranges of keys are the handle's: each is a maximum that probabilities are rounded against and a partial row that is rounded, so other
+    // ranges are other results, and fewer are less exact (784 rows in 3 ranges instead of 4: one round of SMs and 16.1 us, not two and 23.7, but
+    // 2.746e-3 from 64 bits and not 2.724e-3; 10 queries over 487 keys in 11 ranges instead of 13: 2.646e-3 and not 2.574e-3).
+    p.splits = a.splits;
+    p.per = (a.nk + a.splits - 1) / a.splits;
+    p.cols = (p.per + 15) / 16 * 16;                                                          // (at most 256, or the tiles would not be tcgen05 ones)
     p.keys = a.nk;
     p.heads = a.heads;
-    p.items = shared_kv ? row_tiles * best : a.batches * p.query_tiles * a.heads;
+    p.items = shared_kv ? row_tiles * p.splits : a.batches * p.query_tiles * a.heads;
     p.prefix = a.prefix;
     p.scale = a.scale;
     p.out = a.out;
-    p.partial_o = partial_o;
+    p.partial_o = a.partial_o;
+    p.partial_ml = a.partial_ml;
     plan->row_tiles = row_tiles;
     plan->grid = std::min(p.items, std::min(workers, sms));
     const int first = std::max(pieces, (p.cols + 63) / 64) * 16384, kv = pieces * p.cols * 128;     // Q, later P and the output; K or V
@@ -219,14 +205,14 @@ cudaError_t plan_solo_attention(const AttnParams& a, uint16_t* partial_o, size_t
     const cuuint32_t q_box[3] = {64u, 128u, 1u};
     const cuuint64_t kv_ld = static_cast<cuuint64_t>(a.ldkv) * 2u;
     const cuuint64_t kv_dims[3] = {static_cast<cuuint64_t>(a.kv_heads * a.hd_pad), static_cast<cuuint64_t>(a.kv_batch_rows), images}, kv_strides[2] = {kv_ld, kv_ld * static_cast<cuuint64_t>(a.kv_batch_rows)};
-    const cuuint32_t kv_box[3] = {64u, static_cast<cuuint32_t>(p.box_rows), 1u};
+    const cuuint32_t kv_box[3] = {64u, static_cast<cuuint32_t>(p.cols), 1u};
     cudaError_t e = encode(&p.map_q, a.q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, q_dims, q_strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (e == cudaSuccess) e = encode(&p.map_k, a.k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (e == cudaSuccess) e = encode(&p.map_v, a.v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, kv_dims, kv_strides, kv_box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (e != cudaSuccess) return e;
     if (shared_kv) {
-        const cuuint64_t dims[2] = {256u, static_cast<cuuint64_t>(best > 1 ? p.items * 128 : p.rows)}, strides[1] = {512u};
-        return encode(&p.map_out, best > 1 ? static_cast<const void*>(partial_o) : a.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
+        const cuuint64_t dims[2] = {256u, static_cast<cuuint64_t>(p.splits > 1 ? p.items * 128 : p.rows)}, strides[1] = {512u};
+        return encode(&p.map_out, p.splits > 1 ? static_cast<const void*>(a.partial_o) : a.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
     }
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(a.heads * a.head_dim), static_cast<cuuint64_t>(a.nq), images};
     const cuuint64_t strides[2] = {out_bytes, out_bytes * static_cast<cuuint64_t>(a.q_batch_rows)};

@@ -103,8 +103,9 @@ def test_dense_projection_over_a_long_k(rows, n, k, dtype):
 @pytest.mark.parametrize("nq,nk,heads,prefix,splits,workers", [
     (1, 1, 1, None, 1, 148), (1, 16, 8, None, 1, 148), (16, 17, 8, 3, 1, 148),                # one row; whole and ragged pieces of 16 keys
     (17, 256, 8, None, 1, 2), (300, 256, 3, 100, 1, 148),                                     # heads that do not divide the 128 rows of a tile
-    (784, 784, 8, None, 4, 148), (700, 816, 8, None, 4, 148), (769, 819, 8, 0, 4, 40),        # up to 272 keys a tile; several tiles per CTA
+    (784, 784, 8, None, 4, 148), (700, 816, 8, None, 4, 148), (769, 819, 8, 0, 4, 40),        # several tiles per CTA
     (51, 819, 8, 768, 13, 148), (51, 819, 8, 768, 13, 3), (101, 920, 8, 819, 13, 148), (2, 2000, 8, 1500, 32, 148),
+    (300, 300, 8, None, 2, 16), (10, 487, 8, 477, 13, 148), (16, 17, 8, 3, 16, 148),          # few workers; many ranges of few rows; ranges without a key
 ])
 def test_attention_of_heads_with_one_kv_head(nq, nk, heads, prefix, splits, workers):
     g = torch.Generator(device="cuda").manual_seed(nq + nk)
@@ -114,6 +115,12 @@ def test_attention_of_heads_with_one_kv_head(nq, nk, heads, prefix, splits, work
     if prefix is not None:
         scores[:, 0, prefix + 1:] = -torch.inf
     want = torch.einsum("hqk,kd->qhd", scores.softmax(-1), v[0, :, 0].double())
+    error = lambda y: float((y.double() - want).norm() / want.norm())                         # noqa: E731
+    # (rows of Q that do not lie one behind another: the stage of the persistent kernel)
+    wide = torch.nn.functional.pad(q, (0, 0, 0, 1))[:, :, :heads]
+    with ResidentAttention(None, wide, k, v, workers=workers, prefix=prefix, splits=splits, head_dim=256, path="tcgen05") as op:
+        stage = op.forward().reshape(nq, heads, 256).clone()
+        assert op.status()["code"] == 0
     with ResidentAttention(None, q, k, v, workers=workers, prefix=prefix, splits=splits, head_dim=256, path="tcgen05") as op:
         for launch in range(3):
             op.output.fill_(float("nan"))
@@ -121,7 +128,11 @@ def test_attention_of_heads_with_one_kv_head(nq, nk, heads, prefix, splits, work
                 op.poison_partials()
             got = op.forward().reshape(nq, heads, 256).clone()
             assert op.status()["code"] == 0
-            assert float((got.double() - want).norm() / want.norm()) <= 6e-3                  # (probabilities and rows in BF16)
+            # probabilities, partial rows and rows are rounded to BF16, each off by a part in 2^8 / sqrt(3) in the mean at most; the stage rounds
+            # the same ones, and only the row sums add up in another order (FP32), which now and then moves a result to the next BF16 value
+            assert error(got) <= 2 ** -8 * ((3 if splits > 1 else 2) / 3) ** 0.5 and error(got) <= 1.002 * error(stage)
+            off = (got.double() - stage.double()).abs()
+            assert bool((off <= 2 ** -7 * stage.double().abs() + 2 ** -16).all()) and float((off > 0).double().mean()) <= 0.01
             if launch:
                 assert torch.equal(got, first)
             first = got
@@ -144,12 +155,17 @@ def test_attention_of_heads_stored_128_apart(batches, nq, nk, heads, kv_heads, h
     if prefix is not None:
         scores[:, :, 0, prefix + 1:] = -torch.inf
     want = torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1), vd)
+    error = lambda y: float((y - want).norm() / want.norm())                                  # noqa: E731
     with ResidentAttention(None, q, k, v, workers=workers, prefix=prefix, head_dim=head_dim, path="tcgen05") as op:
+        with NativeStageProgram(None, [(op, [])]) as program:
+            stage = program.forward().reshape(want.shape).double()
+            assert program.status()["code"] == 0
         for _ in range(3):
             op.output.fill_(float("nan"))
             got = op.forward().reshape(want.shape).double()
             assert op.status()["code"] == 0
-            assert float((got - want).norm() / want.norm()) <= 6e-3
+            assert error(got) <= 2 ** -8 * (2 / 3) ** 0.5 and error(got) <= 1.002 * error(stage)      # (as above)
+            assert bool(((got - stage).abs() <= 2 ** -7 * stage.abs() + 2 ** -16).all())
 
 
 @pytest.mark.parametrize("rows,width", [(1, 16), (51, 1024), (592, 2048), (593, 1168), (2000, 64)])
