@@ -1320,11 +1320,9 @@ extern "C" int configure_attention_splits(void* handle, int splits) {
     float* partial_ml = nullptr;
     const int groups = a.heads * ((a.nq + kAttnQRows - 1) / kAttnQRows);          // heads x 128-query tiles
     const size_t tasks = static_cast<size_t>(groups) * splits;
-    // (the kernel of its own that a stand-alone launch may take has splits of its own: one round of SMs at most)
-    const size_t room = a.kv_heads == 1 && a.head_dim == 256 ? std::max<size_t>(tasks, sm_count(op->device)) : tasks;
     if (splits > 1) {
-        cudaError_t e = cudaMalloc(&partial_o, room * kAttnQRows * a.head_dim * sizeof(uint16_t));
-        if (e == cudaSuccess) e = cudaMalloc(&partial_ml, room * kAttnQRows * 2 * sizeof(float));
+        cudaError_t e = cudaMalloc(&partial_o, tasks * kAttnQRows * a.head_dim * sizeof(uint16_t));
+        if (e == cudaSuccess) e = cudaMalloc(&partial_ml, tasks * kAttnQRows * 2 * sizeof(float));
         if (e != cudaSuccess) {
             cudaFree(partial_o);
             cudaFree(partial_ml);
@@ -1336,8 +1334,8 @@ extern "C" int configure_attention_splits(void* handle, int splits) {
     cudaFree(op->partial_ml);
     op->partial_o = partial_o;
     op->partial_ml = partial_ml;
-    op->partial_bytes = splits > 1 ? room * kAttnQRows * a.head_dim * sizeof(uint16_t) : 0;
-    op->stat_bytes = splits > 1 ? room * kAttnQRows * 2 * sizeof(float) : 0;
+    op->partial_bytes = splits > 1 ? tasks * kAttnQRows * a.head_dim * sizeof(uint16_t) : 0;
+    op->stat_bytes = splits > 1 ? tasks * kAttnQRows * 2 * sizeof(float) : 0;
     a.splits = splits;
     a.fused_merge = 0;
     a.partial_o = partial_o;

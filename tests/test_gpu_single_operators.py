@@ -141,6 +141,24 @@ def test_attention_of_heads_with_one_kv_head(nq, nk, heads, prefix, splits, work
             assert state["epoch"] == 3 and all(c == 3 * splits for c in state["counts"])
 
 
+def test_partial_rows_of_split_attention():
+    """An operator holds partial rows for its configured ranges and no more, launched by itself or not: 64 of 128 rows here, 4 MiB."""
+    g = torch.Generator(device="cuda").manual_seed(11)
+    q, k = (torch.randn(1, n, h, 256, generator=g, device="cuda").bfloat16() for n, h in ((51, 8), (819, 1)))
+    ops, output = [], torch.empty(1, 51, 8, 256, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    try:
+        for _ in range(32):
+            ops.append(ResidentAttention(None, q, k, k, workers=148, splits=8, head_dim=256, output=output))
+            ops[-1].forward()
+        torch.cuda.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] <= 32 * (4 << 20) * 1.25                 # (statistics, programs, whole pages)
+    finally:
+        for op in ops:
+            op.close()
+
+
 @pytest.mark.parametrize("batches,nq,nk,heads,kv_heads,head_dim,prefix,workers", [
     (1, 1, 1, 1, 1, 72, None, 148), (1, 16, 17, 2, 2, 72, 3, 148),                            # one row; ragged pieces of 16 keys
     (3, 256, 256, 16, 16, 72, None, 148), (2, 129, 240, 16, 16, 72, None, 148),               # one row in an image's second tile
