@@ -632,6 +632,8 @@ int solo_route(Op* op, int sms) {
 }
 cudaError_t launch_route(const Op* op, cudaStream_t stream) {
     SoloRoute& r = *op->route;
+    // (set_native_model_wait_budget may have been called since the route was made)
+    r.norm.guard.budget_ns = r.gemm.args.guard.budget_ns = r.attention.args.guard.budget_ns = op->solo->budget_ns;
     if (r.kind == SoloRoute::ATTENTION) {
         SoloAttn& p = r.attention.args;
         p.target = op->solo->epoch * static_cast<unsigned int>(p.splits) * 4u;

@@ -7,6 +7,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from native_pi0 import _native
 from native_pi0.attention import ResidentAttention
 from native_pi0.dense import ResidentDense
 from native_pi0.linear import NativeStageProgram
@@ -196,3 +197,24 @@ def test_norm(rows, width):
                dict(precision="factor"), dict(precision="fp4", quantize_only=True)):
         with ResidentNorm(None, x, workers=148, row_alignment=128, **kw) as op:
             alone_and_as_a_stage(op)
+
+
+def budget(op, nanoseconds):
+    _native.check(op.library.set_native_model_wait_budget(op.handle, nanoseconds), "wait budget")
+
+
+def test_wait_budget_of_an_operator():
+    """The budget given to an operator handle bounds the waits of its launches, whether it is given before the first or later.  A tile of K =
+    131072 on one SM keeps the draining warps waiting for more than 100 us."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, b = (torch.randn(64, 131072, generator=g, device="cuda").bfloat16() for _ in range(2))
+    with ResidentDense(None, a, b, workers=1) as op:
+        for _ in range(2):
+            budget(op, 20_000)
+            op.forward()
+            status = op.status()
+            assert status["code"] == 2 and status["aborted"] == 1 and status["stage"] == 0
+            budget(op, 2_000_000_000)
+            good = op.forward().clone()
+            assert op.status()["code"] == 0
+            assert float((good.double() - a.double() @ b.double().T).norm() / good.double().norm()) < 3e-3
