@@ -218,3 +218,27 @@ def test_wait_budget_of_an_operator():
             good = op.forward().clone()
             assert op.status()["code"] == 0
             assert float((good.double() - a.double() @ b.double().T).norm() / good.double().norm()) < 3e-3
+
+
+def test_wait_budget_begins_behind_the_kernel_in_front():
+    """CTAs that are let in early do not count their predecessor's time as their own: about a millisecond on one SM, in front of operators that may
+    wait for 100 us."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()                 # noqa: E731
+    with ResidentDense(None, randn(64, 131072), randn(512, 131072), workers=1) as long, \
+            ResidentDense(None, randn(64, 1024), randn(128, 1024), workers=148) as gemm, \
+            ResidentAttention(None, randn(1, 51, 8, 256), randn(1, 819, 1, 256), randn(1, 819, 1, 256), workers=148, splits=13) as attention:
+        for op in (gemm, attention):
+            want = op.forward().clone()
+            budget(op, 100_000)
+            for _ in range(2):
+                start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                start.record()
+                long.forward()
+                end.record()
+                torch.cuda.synchronize()
+                assert start.elapsed_time(end) > 0.3                                          # (three times the budget)
+                long.forward()
+                got = op.forward()
+                assert op.status()["code"] == 0 and torch.equal(got, want)
+        assert long.status()["code"] == 0
