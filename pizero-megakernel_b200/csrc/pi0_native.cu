@@ -623,6 +623,7 @@ int solo_route(Op* op, int sms) {
             expected[band] += p.splits;
         }
         p.tickets = prog->d_counters + prog->stages[0].aux_base;
+        for (int t = 0; p.splits > 1 && t < plan.row_tiles; t++) expected[prog->stages[0].aux_base + t] = 4 * p.splits;
     } else {
         return cudaSuccess;
     }

@@ -74,6 +74,12 @@ __device__ __forceinline__ AttnItem attn_item(const SoloAttn& p, int item) {
     }
 }
 
+// Counter of a finished item: the 128-query band in which its row tile begins, or its tile of an image.
+template <int PIECES>
+__device__ __forceinline__ unsigned int attn_band(const SoloAttn& p, int item) {
+    return PIECES == 4 ? static_cast<unsigned>(item / p.splits) / static_cast<unsigned>(p.heads) : static_cast<unsigned>(item / p.heads);
+}
+
 template <int PIECES>
 __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(const __grid_constant__ SoloAttn p) {
     extern __shared__ uint8_t smem_raw[];
@@ -275,17 +281,17 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                 named_barrier(6 + share, 128);               // the piece is complete
                 if (quarter == 0 && lane == 0) {
                     // rows beyond the last one are left out by the copy engine
-                    if (alive) {
+                    if (!solo_gave_up(&ctl->abort)) {
                         tma_store_2d(&p.map_out, data + share * 16384, share * 64, splits > 1 ? item * 128 : at.row0);
                         bulk_store_wait();
+                        if (splits > 1) red_release_add(p.tickets + row_tile, 1u);
                     }
-                    if (splits > 1) red_release_add(p.tickets + row_tile, 1u);
                     mbar_arrive(&ctl->free);
                 }
             } else {
                 named_barrier(6, 512);
                 if (warp == 2 && lane == 0) {
-                    if (alive) {
+                    if (!solo_gave_up(&ctl->abort)) {
                         tma_store_3d(&p.map_out, data, at.head * p.head_dim, at.row0, at.batch);
                         bulk_store_wait();
                     }
@@ -293,9 +299,7 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                 }
             }
             named_barrier(5, 512);                           // (xm and xl are free for the next item)
-            if (warp == 2 && lane == 0) {
-                atomicAdd(p.guard.counters + (PIECES == 4 ? static_cast<unsigned>(row_tile) * 128u / static_cast<unsigned>(p.heads) / 128u : static_cast<unsigned>(item / p.heads)), 1u);
-            }
+            if (warp == 2 && lane == 0 && !(PIECES == 4 && splits > 1) && !solo_gave_up(&ctl->abort)) atomicAdd(p.guard.counters + attn_band<PIECES>(p, item), 1u);
         }
         if (PIECES == 4 && splits > 1) {
             // A CTA merges a share of the rows of its tiles.  All CTAs of the grid are resident, and none waits before
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                     for (uint32_t spin = 1; ok && static_cast<int>(ld_acquire(p.tickets + row_tile) - p.target) < 0; ++spin) {
                         __nanosleep(20);
                         if ((spin & 63u) == 0u) {
-                            ok = *reinterpret_cast<volatile int*>(&ctl->abort) == 0;
+                            ok = !solo_gave_up(&ctl->abort);
                             const unsigned long long now = global_ns();
                             if (start == 0) start = now;
                             if (now - start > w.budget_ns || ld_relaxed_int(&w.status->abort)) { solo_give_up(w, 0u); ok = 0; }
@@ -317,6 +321,7 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                     }
                 }
                 if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+                if (warp == 2 && lane == 0 && !solo_gave_up(&ctl->abort)) atomicAdd(p.guard.counters + attn_band<PIECES>(p, item), 1u);
                 const float2* ml = reinterpret_cast<const float2*>(p.partial_ml) + static_cast<size_t>(row_tile) * splits * 128 + r0;
                 const uint4* po = reinterpret_cast<const uint4*>(p.partial_o) + (static_cast<size_t>(row_tile) * splits * 128 + r0) * 32 + lane;
                 uint4* out = reinterpret_cast<uint4*>(p.out) + (static_cast<size_t>(row_tile) * 128 + r0) * 32 + lane;
@@ -361,7 +366,7 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
         }
     }
     __syncwarp();
-    if (*reinterpret_cast<volatile int*>(&ctl->abort)) {
+    if (solo_gave_up(&ctl->abort)) {
         const unsigned long long t0 = global_ns();
         while (global_ns() - t0 < 2000000ull) __nanosleep(1000);
     }

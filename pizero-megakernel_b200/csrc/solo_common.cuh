@@ -11,7 +11,7 @@ struct SoloWait {
     unsigned long long budget_ns;
     int* abort;                  // shared memory: somebody of this CTA has given up
 };
-// Out of time: recorded for the host, and every other wait of the CTA ends.  (The first reporter of the operator wins.)
+// Out of time: recorded for the host, and every other wait of the CTA, and of the operator's other CTAs, ends.  (The first reporter wins.)
 static __device__ __noinline__ bool solo_give_up(SoloWait w, uint32_t parity) {
     if (atomicCAS(&w.status->code, 0, 2) == 0) {
         w.status->worker = static_cast<int>(blockIdx.x);
@@ -25,6 +25,8 @@ static __device__ __noinline__ bool solo_give_up(SoloWait w, uint32_t parity) {
     *reinterpret_cast<volatile int*>(w.abort) = 1;
     return false;
 }
+// Whether a wait of this CTA has run out: its tile is not complete, and nobody may be told that it is.
+__device__ __forceinline__ bool solo_gave_up(const int* abort) { return *reinterpret_cast<const volatile int*>(abort) != 0; }
 template <bool CLUSTER>
 __device__ __forceinline__ bool solo_try(uint64_t* bar, uint32_t parity) {
     if constexpr (!CLUSTER) return mbar_try_wait(bar, parity);
@@ -38,11 +40,11 @@ static __device__ __noinline__ bool solo_wait_long(SoloWait w, uint64_t* bar, ui
     unsigned long long start = 0;
     for (uint32_t spin = 1;; ++spin) {
         if (solo_try<CLUSTER>(bar, parity)) return true;     // each try suspends for at most ~1 us
-        if (*reinterpret_cast<volatile int*>(w.abort)) return false;
+        if (solo_gave_up(w.abort)) return false;
         if ((spin & 15u) == 0u) {
             const unsigned long long now = global_ns();
             if (start == 0) start = now;
-            if (now - start > w.budget_ns) return solo_give_up(w, parity);
+            if (now - start > w.budget_ns || ld_relaxed_int(&w.status->abort)) return solo_give_up(w, parity);
         }
     }
 }
@@ -62,11 +64,11 @@ static __device__ __noinline__ bool solo_wait_warp_long(SoloWait w, uint64_t* ba
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
         int stop = 0;
         if (lane_id() == 0) {
-            if (*reinterpret_cast<volatile int*>(w.abort)) stop = 1;
+            if (solo_gave_up(w.abort)) stop = 1;
             else if ((spin & 15u) == 0u) {
                 const unsigned long long now = global_ns();
                 if (start == 0) start = now;
-                if (now - start > w.budget_ns) { solo_give_up(w, parity); stop = 1; }
+                if (now - start > w.budget_ns || ld_relaxed_int(&w.status->abort)) { solo_give_up(w, parity); stop = 1; }
             }
         }
         if (__shfl_sync(0xffffffffu, stop, 0)) return false;
@@ -94,6 +96,9 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void st_cluster_int(uint32_t addr, int v) {
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 // (relaxed: what it tells is that tensor memory has been read, and tcgen05.wait::ld has returned; a release would wait for the draining warp's stores)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {

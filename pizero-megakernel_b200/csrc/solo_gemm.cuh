@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                 gemm_epilogue_chunk<EPI, kLean, true>(g, d, raw, res, row, n0 + c, row_ok, g.alpha, 0.f, unused_a, unused_b);
                 if (c + 32 < col_end) load_residual(c + 32);
             }
-            if (warp == kDrainWarps && lane == 0) atomicAdd(p.guard.counters + (m0 >> 7), 1u);     // (quarter 0, the last columns)
+            if (warp == kDrainWarps && lane == 0 && !solo_gave_up(&ctl->abort)) atomicAdd(p.guard.counters + (m0 >> 7), 1u);     // (quarter 0, the last columns)
         }
     }
 
@@ -310,11 +310,13 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
             const int n_tile = unit / m_tiles;
             const int m0 = ((unit - n_tile * m_tiles) * CG + static_cast<int>(rank)) * p.tile_rows, n0 = n_tile * p.bn;
             const int parts = min(p.bn, g.cols - n0) >> 5;
-            const bool work = warp >= 4 && m0 + quarter * 32 < g.rows;
             const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
             tc_fence_before();
             __syncwarp();
+            if (lane == 0 && solo_gave_up(&ctl->abort))                       // a part of the sum is missing: the tile is nobody's
+                for (int r = 0; r < group; ++r) st_cluster_int(map_to_rank(smem_u32(&ctl->abort), static_cast<uint32_t>(r)), 1);
             cluster_sync();                                                   // all MMAs of the cluster are done
+            const bool whole = !solo_gave_up(&ctl->abort), work = whole && warp >= 4 && m0 + quarter * 32 < g.rows;
             tc_fence_after();
             if (work) {
 #pragma unroll 1
@@ -373,13 +375,13 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                     gemm_epilogue_chunk<EPI, kLean, true>(g, d, raw, res, row, n0 + c * 32, row_ok, g.alpha, 0.f, unused_a, unused_b);
                 }
             }
-            if (warp == 4 && lane == 0 && split == 0 && m0 < g.rows) atomicAdd(p.guard.counters + (m0 >> 7), 1u);
+            if (whole && warp == 4 && lane == 0 && split == 0 && m0 < g.rows) atomicAdd(p.guard.counters + (m0 >> 7), 1u);
         }
     }
 
     // Everybody meets here: every wait above is bounded.  After one that ran out, copies in flight get a moment to land.
     __syncwarp();
-    if (*reinterpret_cast<volatile int*>(&ctl->abort)) {
+    if (solo_gave_up(&ctl->abort)) {
         const unsigned long long t0 = global_ns();
         while (global_ns() - t0 < 2000000ull) __nanosleep(1000);
     }

@@ -1,6 +1,8 @@
 """Operators that are launched by themselves have kernels of their own (``csrc/solo.h``).  They are held to the stage of a program with the
 same handle - bit for bit where both add up in one order - and otherwise to 64-bit arithmetic, at the edges of their tiles and of the
 rules that choose them."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -203,6 +205,14 @@ def budget(op, nanoseconds):
     _native.check(op.library.set_native_model_wait_budget(op.handle, nanoseconds), "wait budget")
 
 
+def counters(op):
+    total = ctypes.c_int()
+    _native.check(op.library.read_native_model_counters(op.handle, None, None, 0, ctypes.byref(total)), "counters")
+    counts, expected = ((ctypes.c_uint * total.value)() for _ in range(2))
+    _native.check(op.library.read_native_model_counters(op.handle, counts, expected, total.value, None), "counters")
+    return list(counts), list(expected)
+
+
 def test_wait_budget_of_an_operator():
     """The budget given to an operator handle bounds the waits of its launches, whether it is given before the first or later.  A tile of K =
     131072 on one SM keeps the draining warps waiting for more than 100 us."""
@@ -242,3 +252,48 @@ def test_wait_budget_begins_behind_the_kernel_in_front():
                 got = op.forward()
                 assert op.status()["code"] == 0 and torch.equal(got, want)
         assert long.status()["code"] == 0
+
+
+@pytest.mark.parametrize("rows,n,k,workers", [(64, 64, 524288, 1), (256, 256, 1048576, 8)])      # one CTA; K split over the pairs of a cluster
+def test_a_tile_that_gave_up_is_not_finished(rows, n, k, workers):
+    """A draining warp whose wait for some 450 us of MMAs runs out leaves its tile unwritten and uncounted, in every pair that shares it."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, b = (torch.randn(r, 4096, generator=g, device="cuda").to(torch.float8_e4m3fn).repeat(1, k // 4096) for r in (rows, n))
+    with ResidentDense(None, a, b, workers=workers) as op:
+        good = op.forward().clone()
+        counts, expected = counters(op)
+        assert op.status()["code"] == 0 and counts == expected and max(counts) > 0
+        for _ in range(2):
+            op.output.fill_(float("nan"))
+            budget(op, 5_000)
+            op.forward()
+            counts, expected = counters(op)
+            assert sum(counts) < sum(expected)
+            assert op.status()["code"] == 2 and bool(torch.isnan(op.output[:rows, :n]).any())
+            budget(op, 2_000_000_000)
+            assert torch.equal(op.forward(), good) and op.status()["code"] == 0
+
+
+def test_attention_whose_partners_do_not_arrive_is_not_finished():
+    """Another stream keeps all but one or two SMs for some 600 us: the first tiles wait for the partial rows of others that have no place to run,
+    give up after 50 us and are not counted; those that come later see it and end."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()                 # noqa: E731
+    other = torch.cuda.Stream()
+    with ResidentDense(None, randn(768, 16384), randn(32768, 16384), workers=147) as long, \
+            ResidentAttention(None, randn(1, 51, 8, 256), randn(1, 819, 1, 256), randn(1, 819, 1, 256), workers=148, splits=13) as op:
+        want = op.forward().clone()
+        counts, expected = counters(op)
+        assert op.status()["code"] == 0 and counts == expected
+        long.forward()
+        torch.cuda.synchronize()
+        budget(op, 50_000)
+        with torch.cuda.stream(other):
+            long.forward()
+        op.forward()
+        counts, expected = counters(op)
+        assert op.status()["code"] == 2 and sum(counts) < sum(expected)
+        budget(op, 2_000_000_000)
+        for _ in range(3):
+            assert torch.equal(op.forward(), want)
+        assert op.status()["code"] == 0 and counters(op)[0] == counters(op)[1]
