@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
                     }
                 }
                 if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+                __syncwarp();                                // (a shuffle orders no memory: lane 0 has acquired for all of them)
                 if (warp == 2 && lane == 0 && !solo_gave_up(&ctl->abort)) atomicAdd(p.guard.counters + attn_band<PIECES>(p, item), 1u);
                 const float2* ml = reinterpret_cast<const float2*>(p.partial_ml) + static_cast<size_t>(row_tile) * splits * 128 + r0;
                 const uint4* po = reinterpret_cast<const uint4*>(p.partial_o) + (static_cast<size_t>(row_tile) * splits * 128 + r0) * 32 + lane;
