@@ -225,6 +225,10 @@ int attention_prepare_handle(void* handle, void** prepare);
 int attention_validate(void* handle);
 /* extension: handle of the merge stage owned by an attention handle with splits > 1 (NULL otherwise). */
 int attention_merge_handle(void* handle, void** merge);
+/* Development diagnostics: how a stand-alone launch of an operator handle runs.  values[0] = 0 as a program of one stage, 1 in the norm's kernel of
+ * its own, 2 in the projection's, 3 in the attention's; [1] CTAs that share a tile (2: a pair), [2] columns of a tile (projections), [3] splits of K or of
+ * the keys, [4] CTAs of the launch.  count >= 5. */
+int operator_launch_form(void* handle, int* values, int count);
 /* Development diagnostics of a split attention handle (splits >= 2), never part of a forward pass.
  * Replaces: native_pi0/attention.cu:629-656 (attention_split_diagnostics, attention_poison_partials).
  * attention_poison_partials fills the partial rows and their (max, sum) statistics with 0xFF bytes on `stream`, so

@@ -739,6 +739,24 @@ __global__ void quantize_rows_kernel(NormParams n) {
 using namespace pi0;
 
 // =====================================================================================================
+extern "C" int operator_launch_form(void* handle, int* values, int count) {
+    Op* op = as_op(handle);
+    if (!op || !values || count < 5) return cudaErrorInvalidValue;
+    int device = 0;
+    cudaError_t ce = cudaGetDevice(&device);
+    if (ce != cudaSuccess) return ce;
+    if (device != op->device) return cudaErrorInvalidDevice;
+    if (int e = solo_program(op)) return e;
+    const SoloRoute* r = op->route.get();
+    values[0] = !r ? 0 : r->kind == SoloRoute::NORM ? 1 : r->kind == SoloRoute::GEMM ? 2 : 3;
+    values[1] = values[0] == 2 ? r->gemm.cg : 1;
+    values[2] = values[0] == 2 ? r->gemm.args.bn : 0;
+    values[3] = values[0] == 2 ? r->gemm.args.splits : values[0] == 3 ? r->attention.args.splits : 1;
+    values[4] = r ? r->grid : op->solo->grid;
+    return cudaSuccess;
+}
+
+// =====================================================================================================
 extern "C" int create_resident_fp4(void** handle, const void* a, const void* b, const void* sfa, const void* sfb, void* out,
                                    int m, int n, int k, int workers, float alpha) {
     if (!handle) return cudaErrorInvalidValue;

@@ -89,6 +89,7 @@ _SIGNATURES = {
     "create_attention": [C.POINTER(_P)] + [_P] * 12 + [_I] * 12 + [_F],
     "launch_attention": [_P, _P],
     "destroy_attention": [_P],
+    "operator_launch_form": [_P, C.POINTER(_I), _I],
     "attention_resources": [C.POINTER(_I), _I],
     "configure_attention_splits": [_P, _I],
     "configure_attention_cache": [_P, _P, _P, _I, _I],

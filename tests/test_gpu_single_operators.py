@@ -28,6 +28,29 @@ def outputs(op):
     return [t.view(torch.uint8) for t in tensors if t is not None]
 
 
+def library(op):
+    return getattr(op, "library", None) or op._library
+
+
+def budget(op, nanoseconds):
+    _native.check(library(op).set_native_model_wait_budget(op.handle, nanoseconds), "wait budget")
+
+
+def counters(op):
+    total = ctypes.c_int()
+    _native.check(library(op).read_native_model_counters(op.handle, None, None, 0, ctypes.byref(total)), "counters")
+    counts, expected = ((ctypes.c_uint * total.value)() for _ in range(2))
+    _native.check(library(op).read_native_model_counters(op.handle, counts, expected, total.value, None), "counters")
+    return list(counts), list(expected)
+
+
+def launch_form(op):
+    """CTAs that share a tile, its columns, splits of K; None where the operator runs as a program of one stage."""
+    values = (ctypes.c_int * 5)()
+    _native.check(library(op).operator_launch_form(op.handle, values, 5), "launch form")
+    return tuple(values[1:4]) if values[0] == 2 else None
+
+
 def alone_and_as_a_stage(op):
     """Three launches of ``op`` give the bits of a program of that one stage, counters included."""
     with NativeStageProgram(None, [(op, [])]) as program:
@@ -42,31 +65,37 @@ def alone_and_as_a_stage(op):
         op.forward()
         status = op.status()
         assert status["code"] == 0 and status["epoch"] == launch + 1
+        counts, expected = counters(op)
+        assert counts == expected and max(counts) > 0
         for got, w in zip(outputs(op), want):
             assert torch.equal(got, w)
 
 
-@pytest.mark.parametrize("rows,n,k,block_n,tiled", [
-    (1, 128, 64, 128, False),            # a single K group, one tile
-    (51, 2560, 1024, 64, True),
-    (51, 640, 320, 32, False),           # 32-wide tiles with scales of their own, half-filled last slot
-    (129, 384, 1152, 128, False),        # one row in the second band
-    (256, 16384, 1024, 128, True),       # pairs of CTAs: 192-wide tiles over blocks of 128 rows, the last one cut
-    (640, 8256 // 128 * 128, 1088, 128, False),      # odd number of row bands, K not in whole slots
-    (300, 16384, 512, 64, True),         # blocks of 64 rows
+@pytest.mark.parametrize("rows,n,k,block_n,tiled,workers,ctas,width", [
+    (1, 128, 64, 128, False, 148, 1, 64),            # a single K group, two tiles
+    (51, 2560, 1024, 64, True, 148, 1, 64),
+    (51, 640, 320, 32, False, 148, 1, 32),           # 32-wide tiles with scales of their own, half-filled last slot
+    (129, 384, 1152, 128, False, 148, 1, 64),        # one row in the second band
+    (640, 8192, 1088, 128, False, 148, 1, 128),      # K not in whole slots
+    (256, 16384, 1024, 128, True, 148, 1, 128),      # tile-major blocks as wide as the tiles
+    (256, 16384, 1024, 128, True, 2, 2, 192),        # one pair of CTAs: 192-wide tiles over blocks of 128 rows, the last of 86 cut
+    (640, 8192, 1088, 128, False, 7, 2, 192),        # three pairs: odd number of row bands, K not in whole groups of scale atoms
+    (300, 4096, 2048, 64, True, 2, 2, 192),          # blocks of 64 rows, a band of 44 rows
+    (768, 32768, 2048, 128, True, 148, 2, 192),      # pairs on all SMs, seven tiles each
 ])
 @pytest.mark.parametrize("out,act", [("f32", "none"), ("bf16", "none"), ("fp4", "none"), ("fp4", "gelu"), ("fp4", "geglu"), ("fp4", "relu2")])
-def test_nvfp4_projection(rows, n, k, block_n, tiled, out, act):
+def test_nvfp4_projection(rows, n, k, block_n, tiled, workers, ctas, width, out, act):
     if act == "geglu" and n % 256:
         pytest.skip("GeGLU takes whole pairs of 128 columns")
     rng, m = np.random.default_rng(rows + n + k), -(-rows // 128) * 128
     g = torch.Generator(device="cuda").manual_seed(rows)
     added = out != "f32" and act != "geglu"
-    with ResidentNVFP4(None, codes(rng, m, k, 1.0), codes(rng, n, k, 0.01), workers=148, rows=rows, block_n=block_n, tiled_weight=tiled,
+    with ResidentNVFP4(None, codes(rng, m, k, 1.0), codes(rng, n, k, 0.01), workers=workers, rows=rows, block_n=block_n, tiled_weight=tiled,
                        output_dtype={"f32": torch.float32, "bf16": torch.bfloat16, "fp4": torch.uint8}[out], output_gelu=act == "gelu",
                        output_geglu=act == "geglu", output_relu2=act == "relu2",
                        bias=torch.randn(n, generator=g, device="cuda") if added else None,
                        residual=torch.randn(m, n, generator=g, device="cuda") if added else None) as op:
+        assert launch_form(op) == (ctas, width, 1)
         alone_and_as_a_stage(op)
 
 
@@ -78,15 +107,22 @@ def test_dense_projection(rows, n, k, dtype, workers):
     randn = lambda *s: torch.randn(*s, generator=g, device="cuda")          # noqa: E731
     for kind in (dict(output_dtype=torch.float32), dict(output_dtype=torch.float32, bias=randn(n), residual=randn(rows, n)), dict(bias=randn(n), residual=randn(rows, n))):
         with ResidentDense(None, randn(rows, k).to(dtype), randn(n, k).to(dtype), alpha=0.05, workers=workers, **kind) as op:
+            if workers == 1 or (rows, workers) == (820, 3):
+                assert launch_form(op)[0] == workers // 3 + 1                                     # (one CTA; one pair with several tiles)
             alone_and_as_a_stage(op)
 
 
-@pytest.mark.parametrize("rows,n,k,dtype", [(768, 2048, 16384, torch.float8_e4m3fn), (513, 1930, 8192, torch.float8_e4m3fn), (300, 1200, 8192, torch.bfloat16)])
-def test_dense_projection_over_a_long_k(rows, n, k, dtype):
+@pytest.mark.parametrize("rows,n,k,dtype,workers,width,splits", [
+    (768, 2048, 16384, torch.float8_e4m3fn, 148, 256, 2), (513, 1930, 8192, torch.float8_e4m3fn, 148, 256, 2), (300, 1200, 8192, torch.bfloat16, 148, 192, 4),
+    (512, 512, 12288, torch.float8_e4m3fn, 148, 64, 3), (256, 64, 16384, torch.float8_e4m3fn, 148, 64, 4),      # two 32-column pieces: pairs without one
+    (256, 200, 24576, torch.float8_e4m3fn, 6, 256, 3), (129, 128, 16384, torch.bfloat16, 6, 128, 3),            # one cluster of six
+])
+def test_dense_projection_over_a_long_k(rows, n, k, dtype, workers, width, splits):
     """K split over the pairs of a cluster: sums of parts, repeated bit for bit and no further from 64 bits than one sum over all of K."""
     g = torch.Generator(device="cuda").manual_seed(k + n)
     a, b = torch.randn(rows, k, generator=g, device="cuda").to(dtype), torch.randn(n, k, generator=g, device="cuda").to(dtype)
-    with ResidentDense(None, a, b, output_dtype=torch.float32, workers=148) as op:
+    with ResidentDense(None, a, b, output_dtype=torch.float32, workers=workers) as op:
+        assert launch_form(op) == (2, width, splits)
         exact = a.double() @ b.double().T
         bound = 2.0 ** -22 * k ** 0.5 * (a.double().abs() @ b.double().abs().T)              # (FP32 sums of K terms)
         with NativeStageProgram(None, [(op, [])]) as program:
@@ -99,7 +135,8 @@ def test_dense_projection_over_a_long_k(rows, n, k, dtype):
             op.output.fill_(float("nan"))
             assert torch.equal(op.forward(), want)
     bias, residual = torch.randn(n, generator=g, device="cuda"), torch.randn(rows, n, generator=g, device="cuda").bfloat16()
-    with ResidentDense(None, a, b, bias=bias, residual=residual, workers=148) as op:
+    with ResidentDense(None, a, b, bias=bias, residual=residual, workers=workers) as op:
+        assert launch_form(op)[2] == splits
         assert torch.equal(op.forward(), (want + residual.float() + bias.bfloat16().float()).bfloat16())
 
 
@@ -199,18 +236,6 @@ def test_norm(rows, width):
                dict(precision="factor"), dict(precision="fp4", quantize_only=True)):
         with ResidentNorm(None, x, workers=148, row_alignment=128, **kw) as op:
             alone_and_as_a_stage(op)
-
-
-def budget(op, nanoseconds):
-    _native.check(op.library.set_native_model_wait_budget(op.handle, nanoseconds), "wait budget")
-
-
-def counters(op):
-    total = ctypes.c_int()
-    _native.check(op.library.read_native_model_counters(op.handle, None, None, 0, ctypes.byref(total)), "counters")
-    counts, expected = ((ctypes.c_uint * total.value)() for _ in range(2))
-    _native.check(op.library.read_native_model_counters(op.handle, counts, expected, total.value, None), "counters")
-    return list(counts), list(expected)
 
 
 def test_wait_budget_of_an_operator():
