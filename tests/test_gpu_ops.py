@@ -1133,10 +1133,10 @@ def test_drains_do_not_depend_on_the_run(m, n, k, rows, block_n):
         assert bool(((decoded - value).abs() <= torch.maximum(step / 4, torch.where(step > 0, value.abs() / 4, value.abs())) + error).all())
 
 
-@pytest.mark.parametrize("columns", [1024, 5632, 6144])
-def test_launches_that_overlap_keep_the_order_of_the_stream(columns):
-    """Launches prepare while the one in front finishes, behind small operators (8 and 44 CTAs; not 48) on SMs that it leaves
-    free: a consumer still reads what its producer, or a copy or an event of another stream in front of it, wrote, and an input
+@pytest.mark.parametrize("columns,ctas", [(1024, 16), (2816, 44), (3072, 48), (8832, 138), (8960, 140), (9472, 148)])
+def test_launches_that_overlap_keep_the_order_of_the_stream(columns, ctas):
+    """Launches prepare while the one in front finishes, behind small operators (16 and 44 CTAs; not 48) on SMs that it leaves
+    free, behind those that take the whole chip (140 and 148 CTAs; not 138) where one of its CTAs has ended: a consumer still reads what its producer, or a copy or an event of another stream in front of it, wrote, and an input
     may be overwritten behind the launch that reads it.  Back to back against one at a time."""
     rng = np.random.default_rng(columns)
     pa = pack_nvfp4(rng.normal(size=(51, 512)).astype(np.float32), row_alignment=128)
@@ -1150,6 +1150,9 @@ def test_launches_that_overlap_keep_the_order_of_the_stream(columns):
     with ResidentNVFP4(None, pa, p0, workers=148, output_dtype=torch.uint8, rows=51) as s0, \
             ResidentNVFP4(None, placeholder, p1, workers=148, rows=51, activation_buffers=(s0.output, s0.output_scales)) as s1, \
             ResidentNorm(None, source, kind="rms", precision="fp4", workers=148, row_alignment=128) as norm:
+        form = (C.c_int * 5)()
+        _native.check(_native.load().operator_launch_form(s0.handle, form, 5), "launch form")
+        assert form[0] == 2 and form[4] == ctas
         def passes(synchronise):
             kept = []
             wait = torch.cuda.synchronize if synchronise else lambda: None
