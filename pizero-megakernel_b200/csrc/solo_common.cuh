@@ -102,7 +102,7 @@ __device__ __forceinline__ void st_cluster_int(uint32_t addr, int v) {
 }
 // (relaxed: what it tells is that tensor memory has been read, and tcgen05.wait::ld has returned; a release would wait for the draining warp's stores)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // ---------------------------------------------------------------- TMA into this CTA's memory; in a pair the barrier may be the other's
