@@ -104,7 +104,7 @@ int encode_bf16_rows(CUtensorMap* map, const void* base, size_t rows, int ld, in
 
 struct Program;
 
-// Stand-alone launch through a kernel of its own (solo.h), made together with the stand-alone program.
+// Stand-alone launch through a kernel of its own (solo.h).
 struct SoloRoute {
     enum { NORM, GEMM, ATTENTION } kind;
     SoloNorm norm{};
@@ -136,9 +136,9 @@ struct Op {
     int attn_path = -1;                // -1 choose by geometry, 0 mma.sync tiles, 1 tcgen05 tiles
     Op* prep = nullptr;                // owned operand-preparation stage (bias / RoPE / head sizes other than 72 and 256)
     void* prep_scratch = nullptr;      // its padded BF16 copies of Q, K and V
-    Program* solo = nullptr;           // lazily built one/two-stage program for stand-alone launches
+    Program* solo = nullptr;           // lazily built one/two-stage program for stand-alone launches; with a route, what counts and reports in its place
     bool solo_dirty = true;
-    std::unique_ptr<SoloRoute> route;  // how such a launch runs instead, where the operator has a kernel of its own (status, counters and epoch stay the program's)
+    std::unique_ptr<SoloRoute> route;  // how such a launch runs instead, where the operator has a kernel of its own
 };
 
 struct Program {
@@ -576,25 +576,46 @@ int gemm_configure(Op* op, bool refresh, Change change) {
 // run (gate/up of 768 rows, 148 CTAs: 34.3 -> 33.5 us; attention of 784 rows, 147: the same).
 int lets_successor_in(int grid, int sms) { return grid <= sms * 3 / 10 || grid >= sms - 8 ? 1 : 0; }
 
-// The kernel of its own that a stand-alone launch of `op` takes, if there is one.  Its finished tiles are counted where the program's
-// would be, so the counters of the handle keep their meaning (expected: per launch and row band).
+// What stands for the program of an operator that has a kernel of its own: counters (per row band, then `tickets`), status, epoch and budget.
+int counter_program(const Op* op, int tickets, std::unique_ptr<Program>* out) {
+    auto prog = std::make_unique<Program>();
+    prog->device = op->device;
+    prog->workers = op->workers;
+    prog->stages.push_back(op->desc);
+    StageDesc& d = prog->stages[0];
+    d.counter_base = 0;
+    d.aux_base = d.bands;
+    prog->expected.assign(d.bands + tickets, 0);
+    const size_t at_status = (sizeof(unsigned int) * prog->expected.size() + 511) / 512 * 512, bytes = at_status + sizeof(VmStatus);
+    cudaError_t e = cudaMalloc(&prog->d_memory, bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(prog->d_memory, 0, bytes, cudaStreamLegacy);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);       // (the caller's stream may not be ordered behind it: see build_program)
+    if (e != cudaSuccess) return e;
+    prog->d_counters = static_cast<unsigned int*>(prog->d_memory);
+    prog->d_status = reinterpret_cast<VmStatus*>(static_cast<uint8_t*>(prog->d_memory) + at_status);
+    *out = std::move(prog);
+    return cudaSuccess;
+}
+
+// The kernel of its own that a stand-alone launch of `op` takes, if there is one, and what stands for its program.  Its finished tiles are
+// counted where the program's would be, so the counters of the handle keep their meaning (expected: per launch and row band).
 int solo_route(Op* op, int sms) {
-    op->route.reset();
     auto route = std::make_unique<SoloRoute>();
-    Program* prog = op->solo;
+    std::unique_ptr<Program> prog;
     const StageDesc& d = op->desc;
-    std::vector<unsigned int> expected(prog->expected.size(), 0);
+    SoloGuard* guard = nullptr;
+    int early = 1;
     if (d.kind == OP_NORM) {
         route->kind = SoloRoute::NORM;
         route->norm.n = d.p.norm;
+        guard = &route->norm.guard;
         // four rows (256 threads) per CTA, eight where that would be more than one round of them
         const int rows = d.p.norm.rows;
         route->groups = (rows + kNormPairRows - 1) / kNormPairRows <= op->workers ? 1 : 2;
         const int per = kNormPairRows * route->groups, blocks = (rows + per - 1) / per;
         route->grid = std::min(blocks, op->workers);
-        for (int b = 0; b < blocks; b++) expected[b * per / kBandRows]++;
-        SoloGuard& guard = route->norm.guard;
-        guard = {prog->d_status, prog->budget_ns, prog->d_counters, 1};
+        if (int e = counter_program(op, 0, &prog)) return e;
+        for (int b = 0; b < blocks; b++) prog->expected[b * per / kBandRows]++;
     } else if (d.kind == OP_GEMM) {
         route->kind = SoloRoute::GEMM;
         const SoloGemmRequest request{&d.p.gemm, op->a, op->b, op->m, op->n, op->k, op->operands, op->workers};
@@ -603,9 +624,11 @@ int solo_route(Op* op, int sms) {
         if (e == cudaErrorNotSupported) return cudaSuccess;
         if (e != cudaSuccess) return e;
         SoloGemm& p = plan.args;
+        guard = &p.guard;
         route->grid = plan.grid;
-        for (int row = 0; row < d.p.gemm.rows; row += p.tile_rows) expected[row / kBandRows] += p.n_tiles;
-        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, lets_successor_in(plan.grid, sms)};
+        early = lets_successor_in(plan.grid, sms);
+        if (int ce = counter_program(op, 0, &prog)) return ce;
+        for (int row = 0; row < d.p.gemm.rows; row += p.tile_rows) prog->expected[row / kBandRows] += p.n_tiles;
     } else if (d.kind == OP_ATTN && !op->prep) {
         route->kind = SoloRoute::ATTENTION;
         SoloAttnPlan& plan = route->attention;
@@ -613,21 +636,25 @@ int solo_route(Op* op, int sms) {
         if (e == cudaErrorNotSupported) return cudaSuccess;
         if (e != cudaSuccess) return e;
         SoloAttn& p = plan.args;
+        guard = &p.guard;
         route->grid = plan.grid;
-        p.guard = {prog->d_status, prog->budget_ns, prog->d_counters, lets_successor_in(plan.grid, sms)};
+        early = lets_successor_in(plan.grid, sms);
+        const int tickets = p.splits > 1 ? plan.row_tiles : 0;
+        if (int ce = counter_program(op, tickets, &prog)) return ce;
         route->band_tiles.assign(d.bands, 0);
-        if (p.head_dim != 256) std::fill(expected.begin(), expected.begin() + d.bands, static_cast<unsigned int>(p.heads));
+        if (p.head_dim != 256) std::fill(prog->expected.begin(), prog->expected.end(), static_cast<unsigned int>(p.heads));
         for (int t = 0; p.head_dim == 256 && t < plan.row_tiles; t++) {
-            const int band = t * 128 / p.heads / 128;
+            const int band = t / p.heads;                      // (the 128-query band in which the tile begins)
             route->band_tiles[band]++;
-            expected[band] += p.splits;
+            prog->expected[band] += p.splits;
         }
-        p.tickets = prog->d_counters + prog->stages[0].aux_base;
-        for (int t = 0; p.splits > 1 && t < plan.row_tiles; t++) expected[prog->stages[0].aux_base + t] = 4 * p.splits;
+        p.tickets = prog->d_counters + d.bands;
+        for (int t = 0; t < tickets; t++) prog->expected[d.bands + t] = 4 * p.splits;
     } else {
         return cudaSuccess;
     }
-    prog->expected = expected;
+    *guard = {prog->d_status, prog->budget_ns, prog->d_counters, early};
+    op->solo = prog.release();
     op->route = std::move(route);
     return cudaSuccess;
 }
@@ -645,11 +672,21 @@ cudaError_t launch_route(const Op* op, cudaStream_t stream) {
                                       : launch_solo_gemm_dense(r.gemm.args, r.gemm.cg, r.grid, r.gemm.smem, stream);
 }
 
-// Stand-alone program of one operator (plus its merge stage when the attention is split).
+// What a stand-alone launch of an operator runs: a kernel of its own, or a program of one stage (plus its merge stage when the attention is split).
+// The first launch pays for it, so the program is built only where it is launched.
 int solo_program(Op* op) {
     if (op->solo && !op->solo_dirty) return cudaSuccess;
     delete op->solo;
     op->solo = nullptr;
+    op->route.reset();
+    int sms = 0;
+    const cudaError_t ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
+    if (ce != cudaSuccess) return ce;
+    if (int e = solo_route(op, sms)) return e;
+    if (op->route) {
+        op->solo_dirty = false;
+        return cudaSuccess;
+    }
     std::vector<StageDesc> stages;
     std::vector<std::pair<int, int>> work;
     StageDesc self = op->desc;
@@ -666,8 +703,6 @@ int solo_program(Op* op) {
             self.p.gemm.tmap_b = op->maps + 2;
         }
     }
-    // (tickets of the split attention's own kernel; a program's stage has them only with the merge inside)
-    if (self.kind == OP_ATTN && self.p.attn.splits > 1) self.aux_count = self.p.attn.heads * self.bands;
     stages.push_back(self);
     work.push_back({self.tiles, op->cost});
     if (op->merge && !op->desc.p.attn.fused_merge) {
@@ -689,11 +724,7 @@ int solo_program(Op* op) {
     // front of 13 or 40: -0.9 to -1.6 throughout.  One operator behind itself gains 0.4 - 0.8 us up to 74 CTAs and then loses
     // (FP8 640 / 768 x 2048 x 16384, 80 / 96 CTAs: 31.1 / 31.9 -> 36.0 / 36.5 us).  So: at most three tenths of the SMs (44 of
     // 148).  Whole models keep their SMs to the end and never let a successor in.
-    int sms = 0;
-    const cudaError_t ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
-    if (ce != cudaSuccess) return ce;
     op->solo->early = op->solo->grid <= sms * 3 / 10;
-    if (int re = solo_route(op, sms)) return re;
     op->solo_dirty = false;
     return cudaSuccess;
 }
