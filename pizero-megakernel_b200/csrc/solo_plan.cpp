@@ -65,10 +65,11 @@ cudaError_t plan_solo_gemm(const SoloGemmRequest& r, SoloGemmPlan* plan) {
     if (!plain || g.row_factor || g.row_sumsq || g.round_before_residual || g.gelu_cols > 0 || g.pad_from > 0 || g.col_center || g.cols != r.n || g.block_n > 128)
         return cudaErrorNotSupported;
     if (scaled && g.epilogue == EPI_F32 && (g.bias || g.residual)) return cudaErrorNotSupported;
-    // At most 88 rows to BF16 over a long K are one tile per CTA whose MMAs are all there is: the persistent kernel's issue loop is as fast and its
-    // first operands are earlier (x 2048 x 16384: 51 rows 14.3 us, 14.7 here, 73 rows 14.4 and 14.6; 128 rows 18.0 and 15.0, 51 rows to FP32
-    // 15.2 and 14.9, 104 to NVFP4 15.2 and 14.9; over a K of 12288 51 rows 12.1 and 11.9).
-    if (scaled && g.rows <= 88 && r.k > 12288 && g.epilogue == EPI_BF16) return cudaErrorNotSupported;
+    // At most 64 rows to BF16 on at most 32 tiles of 64 columns: the MMAs of a long K are all there is, and over 16384 and more the persistent kernel issues
+    // them as fast and has its first operands earlier.  Stage and own kernel (us): x 2048 x 16384 1 row 14.8 and 15.4, 64 rows 15.4 and 15.4; 73
+    // rows, whose tiles copy more of A, 17.3 and 15.5; x 4096 x 16384, where twice the CTAs share L2, 16.6 and 16.0; x 2048 x 12544 51 rows 13.2 and 12.9;
+    // x 2048 x 32768 24.4 and 26.6.  (51 rows to FP32 15.2 and 14.9.)
+    if (scaled && g.epilogue == EPI_BF16 && g.rows <= 64 && r.k >= 16384 && g.block_n == 64 && g.cols <= 32 * 64 && g.cols <= r.workers * 64) return cudaErrorNotSupported;
     const size_t row_bytes = scaled ? static_cast<size_t>(r.k) / 2 : r.operands == GEMM_BF16 ? static_cast<size_t>(r.k) * 2 : static_cast<size_t>(r.k);
     const int chunks = static_cast<int>((row_bytes + 127) / 128), k_groups = static_cast<int>(row_bytes / 32);
     const int few = std::min(128, std::max(scaled ? 32 : 64, (g.rows + 7) / 8 * 8));          // rows copied when there is one row band

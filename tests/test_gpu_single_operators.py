@@ -99,6 +99,19 @@ def test_nvfp4_projection(rows, n, k, block_n, tiled, workers, ctas, width, out,
         alone_and_as_a_stage(op)
 
 
+@pytest.mark.parametrize("rows,n,k,block_n,workers,own", [
+    (64, 2048, 16384, 64, 148, False), (73, 2048, 16384, 64, 148, True), (64, 2176, 16384, 64, 148, True), (64, 2048, 16128, 64, 148, True),
+    (64, 2048, 16384, 128, 148, True), (64, 2048, 16384, 64, 31, True), (1, 256, 32768, 64, 4, False),
+])
+def test_few_rows_over_a_long_k(rows, n, k, block_n, workers, own):
+    """One tile for each of a few CTAs runs as a program of one stage; more rows, tiles, CTAs or a shorter K do not."""
+    rng = np.random.default_rng(n)
+    with ResidentNVFP4(None, codes(rng, 128, k, 1.0), codes(rng, n, k, 0.01), workers=workers, rows=rows, block_n=block_n, output_dtype=torch.bfloat16) as op:
+        assert (launch_form(op) is not None) == own
+        op.forward()
+        assert op.status()["code"] == 0
+
+
 @pytest.mark.parametrize("workers", [1, 3, 148])
 @pytest.mark.parametrize("rows,n,k", [(1, 104, 504), (65, 1000, 1152), (333, 1000, 1152), (820, 4400, 1088), (256, 9000, 640)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float8_e4m3fn])
