@@ -130,8 +130,8 @@ cudaError_t plan_solo_gemm(const SoloGemmRequest& r, SoloGemmPlan* plan) {
     plan->cg = best.cg;
     plan->grid = units * best.cg * best.splits;
     p.stages = std::min({kSoloMaxSlots, kSoloDataBytes / p.stride, rounds * ((p.slots + best.splits - 1) / best.splits)});
-    // (a split of K: the others' sums for this pair's share of the columns, 16 KiB per 32-column piece, take the place of the ring)
-    if (best.splits > 1 && (best.bn / 32 + best.splits - 1) / best.splits * (best.splits - 1) * 16384 > p.stages * p.stride) return cudaErrorNotSupported;
+    // (a split of K: the others' sums for this pair's share of the columns take the place of the ring.  16 KiB per 32-column piece and other pair, at
+    // most 96 KiB - 256 columns in 3 or 4 parts - where the ring of 32 slots and more per part has at least 160)
     plan->smem = kSoloCtlBytes + static_cast<size_t>(p.stages) * p.stride + 1024;
     // tensor memory: one or two accumulators, behind them the scales of two or four slots
     p.acc_bufs = rounds > 1 ? 2 : 1;
