@@ -40,6 +40,7 @@ int configure_resident_fp4_bf16(void* handle, const void* bias, const void* resi
  * gate/up columns (No = N/2), 3 ReLU^2; otherwise No = N.  global_scale is the output's tensor scale. */
 int configure_resident_fp4_quantized(void* handle, const void* bias, const void* residual, void* out, void* scales,
                                      float global_scale, int activation);
+/* (of the persistent kernel that runs programs; a lone projection or attention may have a kernel of its own: operator_launch_form) */
 int resident_fp4_resources(void* handle, int* values, int count);
 int destroy_resident_fp4(void* handle);
 /* extension: fused QKV epilogue - BF16 Q [M, ldq] (heads stored pair-interleaved), rotate-half RoPE with BF16
@@ -189,6 +190,7 @@ int create_attention(void** handle, const void* q, const void* k, const void* v,
                      int ldq, int ldkv, int out_ld, int fp16, int workers, int prefix, float scale);
 int launch_attention(void* handle, void* stream);
 int destroy_attention(void* handle);
+/* (of the persistent kernel: see resident_fp4_resources) */
 int attention_resources(int* values, int count);
 /* Split the key range into `splits` parts; partial (o, m, l) go to library-owned scratch and a merge stage
  * produces the output. */

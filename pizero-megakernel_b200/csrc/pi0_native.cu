@@ -495,10 +495,10 @@ int gemm_tiles(StageDesc& d, int operands, int m, int block_n) {
     return cudaSuccess;
 }
 
-// Tile width of a dense projection that is launched by itself and has not been given one (in a program of several stages it keeps 128).
-// Such a launch is paid by the operand rows that an SM takes in, A's and the tile's own for every tile it gets, and every width
-// gives the same sums over K.  In 24 shapes of 1 to 820 rows, 100 to 4400 columns and K of 504 to 4400 the estimate picks the fastest
-// width (to 2 %) back to back, and behind a flushed L2 too (us, 128 / 64 / 32 columns; flushed, launch and event included, in brackets):
+// Tile width of a dense projection that is launched by itself as a program of one stage (GELU, GeGLU, row factors, rounding before the residual; the
+// others have a kernel of their own) and has not been given one (in a program of several stages it keeps 128).  Such a launch is paid by the operand rows that an SM takes in, A's and the tile's own for every tile it gets, and every width
+// gives the same sums over K.  In 24 shapes of 1 to 820 rows, 100 to 4400 columns and K of 504 to 4400, as stages with plain output, the estimate picks
+// the fastest width (to 2 %) back to back, and behind a flushed L2 too (us, 128 / 64 / 32 columns; flushed, launch and event included, in brackets):
 // BF16 333 x 1000 x 1152 9.4 / 8.7 / 8.2 (17.2 / 15.4 / 14.3), 20 x 4352 x 4352 18.0 / 14.5 / 14.3 (33.7 / 27.6 / 24.6), 768 x 1152 x 4352 19.0 /
 // 15.7 / 21.5 (30.7 / 25.5 / 29.7), 820 x 4400 x 4400 40.0 / 50.1 / 68.0 (54.2 / 65.5 / 80.9), 10 x 100 x 504 6.9 / 5.9 / 5.7 (14.3 / 12.5 / 12.3);
 // FP8 50 x 500 x 4352 11.8 / 10.0 / 8.7 (20.5 / 18.4 / 16.4), 768 x 2048 x 4096 13.3 / 16.2 / 18.1 (22.5 / 24.6 / 26.6).
@@ -571,9 +571,14 @@ int gemm_configure(Op* op, bool refresh, Change change) {
     return cudaSuccess;
 }
 
-// Whether a launch of `grid` CTAs lets its successor's start while it runs: see solo_program for the small ones.  One that takes the whole
-// chip can let it in, too: the successor's CTAs find no other place than the SM of one that has ended, and prepare there while the last ones
-// run (gate/up of 768 rows, 148 CTAs: 34.3 -> 33.5 us; attention of 784 rows, 147: the same).
+// Whether a launch of a kernel of its own with `grid` CTAs lets its successor's start while it runs: a small one, which leaves SMs free, and one that takes
+// the whole chip, where the successor's CTAs find no other place than the SM of one that has ended and prepare there while the last ones run.
+// Early against not (us per launch; q|k|v-like projections of 51 rows and K = 1024, behind themselves, in front of a BF16 one of 96 CTAs and of one of
+// 148): 24 - 44 CTAs -0.14 to -0.17, -0.64 to -0.76, -0.04 to -0.08; 48 - 64 -0.14 to -0.17, -0.68 to -0.76, -0.11 to -0.17; 80 - 138 -0.09 to
+// +0.03, -0.02 to -0.24, -0.14 to +0.04; 140 -0.19, -0.01, -0.29; 148 -0.06, +0.06, +0.22.  Larger ones behind themselves: gate/up of 768 rows, 148
+// CTAs, 34.3 -> 33.5; BF16 820 x 4400 x 1088, 144, 12.2 -> 11.5; BF16 256 x 9000 x 640, 142, 6.6 -> 6.8; attention of 784 rows, 148 of which 48 have two
+// tiles, 22.8 -> 23.6, but 0.5 less in front of projections of 14 to 148 CTAs.  The lower line is the one of programs of one stage (solo_program); up to
+// 64 CTAs these kernels would gain as much above it, beyond that little.
 int lets_successor_in(int grid, int sms) { return grid <= sms * 3 / 10 || grid >= sms - 8 ? 1 : 0; }
 
 // What stands for the program of an operator that has a kernel of its own: counters (per row band, then `tickets`), status, epoch and budget.
@@ -720,8 +725,8 @@ int solo_program(Op* op) {
     // Pairs of launches, early against not: GEMM of 24 / 32 / 37 / 40 / 44 CTAs in front of a BF16 one of 96: -0.36 / -0.19 /
     // -0.26 / -0.29 / -0.15 us; of 48 / 52 / 64: +0.17 / +0.20 / +0.37; in front of 120 or 128 CTAs -0.2 to 0 up to 44, 0 beyond; in
     // front of 13 or 40: -0.9 to -1.6 throughout.  One operator behind itself gains 0.4 - 0.8 us up to 74 CTAs and then loses
-    // (FP8 640 / 768 x 2048 x 16384, 80 / 96 CTAs: 31.1 / 31.9 -> 36.0 / 36.5 us).  So: at most three tenths of the SMs (44 of
-    // 148).  Whole models keep their SMs to the end and never let a successor in.
+    // (FP8 640 / 768 x 2048 x 16384 as stages, 80 / 96 CTAs: 31.1 / 31.9 -> 36.0 / 36.5 us).  So: at most three tenths of the SMs (44 of
+    // 148).  Kernels of single operators: lets_successor_in.  Whole models keep their SMs to the end and never let a successor in.
     op->solo->early = op->solo->grid <= sms * 3 / 10;
     op->solo_dirty = false;
     return cudaSuccess;
