@@ -225,7 +225,8 @@ int attention_prepare_handle(void* handle, void** prepare);
 /* extension: cudaSuccess when the handle can run as configured - an operator with prepared operands or a mask whose key
  * range per tile exceeds 256 (or whose path was forced to mma.sync) cannot; launches and programs refuse it too. */
 int attention_validate(void* handle);
-/* extension: handle of the merge stage owned by an attention handle with splits > 1 (NULL otherwise). */
+/* extension: handle of the merge stage owned by an attention handle with splits > 1 (NULL otherwise).  From then on launches of the attention
+ * handle are programs, whose partial rows a launch of the merge handle reads. */
 int attention_merge_handle(void* handle, void** merge);
 /* Development diagnostics: how a stand-alone launch of an operator handle runs.  values[0] = 0 as a program of one stage, 1 in the norm's kernel of
  * its own, 2 in the projection's, 3 in the attention's; [1] CTAs that share a tile (2: a pair), [2] columns of a tile (projections), [3] splits of K or of
@@ -282,7 +283,7 @@ int configure_linear32_extra_row(void* handle, const float* src, void* dst);
 /* expert input rows: row 0 = state embedding, rows 1..chunk = action embeddings, BF16 [*, width]. */
 int create_suffix_assemble(void** handle, const float* state_emb, const float* action_emb, void* out, int chunk,
                            int width, int workers);
-int launch_op(void* handle, void* stream);      /* any operator handle, as a one-stage program */
+int launch_op(void* handle, void* stream);      /* any operator handle by itself */
 int destroy_op(void* handle);
 /* tiles, 128-row bands and K-cost of an operator handle (what the stream compiler needs). */
 int op_geometry(void* handle, int* tiles, int* bands, int* cost);

@@ -129,6 +129,7 @@ struct Op {
     bool tile_given = false;           // the caller has chosen a tile width
     // attention bookkeeping
     Op* merge = nullptr;               // owned merge stage (splits > 1)
+    bool merge_shared = false;         // its handle has been given out: launched by itself it finds the partial rows of the last launch as the stage lays them out
     uint16_t* partial_o = nullptr;
     float* partial_ml = nullptr;
     size_t partial_bytes = 0, stat_bytes = 0;
@@ -633,7 +634,7 @@ int solo_route(Op* op, int sms) {
         early = lets_successor_in(plan.grid, sms);
         if (int ce = counter_program(op, 0, &prog)) return ce;
         for (int row = 0; row < d.p.gemm.rows; row += p.tile_rows) prog->expected[row / kBandRows] += p.n_tiles;
-    } else if (d.kind == OP_ATTN && !op->prep) {
+    } else if (d.kind == OP_ATTN && !op->prep && !op->merge_shared) {
         route->kind = SoloRoute::ATTENTION;
         SoloAttnPlan& plan = route->attention;
         cudaError_t e = plan_solo_attention(d.p.attn, op->workers, sms, &plan);
@@ -1385,6 +1386,7 @@ extern "C" int configure_attention_splits(void* handle, int splits) {
         }
     }
     if (op->merge) { free_op(op->merge); op->merge = nullptr; }
+    op->merge_shared = false;
     cudaFree(op->partial_o);
     cudaFree(op->partial_ml);
     op->partial_o = partial_o;
@@ -1540,6 +1542,10 @@ extern "C" int attention_merge_handle(void* handle, void** merge) {
     Op* op = as_op(handle);
     if (!op || op->desc.kind != OP_ATTN || !merge) return cudaErrorInvalidValue;
     *merge = op->merge;
+    if (op->merge && !op->merge_shared) {
+        op->merge_shared = true;
+        op->solo_dirty = op->solo_dirty || op->route;
+    }
     return cudaSuccess;
 }
 

@@ -194,6 +194,23 @@ def test_attention_of_heads_with_one_kv_head(nq, nk, heads, prefix, splits, work
             assert state["epoch"] == 3 and all(c == 3 * splits for c in state["counts"])
 
 
+def test_merge_handle_launched_by_itself():
+    """The merge stage of a split attention merges the partial rows of its owner's last launch again, whenever its handle was asked for."""
+    g = torch.Generator(device="cuda").manual_seed(12)
+    q, k = (torch.randn(1, n, h, 256, generator=g, device="cuda").bfloat16() for n, h in ((51, 8), (819, 1)))
+    with ResidentAttention(None, q, k, k, workers=148, splits=13, head_dim=256) as op:
+        alone = op.forward().clone()
+        merge = op.merge_handle
+        for _ in range(2):
+            want = op.forward().clone()
+            op.output.zero_()
+            _native.check(op.library.launch_op(merge, torch.cuda.current_stream().cuda_stream), "merge")
+            assert torch.equal(op.output, want) and op.status()["code"] == 0
+        assert float((want.double() - alone.double()).norm() / want.double().norm()) <= 1e-3
+        state = op.read_split_counts()
+        assert all(c == 13 * state["epoch"] for c in state["counts"])
+
+
 def test_partial_rows_of_split_attention():
     """An operator holds partial rows for its configured ranges and no more, launched by itself or not: 64 of 128 rows here, 4 MiB."""
     g = torch.Generator(device="cuda").manual_seed(11)
