@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(kSoloAttnThreads, 1) pi0_attention_kernel(cons
     } else if (warp == 1) {
         const uint32_t tmem_u = uniform_u32(tmem), q16 = uniform_u32((smem_u32(data) & 0x3FFFFu) >> 4), k16 = uniform_u32((smem_u32(sk) & 0x3FFFFu) >> 4),
                        v16 = uniform_u32((smem_u32(sv) & 0x3FFFFu) >> 4), slab16 = uniform_u32(slab >> 4);
-        grid_dependency_wait();                               // (the time that the kernel in front takes is not this one's)
         if (elect_one()) {
             constexpr uint64_t kKMajor = (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
             constexpr uint32_t kBf16 = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);

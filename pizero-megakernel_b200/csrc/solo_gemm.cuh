@@ -186,7 +186,6 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
         const int k_groups = uniform_i32(g.k_groups), bn = uniform_i32(p.bn), ks_first = uniform_i32(ks_begin), ks_last = uniform_i32(ks_end);
         const bool per_tile = p.sfb_per_tile != 0, two_bufs = uniform_i32(p.acc_bufs) == 2;
         const uint16_t both = static_cast<uint16_t>(3u << uniform_u32(first_rank));
-        grid_dependency_wait();                               // (the time that the kernel in front takes is not this one's)
         if (leader && elect_one()) {
             uint32_t slot = 0, phase = 0, use = 0, it = 0;
             bool alive = true, landed = false;                                // landed: the slot was seen full half-way through the one before
@@ -298,7 +297,7 @@ __global__ void __launch_bounds__(128 + 32 * solo_drain_warps(OPERANDS, EPI), 1)
                 gemm_epilogue_chunk<EPI, kLean, true>(g, d, raw, res, row, n0 + c, row_ok, g.alpha, 0.f, unused_a, unused_b);
                 if (c + 32 < col_end) load_residual(c + 32);
             }
-            if (warp == kDrainWarps && lane == 0 && !solo_gave_up(&ctl->abort)) atomicAdd(p.guard.counters + (m0 >> 7), 1u);     // (quarter 0, the last columns)
+            if (warp == kDrainWarps && lane == 0) atomicAdd(p.guard.counters + (m0 >> 7), solo_gave_up(&ctl->abort) ? 0u : 1u);     // (quarter 0, the last columns)
         }
     }
 
